@@ -24,6 +24,7 @@
 
 #include "../../include/ltl.h"
 #include "packed_core.cuh"
+#include "transfer_core.cuh"
 
 namespace ltl {
 
@@ -342,14 +343,20 @@ static size_t persist_ring_bytes() {
 // ---------------------------------------------------------------------------
 // Dense staging <-> arena (all grids of a list, or one grid)
 // ---------------------------------------------------------------------------
+// (memory-bound like k_transfer.cu's kernels: 16-byte vectors of cells.  A grid's
+// rows are n bytes apart in the staging buffer, so most rows start unaligned.)
 __global__ void k_batch_pack(const uint8_t* __restrict__ cells, uint32_t* __restrict__ arena,
                              const BatchGrid* __restrict__ grids, int first) {
     const BatchGrid g = grids[first + blockIdx.y];
     const uint8_t* c = cells + g.cell_off;
+    const uint8_t* end = c + (size_t)g.n * g.n;
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < g.n * g.nw; t += gridDim.x * blockDim.x) {
         const int i = t / g.nw, w = t % g.nw;
-        uint32_t v = 0u;
-        for (int b = 0; b < 32 && 32 * w + b < g.n; ++b) v |= (uint32_t)(c[(size_t)i * g.n + 32 * w + b] ? 1u : 0u) << b;
+        const uint8_t* p = c + (size_t)i * g.n + 32 * w;
+        const int valid = g.n - 32 * w;
+        uint32_t v = cells16_to_bits<true>(load16(p, c, end));
+        if (valid > 16) v |= cells16_to_bits<true>(load16(p + 16, c, end)) << 16;
+        if (valid < 32) v &= (1u << valid) - 1u;
         arena[g.off + (size_t)(g.HR + i) * g.wp + 1 + w] = v;
     }
 }
@@ -357,11 +364,15 @@ __global__ void k_batch_pack(const uint8_t* __restrict__ cells, uint32_t* __rest
 __global__ void k_batch_unpack(const uint32_t* __restrict__ arena, uint8_t* __restrict__ cells,
                                const BatchGrid* __restrict__ grids, int first) {
     const BatchGrid g = grids[first + blockIdx.y];
-    uint8_t* c = cells + g.cell_off;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < g.n * g.nw; t += gridDim.x * blockDim.x) {
-        const int i = t / g.nw, w = t % g.nw;
-        const uint32_t v = arena[g.off + (size_t)(g.HR + i) * g.wp + 1 + w];
-        for (int b = 0; b < 32 && 32 * w + b < g.n; ++b) c[(size_t)i * g.n + 32 * w + b] = (uint8_t)((v >> b) & 1u);
+    uint8_t* dst = cells + g.cell_off;
+    const int vecs = (g.n + 15) / 16 + 1;  // aligned vectors a row may touch
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < g.n * vecs; t += gridDim.x * blockDim.x) {
+        const int i = t / vecs;
+        uint8_t* row = dst + (size_t)i * g.n;
+        const int c = lead(row) + 16 * (t % vecs);
+        if (c >= g.n) continue;
+        const uint32_t bits = bits16_at(arena + g.off + (size_t)(g.HR + i) * g.wp + 1, c, g.nw);
+        store16(row + c, bits16_to_cells(bits), -c, g.n - c);
     }
 }
 

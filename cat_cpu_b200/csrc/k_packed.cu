@@ -1,4 +1,4 @@
-// k_packed.cu -- K3: bit-packed LtL step (one bit per cell) and the PACK codec.
+// k_packed.cu -- K3: bit-packed LtL step (one bit per cell).
 //
 // Same function as the reference's HostSolver<int> step (kezada94/CAT_cpu,
 // src/CellularAutomata/Solvers/HostSolver.tpp:58-91, torus halo :93-140), with
@@ -9,9 +9,6 @@
 //            (B -= h(r-R); B += h(r+R+1) while a thread walks down its band);
 //   next   = s ? [smin+1 <= B <= smax+1] : [bmin <= B <= bmax]   (B includes the centre)
 // evaluated with bit-sliced comparators.  Every operation acts on 32 cells.
-//
-// The PACK codec (ltl_pack_device / ltl_unpack_device) stores row i of a grid
-// as ceil(cols/64) uint64 words, cell (i, j) = bit j % 64 of word j / 64.
 #include <algorithm>
 
 #include "packed_core.cuh"
@@ -189,169 +186,6 @@ cudaError_t launch_packed_halo(const PackedFrame& f, cudaStream_t s) {
     if (e != cudaSuccess) return e;
     dim3 g2((unsigned)std::max<size_t>(1, std::min<size_t>((f.wpitch + 127) / 128, 64)), (unsigned)(2 * f.HR));
     k_packed_halo_rows<<<g2, 128, 0, s>>>(f.words, f.nrows(), f.HR, f.wpitch);
-    return cudaGetLastError();
-}
-
-// ---------------------------------------------------------------------------
-// Byte frame <-> packed frame (inner cells only; halos are refilled after).
-// ---------------------------------------------------------------------------
-// Four 0/1 bytes of a word -> 4 bits: the multiply places byte k's bit at bit
-// 24 + k with no two partial products overlapping (so no carries), and back:
-// the 4 bits of a nibble spread to bit 0 of each byte by copies 7 bits apart.
-__device__ __forceinline__ uint32_t bytes4_to_bits(uint32_t w) { return ((w & 0x01010101u) * 0x01020408u) >> 24; }
-__device__ __forceinline__ uint32_t bits4_to_bytes(uint32_t nib) { return (nib * 0x00204081u) & 0x01010101u; }
-
-// Inner rows [row0, row0 + nrows) of a packed frame from / to a dense byte
-// buffer whose row i (`pitch` bytes apart, `src`/`dst` = its cell (0, 0)) is
-// frame row row0 + i.  `vec`: buffer and pitch 16-byte aligned, so whole
-// 32-cell words move as two 16-byte vectors.
-__global__ void k_pack_rows(const uint8_t* __restrict__ src, size_t pitch, bool vec, int n, int nw, int HR, int HW,
-                            size_t wp, int row0, int nrows, uint32_t* __restrict__ dst) {
-    const long long total = (long long)nrows * nw;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-         t += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(t / nw), w = (int)(t % nw);
-        const uint8_t* p = src + (size_t)i * pitch + 32 * w;
-        uint32_t v = 0u;
-        if (vec && 32 * w + 32 <= n) {
-            const uint4 a = *(const uint4*)p, b = *(const uint4*)(p + 16);
-            const uint32_t q[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-#pragma unroll
-            for (int k = 0; k < 8; ++k) v |= bytes4_to_bits(q[k]) << (4 * k);
-        } else {
-            for (int b = 0; b < 32 && 32 * w + b < n; ++b) v |= (uint32_t)(p[b] & 1u) << b;
-        }
-        dst[(size_t)(HR + row0 + i) * wp + HW + w] = v;
-    }
-}
-
-__global__ void k_unpack_rows(const uint32_t* __restrict__ src, int n, int nw, int HR, int HW, size_t wp, int row0,
-                              int nrows, uint8_t* __restrict__ dst, size_t pitch, bool vec) {
-    const long long total = (long long)nrows * nw;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-         t += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(t / nw), w = (int)(t % nw);
-        const uint32_t v = src[(size_t)(HR + row0 + i) * wp + HW + w];
-        uint8_t* p = dst + (size_t)i * pitch + 32 * w;
-        if (vec && 32 * w + 32 <= n) {
-            uint32_t q[8];
-#pragma unroll
-            for (int k = 0; k < 8; ++k) q[k] = bits4_to_bytes((v >> (4 * k)) & 0xFu);
-            *(uint4*)p = make_uint4(q[0], q[1], q[2], q[3]);
-            *(uint4*)(p + 16) = make_uint4(q[4], q[5], q[6], q[7]);
-        } else {
-            for (int b = 0; b < 32 && 32 * w + b < n; ++b) p[b] = (uint8_t)((v >> b) & 1u);
-        }
-    }
-}
-
-static bool vec16(const void* p, size_t pitch) { return ((uintptr_t)p % 16 == 0) && (pitch % 16 == 0); }
-
-cudaError_t launch_pack_rows(const uint8_t* src, size_t pitch, const PackedFrame& dst, int row0, int nrows,
-                             cudaStream_t s) {
-    if (nrows <= 0) return cudaSuccess;
-    const long long total = (long long)nrows * dst.nw;
-    const int blocks = (int)std::min<long long>((total + 255) / 256, 148 * 32);
-    k_pack_rows<<<blocks, 256, 0, s>>>(src, pitch, vec16(src, pitch), dst.n, dst.nw, dst.HR, dst.HW, dst.wpitch,
-                                       row0, nrows, dst.words);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_unpack_rows(const PackedFrame& src, int row0, int nrows, uint8_t* dst, size_t pitch,
-                               cudaStream_t s) {
-    if (nrows <= 0) return cudaSuccess;
-    const long long total = (long long)nrows * src.nw;
-    const int blocks = (int)std::min<long long>((total + 255) / 256, 148 * 32);
-    k_unpack_rows<<<blocks, 256, 0, s>>>(src.words, src.n, src.nw, src.HR, src.HW, src.wpitch, row0, nrows, dst,
-                                         pitch, vec16(dst, pitch));
-    return cudaGetLastError();
-}
-
-// byte frame -> packed frame, inner cells only (halos are refilled after)
-cudaError_t launch_pack_frame(const Frame& src, const PackedFrame& dst, cudaStream_t s) {
-    return launch_pack_rows(src.base + (size_t)src.H * src.pitch + src.H, src.pitch, dst, 0, dst.nrows(), s);
-}
-
-cudaError_t launch_unpack_frame(const PackedFrame& src, const Frame& dst, cudaStream_t s) {
-    cudaError_t e =
-        launch_unpack_rows(src, 0, src.nrows(), dst.base + (size_t)dst.H * dst.pitch + dst.H, dst.pitch, s);
-    if (e != cudaSuccess) return e;
-    return launch_halo_fill(dst, s);
-}
-
-// ---------------------------------------------------------------------------
-// PACK codec on dense device buffers.
-// ---------------------------------------------------------------------------
-__global__ void k_pack64(const uint8_t* __restrict__ cells, size_t cp, int rows, int cols, uint64_t* __restrict__ words,
-                         size_t wp) {
-    const int nw = (cols + 63) / 64;
-    const long long total = (long long)rows * nw;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-         t += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(t / nw), w = (int)(t % nw);
-        const uint8_t* p = cells + (size_t)i * cp + 64 * (size_t)w;
-        uint64_t v = 0ull;
-        for (int b = 0; b < 64 && 64 * w + b < cols; ++b) v |= (uint64_t)(p[b] ? 1u : 0u) << b;
-        words[(size_t)i * wp + w] = v;
-    }
-}
-
-__global__ void k_unpack64(const uint64_t* __restrict__ words, size_t wp, int rows, int cols, uint8_t* __restrict__ cells,
-                           size_t cp) {
-    const int nw = (cols + 63) / 64;
-    const long long total = (long long)rows * nw;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-         t += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(t / nw), w = (int)(t % nw);
-        const uint64_t v = words[(size_t)i * wp + w];
-        uint8_t* p = cells + (size_t)i * cp + 64 * (size_t)w;
-        for (int b = 0; b < 64 && 64 * w + b < cols; ++b) p[b] = (uint8_t)((v >> b) & 1ull);
-    }
-}
-
-// Inner words of a packed frame -> PACK-coded rows (uint64 word k of a row =
-// frame words 2k and 2k + 1), bits past n cleared.
-__global__ void k_frame_to_pack64(const uint32_t* __restrict__ src, int n, int rows, int nw, int HR, int HW,
-                                  size_t wp, uint64_t* __restrict__ dst, size_t dst_wp) {
-    const int nw64 = (n + 63) / 64;
-    const long long total = (long long)rows * nw64;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-         t += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(t / nw64), k = (int)(t % nw64);
-        const uint32_t* row = src + (size_t)(HR + i) * wp + HW;
-        uint32_t lo = row[2 * k];
-        uint32_t hi = 2 * k + 1 < nw ? row[2 * k + 1] : 0u;
-        uint64_t v = ((uint64_t)hi << 32) | lo;
-        const int valid = n - 64 * k;  // cells of this word inside the row
-        if (valid < 64) v &= (1ull << valid) - 1ull;
-        dst[(size_t)i * dst_wp + k] = v;
-    }
-}
-
-cudaError_t launch_frame_to_pack64(const PackedFrame& f, uint64_t* dst, size_t dst_pitch_words, cudaStream_t s) {
-    const long long total = (long long)f.nrows() * ((f.n + 63) / 64);
-    if (total == 0) return cudaSuccess;
-    const int blocks = (int)std::min<long long>((total + 255) / 256, 148 * 32);
-    k_frame_to_pack64<<<blocks, 256, 0, s>>>(f.words, f.n, f.nrows(), f.nw, f.HR, f.HW, f.wpitch, dst,
-                                             dst_pitch_words);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_pack(const uint8_t* cells, size_t cell_pitch, int rows, int cols, uint64_t* words,
-                        size_t word_pitch_words, cudaStream_t s) {
-    if (rows == 0 || cols == 0) return cudaSuccess;
-    long long total = (long long)rows * ((cols + 63) / 64);
-    int blocks = (int)std::min<long long>((total + 255) / 256, 148 * 32);
-    k_pack64<<<blocks, 256, 0, s>>>(cells, cell_pitch, rows, cols, words, word_pitch_words);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_unpack(const uint64_t* words, size_t word_pitch_words, int rows, int cols, uint8_t* cells,
-                          size_t cell_pitch, cudaStream_t s) {
-    if (rows == 0 || cols == 0) return cudaSuccess;
-    long long total = (long long)rows * ((cols + 63) / 64);
-    int blocks = (int)std::min<long long>((total + 255) / 256, 148 * 32);
-    k_unpack64<<<blocks, 256, 0, s>>>(words, word_pitch_words, rows, cols, cells, cell_pitch);
     return cudaGetLastError();
 }
 

@@ -1,7 +1,6 @@
 // k_plain.cu -- CUDA-core kernels of libltl_b200:
-//   K5 torus halo fill, K1 plain LtL step (SWAR fast path for R <= 5 and a
-//   fused prefix-sum path for larger R), K6 population / comparison, and the
-//   dense <-> frame copies used by upload/download.
+//   K5 torus halo fill and K1 plain LtL step (SWAR fast path for R <= 5 and a
+//   fused prefix-sum path for larger R).
 //
 // Semantics restated from the reference (kezada94/CAT_cpu):
 //   step  HostSolver<int>::CAStepAlgorithm, src/CellularAutomata/Solvers/HostSolver.tpp:58-73
@@ -991,104 +990,6 @@ cudaError_t launch_plain_generic(const Frame& cur, const Frame& nxt, const Rule&
     if (nt == 128) return launch_wide_rm<false, 8, 128>(cur, nxt, q, band, T, grid, s);
     return cpt == 8 ? launch_wide_rm<false, 8, 256>(cur, nxt, q, band, T, grid, s)
                     : launch_wide_rm<false, 16, 256>(cur, nxt, q, band, T, grid, s);
-}
-
-// ---------------------------------------------------------------------------
-// K6: population and comparison over inner cells.
-// ---------------------------------------------------------------------------
-__global__ void k_population(const uint8_t* __restrict__ g, int n, int rows, int H, size_t pitch,
-                             unsigned long long* out) {
-    unsigned long long acc = 0;
-    const long long total = (long long)rows * n;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-         t += (long long)gridDim.x * blockDim.x) {
-        int i = (int)(t / n), j = (int)(t % n);
-        acc += g[(size_t)(H + i) * pitch + H + j];
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-    if ((threadIdx.x & 31) == 0 && acc) atomicAdd(out, acc);
-}
-
-__global__ void k_compare(const uint8_t* __restrict__ g, int n, int rows, int H, size_t pitch,
-                          const uint8_t* __restrict__ other, size_t opitch, unsigned long long* out) {
-    unsigned long long cnt = 0, first = ~0ull;
-    const long long total = (long long)rows * n;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-         t += (long long)gridDim.x * blockDim.x) {
-        int i = (int)(t / n), j = (int)(t % n);
-        if (g[(size_t)(H + i) * pitch + H + j] != other[(size_t)i * opitch + j]) {
-            ++cnt;
-            if ((unsigned long long)t < first) first = (unsigned long long)t;
-        }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        cnt += __shfl_down_sync(0xffffffffu, cnt, o);
-        unsigned long long f2 = __shfl_down_sync(0xffffffffu, first, o);
-        first = f2 < first ? f2 : first;
-    }
-    if ((threadIdx.x & 31) == 0 && cnt) {
-        atomicAdd(out, cnt);
-        atomicMin(out + 1, first);
-    }
-}
-
-cudaError_t launch_population(const Frame& f, unsigned long long* scratch, cudaStream_t s) {
-    cudaError_t e = cudaMemsetAsync(scratch, 0, sizeof(unsigned long long), s);
-    if (e != cudaSuccess) return e;
-    long long total = (long long)f.nrows() * f.n;
-    int blocks = (int)std::min<long long>((total + 255) / 256, 148 * 16);
-    k_population<<<blocks, 256, 0, s>>>(f.base, f.n, f.nrows(), f.H, f.pitch, scratch);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_compare(const Frame& f, const uint8_t* other, size_t other_pitch,
-                           unsigned long long* scratch, cudaStream_t s) {
-    cudaError_t e = cudaMemsetAsync(scratch, 0, sizeof(unsigned long long), s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(scratch + 1, 0xff, sizeof(unsigned long long), s);
-    if (e != cudaSuccess) return e;
-    long long total = (long long)f.nrows() * f.n;
-    int blocks = (int)std::min<long long>((total + 255) / 256, 148 * 16);
-    k_compare<<<blocks, 256, 0, s>>>(f.base, f.n, f.nrows(), f.H, f.pitch, other, other_pitch, scratch);
-    return cudaGetLastError();
-}
-
-// ---------------------------------------------------------------------------
-// Dense n x n <-> frame inner copies (device to device).
-// ---------------------------------------------------------------------------
-__global__ void k_copy_in(uint8_t* __restrict__ g, int n, int rows, int H, size_t pitch,
-                          const uint8_t* __restrict__ src, size_t sp) {
-    const long long total = (long long)rows * n;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-         t += (long long)gridDim.x * blockDim.x) {
-        int i = (int)(t / n), j = (int)(t % n);
-        g[(size_t)(H + i) * pitch + H + j] = src[(size_t)i * sp + j] ? 1 : 0;
-    }
-}
-
-__global__ void k_copy_out(const uint8_t* __restrict__ g, int n, int rows, int H, size_t pitch,
-                           uint8_t* __restrict__ dst, size_t dp) {
-    const long long total = (long long)rows * n;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-         t += (long long)gridDim.x * blockDim.x) {
-        int i = (int)(t / n), j = (int)(t % n);
-        dst[(size_t)i * dp + j] = g[(size_t)(H + i) * pitch + H + j];
-    }
-}
-
-cudaError_t launch_copy_in(const Frame& f, const uint8_t* src, size_t src_pitch, cudaStream_t s) {
-    long long total = (long long)f.nrows() * f.n;
-    int blocks = (int)std::min<long long>((total + 255) / 256, 148 * 32);
-    k_copy_in<<<blocks, 256, 0, s>>>(f.base, f.n, f.nrows(), f.H, f.pitch, src, src_pitch);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_copy_out(const Frame& f, uint8_t* dst, size_t dst_pitch, cudaStream_t s) {
-    long long total = (long long)f.nrows() * f.n;
-    int blocks = (int)std::min<long long>((total + 255) / 256, 148 * 32);
-    k_copy_out<<<blocks, 256, 0, s>>>(f.base, f.n, f.nrows(), f.H, f.pitch, dst, dst_pitch);
-    return cudaGetLastError();
 }
 
 }  // namespace ltl

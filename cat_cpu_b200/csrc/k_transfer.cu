@@ -1,0 +1,350 @@
+// k_transfer.cu -- everything that moves a grid between its codings on the
+// device: dense byte cells (a caller's buffer or a byte frame), the packed
+// frame's 32-bit words, the PACK codec's 64-bit words; and the reductions over
+// a grid (K6: population, comparison), read from whichever coding holds it.
+//
+// Every kernel here is bound by memory: a byte of cells in or out and an eighth
+// of that in words.  So each thread moves whole 16-byte vectors of cells, in an
+// order that keeps a warp's vectors contiguous, with kRows rows in flight per
+// thread.  Callers' buffers may have any alignment and pitch: the kernels write
+// vectors that are aligned in the destination, and read an unaligned source as
+// aligned 32-bit words shifted together (load16).  Measured on B200, before
+// (one byte, or 64 strided bytes, per thread) and after: 16384^2 cells to PACK
+// words and back 2057 -> 131 us (604 MB, 4.6 TB/s); 16384^2 cells into a packed
+// frame and out again 1376 -> 152 us (the byte frame between is gone too).
+//
+// Reference counterparts (kezada94/CAT_cpu): the host <-> solver copies of
+// src/CellularAutomata/Solvers/AMXSolver.cpp (CASolver.cpp:3-13) and
+// src/CellularAutomata/CADataDomainComparator.tpp:8-27.
+#include <algorithm>
+
+#include "ltl_kernels.h"
+#include "transfer_core.cuh"
+
+namespace ltl {
+
+namespace {
+
+constexpr int kTx = 32;    // threads along a row
+constexpr int kTy = 8;     // rows per block pass
+constexpr int kRows = 4;   // rows per thread in flight
+
+// Byte rows -> word rows: thread = one 32-bit word of a row, kNonzero: a cell is
+// alive if its byte is not 0 (else by its bit 0).  Words past the cells get 0.
+template <bool kNonzero>
+__global__ void __launch_bounds__(kTx * kTy)
+k_cells_to_words(const uint8_t* __restrict__ src, size_t sp, int rows, int cols, uint32_t* __restrict__ dst, size_t dp,
+                 int nwords) {
+    const int w = blockIdx.x * kTx + threadIdx.x;
+    if (w >= nwords) return;
+    const uint8_t* end = src + (size_t)(rows - 1) * sp + cols;
+    const int valid = cols - 32 * w;
+    const uint32_t mask = valid >= 32 ? 0xffffffffu : (valid > 0 ? (1u << valid) - 1u : 0u);
+    for (int r0 = blockIdx.y * (kTy * kRows) + threadIdx.y; r0 < rows; r0 += gridDim.y * (kTy * kRows)) {
+        uint4 a[kRows], b[kRows];
+#pragma unroll
+        for (int k = 0; k < kRows; ++k) {
+            const int r = r0 + k * kTy;
+            const uint8_t* p = src + (size_t)r * sp + 32 * (size_t)w;
+            a[k] = b[k] = make_uint4(0u, 0u, 0u, 0u);
+            if (r < rows && valid > 0) a[k] = load16(p, src, end);
+            if (r < rows && valid > 16) b[k] = load16(p + 16, src, end);
+        }
+#pragma unroll
+        for (int k = 0; k < kRows; ++k) {
+            const int r = r0 + k * kTy;
+            if (r < rows)
+                dst[(size_t)r * dp + w] =
+                    (cells16_to_bits<kNonzero>(a[k]) | (cells16_to_bits<kNonzero>(b[k]) << 16)) & mask;
+        }
+    }
+}
+
+// Word rows -> byte rows: thread = one aligned 16-byte vector of the destination.
+__global__ void __launch_bounds__(kTx * kTy)
+k_words_to_cells(const uint32_t* __restrict__ src, size_t sp, int nwords, int rows, int cols, uint8_t* __restrict__ dst,
+                 size_t dp) {
+    const int v = blockIdx.x * kTx + threadIdx.x;
+    for (int r0 = blockIdx.y * (kTy * kRows) + threadIdx.y; r0 < rows; r0 += gridDim.y * (kTy * kRows)) {
+        uint32_t bits[kRows];
+#pragma unroll
+        for (int k = 0; k < kRows; ++k) {
+            const int r = r0 + k * kTy;
+            const int c = lead(dst + (size_t)r * dp) + 16 * v;
+            bits[k] = r < rows && c < cols ? bits16_at(src + (size_t)r * sp, c, nwords) : 0u;
+        }
+#pragma unroll
+        for (int k = 0; k < kRows; ++k) {
+            const int r = r0 + k * kTy;
+            if (r >= rows) continue;
+            uint8_t* row = dst + (size_t)r * dp;
+            const int c = lead(row) + 16 * v;
+            if (c < cols) store16(row + c, bits16_to_cells(bits[k]), -c, cols - c);
+        }
+    }
+}
+
+// Byte rows -> byte rows (kNonzero: every byte that is not 0 becomes 1).
+// src == dst is allowed: a thread reads only the vectors it writes.
+template <bool kNonzero>
+__global__ void __launch_bounds__(kTx * kTy)
+k_copy_cells(const uint8_t* src, size_t sp, int rows, int cols, uint8_t* dst, size_t dp) {
+    const int v = blockIdx.x * kTx + threadIdx.x;
+    const uint8_t* end = src + (size_t)(rows - 1) * sp + cols;
+    for (int r0 = blockIdx.y * (kTy * kRows) + threadIdx.y; r0 < rows; r0 += gridDim.y * (kTy * kRows)) {
+        uint4 a[kRows];
+#pragma unroll
+        for (int k = 0; k < kRows; ++k) {
+            const int r = r0 + k * kTy;
+            const int c = lead(dst + (size_t)r * dp) + 16 * v;
+            a[k] = make_uint4(0u, 0u, 0u, 0u);
+            if (r < rows && c < cols) a[k] = load16(src + (size_t)r * sp + c, src, end);
+        }
+#pragma unroll
+        for (int k = 0; k < kRows; ++k) {
+            const int r = r0 + k * kTy;
+            if (r >= rows) continue;
+            uint8_t* row = dst + (size_t)r * dp;
+            const int c = lead(row) + 16 * v;
+            if constexpr (kNonzero)
+                a[k] = make_uint4(nonzero4(a[k].x), nonzero4(a[k].y), nonzero4(a[k].z), nonzero4(a[k].w));
+            if (c < cols) store16(row + c, a[k], -c, cols - c);
+        }
+    }
+}
+
+// Rows of a grid as 16-cell groups, from the byte frame (kWords = false) or the
+// packed frame.  Cells past n read as 0.
+struct GridRows {
+    const void* inner;  // cell (0, 0): byte frame (16-byte aligned rows) or word frame
+    size_t pitch;       // bytes or words
+    int n, rows;
+};
+
+__device__ __forceinline__ void keep_cells(uint4& v, int valid) {
+    if (valid >= 16) return;
+    uint32_t q[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int left = valid - 4 * k;
+        q[k] = left >= 4 ? q[k] : (left > 0 ? q[k] & ((1u << (8 * left)) - 1u) : 0u);
+    }
+    v = make_uint4(q[0], q[1], q[2], q[3]);
+}
+
+template <bool kWords>
+__global__ void __launch_bounds__(kTx * kTy) k_population(GridRows g, unsigned long long* out) {
+    unsigned long long acc = 0;
+    constexpr int kCells = kWords ? 32 : 16;
+    const int v = blockIdx.x * kTx + threadIdx.x;
+    const int valid = g.n - kCells * v;
+    if (valid > 0) {
+        for (int r0 = blockIdx.y * (kTy * kRows) + threadIdx.y; r0 < g.rows; r0 += gridDim.y * (kTy * kRows)) {
+            uint32_t cnt = 0;
+#pragma unroll
+            for (int k = 0; k < kRows; ++k) {
+                const int r = r0 + k * kTy;
+                if (r >= g.rows) continue;
+                if constexpr (kWords) {
+                    uint32_t w = __ldg((const uint32_t*)g.inner + (size_t)r * g.pitch + v);
+                    if (valid < 32) w &= (1u << valid) - 1u;
+                    cnt += __popc(w);
+                } else {
+                    // the vector may reach into the right halo: those cells are dropped
+                    uint4 a = __ldg((const uint4*)((const uint8_t*)g.inner + (size_t)r * g.pitch) + v);
+                    keep_cells(a, valid);
+                    cnt += __popc(a.x) + __popc(a.y) + __popc(a.z) + __popc(a.w);  // 0/1 bytes
+                }
+            }
+            acc += cnt;
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+    if (threadIdx.x == 0 && acc) atomicAdd(out, acc);
+}
+
+template <bool kWords>
+__global__ void __launch_bounds__(kTx * kTy)
+k_compare(GridRows g, const uint8_t* __restrict__ other, size_t op, unsigned long long* out) {
+    unsigned long long cnt = 0, first = ~0ull;
+    const int v = blockIdx.x * kTx + threadIdx.x;
+    const int valid = g.n - 16 * v;
+    if (valid > 0) {
+        const uint8_t* end = other + (size_t)(g.rows - 1) * op + g.n;
+        for (int r0 = blockIdx.y * (kTy * kRows) + threadIdx.y; r0 < g.rows; r0 += gridDim.y * (kTy * kRows)) {
+            uint4 a[kRows], b[kRows];
+#pragma unroll
+            for (int k = 0; k < kRows; ++k) {
+                const int r = r0 + k * kTy;
+                a[k] = b[k] = make_uint4(0u, 0u, 0u, 0u);
+                if (r >= g.rows) continue;
+                if constexpr (kWords) {
+                    const uint32_t w = __ldg((const uint32_t*)g.inner + (size_t)r * g.pitch + (v >> 1));
+                    a[k] = bits16_to_cells((v & 1) ? w >> 16 : w & 0xffffu);
+                } else {
+                    a[k] = __ldg((const uint4*)((const uint8_t*)g.inner + (size_t)r * g.pitch) + v);
+                }
+                b[k] = load16(other + (size_t)r * op + 16 * (size_t)v, other, end);
+            }
+#pragma unroll
+            for (int k = 0; k < kRows; ++k) {
+                uint4 d = make_uint4(nonzero4(a[k].x ^ b[k].x), nonzero4(a[k].y ^ b[k].y), nonzero4(a[k].z ^ b[k].z),
+                                     nonzero4(a[k].w ^ b[k].w));
+                keep_cells(d, valid);
+                const uint32_t bits = cells16_to_bits<false>(d);
+                if (bits) {
+                    cnt += __popc(bits);
+                    const unsigned long long at =
+                        (unsigned long long)(r0 + k * kTy) * g.n + 16 * (unsigned)v + __ffs(bits) - 1;
+                    first = at < first ? at : first;
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        cnt += __shfl_down_sync(0xffffffffu, cnt, o);
+        const unsigned long long f2 = __shfl_down_sync(0xffffffffu, first, o);
+        first = f2 < first ? f2 : first;
+    }
+    if (threadIdx.x == 0 && cnt) {
+        atomicAdd(out, cnt);
+        atomicMin(out + 1, first);
+    }
+}
+
+// Inner words of a packed frame -> PACK-coded rows (uint64 word k of a row =
+// frame words 2k and 2k + 1), bits past n cleared.  Thread = one frame word.
+__global__ void __launch_bounds__(kTx * kTy)
+k_words_to_pack(const uint32_t* __restrict__ src, size_t sp, int rows, int n, uint32_t* __restrict__ dst, size_t dp,
+                int nwords) {
+    const int w = blockIdx.x * kTx + threadIdx.x;
+    if (w >= nwords) return;
+    const int valid = n - 32 * w;
+    const uint32_t mask = valid >= 32 ? 0xffffffffu : (valid > 0 ? (1u << valid) - 1u : 0u);
+    for (int r = blockIdx.y * kTy + threadIdx.y; r < rows; r += gridDim.y * kTy)
+        dst[(size_t)r * dp + w] = valid > 0 ? __ldg(src + (size_t)r * sp + w) & mask : 0u;
+}
+
+// `items` threads along a row, `rows` rows, `per` rows per thread.  `cap`
+// bounds the blocks of a reduction (each ends in an atomic).
+dim3 cover(long long items, int rows, int per, long long cap = 0) {
+    const long long gx = std::max<long long>(1, (items + kTx - 1) / kTx);
+    long long gy = std::max<long long>(1, ((long long)rows + kTy * per - 1) / (kTy * per));
+    if (cap > 0) gy = std::min(gy, std::max<long long>(1, cap / gx));
+    return dim3((unsigned)gx, (unsigned)std::min<long long>(gy, 65535));
+}
+
+const dim3 kBlock(kTx, kTy);
+constexpr long long kReduceBlocks = 148 * 16;
+
+GridRows byte_rows(const Frame& f) {
+    return GridRows{f.base + (size_t)f.H * f.pitch + f.H, f.pitch, f.n, f.nrows()};
+}
+uint32_t* word_origin(const PackedFrame& f) { return f.words + (size_t)f.HR * f.wpitch + f.HW; }
+GridRows word_rows(const PackedFrame& f) { return GridRows{word_origin(f), f.wpitch, f.n, f.nrows()}; }
+
+}  // namespace
+
+// --- byte buffers <-> byte frames -------------------------------------------
+cudaError_t launch_copy_in(const Frame& f, const uint8_t* src, size_t src_pitch, cudaStream_t s) {
+    const int rows = f.nrows();
+    k_copy_cells<true><<<cover((f.n + 15) / 16 + 1, rows, kRows), kBlock, 0, s>>>(src, src_pitch, rows, f.n,
+                                                                                 f.inner(0, 0), f.pitch);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_copy_out(const Frame& f, uint8_t* dst, size_t dst_pitch, cudaStream_t s) {
+    const int rows = f.nrows();
+    k_copy_cells<false><<<cover((f.n + 15) / 16 + 1, rows, kRows), kBlock, 0, s>>>(f.cinner(0, 0), f.pitch, rows, f.n,
+                                                                                  dst, dst_pitch);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_binarize(const Frame& f, cudaStream_t s) { return launch_copy_in(f, f.inner(0, 0), f.pitch, s); }
+
+// --- byte buffers <-> packed frames -----------------------------------------
+cudaError_t launch_pack_rows(const uint8_t* src, size_t pitch, bool nonzero, const PackedFrame& dst, int row0,
+                             int nrows, cudaStream_t s) {
+    if (nrows <= 0) return cudaSuccess;
+    uint32_t* d = word_origin(dst) + (size_t)row0 * dst.wpitch;
+    auto kernel = nonzero ? k_cells_to_words<true> : k_cells_to_words<false>;
+    kernel<<<cover(dst.nw, nrows, kRows), kBlock, 0, s>>>(src, pitch, nrows, dst.n, d, dst.wpitch, dst.nw);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_unpack_rows(const PackedFrame& src, int row0, int nrows, uint8_t* dst, size_t pitch,
+                               cudaStream_t s) {
+    if (nrows <= 0) return cudaSuccess;
+    k_words_to_cells<<<cover((src.n + 15) / 16 + 1, nrows, kRows), kBlock, 0, s>>>(
+        word_origin(src) + (size_t)row0 * src.wpitch, src.wpitch, src.nw, nrows, src.n, dst, pitch);
+    return cudaGetLastError();
+}
+
+// --- PACK codec ---------------------------------------------------------------
+cudaError_t launch_pack(const uint8_t* cells, size_t cell_pitch, int rows, int cols, uint64_t* words,
+                        size_t word_pitch_words, cudaStream_t s) {
+    if (rows == 0 || cols == 0) return cudaSuccess;
+    const int nwords = 2 * ((cols + 63) / 64);  // 32-bit halves, little-endian
+    k_cells_to_words<true><<<cover(nwords, rows, kRows), kBlock, 0, s>>>(cells, cell_pitch, rows, cols,
+                                                                       (uint32_t*)words, 2 * word_pitch_words, nwords);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_unpack(const uint64_t* words, size_t word_pitch_words, int rows, int cols, uint8_t* cells,
+                          size_t cell_pitch, cudaStream_t s) {
+    if (rows == 0 || cols == 0) return cudaSuccess;
+    k_words_to_cells<<<cover((cols + 15) / 16 + 1, rows, kRows), kBlock, 0, s>>>(
+        (const uint32_t*)words, 2 * word_pitch_words, 2 * ((cols + 63) / 64), rows, cols, cells, cell_pitch);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_frame_to_pack64(const PackedFrame& f, uint64_t* dst, size_t dst_pitch_words, cudaStream_t s) {
+    const int rows = f.nrows(), nwords = 2 * ((f.n + 63) / 64);
+    k_words_to_pack<<<cover(nwords, rows, 1), kBlock, 0, s>>>(word_origin(f), f.wpitch, rows, f.n, (uint32_t*)dst,
+                                                             2 * dst_pitch_words, nwords);
+    return cudaGetLastError();
+}
+
+// --- K6: population and comparison over the inner cells -----------------------
+cudaError_t launch_population(const Frame& f, unsigned long long* scratch, cudaStream_t s) {
+    cudaError_t e = cudaMemsetAsync(scratch, 0, sizeof(unsigned long long), s);
+    if (e != cudaSuccess) return e;
+    k_population<false><<<cover((f.n + 15) / 16, f.nrows(), kRows, kReduceBlocks), kBlock, 0, s>>>(byte_rows(f),
+                                                                                                  scratch);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_population(const PackedFrame& f, unsigned long long* scratch, cudaStream_t s) {
+    cudaError_t e = cudaMemsetAsync(scratch, 0, sizeof(unsigned long long), s);
+    if (e != cudaSuccess) return e;
+    k_population<true><<<cover(f.nw, f.nrows(), kRows, kReduceBlocks), kBlock, 0, s>>>(word_rows(f), scratch);
+    return cudaGetLastError();
+}
+
+static cudaError_t clear_compare(unsigned long long* scratch, cudaStream_t s) {
+    cudaError_t e = cudaMemsetAsync(scratch, 0, sizeof(unsigned long long), s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(scratch + 1, 0xff, sizeof(unsigned long long), s);
+    return e;
+}
+
+cudaError_t launch_compare(const Frame& f, const uint8_t* other, size_t other_pitch, unsigned long long* scratch,
+                           cudaStream_t s) {
+    cudaError_t e = clear_compare(scratch, s);
+    if (e != cudaSuccess) return e;
+    k_compare<false><<<cover((f.n + 15) / 16, f.nrows(), kRows, kReduceBlocks), kBlock, 0, s>>>(byte_rows(f), other,
+                                                                                               other_pitch, scratch);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_compare(const PackedFrame& f, const uint8_t* other, size_t other_pitch, unsigned long long* scratch,
+                           cudaStream_t s) {
+    cudaError_t e = clear_compare(scratch, s);
+    if (e != cudaSuccess) return e;
+    k_compare<true><<<cover((f.n + 15) / 16, f.nrows(), kRows, kReduceBlocks), kBlock, 0, s>>>(word_rows(f), other,
+                                                                                              other_pitch, scratch);
+    return cudaGetLastError();
+}
+
+}  // namespace ltl

@@ -60,7 +60,6 @@ struct ltl_ctx {
     size_t pwords_bytes = 0;
     // PACK-coded staging rows of ltl_upload_packed / ltl_download_packed (made on first use)
     uint64_t* pstage = nullptr;
-    bool packed_valid = false;  // packed frames hold the current state
     // tensor variant
     TensorPlan* tplan = nullptr;
     unsigned long long wait_ns = 2000000000ull;
@@ -325,41 +324,28 @@ extern "C" int ltl_get_info(const ltl_ctx* c, ltl_info* info) {
     return LTL_OK;
 }
 
-// Make the packed frames hold the byte frame's state (packed variant keeps its
-// state packed between steps; the byte frame is refreshed on download).
+// The packed and tensor variants hold the grid in the packed frames only; their
+// byte frames are staging for host transfers.
 static bool keeps_packed(const ltl_ctx* c) {
     return c->variant == LTL_VARIANT_PACKED || c->variant == LTL_VARIANT_TENSOR;
 }
 
-static int sync_to_packed(ltl_ctx* c) {
-    Frame& f = cur_frame(c);
-    LTL_CUDA(launch_pack_frame(f, cur_packed(c), c->stream));
-    if (c->variant == LTL_VARIANT_PACKED) LTL_CUDA(launch_packed_halo(cur_packed(c), c->stream));
-    c->packed_valid = true;
-    return LTL_OK;
-}
-
-static int sync_from_packed(ltl_ctx* c) {
-    if (!keeps_packed(c) || !c->packed_valid) return LTL_OK;
-    LTL_CUDA(launch_unpack_frame(cur_packed(c), cur_frame(c), c->stream));
-    return LTL_OK;
-}
-
+// After the current frame's inner cells were written: refresh the halo where the
+// step reads one.
 static int after_upload(ltl_ctx* c) {
-    LTL_CUDA(launch_halo_fill(cur_frame(c), c->stream));
-    c->packed_valid = false;
-    if (keeps_packed(c)) return sync_to_packed(c);
+    if (c->variant == LTL_VARIANT_PACKED) LTL_CUDA(launch_packed_halo(cur_packed(c), c->stream));
+    // the SWAR kernels with plain_wrap read inner cells only
+    if (c->variant == LTL_VARIANT_PLAIN && !c->plain_wrap) LTL_CUDA(launch_halo_fill(cur_frame(c), c->stream));
     return LTL_OK;
 }
 
-__global__ void k_binarize(uint8_t* g, int n, int rows, int H, size_t pitch) {
-    const long long total = (long long)rows * n;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-         t += (long long)gridDim.x * blockDim.x) {
-        int i = (int)(t / n), j = (int)(t % n);
-        uint8_t* p = g + (size_t)(H + i) * pitch + H + j;
-        *p = *p ? 1 : 0;
-    }
+// Cells from a device buffer into the current frame (not 0 -> 1).
+static int take_cells(ltl_ctx* c, const uint8_t* dev, size_t pitch) {
+    if (keeps_packed(c))
+        LTL_CUDA(launch_pack_rows(dev, pitch, true, cur_packed(c), 0, c->rows, c->stream));
+    else
+        LTL_CUDA(launch_copy_in(cur_frame(c), dev, pitch, c->stream));
+    return after_upload(c);
 }
 
 extern "C" int ltl_upload(ltl_ctx* c, const uint8_t* inner, size_t pitch) {
@@ -372,11 +358,8 @@ extern "C" int ltl_upload(ltl_ctx* c, const uint8_t* inner, size_t pitch) {
     Frame& f = cur_frame(c);
     LTL_CUDA(cudaMemcpy2DAsync(f.inner(0, 0), f.pitch, inner, pitch, c->n, c->rows, cudaMemcpyHostToDevice,
                                c->stream));
-    long long total = (long long)c->rows * c->n;
-    k_binarize<<<(int)std::min<long long>((total + 255) / 256, 148 * 32), 256, 0, c->stream>>>(
-        f.base, c->n, c->rows, f.H, f.pitch);
-    LTL_CUDA(cudaGetLastError());
-    if (int r = after_upload(c)) return r;
+    // (the plain variant reads and writes the frame in place)
+    if (int r = take_cells(c, f.inner(0, 0), f.pitch)) return r;
     LTL_CUDA(cudaStreamSynchronize(c->stream));
     return LTL_OK;
 }
@@ -388,8 +371,7 @@ extern "C" int ltl_upload_device(ltl_ctx* c, const uint8_t* dev_inner, size_t pi
         return LTL_EINVAL;
     }
     LTL_CUDA(cudaSetDevice(c->device));
-    LTL_CUDA(launch_copy_in(cur_frame(c), dev_inner, pitch, c->stream));
-    return after_upload(c);
+    return take_cells(c, dev_inner, pitch);
 }
 
 extern "C" int ltl_download(ltl_ctx* c, uint8_t* inner, size_t pitch) {
@@ -399,8 +381,9 @@ extern "C" int ltl_download(ltl_ctx* c, uint8_t* inner, size_t pitch) {
         return LTL_EINVAL;
     }
     LTL_CUDA(cudaSetDevice(c->device));
-    if (int r = sync_from_packed(c)) return r;
     Frame& f = cur_frame(c);
+    if (keeps_packed(c))
+        LTL_CUDA(launch_unpack_rows(cur_packed(c), 0, c->rows, f.inner(0, 0), f.pitch, c->stream));
     LTL_CUDA(cudaMemcpy2DAsync(inner, pitch, f.inner(0, 0), f.pitch, c->n, c->rows, cudaMemcpyDeviceToHost,
                                c->stream));
     LTL_CUDA(cudaStreamSynchronize(c->stream));
@@ -441,8 +424,6 @@ extern "C" int ltl_upload_packed(ltl_ctx* c, const uint64_t* words, size_t word_
         LTL_CUDA(cudaMemcpy2DAsync(f.words + (size_t)f.HR * f.wpitch + f.HW, f.wpitch * sizeof(uint32_t), words,
                                    word_pitch_bytes, (size_t)f.nw * sizeof(uint32_t), c->rows,
                                    cudaMemcpyHostToDevice, c->stream));
-        if (c->variant == LTL_VARIANT_PACKED) LTL_CUDA(launch_packed_halo(f, c->stream));
-        c->packed_valid = true;
     } else {
         if (int r = pack_stage(c)) return r;
         const size_t spitch = (size_t)(c->n + 63) / 64;  // words
@@ -450,8 +431,8 @@ extern "C" int ltl_upload_packed(ltl_ctx* c, const uint64_t* words, size_t word_
                                    cudaMemcpyHostToDevice, c->stream));
         Frame& f = cur_frame(c);
         LTL_CUDA(launch_unpack(c->pstage, spitch, c->rows, c->n, f.inner(0, 0), f.pitch, c->stream));
-        if (int r = after_upload(c)) return r;
     }
+    if (int r = after_upload(c)) return r;
     LTL_CUDA(cudaStreamSynchronize(c->stream));
     return LTL_OK;
 }
@@ -462,7 +443,7 @@ extern "C" int ltl_download_packed(ltl_ctx* c, uint64_t* words, size_t word_pitc
     LTL_CUDA(cudaSetDevice(c->device));
     if (int r = pack_stage(c)) return r;
     const size_t spitch = (size_t)(c->n + 63) / 64;  // words
-    if (keeps_packed(c) && c->packed_valid) {
+    if (keeps_packed(c)) {
         LTL_CUDA(launch_frame_to_pack64(cur_packed(c), c->pstage, spitch, c->stream));
     } else {
         Frame& f = cur_frame(c);
@@ -481,8 +462,10 @@ extern "C" int ltl_download_device(ltl_ctx* c, uint8_t* dev_inner, size_t pitch)
         return LTL_EINVAL;
     }
     LTL_CUDA(cudaSetDevice(c->device));
-    if (int r = sync_from_packed(c)) return r;
-    LTL_CUDA(launch_copy_out(cur_frame(c), dev_inner, pitch, c->stream));
+    if (keeps_packed(c))
+        LTL_CUDA(launch_unpack_rows(cur_packed(c), 0, c->rows, dev_inner, pitch, c->stream));
+    else
+        LTL_CUDA(launch_copy_out(cur_frame(c), dev_inner, pitch, c->stream));
     return LTL_OK;
 }
 
@@ -501,7 +484,7 @@ extern "C" int ltl_download_rows_device(ltl_ctx* c, int row0, int nrows, uint8_t
     if (int r = check_rows(c, "ltl_download_rows_device", row0, nrows, dev, pitch)) return r;
     if (nrows == 0) return LTL_OK;
     LTL_CUDA(cudaSetDevice(c->device));
-    if (keeps_packed(c) && c->packed_valid) {
+    if (keeps_packed(c)) {
         // straight from the packed frame: only the asked rows are unpacked
         LTL_CUDA(launch_unpack_rows(cur_packed(c), row0, nrows, dev, pitch, c->stream));
         return LTL_OK;
@@ -518,15 +501,9 @@ extern "C" int ltl_upload_rows_device(ltl_ctx* c, int row0, int nrows, const uin
     if (nrows == 0) return LTL_OK;
     LTL_CUDA(cudaSetDevice(c->device));
     if (keeps_packed(c)) {
-        // straight into the packed frame once it holds the current state (the
-        // byte frame is staging only: every read of a packed grid unpacks it
-        // again), then its halo
-        if (!c->packed_valid) {
-            if (int r = sync_to_packed(c)) return r;
-        }
-        LTL_CUDA(launch_pack_rows(dev, pitch, cur_packed(c), row0, nrows, c->stream));
-        if (c->variant == LTL_VARIANT_PACKED) LTL_CUDA(launch_packed_halo(cur_packed(c), c->stream));
-        return LTL_OK;
+        // straight into the packed frame, then its halo
+        LTL_CUDA(launch_pack_rows(dev, pitch, false, cur_packed(c), row0, nrows, c->stream));
+        return after_upload(c);
     }
     Frame& f = cur_frame(c);
     LTL_CUDA(cudaMemcpy2DAsync(f.inner(row0, 0), f.pitch, dev, pitch, c->n, nrows, cudaMemcpyDeviceToDevice,
@@ -626,9 +603,6 @@ extern "C" int ltl_step(ltl_ctx* c, int steps) {
     }
     if (steps == 0) return LTL_OK;
     LTL_CUDA(cudaSetDevice(c->device));
-    if (keeps_packed(c) && !c->packed_valid) {
-        if (int r = sync_to_packed(c)) return r;
-    }
     int passes = steps / c->depth;
     const int rest = steps % c->depth;  // a last, shorter pass
     while (!c->timing && passes >= kGraphPasses) {
@@ -672,8 +646,8 @@ extern "C" int ltl_population(ltl_ctx* c, uint64_t* live) {
         return LTL_EINVAL;
     }
     LTL_CUDA(cudaSetDevice(c->device));
-    if (int r = sync_from_packed(c)) return r;
-    LTL_CUDA(launch_population(cur_frame(c), c->scratch, c->stream));
+    LTL_CUDA(keeps_packed(c) ? launch_population(cur_packed(c), c->scratch, c->stream)
+                             : launch_population(cur_frame(c), c->scratch, c->stream));
     unsigned long long v = 0;
     LTL_CUDA(cudaMemcpyAsync(&v, c->scratch, sizeof(v), cudaMemcpyDeviceToHost, c->stream));
     LTL_CUDA(cudaStreamSynchronize(c->stream));
@@ -689,8 +663,8 @@ extern "C" int ltl_compare_device(ltl_ctx* c, const uint8_t* dev_expected, size_
         return LTL_EINVAL;
     }
     LTL_CUDA(cudaSetDevice(c->device));
-    if (int r = sync_from_packed(c)) return r;
-    LTL_CUDA(launch_compare(cur_frame(c), dev_expected, pitch, c->scratch, c->stream));
+    LTL_CUDA(keeps_packed(c) ? launch_compare(cur_packed(c), dev_expected, pitch, c->scratch, c->stream)
+                             : launch_compare(cur_frame(c), dev_expected, pitch, c->scratch, c->stream));
     unsigned long long v[2] = {0, 0};
     LTL_CUDA(cudaMemcpyAsync(v, c->scratch, sizeof(v), cudaMemcpyDeviceToHost, c->stream));
     LTL_CUDA(cudaStreamSynchronize(c->stream));

@@ -40,16 +40,6 @@ int plain_wide_cols_per_thread(int radius);
 cudaError_t launch_plain_generic(const Frame& cur, const Frame& nxt, const Rule& rule, int band_rows,
                                  cudaStream_t s);
 
-// K6: population and comparison over the inner n x n cells.  `scratch` holds
-// two uint64 (count, first index) in device memory.
-cudaError_t launch_population(const Frame& f, unsigned long long* scratch, cudaStream_t s);
-cudaError_t launch_compare(const Frame& f, const uint8_t* other, size_t other_pitch,
-                           unsigned long long* scratch, cudaStream_t s);
-
-// Copies between a dense n x n grid (pitch bytes per row) and a frame's inner cells.
-cudaError_t launch_copy_in(const Frame& f, const uint8_t* src, size_t src_pitch, cudaStream_t s);
-cudaError_t launch_copy_out(const Frame& f, uint8_t* dst, size_t dst_pitch, cudaStream_t s);
-
 // K3: bit-packed variant.  Packed frame: 32-bit words, cell (i, j) is bit j % 32
 // of word j / 32 (LSB first; two consecutive words are one little-endian uint64
 // of the PACK codec).  Inner row i is frame row HR + i, inner word w is frame
@@ -71,20 +61,35 @@ cudaError_t launch_packed_step(const PackedFrame& cur, const PackedFrame& nxt, c
 cudaError_t launch_packed_halo(const PackedFrame& f, cudaStream_t s);
 // true when launch_packed_step also refreshes the output frame's halo
 bool packed_fused_halo(const PackedFrame& f, int radius);
-cudaError_t launch_pack_frame(const Frame& src, const PackedFrame& dst, cudaStream_t s);
-cudaError_t launch_unpack_frame(const PackedFrame& src, const Frame& dst, cudaStream_t s);
-// Inner rows [row0, row0 + nrows) of a packed frame to / from a dense byte
-// buffer (buffer row i = frame row row0 + i, `pitch` bytes apart, 0/1 cells).
-// After packing rows in, the frame's halo is stale: refresh it.
+
+// Transfers between codings and reductions (k_transfer.cu).  Callers' byte
+// buffers are dense cells, `pitch` bytes per row, any alignment.
+// Byte frame <- / -> caller's buffer; in, every byte that is not 0 becomes 1.
+cudaError_t launch_copy_in(const Frame& f, const uint8_t* src, size_t src_pitch, cudaStream_t s);
+cudaError_t launch_copy_out(const Frame& f, uint8_t* dst, size_t dst_pitch, cudaStream_t s);
+// Every inner byte of the frame that is not 0 becomes 1.
+cudaError_t launch_binarize(const Frame& f, cudaStream_t s);
+// Inner rows [row0, row0 + nrows) of a packed frame from / to a buffer whose row
+// i is frame row row0 + i.  nonzero: a cell is alive if its byte is not 0, else
+// by its bit 0.  After packing rows in, a halo the step reads is stale.
+cudaError_t launch_pack_rows(const uint8_t* src, size_t pitch, bool nonzero, const PackedFrame& dst, int row0,
+                             int nrows, cudaStream_t s);
 cudaError_t launch_unpack_rows(const PackedFrame& src, int row0, int nrows, uint8_t* dst, size_t pitch, cudaStream_t s);
-cudaError_t launch_pack_rows(const uint8_t* src, size_t pitch, const PackedFrame& dst, int row0, int nrows,
-                             cudaStream_t s);
 // A packed frame's inner words as PACK-coded rows (bits past n cleared).
 cudaError_t launch_frame_to_pack64(const PackedFrame& f, uint64_t* dst, size_t dst_pitch_words, cudaStream_t s);
+// PACK codec on callers' buffers (not 0 -> 1).
 cudaError_t launch_pack(const uint8_t* cells, size_t cell_pitch, int rows, int cols, uint64_t* words,
                         size_t word_pitch_words, cudaStream_t s);
 cudaError_t launch_unpack(const uint64_t* words, size_t word_pitch_words, int rows, int cols, uint8_t* cells,
                           size_t cell_pitch, cudaStream_t s);
+// K6: population and comparison over the inner cells.  `scratch` holds two
+// uint64 (count, first index) in device memory.
+cudaError_t launch_population(const Frame& f, unsigned long long* scratch, cudaStream_t s);
+cudaError_t launch_population(const PackedFrame& f, unsigned long long* scratch, cudaStream_t s);
+cudaError_t launch_compare(const Frame& f, const uint8_t* other, size_t other_pitch, unsigned long long* scratch,
+                           cudaStream_t s);
+cudaError_t launch_compare(const PackedFrame& f, const uint8_t* other, size_t other_pitch, unsigned long long* scratch,
+                           cudaStream_t s);
 
 // K2: tcgen05 banded-product step on packed frames (the tensor variant keeps
 // its grid in the packed layout of K3; the kernel wraps rows and words modulo n
