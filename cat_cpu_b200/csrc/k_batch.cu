@@ -10,12 +10,13 @@
 //     own kernel instantiation, with the rule's bit masks in the constant bank;
 //   - "resident" grids (small enough that two packed copies fit in one SM's
 //     shared memory) are advanced all requested steps in ONE launch: a CTA loads
-//     the grid once, keeps the torus halo in shared memory and writes the grid
-//     back after the last step (temporal blocking of the whole run);
+//     the grid once and writes it back after the last step (temporal blocking
+//     of the whole run);
 //   - larger grids are advanced one generation per launch by a persistent
-//     kernel that walks a (grid, row band, word strip) work list, followed by a
-//     batched halo refresh; the whole step loop is captured in a CUDA graph, and
-//     the resident launches run concurrently on a forked stream.
+//     kernel that walks a (grid, row band, word strip) work list; the whole step
+//     loop is captured in a CUDA graph, and the resident launches run
+//     concurrently on a forked stream.  No form has a halo: the walk wraps rows
+//     and words in its loads.
 #include <algorithm>
 #include <cstring>
 #include <map>
@@ -31,12 +32,10 @@ namespace ltl {
 struct BatchGrid {
     long long off;       // word offset of the grid's packed frame in an arena
     long long cell_off;  // byte offset of the grid in the dense staging buffer
-    int n, nw, HR, wp;   // cells per side, inner words per row, halo rows, words per frame row
+    int n, nw, wp;       // cells per side, words per row, row pitch in words (a multiple of 4)
     int R;
     int cls;             // rule class
 };
-
-#define LTL_BATCH_RADII(X) X(1) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13) X(14) X(15) X(16)
 
 constexpr int kBatchWarps = 4;
 constexpr int kResThreads = 1024;
@@ -45,196 +44,65 @@ constexpr int kResSmemLimit = 220 * 1024;
 // ---------------------------------------------------------------------------
 // Per-step kernel for the streamed grids of one rule class.
 // ---------------------------------------------------------------------------
+// The walk in the form that a side needs, one word per lane.
+template <int R, bool kRing, bool kConst>
+__device__ __forceinline__ void batch_walk(const uint32_t* cur, uint32_t* nxt, const BatchGrid& g, int r0, int r1,
+                                           int w0, uint32_t* ring, int lane, const PackedRule& pr) {
+    if (g.n < 64)
+        packed_walk<R, 1, kRing, kEdgeTiny, kConst>(cur, nxt, g.wp, g.n, g.nw, g.n, r0, r1, w0, ring, lane, pr);
+    else if (g.n % 32 == 0)
+        packed_walk<R, 1, kRing, kEdgeNone, kConst>(cur, nxt, g.wp, g.n, g.nw, g.n, r0, r1, w0, ring, lane, pr);
+    else
+        packed_walk<R, 1, kRing, kEdgeRagged, kConst>(cur, nxt, g.wp, g.n, g.nw, g.n, r0, r1, w0, ring, lane, pr);
+}
+
 template <int R>
 __global__ void __launch_bounds__(kBatchWarps * 32)
 k_batch_step(const uint32_t* __restrict__ cur, uint32_t* __restrict__ nxt, const BatchGrid* __restrict__ grids,
              const int4* __restrict__ items, int n_items, const __grid_constant__ PackedRule pr) {
-    using Ring = PackedRing<R, kBatchWarps>;
-    extern __shared__ uint32_t ring_all[];
+    extern __shared__ __align__(16) uint32_t ring_all[];
     const int lane = threadIdx.x & 31;
     const int wid = threadIdx.x >> 5;
-    uint32_t* ring_lane = ring_all + (size_t)wid * Ring::WARP_WORDS + lane;
+    uint32_t* ring = ring_all + (size_t)wid * PackedRing<R, 1>::WARP_WORDS;
     const int gwarp = blockIdx.x * kBatchWarps + wid;
     const int gwarps = gridDim.x * kBatchWarps;
     for (int it = gwarp; it < n_items; it += gwarps) {
         const int4 item = items[it];  // grid, r0, r1, word strip
         const BatchGrid g = grids[item.x];
         const int w = item.w * 32 + lane;
-        packed_band<R, Ring::fits>(cur + g.off, nxt + g.off, (size_t)g.wp, g.HR, item.y, item.z, 1 + w, w <= g.nw,
-                                   w < g.nw, lane, ring_lane, pr);
-        __syncwarp();
+        if (w < g.nw) batch_walk<R, true, true>(cur + g.off, nxt + g.off, g, item.y, item.z, w, ring, lane, pr);
     }
 }
 
 // ---------------------------------------------------------------------------
-// Halo refresh of packed frames (same rules as k_packed.cu's halo kernels):
-// bit position p of an inner row holds cell (p - 32) mod n, then the top and
-// bottom halo rows are copies of the inner rows they wrap to.
+// Resident kernel: whole grids in shared memory for `steps` generations.  The
+// leaving row is counted again (shared memory holds the two grids, no rings).
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t frame_bit(const uint32_t* row, int cell) {
-    const int p = 32 + cell;
-    return (row[p >> 5] >> (p & 31)) & 1u;
-}
-
-__device__ __forceinline__ uint32_t halo_word_bits(const uint32_t* row, int fw, int n, int nw) {
-    // frame word fw (0 = left halo, nw = last inner, nw + 1 = right halo), bit by bit
-    if (fw == nw) {
-        const int inner_bits = n - 32 * (nw - 1);
-        uint32_t v = inner_bits >= 32 ? row[fw] : (row[fw] & ((1u << inner_bits) - 1u));
-        for (int b = inner_bits; b < 32; ++b) v |= frame_bit(row, (32 * (nw - 1) + b) % n) << b;
-        return v;
-    }
-    uint32_t v = 0u;
-    for (int b = 0; b < 32; ++b) {
-        const int cell = 32 * (fw - 1) + b;
-        v |= frame_bit(row, ((cell % n) + n) % n) << b;
-    }
-    return v;
-}
-
-__device__ __forceinline__ uint32_t halo_word(const uint32_t* row, int fw, int n, int nw) {
-    return packed_halo_word(row, fw, n, nw, [&] { return halo_word_bits(row, fw, n, nw); });
-}
-
-// The three column-halo words of one inner frame row: frame word 0 (cells
-// n-32 .. n-1), the last inner word's bits past n, and frame word nw + 1 (the
-// cells that follow).  For n >= 64 it reads the four inner words they come
-// from once (first two, last two); smaller grids take the bit-by-bit path.
-__device__ __forceinline__ void halo_cols_row(uint32_t* row, int n, int nw) {
-    if (n >= 64) {
-        const uint32_t w1 = row[1], w2 = row[2];  // inner words 0 and 1
-        const uint32_t wl = row[nw], wp = row[nw - 1];  // inner words nw - 1 and nw - 2
-        const int ib = n - 32 * (nw - 1);  // inner bits of the last word, 1..32
-        // the last inner word with its bits past n filled from the row's start
-        const uint32_t last = ib >= 32 ? wl : ((wl & ((1u << ib) - 1u)) | (w1 << ib));
-        // frame word 0: cells n-32 .. n-1 = the 32 bits that end at inner bit ib of the last word
-        const uint32_t left = ib >= 32 ? wl : __funnelshift_r(wp, wl, ib);
-        // frame word nw + 1: cells 32 nw - n .. (the row's start shifted by the bits past n)
-        const int c = 32 * nw - n;
-        const uint32_t right = c ? __funnelshift_r(w1, w2, c) : w1;
-        row[0] = left;
-        row[nw] = last;
-        row[nw + 1] = right;
-    } else {
-        for (int k = 0; k < 3; ++k) {
-            const int fw = k == 0 ? 0 : nw + (k - 1);
-            row[fw] = halo_word(row, fw, n, nw);
-        }
-    }
-}
-
-// One thread per inner row writes the row's three column-halo words.
-__global__ void k_batch_halo_cols(uint32_t* __restrict__ arena, const BatchGrid* __restrict__ grids,
-                                  const int* __restrict__ list) {
-    const BatchGrid g = grids[list[blockIdx.y]];
-    uint32_t* f = arena + g.off;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < g.n; i += gridDim.x * blockDim.x)
-        halo_cols_row(f + (size_t)(g.HR + i) * g.wp, g.n, g.nw);
-}
-
-__global__ void k_batch_halo_rows(uint32_t* __restrict__ arena, const BatchGrid* __restrict__ grids,
-                                  const int* __restrict__ list) {
-    const BatchGrid g = grids[list[blockIdx.y]];
-    uint32_t* f = arena + g.off;
-    const int total = 2 * g.HR * g.wp;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
-        const int band = t / g.wp, w = t % g.wp;
-        const int r = band < g.HR ? band : g.n + band;
-        const int src = g.HR + (((r - g.HR) % g.n) + g.n) % g.n;
-        f[(size_t)r * g.wp + w] = f[(size_t)src * g.wp + w];
-    }
-}
-
-// ---------------------------------------------------------------------------
-// Resident kernel: whole grids in shared memory for `steps` generations.
-// ---------------------------------------------------------------------------
-__device__ void smem_halo(uint32_t* buf, int n, int nw, int HR, int wp) {
-    for (int t = threadIdx.x; t < n * 3; t += blockDim.x) {
-        const int i = t / 3, k = t % 3;
-        const int fw = k == 0 ? 0 : nw + (k - 1);
-        uint32_t* row = buf + (size_t)(HR + i) * wp;
-        row[fw] = halo_word(row, fw, n, nw);
-    }
-    __syncthreads();
-    for (int t = threadIdx.x; t < 2 * HR * wp; t += blockDim.x) {
-        const int band = t / wp, w = t % wp;
-        const int r = band < HR ? band : n + band;
-        const int src = HR + (((r - HR) % n) + n) % n;
-        buf[(size_t)r * wp + w] = buf[(size_t)src * wp + w];
-    }
-    __syncthreads();
-}
-
 template <int R>
 __global__ void __launch_bounds__(kResThreads, 1)
 k_batch_resident(const uint32_t* __restrict__ src, uint32_t* __restrict__ dst, const BatchGrid* __restrict__ grids,
                  const int* __restrict__ list, int n_list, int steps, const __grid_constant__ PackedRule pr) {
-    constexpr int PH = bits_for(2 * R + 1);
-    constexpr int PB = bits_for((2 * R + 1) * (2 * R + 1));
-    extern __shared__ uint32_t sm[];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    extern __shared__ __align__(16) uint32_t sm[];
     for (int li = blockIdx.x; li < n_list; li += gridDim.x) {
         const BatchGrid g = grids[list[li]];
-        const int rows = g.n + 2 * g.HR;
+        const int words = g.n * g.wp;
         uint32_t* bufA = sm;
-        uint32_t* bufB = sm + (size_t)rows * g.wp;
-        // inner words in, halos built in shared memory
-        for (int t = threadIdx.x; t < g.n * g.nw; t += blockDim.x) {
-            const int i = t / g.nw, w = t % g.nw;
-            bufA[(size_t)(g.HR + i) * g.wp + 1 + w] = src[g.off + (size_t)(g.HR + i) * g.wp + 1 + w];
-        }
+        uint32_t* bufB = sm + words;
+        for (int t = threadIdx.x; t < words; t += blockDim.x) bufA[t] = src[g.off + t];
         __syncthreads();
-        smem_halo(bufA, g.n, g.nw, g.HR, g.wp);
-        // work split: every warp owns a band of rows of one 32-word strip
-        const int strips = (g.nw + 31) / 32;
-        const int warps = blockDim.x >> 5;
-        const int bands = max(1, warps / strips);
+        const int bands = min(g.n, max(1, (int)blockDim.x / g.nw));
         const int band_rows = (g.n + bands - 1) / bands;
         for (int s = 0; s < steps; ++s) {
-            for (int it = wid; it < strips * bands; it += warps) {
-                const int ws = it % strips, band = it / strips;
-                const int r0 = band * band_rows, r1 = min(r0 + band_rows, g.n);
-                if (r0 >= r1) continue;  // warp-uniform
-                const int w = ws * 32 + lane;
-                const bool active = w <= g.nw, outputs = w < g.nw;
-                const int fw = 1 + w;
-                auto rowp = [&](int r) { return bufA + (size_t)(g.HR + r) * g.wp; };
-                uint32_t B[PB];
-#pragma unroll
-                for (int i = 0; i < PB; ++i) B[i] = 0u;
-#pragma unroll 1
-                for (int dy = -R; dy <= R; ++dy) {
-                    uint32_t h[PH];
-                    hcount<R, PH, false>(rowp(r0 + dy), fw, active, lane, h);
-                    planes_add<PB, PH>(B, h);
-                }
-#pragma unroll 1
-                for (int r = r0; r < r1; ++r) {
-                    if (outputs) {
-                        const uint32_t sv = rowp(r)[fw];
-                        const uint32_t in1 = planes_in<PB>(B, pr.lo[1], pr.hi[1]) & pr.keep[1];
-                        const uint32_t in0 = planes_in<PB>(B, pr.lo[0], pr.hi[0]) & pr.keep[0];
-                        bufB[(size_t)(g.HR + r) * g.wp + fw] = (sv & in1) | (~sv & in0);
-                    }
-                    if (r + 1 < r1) {
-                        uint32_t h[PH];
-                        hcount<R, PH, false>(rowp(r - R), fw, active, lane, h);
-                        planes_sub<PB, PH>(B, h);
-                        hcount<R, PH, false>(rowp(r + R + 1), fw, active, lane, h);
-                        planes_add<PB, PH>(B, h);
-                    }
-                }
+            for (int it = threadIdx.x; it < g.nw * bands; it += blockDim.x) {
+                const int band = it / g.nw, r0 = band * band_rows, r1 = min(r0 + band_rows, g.n);
+                if (r0 < r1) batch_walk<R, false, false>(bufA, bufB, g, r0, r1, it - band * g.nw, nullptr, 0, pr);
             }
             __syncthreads();
-            smem_halo(bufB, g.n, g.nw, g.HR, g.wp);
             uint32_t* t = bufA;
             bufA = bufB;
             bufB = t;
         }
-        for (int t = threadIdx.x; t < g.n * g.nw; t += blockDim.x) {
-            const int i = t / g.nw, w = t % g.nw;
-            dst[g.off + (size_t)(g.HR + i) * g.wp + 1 + w] = bufA[(size_t)(g.HR + i) * g.wp + 1 + w];
-        }
+        for (int t = threadIdx.x; t < words; t += blockDim.x) dst[g.off + t] = bufA[t];
         __syncthreads();
     }
 }
@@ -244,76 +112,41 @@ k_batch_resident(const uint32_t* __restrict__ src, uint32_t* __restrict__ dst, c
 // the generations of one ltl_batch_step.  A CTA takes whole grids from a device
 // counter, the most work first, and runs a grid's generations back to back with
 // CTA barriers between them, so the grid stays in this SM's L1 and the L2 for
-// the whole run (temporal blocking of the run) and no per-generation launch or
-// halo launch is made.  The grid's radius selects the band walk (a switch over
-// the compiled radii) and its rule class the comparator masks, which are loaded
-// once per grid.  Rows of fewer than 32 words are handled by segments of a warp
-// working on different row bands.
+// the whole run (temporal blocking of the run) and no per-generation launch is
+// made.  The grid's radius selects the band walk (a switch over the compiled radii)
+// and its rule class the comparator masks, which are loaded once per grid.  Lanes
+// are numbered over (band, word), so none idles on narrow rows.
 // ---------------------------------------------------------------------------
 constexpr int kPersistWarps = 8;
-
-// Halo of one frame in global memory, by the whole CTA: the column words of
-// every inner row, then the top and bottom halo rows (copies of whole frame
-// rows, their column words included).  Plain loads: the CTA reads what it
-// wrote before the barrier.
-__device__ void frame_halo_cta(uint32_t* f, const BatchGrid& g) {
-    for (int i = threadIdx.x; i < g.n; i += blockDim.x) halo_cols_row(f + (size_t)(g.HR + i) * g.wp, g.n, g.nw);
-    __syncthreads();
-    const int total = 2 * g.HR * g.wp;
-    for (int t = threadIdx.x; t < total; t += blockDim.x) {
-        const int band = t / g.wp, w = t % g.wp;
-        const int r = band < g.HR ? band : g.n + band;
-        const int src = g.HR + (((r - g.HR) % g.n) + g.n) % g.n;
-        f[(size_t)r * g.wp + w] = f[(size_t)src * g.wp + w];
-    }
-    __syncthreads();
-}
 
 // All generations of one grid by the whole CTA (radius R).
 template <int R>
 __device__ void persist_grid(const BatchGrid& g, uint32_t* a0, uint32_t* a1, int steps, const PackedRule& rule,
                              uint32_t* ring_all) {
-    using Ring = PackedRing<R, kPersistWarps>;
     const PackedRule pr = rule;  // the masks the comparators use, kept in registers
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    uint32_t* ring_lane = ring_all + (size_t)wid * Ring::WARP_WORDS + lane;
+    uint32_t* ring = ring_all + (size_t)wid * PackedRing<R, 1>::WARP_WORDS;
     uint32_t* f0 = a0 + g.off;
     uint32_t* f1 = a1 + g.off;
-    frame_halo_cta(f0, g);
-    // lanes per segment: the row's words rounded up to a power of two, at most 32
-    const int seg = g.nw >= 32 ? 32 : (g.nw <= 1 ? 1 : 1 << (32 - __clz(g.nw - 1)));
-    const int ns = 32 / seg;  // segments per warp
-    const int strips = (g.nw + seg - 1) / seg;
-    // enough bands for every segment of the CTA, none shorter than 2 (2R + 1)
-    // rows (a band first counts 2R + 1 rows to start its window)
-    const int want = max(1, kPersistWarps * ns / strips);
-    const int band_rows = min(g.n, max((g.n + want - 1) / want, 4 * R + 2));
-    const int bands = (g.n + band_rows - 1) / band_rows;
-    const int items = strips * bands;
-    const int wl = lane & (seg - 1), sidx = lane / seg;
+    // a lane per (word, band): as many bands as there are lanes for
+    const int bands = min(g.n, max(1, kPersistWarps * 32 / g.nw));
+    const int band_rows = (g.n + bands - 1) / bands;
+    const int items = g.nw * bands;
     for (int s = 0; s < steps; ++s) {
         const uint32_t* src = (s & 1) ? f1 : f0;
         uint32_t* dst = (s & 1) ? f0 : f1;
-        for (int base = wid * ns; base < items; base += kPersistWarps * ns) {  // warp-uniform
-            const int item = base + sidx;
-            const bool valid = item < items;
-            const int strip = valid ? item % strips : 0;
-            const int band = valid ? item / strips : 0;
-            const int r0 = band * band_rows, r1 = min(r0 + band_rows, g.n);
-            const int w = strip * seg + wl;
-            const bool active = valid && w < g.nw;
-            packed_band_seg<R, Ring::fits>(src, dst, (size_t)g.wp, g.HR, r0, r1, band_rows, 1 + w, active, wl == 0,
-                                           wl == seg - 1 || w == g.nw - 1, ring_lane, pr);
+        for (int it = threadIdx.x; it < items; it += kPersistWarps * 32) {
+            const int band = it / g.nw, r0 = band * band_rows, r1 = min(r0 + band_rows, g.n);
+            if (r0 < r1) batch_walk<R, true, false>(src, dst, g, r0, r1, it - band * g.nw, ring, lane, pr);
         }
         __syncthreads();
-        frame_halo_cta(dst, g);
     }
 }
 
 __global__ void __launch_bounds__(kPersistWarps * 32)
 k_batch_persist(uint32_t* a0, uint32_t* a1, const BatchGrid* __restrict__ grids, const PackedRule* __restrict__ rules,
                 const int* __restrict__ order, int n_order, int* next, int steps) {
-    extern __shared__ uint32_t ring_all[];
+    extern __shared__ __align__(16) uint32_t ring_all[];
     __shared__ int s_item;
     while (true) {
         if (threadIdx.x == 0) s_item = atomicAdd(next, 1);
@@ -333,11 +166,10 @@ k_batch_persist(uint32_t* a0, uint32_t* a1, const BatchGrid* __restrict__ grids,
 }
 
 // Shared memory of the persistent kernel for a batch whose largest radius is R:
-// 8 warps' h rings when they fit (else the walk counts leaving rows again).
+// 8 warps' rings of window counts.
 template <int R>
 static size_t persist_ring_bytes() {
-    using Ring = PackedRing<R, kPersistWarps>;
-    return Ring::fits ? (size_t)Ring::BYTES : 0;
+    return (size_t)kPersistWarps * PackedRing<R, 1>::WARP_WORDS * 4;
 }
 
 // ---------------------------------------------------------------------------
@@ -357,7 +189,7 @@ __global__ void k_batch_pack(const uint8_t* __restrict__ cells, uint32_t* __rest
         uint32_t v = cells16_to_bits<true>(load16(p, c, end));
         if (valid > 16) v |= cells16_to_bits<true>(load16(p + 16, c, end)) << 16;
         if (valid < 32) v &= (1u << valid) - 1u;
-        arena[g.off + (size_t)(g.HR + i) * g.wp + 1 + w] = v;
+        arena[g.off + (size_t)i * g.wp + w] = v;
     }
 }
 
@@ -371,7 +203,7 @@ __global__ void k_batch_unpack(const uint32_t* __restrict__ arena, uint8_t* __re
         uint8_t* row = dst + (size_t)i * g.n;
         const int c = lead(row) + 16 * (t % vecs);
         if (c >= g.n) continue;
-        const uint32_t bits = bits16_at(arena + g.off + (size_t)(g.HR + i) * g.wp + 1, c, g.nw);
+        const uint32_t bits = bits16_at(arena + g.off + (size_t)i * g.wp, c, g.nw);
         store16(row + c, bits16_to_cells(bits), -c, g.n - c);
     }
 }
@@ -382,15 +214,14 @@ __global__ void k_batch_unpack(const uint32_t* __restrict__ arena, uint8_t* __re
 template <int R>
 static size_t res_smem_bytes(int n) {
     const int nw = (n + 31) / 32;
-    const int wp = (nw + 3 + 3) / 4 * 4;
-    return 2ull * (size_t)(n + 2 * (R + 1)) * wp * 4;
+    const int wp = (nw + 3) / 4 * 4;
+    return 2ull * (size_t)n * wp * 4;
 }
 
 template <int R>
 static cudaError_t launch_batch_step_r(const uint32_t* cur, uint32_t* nxt, const BatchGrid* grids, const int4* items,
                                        int n_items, const PackedRule& pr, int sms, cudaStream_t s) {
-    using Ring = PackedRing<R, kBatchWarps>;
-    const int smem = Ring::fits ? Ring::BYTES : 0;
+    const int smem = kBatchWarps * PackedRing<R, 1>::WARP_WORDS * 4;
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_step<R>, kBatchWarps * 32, smem);
     if (per_sm < 1) per_sm = 1;
@@ -403,9 +234,8 @@ static cudaError_t launch_batch_step_r(const uint32_t* cur, uint32_t* nxt, const
 // radius outside any stream capture.
 template <int R>
 static cudaError_t prepare_batch_step_r() {
-    using Ring = PackedRing<R, kBatchWarps>;
-    if (!Ring::fits || Ring::BYTES <= 48 * 1024) return cudaSuccess;
-    return cudaFuncSetAttribute(k_batch_step<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, Ring::BYTES);
+    return cudaFuncSetAttribute(k_batch_step<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                kBatchWarps * PackedRing<R, 1>::WARP_WORDS * 4);
 }
 
 template <int R>
@@ -510,8 +340,6 @@ struct ltl_batch {
     int stream_band_rows = 64;
     long long resident_max = 0;
     BatchGrid* d_grids = nullptr;
-    int* d_streamed_all = nullptr;
-    int n_streamed_all = 0;
     uint32_t* arena[2] = {nullptr, nullptr};
     size_t arena_words = 0;
     uint8_t* staging = nullptr;
@@ -545,7 +373,6 @@ static void batch_release(ltl_batch* b) {
     if (b->d_order) cudaFree(b->d_order);
     if (b->d_rules) cudaFree(b->d_rules);
     if (b->d_grids) cudaFree(b->d_grids);
-    if (b->d_streamed_all) cudaFree(b->d_streamed_all);
     for (auto& a : b->arena)
         if (a) cudaFree(a);
     if (b->staging) cudaFree(b->staging);
@@ -566,7 +393,6 @@ static void batch_release(ltl_batch* b) {
     } while (0)
 
 static uint32_t* cur_arena(ltl_batch* b);
-static cudaError_t refresh_streamed_halo(ltl_batch* b, uint32_t* arena, cudaStream_t s);
 
 // Work plan: which grids are resident, and the streamed work lists.  Rebuilt
 // when a shape parameter changes (the arenas' layout does not depend on it).
@@ -586,9 +412,6 @@ static int batch_plan(ltl_batch* b) {
     if (b->d_order) cudaFree(b->d_order);
     b->d_order = nullptr;
     b->n_order = 0;
-    if (b->d_streamed_all) cudaFree(b->d_streamed_all);
-    b->d_streamed_all = nullptr;
-    b->n_streamed_all = 0;
     const int count = (int)b->grids.size();
     if (b->persistent) {
         // one list of every grid, the most work first (cells x a cost that grows
@@ -612,7 +435,6 @@ static int batch_plan(ltl_batch* b) {
         BATCH_CUDA(cudaMemcpy(b->d_order, order.data(), sizeof(int) * count, cudaMemcpyHostToDevice));
         return LTL_OK;
     }
-    std::vector<int> streamed_all;
     for (int i = 0; i < count; ++i) {
         BatchClass& c = b->classes[b->cls_id[i]];
         const size_t need = res_smem_dispatch(b->grids[i].R, b->grids[i].n);
@@ -621,14 +443,7 @@ static int batch_plan(ltl_batch* b) {
             c.res_smem = std::max(c.res_smem, need);
         } else {
             c.streamed.push_back(i);
-            streamed_all.push_back(i);
         }
-    }
-    b->n_streamed_all = (int)streamed_all.size();
-    if (!streamed_all.empty()) {
-        BATCH_CUDA(cudaMalloc(&b->d_streamed_all, sizeof(int) * streamed_all.size()));
-        BATCH_CUDA(cudaMemcpy(b->d_streamed_all, streamed_all.data(), sizeof(int) * streamed_all.size(),
-                              cudaMemcpyHostToDevice));
     }
     // one shared-memory limit per kernel instantiation (radius): the largest any class of that radius needs
     std::map<int, size_t> smem_by_radius;
@@ -657,11 +472,6 @@ static int batch_plan(ltl_batch* b) {
             BATCH_CUDA(cudaMemcpy(c.d_items, items.data(), sizeof(int4) * items.size(), cudaMemcpyHostToDevice));
         }
     }
-    // the streamed kernels read halos that an upload made in persistent mode left unset
-    if (b->stream && b->arena[0]) {
-        BATCH_CUDA(refresh_streamed_halo(b, cur_arena(b), b->stream));
-        BATCH_CUDA(cudaStreamSynchronize(b->stream));
-    }
     return LTL_OK;
 }
 
@@ -689,12 +499,11 @@ static int batch_build(ltl_batch* b, int flags) {
         BatchGrid g{};
         g.n = d.n;
         g.nw = (d.n + 31) / 32;
-        g.HR = d.radius + 1;
-        g.wp = (g.nw + 3 + 3) / 4 * 4;
+        g.wp = (g.nw + 3) / 4 * 4;
         g.R = d.radius;
         g.off = (long long)words;
         g.cell_off = cells;
-        words += (size_t)(g.n + 2 * g.HR) * g.wp;
+        words += (size_t)g.n * g.wp;
         words = (words + 31) / 32 * 32;
         cells += (long long)g.n * g.n;
         g.cls = it->second;
@@ -829,17 +638,6 @@ extern "C" int ltl_batch_set_stream(ltl_batch* b, void* stream) {
 static uint32_t* cur_arena(ltl_batch* b) { return b->arena[b->cur_is_a ? 0 : 1]; }
 static uint32_t* nxt_arena(ltl_batch* b) { return b->arena[b->cur_is_a ? 1 : 0]; }
 
-static cudaError_t refresh_streamed_halo(ltl_batch* b, uint32_t* arena, cudaStream_t s) {
-    if (b->n_streamed_all == 0) return cudaSuccess;
-    // one block row per grid; launches of at most 65535 grids (the grid-y limit)
-    for (int first = 0; first < b->n_streamed_all; first += 65535) {
-        dim3 g1(8, (unsigned)std::min(65535, b->n_streamed_all - first));
-        k_batch_halo_cols<<<g1, 128, 0, s>>>(arena, b->d_grids, b->d_streamed_all + first);
-        k_batch_halo_rows<<<g1, 128, 0, s>>>(arena, b->d_grids, b->d_streamed_all + first);
-    }
-    return cudaGetLastError();
-}
-
 extern "C" int ltl_batch_upload_all(ltl_batch* b, const uint8_t* cells) {
     if (!b || !cells) {
         ltl_set_error("ltl_batch_upload_all: bad arguments");
@@ -853,7 +651,6 @@ extern "C" int ltl_batch_upload_all(ltl_batch* b, const uint8_t* cells) {
         k_batch_pack<<<g, 256, 0, b->stream>>>(b->staging, cur_arena(b), b->d_grids, first);
     }
     BATCH_CUDA(cudaGetLastError());
-    BATCH_CUDA(refresh_streamed_halo(b, cur_arena(b), b->stream));
     BATCH_CUDA(cudaStreamSynchronize(b->stream));
     return LTL_OK;
 }
@@ -886,7 +683,6 @@ extern "C" int ltl_batch_upload(ltl_batch* b, int grid, const uint8_t* inner, si
                                  b->stream));
     k_batch_pack<<<dim3(16, 1), 256, 0, b->stream>>>(b->staging, cur_arena(b), b->d_grids, grid);
     BATCH_CUDA(cudaGetLastError());
-    BATCH_CUDA(refresh_streamed_halo(b, cur_arena(b), b->stream));
     BATCH_CUDA(cudaStreamSynchronize(b->stream));
     return LTL_OK;
 }
@@ -952,10 +748,6 @@ static cudaError_t enqueue_steps(ltl_batch* b, int steps, const char** what) {
             *what = "streamed step kernel launch";
             e = batch_step_dispatch(c.rule.radius, src, dst, b->d_grids, c.d_items, c.n_items, c.pr, b->sms,
                                     b->stream);
-        }
-        if (e == cudaSuccess) {
-            *what = "halo kernel launch";
-            e = refresh_streamed_halo(b, dst, b->stream);
         }
     }
     if (any_res && e == cudaSuccess) {

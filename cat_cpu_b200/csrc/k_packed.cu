@@ -3,107 +3,385 @@
 // Same function as the reference's HostSolver<int> step (kezada94/CAT_cpu,
 // src/CellularAutomata/Solvers/HostSolver.tpp:58-91, torus halo :93-140), with
 // 32 cells per 32-bit word and the neighbour count kept bit-sliced:
-//   h(row) = horizontal (2R+1)-window count of one row, as PH bit planes, by a
-//            carry-save (Wallace) reduction of the 2R+1 shifted row words;
+//   h(row) = horizontal (2R+1)-window count of one row, as PH bit planes
+//            (window_counts in packed_core.cuh);
 //   B      = vertical sliding sum of h over 2R+1 rows, as PB bit planes
-//            (B -= h(r-R); B += h(r+R+1) while a thread walks down its band);
+//            (B += h(r+R+1) - h(r-R) while a lane walks down its band);
 //   next   = s ? [smin+1 <= B <= smax+1] : [bmin <= B <= bmax]   (B includes the centre)
 // evaluated with bit-sliced comparators.  Every operation acts on 32 cells.
+//
+// Bound by the ALU pipe (16 lanes per scheduler and clock; measured 2.0 cycles per
+// warp for lop3 and funnel shifts alike, and multiply-adds on the otherwise idle FMA
+// pipe cannot do either).  At R = 5 a word costs 67 such operations: window count
+// 23.5, moving B 21, rule 23.  Measured per generation at 16384^2, R = 5: 71.9 us
+// before (a halo'd frame, one word per lane, neighbours by shuffle, 90 operations and
+// as many again around them, 71% of the ALU), 44.3 now (about 84%).
 #include <algorithm>
 
+#include "grid_barrier.cuh"
 #include "packed_core.cuh"
+#include "packed_tile.cuh"
 
 namespace ltl {
 
-constexpr int kPackedWarps = 4;
+constexpr int kPackedWarps = 4;      // band walk: one warp per scheduler, so that k CTAs load all four alike
+constexpr int kTileThreads = 512;
+constexpr int kTileMaxRadius = 16;   // radii of the tile kernels
+constexpr size_t kTileSmem = 220 * 1024;
 
-// Rows per work item when no tuned value applies: as few bands as fill every
-// resident warp once (each band re-counts 2R+1 rows to start its window, so
-// fewer, longer bands waste less), split further only where a band would be
-// longer than 256 rows.
-static int packed_band_rows(int n, int n_wstrips, int resident_warps) {
-    const int per_wave = std::max(1, resident_warps / std::max(n_wstrips, 1));
-    int bands = per_wave;
-    while ((n + bands - 1) / bands > 256) bands += per_wave;
-    return std::max(16, (n + bands - 1) / bands);
+// Words per lane and ring of the band walk, measured at 16384^2 (us): two words
+// per lane share their neighbours' loads and half the loop's bookkeeping (R = 1
+// 26 against 33, R = 5 53 / 58, R = 8 75 / 78), until the ring's share of shared
+// memory leaves too few warps (R = 12 104 / 96, R = 16 128 / 104).  From R = 29 on
+// a ring leaves one or two warps per SM, and counting the leaving row again is
+// cheaper (R = 32 283 against 340, R = 24 226 against 169).
+template <int R>
+constexpr int packed_words() { return R <= 8 ? 2 : 1; }
+template <int R>
+constexpr bool packed_ring() { return R <= 28; }
+
+// Rows per band.  All bands of a step run at once, k CTAs on each SM, and each
+// counts 2R+1 rows (at about 0.6 of an output row's cost) before its first output
+// row: more CTAs per SM keep the ALU busier, fewer repeat less.  Time of a row
+// relative to three or more CTAs per SM, measured on B200 at R = 5 (16384^2: 50.6,
+// 44.6, 46.0 us at k = 2, 3, 4; 4096^2: k = 1 1.5 times): 1.5, 1.12, 1, 1.
+static int packed_band_rows(int rows, int groups, int R, int sms, int per_sm) {
+    static const double rate[] = {1.5, 1.12, 1.0, 1.0};
+    double best = 0;
+    int best_rows = rows;
+    for (int k = 1; k <= std::min(per_sm, 4); ++k) {
+        const long long bands = (long long)sms * k * kPackedWarps * 32 / groups;
+        const int b = bands < 1 ? rows : std::max(2, (int)((rows + bands - 1) / bands));
+        const double t = k * rate[k - 1] * (0.6 * (2 * R + 1) + b);
+        if (best == 0 || t < best) {
+            best = t;
+            best_rows = b;
+        }
+    }
+    return std::min(best_rows, rows);
 }
 
-template <int R, bool FUSE>
-__global__ void __launch_bounds__(kPackedWarps * 32)
-k_packed_step(const uint32_t* __restrict__ cur, uint32_t* __restrict__ nxt, int rows, int nw, int HR, int HW,
-              size_t wp, int n_wstrips, int n_items, int band_rows, const __grid_constant__ PackedRule pr) {
-    using Ring = PackedRing<R, kPackedWarps>;
-    extern __shared__ uint32_t ring_all[];
-    const int lane = threadIdx.x & 31;
-    const int wid = threadIdx.x >> 5;
-    uint32_t* ring_lane = ring_all + (size_t)wid * Ring::WARP_WORDS + lane;
-    const int gwarp = blockIdx.x * kPackedWarps + wid;
-    const int gwarps = gridDim.x * kPackedWarps;
+// Work split of a step: `groups` lanes along a row (W words each) by `bands` row
+// bands, lanes numbered row by row.
+struct PackedSplit {
+    int groups, bands, band_rows;
+    __device__ __forceinline__ bool item(int id, int rows, int W, int& w0, int& r0, int& r1) const {
+        const int band = id / groups;
+        if (band >= bands) return false;
+        w0 = W * (id - band * groups);
+        r0 = band * band_rows;
+        r1 = min(r0 + band_rows, rows);
+        return true;
+    }
+};
 
-    for (int item = gwarp; item < n_items; item += gwarps) {
-        const int ws = item % n_wstrips;
-        const int band = item / n_wstrips;
-        const int r0 = band * band_rows;
-        const int r1 = min(r0 + band_rows, rows);
-        const int w = ws * 32 + lane;     // inner word
-        const bool active = w <= nw;      // w == nw is the right halo word (neighbour of the last word)
-        const bool outputs = w < nw;
-        packed_band<R, Ring::fits, FUSE>(cur, nxt, wp, HR, r0, r1, HW + w, active, outputs, lane, ring_lane, pr,
-                                         rows, nw);
-        __syncwarp();
+// One generation.
+template <int R, int W, bool kRing, int EDGE>
+__global__ void __launch_bounds__(kPackedWarps * 32)
+k_packed_step(const uint32_t* __restrict__ cur, uint32_t* __restrict__ nxt, int wp, int n, int nw, int rows,
+              PackedSplit split, const __grid_constant__ PackedRule pr) {
+    extern __shared__ __align__(16) uint32_t ring_all[];
+    uint32_t* ring = ring_all + (kRing ? (threadIdx.x >> 5) * PackedRing<R, W>::WARP_WORDS : 0);
+    int w0, r0, r1;
+    if (split.item(blockIdx.x * (kPackedWarps * 32) + threadIdx.x, rows, W, w0, r0, r1))
+        packed_walk<R, W, kRing, EDGE, true>(cur, nxt, wp, n, nw, rows, r0, r1, w0, ring, threadIdx.x & 31, pr);
+}
+
+// `steps` generations in one cooperative launch, a tile per CTA (packed_tile.cuh), a
+// grid barrier between generations.
+struct TileSplit {
+    int tile_rows, tile_words;  // of a tile (the last ones of the grid are smaller)
+    int tiles_x, tiles;
+};
+
+template <int R, int EDGE>
+__global__ void __launch_bounds__(kTileThreads, 1)
+k_packed_tiles(uint32_t* a, uint32_t* b, int steps, int wp, int n, int nw, int rows, TileSplit split,
+               GridBarrier* barrier, unsigned int* err, const __grid_constant__ PackedRule pr) {
+    extern __shared__ __align__(16) uint32_t counts[];
+    GridBarrierWait all(barrier, gridDim.x);
+    const int step = kTileThreads / split.tile_words;  // rows of the tile that the CTA's threads take at once
+    const int first = threadIdx.x / split.tile_words, col = threadIdx.x - first * split.tile_words;
+    const int ty = blockIdx.x / split.tiles_x;
+    const int r0 = ty * split.tile_rows, w0 = (blockIdx.x - ty * split.tiles_x) * split.tile_words + col;
+    const int tr = min(split.tile_rows, rows - r0);
+    const bool works = first < step && w0 < nw;
+    const int band = (tr + step - 1) / step, b0 = first * band;
+    for (int s = 0; s < steps; ++s) {
+        const uint32_t* cur = s & 1 ? b : a;
+        uint32_t* nxt = s & 1 ? a : b;
+        if (works) tile_counts<R, EDGE, false>(cur, wp, n, nw, rows, r0, tr, w0, first, step, counts + col);
+        __syncthreads();
+        if (works && b0 < tr) tile_rows<R, false>(cur, nxt, wp, r0, b0, min(b0 + band, tr), w0, counts + col, pr);
+        if (s + 1 < steps && !all.wait(err)) return;
+    }
+}
+
+// The same for grids of at most kTileWords words per row: the generations are done
+// in `blocks` blocks, and a CTA keeps its rows in shared memory for all d generations
+// of a block.  It loads R d rows more on each side, and each generation is exact on R
+// fewer of them.  A grid that is one CTA's alone (blocks = 1) wraps its rows in shared
+// memory and needs no halo.  `blocks` is odd or even as `steps` is, so that the grid
+// ends in the frame where single generations would have left it.
+template <int R, int EDGE>
+__global__ void __launch_bounds__(kTileThreads, 1)
+k_packed_small(uint32_t* a, uint32_t* b, int steps, int blocks, int wp, int n, int nw, int rows, int band_rows,
+               GridBarrier* barrier, unsigned int* err, const __grid_constant__ PackedRule pr) {
+    extern __shared__ __align__(16) uint32_t counts[];
+    const bool whole = gridDim.x == 1;
+    const int ext_max = whole ? rows : band_rows + 2 * R * ((steps + blocks - 1) / blocks);
+    uint32_t* s_in = counts + (size_t)(whole ? rows + 2 * R : ext_max) * PackedTile<R>::ROW;
+    uint32_t* s_out = s_in + (size_t)ext_max * kTileStride;
+    GridBarrierWait all(barrier, gridDim.x);
+    const int step = kTileThreads / nw;
+    const int first = threadIdx.x / nw, col = threadIdx.x - first * nw;
+    const bool works = first < step;
+    const int r0 = blockIdx.x * band_rows, tr = min(band_rows, rows - r0);
+    const uint32_t* cur = a;
+    uint32_t* nxt = b;
+    for (int s = 0; s < steps; --blocks) {
+        const int d = (steps - s + blocks - 1) / blocks;
+        const int halo = whole ? 0 : R * d, ext = tr + 2 * halo;
+        if (works)
+            for (int i = first; i < ext; i += step) {
+                int r = r0 - halo + i;
+                r += r < 0 ? rows : (r >= rows ? -rows : 0);
+                s_in[i * kTileStride + col] = cur[(size_t)r * wp + col];
+            }
+        __syncthreads();
+        for (int k = 1; k <= d; ++k) {
+            const int lo = whole ? 0 : R * k, hi = whole ? rows : ext - R * k;
+            if (works) tile_counts<R, EDGE, false>(s_in, kTileStride, n, nw, ext, lo, hi - lo, col, first, step, counts + col);
+            __syncthreads();
+            const int band = (hi - lo + step - 1) / step, b0 = first * band;
+            if (works && b0 < hi - lo)
+                tile_rows<R, false>(s_in, s_out, kTileStride, lo, b0, min(b0 + band, hi - lo), col, counts + col, pr);
+            __syncthreads();
+            uint32_t* t = s_in;
+            s_in = s_out;
+            s_out = t;
+        }
+        if (whole && steps % 2 == 0) nxt = a;  // (its only block, all read by now)
+        if (works)
+            for (int i = first; i < tr; i += step) nxt[(size_t)(r0 + i) * wp + col] = s_in[(halo + i) * kTileStride + col];
+        s += d;
+        if (s < steps && !all.wait(err)) return;
+        const uint32_t* t = cur;
+        cur = nxt;
+        nxt = (uint32_t*)t;
     }
 }
 
 bool packed_supported(int n, int radius) { return radius >= 1 && radius <= 32 && n >= radius; }
 
-// The step writes the output frame's halo itself (packed_band's kFuse) where
-// every halo word is a whole inner word: n a multiple of 32, one halo word.
-bool packed_fused_halo(const PackedFrame& f, int radius) {
-    return f.HW == 1 && f.n % 32 == 0 && f.n >= 64 && f.nrows() >= 2 * radius + 2;
+template <int R, int W, int EDGE>
+struct PackedLaunch {
+    static constexpr bool kRing = packed_ring<R>();
+    static constexpr int smem = kRing ? kPackedWarps * PackedRing<R, W>::WARP_WORDS * 4 : 0;
+
+    static cudaError_t prepare() {
+        return cudaFuncSetAttribute(k_packed_step<R, W, kRing, EDGE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    smem);
+    }
+    template <class K>
+    static PackedSplit split(K kernel, const PackedFrame& c, int band_rows, unsigned& ctas) {
+        int dev = 0, sms = 148, per_sm = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kPackedWarps * 32, smem);
+        const int rows = c.nrows(), groups = (c.nw + W - 1) / W;
+        if (band_rows <= 0) band_rows = packed_band_rows(rows, groups, R, sms, std::max(per_sm, 1));
+        const int bands = (rows + band_rows - 1) / band_rows;
+        const long long items = (long long)groups * bands;
+        ctas = (unsigned)((items + kPackedWarps * 32 - 1) / (kPackedWarps * 32));
+        return PackedSplit{groups, bands, band_rows};
+    }
+    static cudaError_t step(const PackedFrame& c, const PackedFrame& x, const PackedRule& pr, int band_rows,
+                            cudaStream_t s) {
+        auto kernel = k_packed_step<R, W, kRing, EDGE>;
+        unsigned ctas;
+        const PackedSplit sp = split(kernel, c, band_rows, ctas);
+        kernel<<<ctas, kPackedWarps * 32, smem, s>>>(c.words, x.words, (int)c.wpitch, c.n, c.nw, c.nrows(), sp, pr);
+        return cudaGetLastError();
+    }
+};
+
+// A launch whose CTAs wait for one another (`waits`) has to be cooperative.
+template <class... P, class... A>
+static cudaError_t launch_group(void (*kernel)(P...), unsigned ctas, size_t smem, bool waits, cudaStream_t s,
+                                A... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(kTileThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeCooperative;
+    at.val.cooperative = ctas > 1 && waits;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
+template <int R, int EDGE>
+struct TileLaunch {
+    static cudaError_t prepare() {
+        return cudaFuncSetAttribute(k_packed_tiles<R, EDGE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)kTileSmem);
+    }
+    // one tile per SM
+    static TileSplit split(int rows, int nw, int sms) {
+        TileSplit sp;
+        const int tx = (nw + kTileWords - 1) / kTileWords;
+        sp.tile_words = (nw + tx - 1) / tx;
+        sp.tiles_x = (nw + sp.tile_words - 1) / sp.tile_words;
+        const int bands = std::max(1, sms / sp.tiles_x);
+        sp.tile_rows = (rows + bands - 1) / bands;
+        sp.tiles = sp.tiles_x * ((rows + sp.tile_rows - 1) / sp.tile_rows);
+        return sp;
+    }
+    static bool fits(int rows, int nw, int sms) {
+        const TileSplit sp = split(rows, nw, sms);
+        return sp.tiles <= sms && PackedTile<R>::bytes(sp.tile_rows) <= kTileSmem;
+    }
+    static cudaError_t run(const PackedFrame& c, const PackedFrame& x, const PackedRule& pr, int steps, int sms,
+                           const PackedRun& run, cudaStream_t s) {
+        const TileSplit sp = split(c.nrows(), c.nw, sms);
+        return launch_group(k_packed_tiles<R, EDGE>, (unsigned)sp.tiles, PackedTile<R>::bytes(sp.tile_rows), steps > 1,
+                            s, c.words, x.words, steps, (int)c.wpitch, c.n, c.nw, c.nrows(), sp, run.barrier,
+                            run.err, pr);
+    }
+};
+
+template <int R, int EDGE>
+struct SmallLaunch {
+    static cudaError_t prepare() {
+        return cudaFuncSetAttribute(k_packed_small<R, EDGE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)kTileSmem);
+    }
+    static size_t bytes(int rows, int tile_rows, int depth) {
+        const int ext = tile_rows >= rows ? rows : tile_rows + 2 * R * depth;
+        return PackedTile<R>::bytes(tile_rows >= rows ? rows : ext - 2 * R) + 2ull * ext * kTileStride * 4;
+    }
+    // rows per CTA: all SMs, but bands of at least 4 rows; grids of at most 256 words
+    // are one CTA's (64^2 at R = 5: 0.78 us per generation against 1.03 in four bands
+    // or more; 128^2 1.29 against 1.03)
+    static int tile_rows(int rows, int nw, int sms) {
+        return rows * nw <= 256 ? rows : std::min(rows, std::max(4, (rows + sms - 1) / sms));
+    }
+    static bool fits(int rows, int nw, int sms) {
+        const int tr = tile_rows(rows, nw, sms);
+        return nw <= kTileWords && bytes(rows, tr, 1) <= kTileSmem && (tr == rows || R <= rows);
+    }
+    static cudaError_t run(const PackedFrame& c, const PackedFrame& x, const PackedRule& pr, int steps, int sms,
+                           const PackedRun& run, cudaStream_t s) {
+        const int rows = c.nrows(), tr = tile_rows(rows, c.nw, sms);
+        const unsigned ctas = (unsigned)((rows + tr - 1) / tr);
+        // generations per block: a barrier and the reload cost about 1.5 us, a generation
+        // 0.5 us and the rows that the tile has more.  Best measured (us per generation
+        // at that depth and at 1): 1000^2 R = 2 1.33 at 6 (2.49), R = 5 2.19 at 4 (3.00),
+        // R = 8 2.90 at 2 (3.38), R = 12 3.85 at 1; 128^2 R = 5 0.99 at 8 (2.31), R = 16
+        // 2.48 at 2 (2.87)
+        const int reach = c.nw <= 4 ? 28 : 18;
+        int depth = std::min(steps, std::max(1, std::min(12, (2 * reach + R - 1) / (2 * R))));
+        while (tr < rows && depth > 1 && (bytes(rows, tr, depth) > kTileSmem || R * depth > rows)) --depth;
+        int blocks = (steps + depth - 1) / depth;
+        if (blocks % 2 != steps % 2) ++blocks;  // (then blocks < steps)
+        if (ctas == 1) blocks = 1;
+        depth = (steps + blocks - 1) / blocks;
+        return launch_group(k_packed_small<R, EDGE>, ctas, bytes(rows, tr, depth), blocks > 1, s, c.words, x.words,
+                            steps, blocks, (int)c.wpitch, c.n, c.nw, rows, tr, run.barrier, run.err, pr);
+    }
+};
+
+template <int R>
+static cudaError_t launch_packed_r(const PackedFrame& c, const PackedFrame& x, const PackedRule& pr, int band_rows,
+                                   cudaStream_t s) {
+    constexpr int W = packed_words<R>();
+    if (c.n < 64) return PackedLaunch<R, 1, kEdgeTiny>::step(c, x, pr, band_rows, s);
+    if (packed_edge(c.n, W) == kEdgeNone) return PackedLaunch<R, W, kEdgeNone>::step(c, x, pr, band_rows, s);
+    return PackedLaunch<R, W, kEdgeRagged>::step(c, x, pr, band_rows, s);
+}
+
+// Which kernel advances a grid, by its words and R.  Measured per generation (us, 48
+// per call; walk = one launch of the band walk each): 1024^2 R = 5 small 2.0, walk
+// 4.4; 2048^2 R = 5 tiles 3.0, walk 5.4; 4096^2 R = 16 tiles 9.4, walk 15.3.  Tiles
+// repeat 2R rows per tile and sum 2R+1 counts per thread, which the walk's long
+// bands amortise on larger grids: at R = 1 and 2 the walk is ahead from 6400^2 on
+// (6.9 against 7.4), at R = 3 to 12 tiles still are (9.2 / 10.3 to 15.5 / 22.1), and
+// at 8192^2 the walk is (R = 5 15.3 against 27.6).
+enum PackedRoute { kRouteWalk, kRouteTiles, kRouteSmall };
+
+template <int R>
+static PackedRoute packed_route_r(int rows, int nw, int sms) {
+    if constexpr (R <= kTileMaxRadius) {
+        if (SmallLaunch<R, kEdgeNone>::fits(rows, nw, sms)) return kRouteSmall;
+        const long long words = (long long)rows * nw;
+        if (words <= (R <= 2 ? 1000000 : 1280000) && TileLaunch<R, kEdgeNone>::fits(rows, nw, sms)) return kRouteTiles;
+    }
+    return kRouteWalk;
+}
+
+template <int R, int EDGE>
+static cudaError_t prepare_packed_edge(PackedRoute route) {
+    return route == kRouteSmall ? SmallLaunch<R, EDGE>::prepare() : TileLaunch<R, EDGE>::prepare();
+}
+
+template <int R, int EDGE>
+static cudaError_t run_packed_edge(const PackedFrame& c, const PackedFrame& x, const PackedRule& pr, int steps,
+                                   PackedRoute route, int sms, const PackedRun& run, cudaStream_t s) {
+    return route == kRouteSmall ? SmallLaunch<R, EDGE>::run(c, x, pr, steps, sms, run, s)
+                                : TileLaunch<R, EDGE>::run(c, x, pr, steps, sms, run, s);
 }
 
 template <int R>
-static cudaError_t launch_packed_r(const PackedFrame& c, const PackedFrame& x, const PackedRule& pr,
-                                   int band_override, cudaStream_t s) {
-    int dev = 0, sms = 148, per_sm = 0;
+static cudaError_t run_packed_r(const PackedFrame& c, const PackedFrame& x, const PackedRule& pr, int steps, int sms,
+                                const PackedRun& run, cudaStream_t s) {
+    if constexpr (R <= kTileMaxRadius) {
+        const PackedRoute route = packed_route_r<R>(c.nrows(), c.nw, sms);
+        if (route == kRouteWalk) return cudaErrorInvalidValue;
+        switch (packed_edge(c.n, 1)) {
+            case kEdgeNone: return run_packed_edge<R, kEdgeNone>(c, x, pr, steps, route, sms, run, s);
+            case kEdgeRagged: return run_packed_edge<R, kEdgeRagged>(c, x, pr, steps, route, sms, run, s);
+            default: return run_packed_edge<R, kEdgeTiny>(c, x, pr, steps, route, sms, run, s);
+        }
+    }
+    return cudaErrorInvalidValue;
+}
+
+static int device_sms() {
+    int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    // strips of 32 words cover the inner words; a lane whose word is the right
-    // halo word (w == nw) only feeds its left neighbour, and lane 31 loads the
-    // word past its own directly, so no strip is needed for the halo alone
-    const int n_wstrips = (c.nw + 31) / 32;
-    const int smem = PackedRing<R, kPackedWarps>::fits ? PackedRing<R, kPackedWarps>::BYTES : 0;
-    const bool fuse = packed_fused_halo(x, R);
-    auto kernel = fuse ? k_packed_step<R, true> : k_packed_step<R, false>;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kPackedWarps * 32, smem);
-    if (per_sm < 1) per_sm = 1;
-    const int band_rows =
-        band_override > 0 ? band_override : packed_band_rows(c.nrows(), n_wstrips, sms * per_sm * kPackedWarps);
-    const int bands = (c.nrows() + band_rows - 1) / band_rows;
-    const int items = n_wstrips * bands;
-    int ctas = std::min((items + kPackedWarps - 1) / kPackedWarps, sms * per_sm);
-    kernel<<<ctas, kPackedWarps * 32, smem, s>>>(c.words, x.words, c.nrows(), c.nw, c.HR, c.HW, c.wpitch,
-                                                           n_wstrips, items, band_rows, pr);
-    return cudaGetLastError();
+    return sms;
 }
 
+// Attributes of the kernels that a grid's calls may launch (each one costs about
+// 3 us here, so not those of every form).
 template <int R>
-static cudaError_t prepare_packed_r() {
-    const int smem = PackedRing<R, kPackedWarps>::fits ? PackedRing<R, kPackedWarps>::BYTES : 0;
-    if (smem <= 48 * 1024) return cudaSuccess;
-    cudaError_t e = cudaFuncSetAttribute(k_packed_step<R, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(k_packed_step<R, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+static cudaError_t prepare_packed_r(const PackedFrame& f, int sms) {
+    constexpr int W = packed_words<R>();
+    cudaError_t e = f.n < 64 ? PackedLaunch<R, 1, kEdgeTiny>::prepare()
+                             : (packed_edge(f.n, W) == kEdgeNone ? PackedLaunch<R, W, kEdgeNone>::prepare()
+                                                                : PackedLaunch<R, W, kEdgeRagged>::prepare());
+    if constexpr (R <= kTileMaxRadius) {
+        const PackedRoute route = packed_route_r<R>(f.nrows(), f.nw, sms);
+        if (e != cudaSuccess || route == kRouteWalk) return e;
+        switch (packed_edge(f.n, 1)) {
+            case kEdgeNone: return prepare_packed_edge<R, kEdgeNone>(route);
+            case kEdgeRagged: return prepare_packed_edge<R, kEdgeRagged>(route);
+            default: return prepare_packed_edge<R, kEdgeTiny>(route);
+        }
+    }
+    return e;
 }
 
-cudaError_t packed_prepare(int radius) {
+cudaError_t packed_prepare(const PackedFrame& f, int radius) {
+    const int sms = device_sms();
     switch (radius) {
 #define LTL_PP(r) \
-    case r: return prepare_packed_r<r>();
-        LTL_PP(1) LTL_PP(2) LTL_PP(3) LTL_PP(4) LTL_PP(5) LTL_PP(6) LTL_PP(7) LTL_PP(8)
-        LTL_PP(9) LTL_PP(10) LTL_PP(11) LTL_PP(12) LTL_PP(13) LTL_PP(14) LTL_PP(15) LTL_PP(16)
-        LTL_PP(17) LTL_PP(18) LTL_PP(19) LTL_PP(20) LTL_PP(21) LTL_PP(22) LTL_PP(23) LTL_PP(24)
-        LTL_PP(25) LTL_PP(26) LTL_PP(27) LTL_PP(28) LTL_PP(29) LTL_PP(30) LTL_PP(31) LTL_PP(32)
+    case r: return prepare_packed_r<r>(f, sms);
+        LTL_PACKED_RADII(LTL_PP)
 #undef LTL_PP
         default: return cudaSuccess;
     }
@@ -111,82 +389,38 @@ cudaError_t packed_prepare(int radius) {
 
 cudaError_t launch_packed_step(const PackedFrame& cur, const PackedFrame& nxt, const Rule& rule, int band_rows,
                                cudaStream_t s) {
-    PackedRule pr = make_packed_rule(rule);
+    const PackedRule pr = make_packed_rule(rule);
     switch (rule.radius) {
 #define LTL_PR(r) \
     case r: return launch_packed_r<r>(cur, nxt, pr, band_rows, s);
-        LTL_PR(1) LTL_PR(2) LTL_PR(3) LTL_PR(4) LTL_PR(5) LTL_PR(6) LTL_PR(7) LTL_PR(8)
-        LTL_PR(9) LTL_PR(10) LTL_PR(11) LTL_PR(12) LTL_PR(13) LTL_PR(14) LTL_PR(15) LTL_PR(16)
-        LTL_PR(17) LTL_PR(18) LTL_PR(19) LTL_PR(20) LTL_PR(21) LTL_PR(22) LTL_PR(23) LTL_PR(24)
-        LTL_PR(25) LTL_PR(26) LTL_PR(27) LTL_PR(28) LTL_PR(29) LTL_PR(30) LTL_PR(31) LTL_PR(32)
+        LTL_PACKED_RADII(LTL_PR)
 #undef LTL_PR
         default: return cudaErrorInvalidValue;
     }
 }
 
-// ---------------------------------------------------------------------------
-// Packed halo: column halo bits of inner rows (bit position p of the frame row
-// holds cell (p - 32*HW) mod n), then whole top/bottom rows copied from the
-// inner rows they wrap to.
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t packed_bit(const uint32_t* row, int HW, int cell) {
-    int p = 32 * HW + cell;
-    return (row[p >> 5] >> (p & 31)) & 1u;
-}
-
-__global__ void k_packed_halo_cols(uint32_t* __restrict__ g, int n, int rows, int nw, int HR, int HW, size_t wp) {
-    // per inner row: words [0, HW) and [HW + nw - 1, HW + nw + HW)
-    const int per_row = 2 * HW + 1;
-    const long long total = (long long)rows * per_row;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-         t += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(t / per_row);
-        const int k = (int)(t % per_row);
-        const int fw = k < HW ? k : HW + nw - 1 + (k - HW);
-        uint32_t* row = g + (size_t)(HR + i) * wp;
-        auto slow = [&]() -> uint32_t {
-            uint32_t v = 0u;
-            if (fw == HW + nw - 1) {
-                // last inner word: keep its inner bits, rewrite the bits past n
-                const int inner_bits = n - 32 * (nw - 1);
-                v = inner_bits >= 32 ? row[fw] : (row[fw] & ((1u << inner_bits) - 1u));
-                for (int b = inner_bits; b < 32; ++b) {
-                    int cell = 32 * (nw - 1) + b;
-                    v |= packed_bit(row, HW, cell % n) << b;
-                }
-            } else {
-                for (int b = 0; b < 32; ++b) {
-                    int cell = 32 * (fw - HW) + b;
-                    int src = ((cell % n) + n) % n;
-                    v |= packed_bit(row, HW, src) << b;
-                }
-            }
-            return v;
-        };
-        const uint32_t v = HW == 1 ? packed_halo_word(row, fw, n, nw, slow) : slow();
-        // the halo words only read inner bits (< n), never bits written here
-        row[fw] = v;
+bool packed_runs(const PackedFrame& f, int radius) {
+    const int sms = device_sms();
+    switch (radius) {
+#define LTL_PR(r) \
+    case r: return packed_route_r<r>(f.nrows(), f.nw, sms) != kRouteWalk;
+        LTL_PACKED_RADII(LTL_PR)
+#undef LTL_PR
+        default: return false;
     }
 }
 
-__global__ void k_packed_halo_rows(uint32_t* __restrict__ g, int rows, int HR, size_t wp) {
-    const int band = blockIdx.y;  // 0 .. 2HR-1
-    const int r = band < HR ? band : rows + band;
-    const int src = HR + (((r - HR) % rows) + rows) % rows;
-    uint32_t* d = g + (size_t)r * wp;
-    const uint32_t* sp = g + (size_t)src * wp;
-    for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < (int)wp; w += gridDim.x * blockDim.x) d[w] = sp[w];
-}
-
-cudaError_t launch_packed_halo(const PackedFrame& f, cudaStream_t s) {
-    const long long total = (long long)f.nrows() * (2 * f.HW + 1);
-    int blocks = (int)std::min<long long>((total + 127) / 128, 4096);
-    k_packed_halo_cols<<<blocks, 128, 0, s>>>(f.words, f.n, f.nrows(), f.nw, f.HR, f.HW, f.wpitch);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    dim3 g2((unsigned)std::max<size_t>(1, std::min<size_t>((f.wpitch + 127) / 128, 64)), (unsigned)(2 * f.HR));
-    k_packed_halo_rows<<<g2, 128, 0, s>>>(f.words, f.nrows(), f.HR, f.wpitch);
-    return cudaGetLastError();
+cudaError_t launch_packed_run(const PackedFrame& cur, const PackedFrame& nxt, const Rule& rule, int steps,
+                              const PackedRun& run, cudaStream_t s) {
+    const PackedRule pr = make_packed_rule(rule);
+    const int sms = device_sms();
+    switch (rule.radius) {
+#define LTL_PR(r) \
+    case r: return run_packed_r<r>(cur, nxt, pr, steps, sms, run, s);
+        LTL_PACKED_RADII(LTL_PR)
+#undef LTL_PR
+        default: return cudaErrorInvalidValue;
+    }
 }
 
 }  // namespace ltl

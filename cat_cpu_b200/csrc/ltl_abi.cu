@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "../../include/ltl.h"
+#include "grid_barrier.cuh"
 #include "ltl_kernels.h"
 
 using namespace ltl;
@@ -58,6 +59,9 @@ struct ltl_ctx {
     PackedFrame pa{}, pb{};
     uint32_t* pwords = nullptr;
     size_t pwords_bytes = 0;
+    bool runs = false;          // packed, small grid: many generations per launch
+    PackedRun run{};            // barrier and error word of those launches
+    bool run_unchecked = false; // such a launch was made since its error word was last read
     // PACK-coded staging rows of ltl_upload_packed / ltl_download_packed (made on first use)
     uint64_t* pstage = nullptr;
     // tensor variant
@@ -75,6 +79,7 @@ struct ltl_ctx {
 };
 
 static constexpr int kGraphPasses = 8;
+static constexpr int kRunSteps = 512;  // generations per launch of a small packed grid
 
 static Frame& cur_frame(ltl_ctx* c) { return c->cur_is_a ? c->fa : c->fb; }
 static Frame& nxt_frame(ltl_ctx* c) { return c->cur_is_a ? c->fb : c->fa; }
@@ -195,7 +200,13 @@ static int create_impl(ltl_ctx** out, int device, int rows, int n, int radius, i
     c->frames_bytes = 2 * one;
     e = cudaMalloc(&c->frames, c->frames_bytes);
     if (e == cudaSuccess) e = cudaMemsetAsync(c->frames, 0, c->frames_bytes, c->stream);
-    if (e == cudaSuccess) e = cudaMalloc(&c->scratch, 4 * sizeof(unsigned long long));
+    if (e == cudaSuccess) e = cudaMalloc(&c->scratch, 8 * sizeof(unsigned long long));
+    if (e == cudaSuccess) e = cudaMemsetAsync(c->scratch, 0, 8 * sizeof(unsigned long long), c->stream);
+    if (e == cudaSuccess) {
+        // words 0..3: reductions; 4: barrier; 5: error word
+        c->run.barrier = (GridBarrier*)(c->scratch + 4);
+        c->run.err = (unsigned int*)(c->scratch + 5);
+    }
     if (e != cudaSuccess) {
         ltl_set_error("ltl_create: device allocation of %zu bytes failed: %s", c->frames_bytes,
                       cudaGetErrorString(e));
@@ -218,22 +229,21 @@ static int create_impl(ltl_ctx** out, int device, int rows, int n, int radius, i
     if (variant == LTL_VARIANT_PACKED) c->packed_band_rows = (int)tuning_lookup("packed", radius, n, "band_rows", 0);
     if (variant == LTL_VARIANT_PLAIN) e = plain_prepare(radius);
     if (variant == LTL_VARIANT_PLAIN && e == cudaSuccess) e = plain_tb_prepare(radius);
-    if (variant == LTL_VARIANT_PACKED) e = packed_prepare(radius);
     if (e != cudaSuccess) {
         ltl_set_error("ltl_create: kernel setup failed: %s", cudaGetErrorString(e));
         release(c);
         return LTL_ECUDA;
     }
     if (variant == LTL_VARIANT_PACKED || variant == LTL_VARIANT_TENSOR) {
-        // the packed step reads R + 1 halo rows; the tensor step wraps rows and
-        // words itself and only needs the right halo word to exist
+        // both steps wrap rows and words themselves; the packed step wants 16-byte
+        // aligned rows without a halo, the tensor step a halo word to exist
         PackedFrame p{};
         p.n = n;
         p.rows = rows;
         p.nw = (n + 31) / 32;
-        p.HR = variant == LTL_VARIANT_PACKED ? radius + 1 : 1;
-        p.HW = 1;
-        p.wpitch = round_up((size_t)p.nw + 2 * p.HW + 1, 4);  // +1: edge lanes read one word past the halo
+        p.HR = variant == LTL_VARIANT_PACKED ? 0 : 1;
+        p.HW = variant == LTL_VARIANT_PACKED ? 0 : 1;
+        p.wpitch = round_up((size_t)p.nw + (p.HW ? 2 * p.HW + 1 : 0), 4);
         size_t prow = (size_t)rows + 2 * p.HR;
         size_t pone = round_up(prow * p.wpitch * sizeof(uint32_t), 4096);
         c->pwords_bytes = 2 * pone;
@@ -248,6 +258,12 @@ static int create_impl(ltl_ctx** out, int device, int rows, int n, int radius, i
         c->pa.words = c->pwords;
         c->pb = p;
         c->pb.words = (uint32_t*)((uint8_t*)c->pwords + pone);
+        c->runs = variant == LTL_VARIANT_PACKED && packed_runs(p, radius);
+        if (variant == LTL_VARIANT_PACKED && (e = packed_prepare(p, radius)) != cudaSuccess) {
+            ltl_set_error("ltl_create: kernel setup failed: %s", cudaGetErrorString(e));
+            release(c);
+            return LTL_ECUDA;
+        }
     }
     if (variant == LTL_VARIANT_TENSOR) {
         c->tplan = tensor_plan_create(c->pa, c->pb, c->rule, device, why, sizeof(why));
@@ -333,8 +349,7 @@ static bool keeps_packed(const ltl_ctx* c) {
 // After the current frame's inner cells were written: refresh the halo where the
 // step reads one.
 static int after_upload(ltl_ctx* c) {
-    if (c->variant == LTL_VARIANT_PACKED) LTL_CUDA(launch_packed_halo(cur_packed(c), c->stream));
-    // the SWAR kernels with plain_wrap read inner cells only
+    // the packed and tensor steps and the SWAR kernels with plain_wrap read inner cells only
     if (c->variant == LTL_VARIANT_PLAIN && !c->plain_wrap) LTL_CUDA(launch_halo_fill(cur_frame(c), c->stream));
     return LTL_OK;
 }
@@ -418,8 +433,7 @@ extern "C" int ltl_upload_packed(ltl_ctx* c, const uint64_t* words, size_t word_
     LTL_CUDA(cudaSetDevice(c->device));
     if (keeps_packed(c)) {
         // straight into the packed frame: a little-endian uint64 row is its 32-bit
-        // word row; bits past n are rewritten by the halo pass (packed) or masked
-        // by the step (tensor)
+        // word row; the steps mask the bits past n
         PackedFrame& f = cur_packed(c);
         LTL_CUDA(cudaMemcpy2DAsync(f.words + (size_t)f.HR * f.wpitch + f.HW, f.wpitch * sizeof(uint32_t), words,
                                    word_pitch_bytes, (size_t)f.nw * sizeof(uint32_t), c->rows,
@@ -501,7 +515,7 @@ extern "C" int ltl_upload_rows_device(ltl_ctx* c, int row0, int nrows, const uin
     if (nrows == 0) return LTL_OK;
     LTL_CUDA(cudaSetDevice(c->device));
     if (keeps_packed(c)) {
-        // straight into the packed frame, then its halo
+        // straight into the packed frame
         LTL_CUDA(launch_pack_rows(dev, pitch, false, cur_packed(c), row0, nrows, c->stream));
         return after_upload(c);
     }
@@ -510,6 +524,9 @@ extern "C" int ltl_upload_rows_device(ltl_ctx* c, int row0, int nrows, const uin
                                c->stream));
     return after_upload(c);
 }
+
+// Small packed grids, unless the caller set the band walk's shape.
+static bool runs_packed(const ltl_ctx* c) { return c->runs && c->packed_band_rows <= 0; }
 
 // One pass = `gens` generations (c->depth, or fewer for the remainder of a
 // step count; only the temporally blocked plain kernel takes more than 1).
@@ -546,11 +563,12 @@ static cudaError_t enqueue_pass(ltl_ctx* c, int gens) {
             break;
         }
         case LTL_VARIANT_PACKED: {
-            e = launch_packed_step(cur_packed(c), nxt_packed(c), c->rule, c->packed_band_rows, c->stream);
+            e = runs_packed(c)
+                    ? launch_packed_run(cur_packed(c), nxt_packed(c), c->rule, 1, c->run, c->stream)
+                    : launch_packed_step(cur_packed(c), nxt_packed(c), c->rule, c->packed_band_rows, c->stream);
             step_kernels = 1;
             if (c->timing && e == cudaSuccess) e = cudaEventRecord(e1, c->stream);
-            if (packed_fused_halo(nxt_packed(c), c->rule.radius)) halo_kernels = 0;
-            else if (e == cudaSuccess) e = launch_packed_halo(nxt_packed(c), c->stream);
+            halo_kernels = 0;
             break;
         }
         case LTL_VARIANT_TENSOR: {
@@ -595,6 +613,15 @@ static int build_graph(ltl_ctx* c, int which) {
     return LTL_OK;
 }
 
+// One launch for up to kRunSteps generations (a kernel holds its SMs until its last).
+static cudaError_t enqueue_run(ltl_ctx* c, int steps) {
+    cudaError_t e = launch_packed_run(cur_packed(c), nxt_packed(c), c->rule, steps, c->run, c->stream);
+    if (e != cudaSuccess) return e;
+    c->run_unchecked = true;
+    if (steps % 2) c->cur_is_a = !c->cur_is_a;
+    return e;
+}
+
 extern "C" int ltl_step(ltl_ctx* c, int steps) {
     if (int r = check_ctx(c)) return r;
     if (steps < 0) {
@@ -603,6 +630,10 @@ extern "C" int ltl_step(ltl_ctx* c, int steps) {
     }
     if (steps == 0) return LTL_OK;
     LTL_CUDA(cudaSetDevice(c->device));
+    if (!c->timing && runs_packed(c)) {
+        for (; steps > 0; steps -= kRunSteps) LTL_CUDA(enqueue_run(c, std::min(steps, kRunSteps)));
+        return LTL_OK;
+    }
     int passes = steps / c->depth;
     const int rest = steps % c->depth;  // a last, shorter pass
     while (!c->timing && passes >= kGraphPasses) {
@@ -623,6 +654,17 @@ extern "C" int ltl_synchronize(ltl_ctx* c) {
     if (int r = check_ctx(c)) return r;
     LTL_CUDA(cudaSetDevice(c->device));
     LTL_CUDA(cudaStreamSynchronize(c->stream));
+    if (c->run_unchecked) {
+        unsigned int flag = 0;
+        LTL_CUDA(cudaMemcpy(&flag, c->run.err, sizeof(flag), cudaMemcpyDeviceToHost));
+        c->run_unchecked = false;
+        if (flag) {
+            LTL_CUDA(cudaMemset(c->scratch + 4, 0, 2 * sizeof(unsigned long long)));
+            ltl_set_error("packed kernel reported a bounded-wait timeout; the grid state is unspecified until the "
+                          "next upload");
+            return LTL_ETIMEOUT;
+        }
+    }
     if (c->tplan) {
         unsigned int flag = 0;
         LTL_CUDA(cudaMemcpy(&flag, tensor_plan_error_flag(c->tplan), sizeof(flag), cudaMemcpyDeviceToHost));

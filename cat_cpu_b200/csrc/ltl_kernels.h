@@ -17,7 +17,6 @@ bool plain_swar8_supported(int radius);
 // One-time function attributes (dynamic shared memory) so that launches can be
 // captured in CUDA graphs without configuration calls.
 cudaError_t plain_prepare(int radius);
-cudaError_t packed_prepare(int radius);
 // wrap: read every cell from its inner position (torus wrap inside the kernel),
 // so the frame halo is neither read nor needed; requires plain_wrap_supported(n).
 bool plain_wrap_supported(int n, int rows);
@@ -43,24 +42,36 @@ cudaError_t launch_plain_generic(const Frame& cur, const Frame& nxt, const Rule&
 // K3: bit-packed variant.  Packed frame: 32-bit words, cell (i, j) is bit j % 32
 // of word j / 32 (LSB first; two consecutive words are one little-endian uint64
 // of the PACK codec).  Inner row i is frame row HR + i, inner word w is frame
-// column HW + w; halo bits hold torus copies, like the byte frame.
+// column HW + w.  No step reads a halo: rows and words wrap in the loads.  Bits
+// past n in a row's last word hold anything; readers mask them.
 struct PackedFrame {
     uint32_t* words;
     int n;          // cells per side
     int nw;         // inner words per row = ceil(n / 32)
-    int HR;         // halo rows (>= R + 1)
-    int HW;         // halo words on each side (1: radius <= 32)
+    int HR;         // rows before inner row 0
+    int HW;         // words before inner word 0 (packed step: 0, 16-byte aligned rows)
     size_t wpitch;  // words per frame row
     int rows = 0;   // inner rows of a rectangular torus (0: square, n rows)
     __host__ __device__ int nrows() const { return rows ? rows : n; }
 };
 bool packed_supported(int n, int radius);
+// as plain_prepare, for a grid's frames
+cudaError_t packed_prepare(const PackedFrame& f, int radius);
 // band_rows <= 0: built-in heuristic; > 0: rows per work item (tuning table / ltl_set_param)
 cudaError_t launch_packed_step(const PackedFrame& cur, const PackedFrame& nxt, const Rule& rule, int band_rows,
                                cudaStream_t s);
-cudaError_t launch_packed_halo(const PackedFrame& f, cudaStream_t s);
-// true when launch_packed_step also refreshes the output frame's halo
-bool packed_fused_halo(const PackedFrame& f, int radius);
+// Grids that are advanced many generations per launch (packed_runs: small ones, by
+// sides and radius alone): `steps` generations from cur, to nxt if `steps` is odd,
+// else back in cur; both frames are written.
+struct GridBarrier;
+struct PackedRun {
+    GridBarrier* barrier = nullptr;  // device, zero at first; one per grid, which always has the same CTAs
+    unsigned int* err = nullptr;     // device, zero at first; set if a barrier wait ran out: the grid
+                                     // is then unspecified and the barrier has to be zeroed
+};
+bool packed_runs(const PackedFrame& f, int radius);
+cudaError_t launch_packed_run(const PackedFrame& cur, const PackedFrame& nxt, const Rule& rule, int steps,
+                              const PackedRun& run, cudaStream_t s);
 
 // Transfers between codings and reductions (k_transfer.cu).  Callers' byte
 // buffers are dense cells, `pitch` bytes per row, any alignment.
@@ -71,7 +82,7 @@ cudaError_t launch_copy_out(const Frame& f, uint8_t* dst, size_t dst_pitch, cuda
 cudaError_t launch_binarize(const Frame& f, cudaStream_t s);
 // Inner rows [row0, row0 + nrows) of a packed frame from / to a buffer whose row
 // i is frame row row0 + i.  nonzero: a cell is alive if its byte is not 0, else
-// by its bit 0.  After packing rows in, a halo the step reads is stale.
+// by its bit 0.
 cudaError_t launch_pack_rows(const uint8_t* src, size_t pitch, bool nonzero, const PackedFrame& dst, int row0,
                              int nrows, cudaStream_t s);
 cudaError_t launch_unpack_rows(const PackedFrame& src, int row0, int nrows, uint8_t* dst, size_t pitch, cudaStream_t s);

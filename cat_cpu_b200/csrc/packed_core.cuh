@@ -7,8 +7,15 @@
 #pragma once
 
 #include <algorithm>
+#include <type_traits>
 
 #include "ltl_kernels.h"
+
+// Radii of the bit-packed kernels (single grids; batches stop at 16).
+#define LTL_BATCH_RADII(X) X(1) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13) X(14) X(15) X(16)
+#define LTL_PACKED_RADII(X)                                                                            \
+    LTL_BATCH_RADII(X) X(17) X(18) X(19) X(20) X(21) X(22) X(23) X(24) X(25) X(26) X(27) X(28) X(29) X(30) \
+    X(31) X(32)
 
 namespace ltl {
 
@@ -23,21 +30,28 @@ __host__ __device__ constexpr int bits_for(int v) {
 //   xor3    a ^ b ^ c                       (sum of a full adder)     0x96
 //   maj3    (a & b) | (a & c) | (b & c)     (carry of a full adder)   0xE8
 //   borrow3 (~a & (b | c)) | (b & c)        (borrow out of a - b - c) 0x8E
-__device__ __forceinline__ uint32_t xor3(uint32_t a, uint32_t b, uint32_t c) {
-    uint32_t d;
-    asm("lop3.b32 %0, %1, %2, %3, 0x96;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
-    return d;
-}
-__device__ __forceinline__ uint32_t maj3(uint32_t a, uint32_t b, uint32_t c) {
-    uint32_t d;
-    asm("lop3.b32 %0, %1, %2, %3, 0xE8;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
-    return d;
-}
-__device__ __forceinline__ uint32_t borrow3(uint32_t a, uint32_t b, uint32_t c) {
-    uint32_t d;
-    asm("lop3.b32 %0, %1, %2, %3, 0x8E;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
-    return d;
-}
+// LTL_LOP3(table, the same function in C, for builds of this header without a GPU).
+#ifdef __CUDACC__
+#define LTL_LOP3(name, table, expr)                                                          \
+    __device__ __forceinline__ uint32_t name(uint32_t a, uint32_t b, uint32_t c) {           \
+        uint32_t d;                                                                          \
+        asm("lop3.b32 %0, %1, %2, %3, " #table ";" : "=r"(d) : "r"(a), "r"(b), "r"(c));      \
+        return d;                                                                            \
+    }
+#else
+#define LTL_LOP3(name, table, expr) \
+    inline uint32_t name(uint32_t a, uint32_t b, uint32_t c) { return expr; }
+#endif
+LTL_LOP3(xor3, 0x96, a ^ b ^ c)
+LTL_LOP3(maj3, 0xE8, (a & b) | (a & c) | (b & c))
+LTL_LOP3(borrow3, 0x8E, (~a & (b | c)) | (b & c))
+// One step of each comparator chain as a single three-input logic operation
+// (written as lop3 so that the run-time mask operand costs one instruction):
+//   ge_step(m, b, ge) = m ? (b & ge) : (b | ge)
+//   le_step(m, b, le) = m ? (~b | le) : (~b & le)
+LTL_LOP3(ge_step, 0x8E, (a & (b & c)) | (~a & (b | c)))
+LTL_LOP3(le_step, 0xB2, (a & (~b | c)) | (~a & (~b & c)))
+#undef LTL_LOP3
 
 // Wallace reduction: out[0..P) = bit planes of the number of set inputs per lane.
 template <int M, int L, int P>
@@ -70,23 +84,6 @@ __device__ __forceinline__ void wallace(const uint32_t* v, uint32_t* out) {
     }
 }
 
-// B -= h (h <= B per lane), B has PB planes, h has PH planes.
-template <int PB, int PH>
-__device__ __forceinline__ void planes_sub(uint32_t (&B)[PB], const uint32_t (&h)[PH]) {
-    uint32_t br = 0u;
-#pragma unroll
-    for (int i = 0; i < PB; ++i) {
-        const uint32_t b = B[i];
-        if (i < PH) {
-            B[i] = xor3(b, h[i], br);
-            br = borrow3(b, h[i], br);
-        } else {
-            B[i] = b ^ br;
-            br = ~b & br;
-        }
-    }
-}
-
 // B += h
 template <int PB, int PH>
 __device__ __forceinline__ void planes_add(uint32_t (&B)[PB], const uint32_t (&h)[PH]) {
@@ -104,304 +101,457 @@ __device__ __forceinline__ void planes_add(uint32_t (&B)[PB], const uint32_t (&h
     }
 }
 
-// One step of each comparator chain as a single three-input logic operation
-// (written as lop3 so that the run-time mask operand costs one instruction):
-//   ge_step(m, b, ge) = m ? (b & ge) : (b | ge)      truth table 0x8E
-//   le_step(m, b, le) = m ? (~b | le) : (~b & le)    truth table 0xB2
-__device__ __forceinline__ uint32_t ge_step(uint32_t m, uint32_t b, uint32_t ge) {
-    uint32_t d;
-    asm("lop3.b32 %0, %1, %2, %3, 0x8E;" : "=r"(d) : "r"(m), "r"(b), "r"(ge));
-    return d;
-}
-__device__ __forceinline__ uint32_t le_step(uint32_t m, uint32_t b, uint32_t le) {
-    uint32_t d;
-    asm("lop3.b32 %0, %1, %2, %3, 0xB2;" : "=r"(d) : "r"(m), "r"(b), "r"(le));
-    return d;
-}
-
-// Lanes where lo <= B <= hi, given the thresholds as per-plane masks (all-ones
-// where the threshold's bit is set); lo, hi < 2^PB.  Two carry chains from the
-// least significant plane up:
-//   ge = carry out of B + ~lo + 1,  le = carry out of hi + ~B + 1.
-template <int PB>
-__device__ __forceinline__ uint32_t planes_in(const uint32_t (&B)[PB], const uint32_t* lm, const uint32_t* hm) {
-    uint32_t ge = 0xffffffffu, le = 0xffffffffu;
-#pragma unroll
-    for (int i = 0; i < PB; ++i) {
-        ge = ge_step(lm[i], B[i], ge);
-        le = le_step(hm[i], B[i], le);
-    }
-    return ge & le;
-}
-
 constexpr int kMaxPlanes = 16;
 
-// Birth (dead cell, index 0) and survival (live cell, index 1) intervals on the
-// box count B, as per-plane bit masks (kernel parameters, so the comparator
-// reads them from the constant bank).  `keep` is ~0u, or 0 for an empty interval.
+// Interval rule on the box count B (centre included), for counts kept as
+// B' = (B - o) mod 2^PB, o = the lower birth bound.  The offset costs nothing (B'
+// starts at -o instead of 0) and turns the birth interval into one comparison,
+// B' <= hi - lo; the survival interval needs two, [lo', hi'] modulo 2^PB, joined
+// by AND, or by OR where the interval wraps.  Three carry chains instead of four,
+// and no select for empty intervals: (2R+1)^2 <= 2^PB - 2 always (a square is not
+// 2^k - 1 for k > 1), so an empty interval is the one value no count takes.
+// Thresholds are per-plane masks (all-ones where the threshold's bit is set).
 struct PackedRule {
-    uint32_t lo[2][kMaxPlanes];
-    uint32_t hi[2][kMaxPlanes];
-    uint32_t keep[2];
+    uint32_t init[kMaxPlanes];     // -o
+    uint32_t birth_hi[kMaxPlanes];
+    uint32_t live_lo[kMaxPlanes];
+    uint32_t live_hi[kMaxPlanes];
+    uint32_t live_wraps;           // ~0 where live_lo > live_hi
 };
+
+__host__ __device__ constexpr int planes_for_radius(int R) { return bits_for((2 * R + 1) * (2 * R + 1)); }
 
 inline PackedRule make_packed_rule(const Rule& r) {
     const int maxB = (2 * r.radius + 1) * (2 * r.radius + 1);
+    const int M = 1 << planes_for_radius(r.radius);
+    const int blo = std::max(r.bmin, 0), bhi = std::min(r.bmax, maxB);
+    // on B = k + 1 (clamped before the addition)
+    const int slo = std::min(std::max(r.smin, -1), maxB) + 1, shi = std::min(r.smax, maxB - 1) + 1;
+    const bool no_birth = blo > bhi, no_live = slo > shi;
+    const int o = no_birth ? maxB + 1 : blo;
+    const int width = no_birth ? 0 : bhi - blo;
+    const int lo = ((no_live ? maxB + 1 : slo) - o + M) % M, hi = ((no_live ? maxB + 1 : shi) - o + M) % M;
     PackedRule p{};
-    const int los[2] = {r.bmin, r.smin + 1};
-    const int his[2] = {r.bmax, r.smax + 1};
-    for (int k = 0; k < 2; ++k) {
-        int lo = std::max(los[k], 0), hi = std::min(his[k], maxB);
-        p.keep[k] = lo > hi ? 0u : 0xffffffffu;
-        if (lo > hi) lo = hi = 0;
-        for (int i = 0; i < kMaxPlanes; ++i) {
-            p.lo[k][i] = ((lo >> i) & 1) ? 0xffffffffu : 0u;
-            p.hi[k][i] = ((hi >> i) & 1) ? 0xffffffffu : 0u;
-        }
+    p.live_wraps = lo > hi ? 0xffffffffu : 0u;
+    const int init = (M - o) % M;
+    for (int i = 0; i < kMaxPlanes; ++i) {
+        p.init[i] = ((init >> i) & 1) ? 0xffffffffu : 0u;
+        p.birth_hi[i] = ((width >> i) & 1) ? 0xffffffffu : 0u;
+        p.live_lo[i] = ((lo >> i) & 1) ? 0xffffffffu : 0u;
+        p.live_hi[i] = ((hi >> i) & 1) ? 0xffffffffu : 0u;
     }
     return p;
 }
 
-// Horizontal window count of one frame row for word column fw (frame column).
-// All lanes of the warp must call it together (shuffles).  kGlobal selects the
-// read-only global load path; rows in shared memory use plain loads.
-template <int R, int PH, bool kGlobal = true>
-__device__ __forceinline__ void hcount(const uint32_t* __restrict__ row, int fw, bool active, int lane,
-                                       uint32_t (&h)[PH]) {
-    auto ld = [&](int i) -> uint32_t {
-        if constexpr (kGlobal) {
-            return __ldg(row + i);
-        } else {
-            return row[i];
-        }
-    };
-    uint32_t own = active ? ld(fw) : 0u;
-    uint32_t left = __shfl_up_sync(0xffffffffu, own, 1);
-    uint32_t right = __shfl_down_sync(0xffffffffu, own, 1);
-    if (lane == 0 && active) left = ld(fw - 1);
-    if (lane == 31 && active) right = ld(fw + 1);
-    uint32_t x[2 * R + 1];
+// Next generation of 32 cells: B = planes of B', s = the centre cells.  Each
+// chain is a carry out, from the least significant plane up: ge of B' + ~lo + 1,
+// le of hi + ~B' + 1.
+template <int PB>
+__device__ __forceinline__ uint32_t rule_planes(const uint32_t (&B)[PB], uint32_t s, const PackedRule& pr) {
+    uint32_t born = 0xffffffffu, ge = 0xffffffffu, le = 0xffffffffu;
 #pragma unroll
-    for (int d = -R; d <= R; ++d) {
-        uint32_t v;
-        if (d == 0)
-            v = own;
-        else if (d > 0)
-            v = __funnelshift_rc(own, right, d);   // cells j + d: higher bits, then the right word
-        else
-            v = __funnelshift_lc(left, own, -d);   // cells j - |d|: lower bits, then the left word
-        x[d + R] = v;
+    for (int i = 0; i < PB; ++i) {
+        born = le_step(pr.birth_hi[i], B[i], born);
+        ge = ge_step(pr.live_lo[i], B[i], ge);
+        le = le_step(pr.live_hi[i], B[i], le);
     }
-    wallace<2 * R + 1, 0, PH>(x, h);
+    const uint32_t lives = maj3(ge, le, pr.live_wraps);  // wraps ? ge | le : ge & le
+    return (s & lives) | (~s & born);
 }
 
-// Shared-memory ring of the last 2R+2 row counts h (PH planes per lane, one
-// ring per warp), so that each row's horizontal count is computed once on
-// entry and read back on exit.  Without it (kRing = false) the leaving row is
-// counted again.
-template <int R, int kWarps>
-struct PackedRing {
-    static constexpr int PH = bits_for(2 * R + 1);
-    static constexpr int ROWS = 2 * R + 2;
-    static constexpr int WARP_WORDS = ROWS * PH * 32;
-    static constexpr int BYTES = WARP_WORDS * 4 * kWarps;
-    static constexpr bool fits = BYTES <= 96 * 1024;
+// B += in - out for window counts in, out (mod 2^PB): one borrow chain over the
+// PH planes, then one signed add.
+template <int PB, int PH>
+__device__ __forceinline__ void planes_move(uint32_t (&B)[PB], const uint32_t (&in)[PH], const uint32_t (&out)[PH]) {
+    uint32_t d[PH], br = 0u;
+#pragma unroll
+    for (int i = 0; i < PH; ++i) {
+        d[i] = xor3(in[i], out[i], br);
+        br = borrow3(in[i], out[i], br);
+    }
+    uint32_t cy = 0u;
+#pragma unroll
+    for (int i = 0; i < PB; ++i) {
+        const uint32_t b = B[i], x = i < PH ? d[i < PH ? i : 0] : br;  // br: the sign planes
+        B[i] = xor3(b, x, cy);
+        cy = maj3(b, x, cy);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Horizontal window counts h of W consecutive words of one row, given the word
+// left of them, the words and the word right of them (x[0 .. W + 1]).
+//
+// R <= 3: a carry-save tree over the 2R+1 shifted copies of each word.
+// R >= 4: the sums of three neighbouring cells are made once (one full adder on
+// x shifted by 0, 1, 2: two planes) and shifted instead of the cells; windows of
+// 2R+1 = 3 q + rest cells are the tree over q such sums and the rest.  The words
+// are first moved by R cells, so that every shift goes one way and W + 1 words
+// (W + 2 above R = 16) of sums serve W words of windows.  Operations per word at
+// W = 2 (shifts and logic): R = 5 23.5 instead of 26, R = 8 37.5 instead of 46,
+// R = 16 67 instead of 94.
+// ---------------------------------------------------------------------------
+
+// Carry-save tree whose weight-1 inputs are v0[M0] and weight-2 inputs v1[M1].
+template <int M0, int M1, int P>
+__device__ __forceinline__ void wallace2(const uint32_t (&v0)[M0], const uint32_t (&v1)[M1], uint32_t (&out)[P]) {
+    constexpr int NF = (M0 - 1) / 2, NH = (M0 - 2 * NF == 2) ? 1 : 0, NC = NF + NH;
+    uint32_t v[M1 + NC];
+#pragma unroll
+    for (int i = 0; i < M1; ++i) v[i] = v1[i];
+    uint32_t acc = v0[0];
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
+        v[M1 + f] = maj3(acc, v0[1 + 2 * f], v0[2 + 2 * f]);
+        acc = xor3(acc, v0[1 + 2 * f], v0[2 + 2 * f]);
+    }
+    if constexpr (NH == 1) {
+        v[M1 + NF] = acc & v0[M0 - 1];
+        acc ^= v0[M0 - 1];
+    }
+    out[0] = acc;
+    wallace<M1 + NC, 1, P>(v, out);
+}
+
+// Bits [32 w + o, 32 w + o + 32) of a row of words (o >= 0 at compile time).
+template <int O, int N>
+__device__ __forceinline__ uint32_t bits_from(const uint32_t (&v)[N], int w) {
+    const int i = w + O / 32;
+    if constexpr (O % 32 == 0) {
+        return v[i];
+    } else {
+        return __funnelshift_r(v[i], i + 1 < N ? v[i + 1] : 0u, O % 32);
+    }
+}
+
+template <int R, int W, int Q, int REST, int N>
+struct WindowInputs {
+    // weight-1 inputs: Q low planes at offsets 0, 3, .., REST raw cells after them
+    template <int K>
+    static __device__ __forceinline__ void low(const uint32_t (&y)[N], const uint32_t (&t0)[N], int w,
+                                               uint32_t (&v)[Q + REST]) {
+        if constexpr (K < Q) {
+            v[K] = bits_from<3 * K>(t0, w);
+            low<K + 1>(y, t0, w, v);
+        } else if constexpr (K < Q + REST) {
+            v[K] = bits_from<3 * Q + (K - Q)>(y, w);
+            low<K + 1>(y, t0, w, v);
+        }
+    }
+    template <int K>
+    static __device__ __forceinline__ void high(const uint32_t (&t1)[N], int w, uint32_t (&v)[Q]) {
+        if constexpr (K < Q) {
+            v[K] = bits_from<3 * K>(t1, w);
+            high<K + 1>(t1, w, v);
+        }
+    }
 };
 
-// One warp's band of output rows [r0, r1) of a packed frame, word column fw
-// of each lane: next = s ? [smin+1 <= B <= smax+1] : [bmin <= B <= bmax] with
-// B the box count (centre included), kept as PB bit planes and slid down the
-// band (B -= h(r - R), B += h(r + R + 1)).  `cur`/`nxt` point at frame row 0,
-// `HR` halo rows, `wp` words per frame row.  ring_lane = this warp's ring + lane
-// (unused when !kRing).  All lanes of the warp must call it together.
-// kFuse: the output frame's halo is written here too (one halo word per side,
-// n a multiple of 32 and n >= 2R + 2): every halo word and halo row is a copy of
-// an inner word or row, so the lane that computes a word also stores it where
-// the torus repeats it -- inner word nw - 1 in the left halo word, word 0 in
-// the right one, rows n - R .. n - 1 above the grid, rows 0 .. R below -- and
-// no halo pass runs between generations.
-template <int R, bool kRing, bool kFuse = false>
-__device__ __forceinline__ void packed_band(const uint32_t* __restrict__ cur, uint32_t* __restrict__ nxt, size_t wp,
-                                            int HR, int r0, int r1, int fw, bool active, bool outputs, int lane,
-                                            uint32_t* ring_lane, const PackedRule& pr, int n = 0, int nw = 0) {
-    constexpr int PH = bits_for(2 * R + 1);
-    constexpr int PB = bits_for((2 * R + 1) * (2 * R + 1));
-    constexpr int RING = 2 * R + 2;
-    // row pointers advance by one frame row per output row; the ring slots of
-    // rows r - R (read back) and r + R + 1 (written) advance with them
-    const uint32_t* rin = cur + (size_t)(HR + r0 - R) * wp;   // next row to count
-    const uint32_t* rs = cur + (size_t)(HR + r0) * wp + fw;   // centre row
-    uint32_t* ro = nxt + (size_t)(HR + r0) * wp + fw;         // output row
-    // kFuse: where this lane's word repeats in the same row (the other halo
-    // word column, or 0), and the row distance of a repeated row
-    const ptrdiff_t fdc = !kFuse ? 0 : fw - 1 == nw - 1 ? -(ptrdiff_t)nw : (fw - 1 == 0 ? (ptrdiff_t)nw : 0);
-    const ptrdiff_t fnr = (ptrdiff_t)n * (ptrdiff_t)wp;
-    uint32_t B[PB];
+template <int R, int W, int PH>
+__device__ __forceinline__ void window_counts(const uint32_t (&x)[W + 2], uint32_t (&h)[W][PH]) {
+    if constexpr (R <= 3) {
 #pragma unroll
-    for (int i = 0; i < PB; ++i) B[i] = 0u;
-#pragma unroll 1
-    for (int k = 0; k < 2 * R + 1; ++k, rin += wp) {
-        uint32_t h[PH];
-        hcount<R, PH>(rin, fw, active, lane, h);
-        planes_add<PB, PH>(B, h);
-        if constexpr (kRing) {
-            uint32_t* sl = ring_lane + k * PH * 32;
+        for (int w = 0; w < W; ++w) {
+            uint32_t v[2 * R + 1];
 #pragma unroll
-            for (int i = 0; i < PH; ++i) sl[32 * i] = h[i];
+            for (int d = -R; d <= R; ++d)
+                v[d + R] = d == 0 ? x[w + 1]
+                                  : (d > 0 ? __funnelshift_r(x[w + 1], x[w + 2], d) : __funnelshift_l(x[w], x[w + 1], -d));
+            wallace<2 * R + 1, 0, PH>(v, h[w]);
+        }
+    } else {
+        constexpr int N = W + (R <= 16 ? 1 : 2);
+        constexpr int Q = (2 * R + 1) / 3, REST = (2 * R + 1) % 3;
+        uint32_t y[N], t0[N], t1[N];  // y: cells from R before the word on; t0, t1: sums of three
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            if constexpr (R == 32) {
+                y[i] = x[i];
+            } else {
+                y[i] = __funnelshift_r(x[i], i + 1 < W + 2 ? x[i + 1 < W + 2 ? i + 1 : 0] : 0u, 32 - R);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            const uint32_t nx = i + 1 < N ? y[i + 1 < N ? i + 1 : 0] : 0u;
+            const uint32_t a = __funnelshift_r(y[i], nx, 1), b = __funnelshift_r(y[i], nx, 2);
+            t0[i] = xor3(y[i], a, b);
+            t1[i] = maj3(y[i], a, b);
+        }
+#pragma unroll
+        for (int w = 0; w < W; ++w) {
+            uint32_t v0[Q + REST], v1[Q];
+            WindowInputs<R, W, Q, REST, N>::template low<0>(y, t0, w, v0);
+            WindowInputs<R, W, Q, REST, N>::template high<0>(t1, w, v1);
+            wallace2<Q + REST, Q, PH>(v0, v1, h[w]);
         }
     }
-    int out_slot = 0;  // ring slot of row r - R; row r + R + 1 goes to the slot before it
-#pragma unroll 1
-    for (int r = r0; r < r1; ++r, rs += wp, ro += wp, rin += wp) {
-        if (outputs) {
-            const uint32_t sv = __ldg(rs);
-            const uint32_t in1 = planes_in<PB>(B, pr.lo[1], pr.hi[1]) & pr.keep[1];
-            const uint32_t in0 = planes_in<PB>(B, pr.lo[0], pr.hi[0]) & pr.keep[0];
-            const uint32_t val = (sv & in1) | (~sv & in0);
-            *ro = val;
-            if constexpr (kFuse) {
-                if (fdc) ro[fdc] = val;
-                if (r <= R || r >= n - R) {  // a row the torus repeats above or below the grid
-                    const ptrdiff_t dr = r <= R ? fnr : -fnr;
-                    ro[dr] = val;
-                    if (fdc) ro[dr + fdc] = val;
+}
+
+// ---------------------------------------------------------------------------
+// The band walk: one lane advances W words of a row (from word w0 on) down the
+// output rows [r0, r1).  B' (PB bit planes per word) slides down the band; the
+// window counts h of the last 2R+1 rows wait in a ring in shared memory, private
+// to the lane (kRing; else the leaving row is counted again).  Lanes do not talk
+// to each other: the words left and right of the lane's come from memory (L1),
+// so any mapping of lanes to (word group, band) works and no lane idles at the
+// end of a row.  The torus is applied to the loads: rows wrap by index, and the
+// first and last lane of a row take their neighbours from the row's other end
+// (EDGE), so no frame has a halo and no pass refreshes one.  The next row's words
+// are loaded one iteration ahead of their use.
+// ---------------------------------------------------------------------------
+enum PackedEdge {
+    kEdgeNone = 0,    // 32 W divides n: neighbours are whole words
+    kEdgeRagged = 1,  // a row's last lane holds cells past n (n >= 64, and nw > W)
+    kEdgeTiny = 2     // n < 64 (W = 1): a row is at most two words, wrapped bit by bit
+};
+
+// Which form a side needs, for W words per lane.
+__host__ __device__ inline int packed_edge(int n, int W) {
+    return n < 64 ? kEdgeTiny : (n % (32 * W) == 0 ? kEdgeNone : kEdgeRagged);
+}
+// Two words per lane need a row of more than two words, or exactly two whole ones.
+__host__ __device__ inline bool packed_two_words(int n) { return n >= 64 && (n + 31) / 32 > 2; }
+
+// The ring of one warp: 2R+1 rows of PH planes of W words per lane, laid out so
+// that a lane's planes are 16-byte vectors and a warp's vectors are contiguous.
+template <int R, int W>
+struct PackedRing {
+    static constexpr int PH = bits_for(2 * R + 1);
+    static constexpr int LANE_WORDS = PH * W;
+    static constexpr int ROW_WORDS = LANE_WORDS * 32;
+    static constexpr int WARP_WORDS = (2 * R + 1) * ROW_WORDS;
+
+    static __device__ __forceinline__ void put(uint32_t* row, int lane, const uint32_t (&h)[W][PH]) {
+        constexpr int V = LANE_WORDS / 4, REM = LANE_WORDS % 4;
+#pragma unroll
+        for (int v = 0; v < V; ++v)
+            *(uint4*)(row + 128 * v + 4 * lane) =
+                make_uint4(h[(4 * v) / PH][(4 * v) % PH], h[(4 * v + 1) / PH][(4 * v + 1) % PH],
+                           h[(4 * v + 2) / PH][(4 * v + 2) % PH], h[(4 * v + 3) / PH][(4 * v + 3) % PH]);
+        if constexpr (REM >= 2)
+            *(uint2*)(row + 128 * V + 2 * lane) =
+                make_uint2(h[(4 * V) / PH][(4 * V) % PH], h[(4 * V + 1) / PH][(4 * V + 1) % PH]);
+        if constexpr (REM % 2 == 1)
+            row[128 * V + (REM == 3 ? 64 : 0) + lane] = h[W - 1][PH - 1];
+    }
+    static __device__ __forceinline__ void get(const uint32_t* row, int lane, uint32_t (&h)[W][PH]) {
+        constexpr int V = LANE_WORDS / 4, REM = LANE_WORDS % 4;
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+            const uint4 q = *(const uint4*)(row + 128 * v + 4 * lane);
+            h[(4 * v) / PH][(4 * v) % PH] = q.x;
+            h[(4 * v + 1) / PH][(4 * v + 1) % PH] = q.y;
+            h[(4 * v + 2) / PH][(4 * v + 2) % PH] = q.z;
+            h[(4 * v + 3) / PH][(4 * v + 3) % PH] = q.w;
+        }
+        if constexpr (REM >= 2) {
+            const uint2 q = *(const uint2*)(row + 128 * V + 2 * lane);
+            h[(4 * V) / PH][(4 * V) % PH] = q.x;
+            h[(4 * V + 1) / PH][(4 * V + 1) % PH] = q.y;
+        }
+        if constexpr (REM % 2 == 1) h[W - 1][PH - 1] = row[128 * V + (REM == 3 ? 64 : 0) + lane];
+    }
+};
+
+// 32 cells from cell a on (0 <= a < n) of a periodic row of n < 64 cells whose
+// first 64 bits are v (copies of the row from bit n on).
+__device__ __forceinline__ uint32_t tiny_cells(uint64_t v, int n, int a) {
+    // bits past 64 continue the period: cell 64 + i is cell 64 % n + i
+    return (uint32_t)(a == 0 ? v : (v >> a) | ((v >> (64 % n)) << (64 - a)));
+}
+
+// One row's words for a lane, as loaded: x[0] left, x[1 .. W] own, x[W + 1]
+// right, e the extra word that an edge lane needs.  fix() turns them into the
+// torus's words.
+template <int W, int EDGE>
+struct RowWords {
+    uint32_t x[W + 2];
+    uint32_t e;
+};
+
+template <int W, int EDGE, bool kConst>
+struct RowReader {
+    int n, nw, w0;
+    int dl, dr, de;   // offsets of the left, right and extra word from the lane's first
+    int jl;           // index of the row's last word among the lane's own
+    int ib;           // cells in the row's last word, 1..32
+
+    __device__ __forceinline__ RowReader(int n_, int nw_, int w0_) : n(n_), nw(nw_), w0(w0_) {
+        jl = nw - 1 - w0;
+        ib = n - 32 * (nw - 1);
+        dl = w0 == 0 ? nw - 1 : -1;
+        dr = jl < W ? -w0 : W;
+        de = w0 == 0 ? nw - 2 : (jl == W ? -w0 : 1 - w0);
+    }
+    static __device__ __forceinline__ uint32_t ld(const uint32_t* p) {
+        if constexpr (kConst) return __ldg(p);
+        else return *p;
+    }
+    // p: the lane's first word in the row
+    __device__ __forceinline__ void load(const uint32_t* p, RowWords<W, EDGE>& r) const {
+        if constexpr (EDGE == kEdgeTiny) {
+            r.x[1] = ld(p - w0);
+            r.e = nw > 1 ? ld(p - w0 + 1) : 0u;
+        } else {
+            own(p, r.x + 1);
+            r.x[0] = ld(p + dl);
+            r.x[W + 1] = ld(p + dr);
+            if constexpr (EDGE == kEdgeRagged)
+                if (w0 == 0 || jl <= W) r.e = ld(p + de);
+        }
+    }
+    __device__ __forceinline__ void own(const uint32_t* p, uint32_t* o) const {
+        if constexpr (W == 2) {
+            uint2 q;
+            if constexpr (kConst) q = __ldg((const uint2*)p);
+            else q = *(const uint2*)p;
+            o[0] = q.x;
+            o[1] = q.y;
+        } else {
+#pragma unroll
+            for (int j = 0; j < W; ++j) o[j] = ld(p + j);
+        }
+    }
+    __device__ __forceinline__ void fix(RowWords<W, EDGE>& r) const {
+        if constexpr (EDGE == kEdgeTiny) {
+            uint64_t v = ((uint64_t)r.e << 32) | r.x[1];
+            v &= (1ull << n) - 1ull;
+            for (int p = n; p < 64; p *= 2) v |= v << p;
+            const int a = (32 * w0) % n;
+            r.x[0] = tiny_cells(v, n, (a + n - 32 % n) % n);
+            r.x[1] = tiny_cells(v, n, a);
+            r.x[2] = tiny_cells(v, n, (a + 32) % n);
+        } else if constexpr (EDGE == kEdgeRagged) {
+            // the last word continues with the row's first cells
+            auto joined = [&](uint32_t last, uint32_t first) {
+                return (last & (0xffffffffu >> (32 - ib))) | __funnelshift_lc(0u, first, ib);
+            };
+            if (jl == W) r.x[W + 1] = joined(r.x[W + 1], w0 == 0 ? r.x[1] : r.e);
+            if (w0 == 0) {
+                // cells n - 32 .. n - 1: the last word's ib cells and the end of the word before
+                r.x[0] = __funnelshift_rc(r.e, r.x[0], ib);
+            } else if (jl < W) {
+                // so do the words after it
+                const uint32_t first = r.x[W + 1];
+                const uint32_t next = __funnelshift_r(first, r.e, 32 - ib);
+#pragma unroll
+                for (int j = 0; j < W; ++j) {
+                    if (j == jl) r.x[1 + j] = joined(r.x[1 + j], first);
+                    if (j == jl + 1) r.x[1 + j] = next;
                 }
+                if (jl == W - 1) r.x[W + 1] = next;
             }
         }
-        if (r + 1 < r1) {
-            uint32_t h[PH];
-            const int in_slot = out_slot == 0 ? RING - 1 : out_slot - 1;
-            if constexpr (kRing) {
-                const uint32_t* sl = ring_lane + out_slot * PH * 32;
-#pragma unroll
-                for (int i = 0; i < PH; ++i) h[i] = sl[32 * i];
-            } else {
-                hcount<R, PH>(rin - (size_t)(2 * R + 1) * wp, fw, active, lane, h);
-            }
-            planes_sub<PB, PH>(B, h);
-            hcount<R, PH>(rin, fw, active, lane, h);
-            planes_add<PB, PH>(B, h);
-            if constexpr (kRing) {
-                uint32_t* sl = ring_lane + in_slot * PH * 32;
-#pragma unroll
-                for (int i = 0; i < PH; ++i) sl[32 * i] = h[i];
-            }
-            out_slot = out_slot + 1 == RING ? 0 : out_slot + 1;
-        }
     }
-}
+};
 
-// Horizontal window count for the segmented band walk below: lanes work in
-// segments, and a lane at a segment's edge (edge_l / edge_r) loads its
-// neighbouring word itself instead of taking it from the next lane.  Loads go
-// through L1 without the read-only path (ld.global.ca), so words this CTA wrote
-// before a __syncthreads are seen.
-template <int R, int PH>
-__device__ __forceinline__ void hcount_seg(const uint32_t* row, int fw, bool active, bool edge_l, bool edge_r,
-                                           uint32_t (&h)[PH]) {
-    const uint32_t own = active ? __ldca(row + fw) : 0u;
-    uint32_t left = __shfl_up_sync(0xffffffffu, own, 1);
-    uint32_t right = __shfl_down_sync(0xffffffffu, own, 1);
-    if (edge_l && active) left = __ldca(row + fw - 1);
-    if (edge_r && active) right = __ldca(row + fw + 1);
-    uint32_t x[2 * R + 1];
-#pragma unroll
-    for (int d = -R; d <= R; ++d) {
-        uint32_t v;
-        if (d == 0)
-            v = own;
-        else if (d > 0)
-            v = __funnelshift_rc(own, right, d);
-        else
-            v = __funnelshift_lc(left, own, -d);
-        x[d + R] = v;
-    }
-    wallace<2 * R + 1, 0, PH>(x, h);
-}
-
-// packed_band for warps whose lanes work on different row bands: every lane
-// has its own band [r0, r1) (the same for the lanes of one segment), and the
-// whole warp runs `len` >= r1 - r0 iterations so that its shuffles stay
-// converged; a lane stops loading and writing once its band has ended.  The
-// h ring (kRing) is per lane, as in packed_band.  All lanes call it together.
-template <int R, bool kRing>
-__device__ __forceinline__ void packed_band_seg(const uint32_t* cur, uint32_t* nxt, size_t wp, int HR, int r0, int r1,
-                                                int len, int fw, bool active, bool edge_l, bool edge_r,
-                                                uint32_t* ring_lane, const PackedRule& pr) {
+// cur, nxt: word 0 of row 0; wp words per row (a multiple of 4; the row's words
+// up to a multiple of W may be written).  kConst: cur is not written while the
+// kernel runs (read-only loads).  ring: this warp's ring.
+template <int R, int W, bool kRing, int EDGE, bool kConst>
+__device__ __forceinline__ void packed_walk(const uint32_t* cur, uint32_t* nxt, int wp, int n, int nw, int rows, int r0,
+                                            int r1, int w0, uint32_t* ring, int lane, const PackedRule& pr) {
+    using Ring = PackedRing<R, W>;
     constexpr int PH = bits_for(2 * R + 1);
-    constexpr int PB = bits_for((2 * R + 1) * (2 * R + 1));
-    constexpr int RING = 2 * R + 2;
-    const uint32_t* rin = cur + (size_t)(HR + r0 - R) * wp;  // next row to count
-    const uint32_t* rs = cur + (size_t)(HR + r0) * wp + fw;  // centre row
-    uint32_t* ro = nxt + (size_t)(HR + r0) * wp + fw;        // output row
-    uint32_t B[PB];
+    constexpr int PB = planes_for_radius(R);
+    const RowReader<W, EDGE, kConst> rd(n, nw, w0);
+    const size_t all = (size_t)rows * wp;
+    auto wrap = [&](const uint32_t*& p, int& r) {
+        if (r == rows) {
+            r = 0;
+            p -= all;
+        }
+    };
+    // entering row (ri, pi), leaving row (ro, po, without a ring), centre row, output row
+    int ri = r0 - R < 0 ? r0 - R + rows : r0 - R, ro = ri;
+    const uint32_t* pi = cur + (size_t)ri * wp + w0;
+    const uint32_t* po = pi;
+    const uint32_t* pc = cur + (size_t)r0 * wp + w0;
+    uint32_t* pn = nxt + (size_t)r0 * wp + w0;
+    uint32_t cen[W];
+    rd.own(pc, cen);
+    uint32_t B[W][PB];
 #pragma unroll
-    for (int i = 0; i < PB; ++i) B[i] = 0u;
-    const bool live0 = active && r0 < r1;
+    for (int w = 0; w < W; ++w)
+#pragma unroll
+        for (int i = 0; i < PB; ++i) B[w][i] = pr.init[i];
+    uint32_t* slot = ring;
+    // The window's first 2R+1 rows, kChunk loads in flight at a time: a band of a
+    // few rows (a small grid) is little but this, and waits for L2 once per chunk.
+    constexpr int kChunk = 4;
+    auto start_rows = [&](auto count) {
+        constexpr int kCount = decltype(count)::value;
+        RowWords<W, EDGE> x[kCount];
+#pragma unroll
+        for (int k = 0; k < kCount; ++k) {
+            rd.load(pi, x[k]);
+            pi += wp;
+            ++ri;
+            wrap(pi, ri);
+        }
+#pragma unroll
+        for (int k = 0; k < kCount; ++k) {
+            rd.fix(x[k]);
+            uint32_t h[W][PH];
+            window_counts<R, W, PH>(x[k].x, h);
+#pragma unroll
+            for (int w = 0; w < W; ++w) planes_add<PB, PH>(B[w], h[w]);
+            if constexpr (kRing) {
+                Ring::put(slot, lane, h);
+                slot += Ring::ROW_WORDS;
+            }
+        }
+    };
 #pragma unroll 1
-    for (int k = 0; k < 2 * R + 1; ++k, rin += wp) {
-        uint32_t h[PH];
-        hcount_seg<R, PH>(rin, fw, live0, edge_l, edge_r, h);
-        planes_add<PB, PH>(B, h);
+    for (int k = 0; k < (2 * R + 1) / kChunk; ++k) start_rows(std::integral_constant<int, kChunk>{});
+    if constexpr ((2 * R + 1) % kChunk != 0) start_rows(std::integral_constant<int, (2 * R + 1) % kChunk>{});
+    slot = ring;
+    const uint32_t* const ring_end = ring + Ring::WARP_WORDS;
+    RowWords<W, EDGE> next;
+    if (r0 + 1 < r1) rd.load(pi, next);
+#pragma unroll 1
+    for (int r = r0;; ++r) {
+        uint32_t val[W];
+#pragma unroll
+        for (int w = 0; w < W; ++w) val[w] = rule_planes<PB>(B[w], cen[w], pr);
+        if constexpr (W == 2) {
+            *(uint2*)pn = make_uint2(val[0], val[1]);
+        } else {
+#pragma unroll
+            for (int w = 0; w < W; ++w) pn[w] = val[w];
+        }
+        if (r + 1 >= r1) break;
+        pn += wp;
+        pc += wp;
+        rd.own(pc, cen);
+        RowWords<W, EDGE> x = next;
+        pi += wp;
+        ++ri;
+        wrap(pi, ri);
+        if (r + 2 < r1) rd.load(pi, next);
+        rd.fix(x);
+        uint32_t in[W][PH], out[W][PH];
         if constexpr (kRing) {
-            uint32_t* sl = ring_lane + k * PH * 32;
+            Ring::get(slot, lane, out);
+        } else {
+            RowWords<W, EDGE> y;
+            rd.load(po, y);
+            po += wp;
+            ++ro;
+            wrap(po, ro);
+            rd.fix(y);
+            window_counts<R, W, PH>(y.x, out);
+        }
+        window_counts<R, W, PH>(x.x, in);
 #pragma unroll
-            for (int i = 0; i < PH; ++i) sl[32 * i] = h[i];
+        for (int w = 0; w < W; ++w) planes_move<PB, PH>(B[w], in[w], out[w]);
+        if constexpr (kRing) {
+            Ring::put(slot, lane, in);  // the entering row takes the leaving row's place
+            slot += Ring::ROW_WORDS;
+            if (slot == ring_end) slot = ring;
         }
     }
-    int out_slot = 0;  // ring slot of row r - R; row r + R + 1 goes to the slot before it
-#pragma unroll 1
-    for (int k = 0; k < len; ++k, rs += wp, ro += wp, rin += wp) {
-        const int r = r0 + k;
-        if (active && r < r1) {
-            const uint32_t sv = __ldca(rs);
-            const uint32_t in1 = planes_in<PB>(B, pr.lo[1], pr.hi[1]) & pr.keep[1];
-            const uint32_t in0 = planes_in<PB>(B, pr.lo[0], pr.hi[0]) & pr.keep[0];
-            *ro = (sv & in1) | (~sv & in0);
-        }
-        if (k + 1 < len) {
-            const bool live = active && r + 1 < r1;
-            uint32_t h[PH];
-            const int in_slot = out_slot == 0 ? RING - 1 : out_slot - 1;
-            if constexpr (kRing) {
-                const uint32_t* sl = ring_lane + out_slot * PH * 32;
-#pragma unroll
-                for (int i = 0; i < PH; ++i) h[i] = sl[32 * i];
-            } else {
-                hcount_seg<R, PH>(rin - (size_t)(2 * R + 1) * wp, fw, live, edge_l, edge_r, h);
-            }
-            planes_sub<PB, PH>(B, h);
-            hcount_seg<R, PH>(rin, fw, live, edge_l, edge_r, h);
-            planes_add<PB, PH>(B, h);
-            if constexpr (kRing) {
-                uint32_t* sl = ring_lane + in_slot * PH * 32;
-#pragma unroll
-                for (int i = 0; i < PH; ++i) sl[32 * i] = h[i];
-            }
-            out_slot = out_slot + 1 == RING ? 0 : out_slot + 1;
-        }
-    }
-}
-
-// Halo word fw of a packed frame row with one halo word per side (inner word w
-// at frame word 1 + w): fw = 0 is the left halo (cells n-32 .. n-1), fw = nw
-// the last inner word with its bits past n rewritten (cells 0 ..), fw = nw + 1
-// the right halo (cells 32 nw - n .. 32 nw - n + 31).  For n >= 64 each is a
-// funnel shift of two inner words; `slow` handles smaller grids bit by bit.
-// Only inner bits (< n) are read, so concurrent writers of other halo words
-// of the same row do not matter.
-template <class Slow>
-__device__ __forceinline__ uint32_t packed_halo_word(const uint32_t* row, int fw, int n, int nw, Slow&& slow) {
-    if (n >= 64) {
-        if (fw == nw) {
-            const int ib = n - 32 * (nw - 1);  // inner bits of the last word, 1..32
-            return ib >= 32 ? row[fw] : ((row[fw] & ((1u << ib) - 1u)) | (row[1] << ib));
-        }
-        const int c = fw == 0 ? n - 32 : 32 * nw - n;  // first cell of the word
-        const uint32_t lo = row[1 + (c >> 5)];
-        return (c & 31) ? __funnelshift_r(lo, row[2 + (c >> 5)], c & 31) : lo;
-    }
-    return slow();
 }
 
 }  // namespace ltl

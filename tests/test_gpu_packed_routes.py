@@ -1,0 +1,71 @@
+"""The bit-packed step's kernels at the sides where one takes over from another
+(one CTA, several CTAs with blocked generations, tiles, band walk) and where a row
+ends inside, at or after a word; square and rectangular, one generation and
+several per call (odd and even counts leave the grid in different frames), and
+under stream capture.  Bit-exact against the oracle."""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+from tests.test_packed_walk import rows_cols_step
+
+pytestmark = pytest.mark.gpu
+
+
+def rule_of(r):
+    N = (2 * r + 1) ** 2
+    return (N // 3, N // 2, int(0.4 * N), int(0.46 * N))
+
+
+@pytest.mark.parametrize("radius", [1, 2, 5, 8, 12, 16, 17])
+def test_sides_vs_oracle(radius):
+    import cat_cpu_b200 as C
+    rng = np.random.default_rng(radius)
+    rule = rule_of(radius)
+    for n in (40, 63, 64, 65, 90, 91, 127, 128, 129, 300, 1000, 1024, 1025, 1057, 2111):
+        g = (rng.random((n, n)) < 0.45).astype(np.uint8)
+        with C.CUDASolver(n, radius, rule, variant=C.VARIANT_PACKED) as s:
+            s.setState(g)
+            for steps in (1, 2, 7, 12) if n < 2000 else (3,):
+                s.doSteps(steps)
+                g = O.run(g, radius, rule, steps)
+                assert np.array_equal(s.getCurrentState(), g), (n, radius, steps)
+            s.synchronize()
+
+
+@pytest.mark.parametrize("rows,n,radius", [(17, 96, 16), (5, 1024, 5), (8, 40, 8), (700, 64, 3), (33, 1500, 4), (1200, 50, 2)])
+def test_rectangles_vs_numpy(rows, n, radius):
+    import cat_cpu_b200 as C
+    rng = np.random.default_rng(rows)
+    rule = rule_of(radius)
+    g = (rng.random((rows, n)) < 0.45).astype(np.uint8)
+    with C.CUDASolver(n, radius, rule, variant=C.VARIANT_PACKED, rows=rows) as s:
+        s.setState(g)
+        for steps in (1, 6):
+            s.doSteps(steps)
+            for _ in range(steps):
+                g = rows_cols_step(g, radius, rule)
+            assert np.array_equal(s.getCurrentState(), g), (rows, n, radius, steps)
+
+
+@pytest.mark.parametrize("n,radius", [(64, 5), (300, 5), (2048, 8), (6500, 1)])
+def test_captured_steps_replay(n, radius):
+    """An even number of generations captured into a caller's graph advances the
+    grid on every replay."""
+    import torch
+    import cat_cpu_b200 as C
+    rule = rule_of(radius)
+    g = (np.random.default_rng(n).random((n, n)) < 0.45).astype(np.uint8)
+    stream = torch.cuda.Stream()
+    with C.CUDASolver(n, radius, rule, variant=C.VARIANT_PACKED) as s:
+        s.set_stream(stream.cuda_stream)
+        s.setState(g)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            s.doSteps(4)
+        with torch.cuda.stream(stream):
+            graph.replay()
+            graph.replay()
+        torch.cuda.synchronize()
+        assert np.array_equal(s.getCurrentState(), O.run(g, radius, rule, 8))
+        del graph
