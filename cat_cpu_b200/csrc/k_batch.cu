@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "../../include/ltl.h"
+#include "grid_barrier.cuh"
 #include "packed_core.cuh"
 #include "transfer_core.cuh"
 
@@ -108,68 +109,169 @@ k_batch_resident(const uint32_t* __restrict__ src, uint32_t* __restrict__ dst, c
 }
 
 // ---------------------------------------------------------------------------
-// Persistent kernel: one launch advances every grid of the batch through all
-// the generations of one ltl_batch_step.  A CTA takes whole grids from a device
-// counter, the most work first, and runs a grid's generations back to back with
-// CTA barriers between them, so the grid stays in this SM's L1 and the L2 for
-// the whole run (temporal blocking of the run) and no per-generation launch is
-// made.  The grid's radius selects the band walk (a switch over the compiled radii)
-// and its rule class the comparator masks, which are loaded once per grid.  Lanes
-// are numbered over (band, word), so none idles on narrow rows.
+// Persistent kernel: one launch advances every grid of the batch through all the
+// generations of one ltl_batch_step.  Grids whose share of the work is more than
+// one CTA's get a group of CTAs each (batch_split decides; a group barrier between
+// generations, so the launch is cooperative); when its group is done, and from the
+// start where it has none, a CTA takes whole grids from a device counter, the most
+// work first, with only CTA barriers between generations.  A grid stays in L1 and
+// L2 for the whole run, and no per-generation launch is made.
+//
+// A CTA is four warps (one per scheduler) and walks long bands; several CTAs per SM
+// on different grids fill the ALU and cover each other's barriers.  The band walk
+// has two words per lane up to R = 5 and lanes numbered over
+// (band, word group), so none idles on narrow rows.  Bound by the ALU where there are
+// many grids (512 grids of R <= 2: 6340 GCUPS), by barriers and band starts where
+// there are few.  256 generations of 64 and of 1024 grids of sides 64..2048, R 1..8
+// (without transfers): 52 and 70 ms with one CTA of eight warps per grid, 3.8 and
+// 42 ms so.
 // ---------------------------------------------------------------------------
-constexpr int kPersistWarps = 8;
+constexpr int kPersistWarps = 4;
+constexpr int kPersistThreads = kPersistWarps * 32;
 
-// All generations of one grid by the whole CTA (radius R).
-template <int R>
-__device__ void persist_grid(const BatchGrid& g, uint32_t* a0, uint32_t* a1, int steps, const PackedRule& rule,
-                             uint32_t* ring_all) {
+// Words per lane.  The shared memory of a CTA is the largest ring of any radius in the
+// batch: with two words at R = 6 to 8 it would be 61 to 87 KB and leave two CTAs per SM
+// to every grid of the batch (the 1024-grid ensemble of R 1..8: 61.9 ms against 48.8).
+constexpr int persist_words(int R) { return R <= 5 ? 2 : 1; }
+
+// A CTA's first task: its rank in the group of grid `grid` (size 0: none).
+struct BatchGroup {
+    int grid, rank, size;
+};
+
+// Not inlined: forms and radii that share one function share its registers (255 and
+// spills; one by one they fit the 128 that four CTAs per SM leave).
+template <int R, int W, int EDGE>
+__device__ __noinline__ bool persist_form(const BatchGrid& g, uint32_t* f0, uint32_t* f1, int steps, int rank,
+                                          int size, GridBarrier* barrier, unsigned int* err, const PackedRule& rule,
+                                          uint32_t* ring) {
     const PackedRule pr = rule;  // the masks the comparators use, kept in registers
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    uint32_t* ring = ring_all + (size_t)wid * PackedRing<R, 1>::WARP_WORDS;
-    uint32_t* f0 = a0 + g.off;
-    uint32_t* f1 = a1 + g.off;
-    // a lane per (word, band): as many bands as there are lanes for
-    const int bands = min(g.n, max(1, kPersistWarps * 32 / g.nw));
+    GridBarrierWait group(barrier, size);
+    const int lanes = size * kPersistThreads, id = rank * kPersistThreads + threadIdx.x;
+    const int groups = (g.nw + W - 1) / W;
+    const int bands = min(g.n, max(1, lanes / groups));
     const int band_rows = (g.n + bands - 1) / bands;
-    const int items = g.nw * bands;
+    const int items = groups * ((g.n + band_rows - 1) / band_rows);
     for (int s = 0; s < steps; ++s) {
         const uint32_t* src = (s & 1) ? f1 : f0;
         uint32_t* dst = (s & 1) ? f0 : f1;
-        for (int it = threadIdx.x; it < items; it += kPersistWarps * 32) {
-            const int band = it / g.nw, r0 = band * band_rows, r1 = min(r0 + band_rows, g.n);
-            if (r0 < r1) batch_walk<R, true, false>(src, dst, g, r0, r1, it - band * g.nw, ring, lane, pr);
+        for (int it = id; it < items; it += lanes) {
+            const int band = it / groups, r0 = band * band_rows;
+            packed_walk<R, W, true, EDGE, false>(src, dst, g.wp, g.n, g.nw, g.n, r0, min(r0 + band_rows, g.n),
+                                                 W * (it - band * groups), ring, threadIdx.x & 31, pr);
         }
-        __syncthreads();
+        if (!group.wait(err)) return false;
     }
+    return true;
 }
 
-__global__ void __launch_bounds__(kPersistWarps * 32)
+// All generations of one grid (radius R) by this CTA, or its part of them.
+template <int R>
+__device__ __forceinline__ bool persist_grid(const BatchGrid& g, uint32_t* a0, uint32_t* a1, int steps, int rank, int size,
+                             GridBarrier* barrier, unsigned int* err, const PackedRule& rule, uint32_t* ring_all) {
+    constexpr int W = persist_words(R);
+    uint32_t* ring = ring_all + (threadIdx.x >> 5) * PackedRing<R, W>::WARP_WORDS;
+    uint32_t* f0 = a0 + g.off;
+    uint32_t* f1 = a1 + g.off;
+    if (g.n < 64) return persist_form<R, 1, kEdgeTiny>(g, f0, f1, steps, rank, size, barrier, err, rule, ring);
+    if (packed_edge(g.n, W) == kEdgeNone)
+        return persist_form<R, W, kEdgeNone>(g, f0, f1, steps, rank, size, barrier, err, rule, ring);
+    return persist_form<R, W, kEdgeRagged>(g, f0, f1, steps, rank, size, barrier, err, rule, ring);
+}
+
+__global__ void __launch_bounds__(kPersistThreads, 4)
 k_batch_persist(uint32_t* a0, uint32_t* a1, const BatchGrid* __restrict__ grids, const PackedRule* __restrict__ rules,
-                const int* __restrict__ order, int n_order, int* next, int steps) {
+                const BatchGroup* __restrict__ first, GridBarrier* barriers, const int* __restrict__ order, int n_order,
+                int* next, unsigned int* err, int steps) {
     extern __shared__ __align__(16) uint32_t ring_all[];
     __shared__ int s_item;
+    BatchGroup task = first[blockIdx.x];
     while (true) {
-        if (threadIdx.x == 0) s_item = atomicAdd(next, 1);
-        __syncthreads();
-        const int li = s_item;
-        __syncthreads();  // every thread has read s_item before it is overwritten
-        if (li >= n_order) break;
-        const BatchGrid g = grids[order[li]];
+        if (task.size == 0) {
+            if (threadIdx.x == 0) s_item = atomicAdd(next, 1);
+            __syncthreads();
+            const int li = s_item;
+            __syncthreads();  // every thread has read s_item before it is overwritten
+            if (li >= n_order) break;
+            task = BatchGroup{order[li], 0, 1};
+        }
+        const BatchGrid g = grids[task.grid];
+        bool ok = true;
         switch (g.R) {
-#define LTL_C(r) \
-    case r: persist_grid<r>(g, a0, a1, steps, rules[g.cls], ring_all); break;
+#define LTL_C(r)                                                                                                    \
+    case r:                                                                                                         \
+        ok = persist_grid<r>(g, a0, a1, steps, task.rank, task.size, barriers + task.grid, err, rules[g.cls],       \
+                             ring_all);                                                                             \
+        break;
             LTL_BATCH_RADII(LTL_C)
 #undef LTL_C
             default: break;
         }
+        if (!ok) break;
+        task.size = 0;
     }
 }
 
 // Shared memory of the persistent kernel for a batch whose largest radius is R:
-// 8 warps' rings of window counts.
+// its warps' rings of window counts.
 template <int R>
 static size_t persist_ring_bytes() {
-    return (size_t)kPersistWarps * PackedRing<R, 1>::WARP_WORDS * 4;
+    return (size_t)kPersistWarps * PackedRing<R, persist_words(R)>::WARP_WORDS * 4;
+}
+
+// Which grids get groups of CTAs.  Model of one generation (us) by `size` CTAs on a
+// chip that holds `per_sm` CTAs on each SM: a band's rows, 0.6 of a row for each of the
+// 2R+1 rows that it counts first, and a group barrier.  A row of one CTA among three or
+// more per SM takes `row` times their number; the rates and rows are fitted to single
+// grids at 16384^2 (k_packed.cu).
+struct BatchCost {
+    int n, groups, R;
+    double row;
+    BatchCost(int n_, int nw, int R_, int per_sm) : n(n_), R(R_) {
+        static const double rate[] = {1.5, 1.12, 1.0};
+        const int W = n < 64 ? 1 : persist_words(R);
+        groups = (nw + W - 1) / W;
+        row = per_sm * rate[std::min(per_sm, 3) - 1] * (W == 2 ? 0.098 + 0.0156 * R : 0.090 + 0.0063 * R);
+    }
+    double start() const { return 0.6 * (2 * R + 1); }
+    static constexpr double kBarrier = 1.3, kSingle = 0.3;
+    double time(int size) const {
+        const int lanes = size * kPersistThreads;
+        const int bands = std::min(n, std::max(1, lanes / groups));
+        const int turns = groups > lanes ? (groups + lanes - 1) / lanes : 1;
+        return turns * row * (start() + (n + bands - 1) / bands) + (size > 1 ? kBarrier : kSingle);
+    }
+    // CTAs that bring a generation under t, 0 if none do
+    int size_for(double t) const {
+        if (time(1) <= t) return 1;
+        const int b = (int)((t - kBarrier) / row - start());
+        if (b < 1) return 0;
+        return (int)(((long long)((n + b - 1) / b) * groups + kPersistThreads - 1) / kPersistThreads);
+    }
+};
+
+// The smallest common time t for which all grids fit into `ctas` CTAs: groups side
+// by side, and the sum of all CTAs' time within ctas * t.  sizes: CTAs per grid.
+static void batch_split(const std::vector<BatchCost>& grids, int ctas, std::vector<int>& sizes) {
+    auto fits = [&](double t) {
+        double area = 0;
+        long long grouped = 0;
+        for (const BatchCost& g : grids) {
+            const int k = g.size_for(t);
+            if (k == 0) return false;
+            area += k * g.time(k);
+            if (k > 1) grouped += k;
+        }
+        return grouped <= ctas && area <= ctas * t;
+    };
+    double hi = 0, lo = 0;
+    for (const BatchCost& g : grids) hi += g.time(1);  // one CTA each, one after the other
+    for (int i = 0; i < 24 && hi - lo > 0.01 * hi; ++i) {
+        const double t = 0.5 * (lo + hi);
+        (fits(t) ? hi : lo) = t;
+    }
+    sizes.assign(grids.size(), 1);
+    for (size_t i = 0; i < grids.size(); ++i) sizes[i] = std::max(1, grids[i].size_for(hi));
 }
 
 // ---------------------------------------------------------------------------
@@ -188,7 +290,14 @@ __global__ void k_batch_pack(const uint8_t* __restrict__ cells, uint32_t* __rest
         const int valid = g.n - 32 * w;
         uint32_t v = cells16_to_bits<true>(load16(p, c, end));
         if (valid > 16) v |= cells16_to_bits<true>(load16(p + 16, c, end)) << 16;
-        if (valid < 32) v &= (1u << valid) - 1u;
+        if (valid < 32) {
+            v &= (1u << valid) - 1u;
+            if (g.n >= 64) {
+                const uint8_t* q = c + (size_t)i * g.n;
+                v = join_word(v, cells16_to_bits<true>(load16(q, c, end)) |
+                                     (cells16_to_bits<true>(load16(q + 16, c, end)) << 16), g.n);
+            }
+        }
         arena[g.off + (size_t)i * g.wp + w] = v;
     }
 }
@@ -353,8 +462,13 @@ struct ltl_batch {
     int n_order = 0;
     int* d_next = nullptr;
     PackedRule* d_rules = nullptr;
+    BatchGroup* d_first = nullptr;     // each CTA's first task
+    GridBarrier* d_barriers = nullptr; // one per grid
+    unsigned int* d_err = nullptr;     // set if a group's barrier wait ran out
     int persist_ctas = 0;
     size_t persist_smem = 0;
+    bool grouped = false;              // some grid has more than one CTA: cooperative launch
+    bool unchecked = false;            // a grouped launch was made since d_err was last read
     cudaStream_t own = nullptr, stream = nullptr, aux = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr;
     // graph cache: (steps, parity) -> exec
@@ -371,6 +485,9 @@ static void batch_release(ltl_batch* b) {
     }
     if (b->d_next) cudaFree(b->d_next);
     if (b->d_order) cudaFree(b->d_order);
+    if (b->d_first) cudaFree(b->d_first);
+    if (b->d_barriers) cudaFree(b->d_barriers);
+    if (b->d_err) cudaFree(b->d_err);
     if (b->d_rules) cudaFree(b->d_rules);
     if (b->d_grids) cudaFree(b->d_grids);
     for (auto& a : b->arena)
@@ -410,29 +527,44 @@ static int batch_plan(ltl_batch* b) {
         c.res_smem = 0;
     }
     if (b->d_order) cudaFree(b->d_order);
+    if (b->d_first) cudaFree(b->d_first);
     b->d_order = nullptr;
+    b->d_first = nullptr;
     b->n_order = 0;
+    b->grouped = false;
     const int count = (int)b->grids.size();
     if (b->persistent) {
-        // one list of every grid, the most work first (cells x a cost that grows
-        // with R), which the CTAs of the one launch take in order
-        std::vector<int> order(count);
         size_t smem = 0;
-        for (int i = 0; i < count; ++i) {
-            order[i] = i;
-            smem = std::max(smem, persist_ring_dispatch(b->grids[i].R));
-        }
-        auto cost = [&](int i) { return (double)b->grids[i].n * b->grids[i].n * (4.0 + b->grids[i].R); };
-        std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cost(x) > cost(y); });
+        for (const BatchGrid& g : b->grids) smem = std::max(smem, persist_ring_dispatch(g.R));
         // always raised: the kernel's own static shared memory counts against the default 48 KiB too
         BATCH_CUDA(cudaFuncSetAttribute(k_batch_persist, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         int per_sm = 0;
-        BATCH_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_persist, kPersistWarps * 32, smem));
+        BATCH_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_persist, kPersistThreads, smem));
+        per_sm = std::max(per_sm, 1);
+        const int ctas = b->sms * per_sm;
+        std::vector<BatchCost> cost;
+        for (const BatchGrid& g : b->grids) cost.emplace_back(g.n, g.nw, g.R, per_sm);
+        std::vector<int> sizes;
+        batch_split(cost, ctas, sizes);
+        std::vector<BatchGroup> first;
+        std::vector<int> order;
+        for (int i = 0; i < count; ++i) {
+            if (sizes[i] <= 1) order.push_back(i);
+            else
+                for (int r = 0; r < sizes[i]; ++r) first.push_back(BatchGroup{i, r, sizes[i]});
+        }
+        std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cost[x].time(1) > cost[y].time(1); });
+        b->grouped = !first.empty();
         b->persist_smem = smem;
-        b->persist_ctas = std::max(1, std::min(count, b->sms * std::max(per_sm, 1)));
-        b->n_order = count;
+        b->persist_ctas = (int)std::min<size_t>(ctas, first.size() + order.size());
+        first.resize(b->persist_ctas, BatchGroup{0, 0, 0});
+        b->n_order = (int)order.size();
+        order.resize(count);  // (never empty)
         BATCH_CUDA(cudaMalloc(&b->d_order, sizeof(int) * count));
         BATCH_CUDA(cudaMemcpy(b->d_order, order.data(), sizeof(int) * count, cudaMemcpyHostToDevice));
+        BATCH_CUDA(cudaMalloc(&b->d_first, sizeof(BatchGroup) * first.size()));
+        BATCH_CUDA(cudaMemcpy(b->d_first, first.data(), sizeof(BatchGroup) * first.size(), cudaMemcpyHostToDevice));
+        BATCH_CUDA(cudaMemset(b->d_barriers, 0, sizeof(GridBarrier) * count));
         return LTL_OK;
     }
     for (int i = 0; i < count; ++i) {
@@ -517,6 +649,9 @@ static int batch_build(ltl_batch* b, int flags) {
                                                      : tuning_lookup("batch", -1, 0, "resident_max_bytes", kResSmemLimit);
     b->persistent = !(flags & LTL_BATCH_STREAM_ALL) && tuning_lookup("batch", -1, 0, "persistent", 1) != 0;
     BATCH_CUDA(cudaMalloc(&b->d_next, sizeof(int)));
+    BATCH_CUDA(cudaMalloc(&b->d_err, sizeof(unsigned int)));
+    BATCH_CUDA(cudaMemset(b->d_err, 0, sizeof(unsigned int)));
+    BATCH_CUDA(cudaMalloc(&b->d_barriers, sizeof(GridBarrier) * count));
     {
         std::vector<PackedRule> rules;
         for (auto& c : b->classes) rules.push_back(c.pr);
@@ -638,6 +773,19 @@ extern "C" int ltl_batch_set_stream(ltl_batch* b, void* stream) {
 static uint32_t* cur_arena(ltl_batch* b) { return b->arena[b->cur_is_a ? 0 : 1]; }
 static uint32_t* nxt_arena(ltl_batch* b) { return b->arena[b->cur_is_a ? 1 : 0]; }
 
+// After the stream was waited for: did a group's barrier wait run out?
+static int check_groups(ltl_batch* b) {
+    if (!b->unchecked) return LTL_OK;
+    unsigned int flag = 0;
+    BATCH_CUDA(cudaMemcpy(&flag, b->d_err, sizeof(flag), cudaMemcpyDeviceToHost));
+    b->unchecked = false;
+    if (!flag) return LTL_OK;
+    BATCH_CUDA(cudaMemset(b->d_err, 0, sizeof(flag)));
+    BATCH_CUDA(cudaMemset(b->d_barriers, 0, sizeof(GridBarrier) * b->grids.size()));
+    ltl_set_error("batch kernel reported a bounded-wait timeout; the grids are unspecified until the next upload");
+    return LTL_ETIMEOUT;
+}
+
 extern "C" int ltl_batch_upload_all(ltl_batch* b, const uint8_t* cells) {
     if (!b || !cells) {
         ltl_set_error("ltl_batch_upload_all: bad arguments");
@@ -669,7 +817,7 @@ extern "C" int ltl_batch_download_all(ltl_batch* b, uint8_t* cells) {
     BATCH_CUDA(cudaGetLastError());
     BATCH_CUDA(cudaMemcpyAsync(cells, b->staging, (size_t)b->total_cells, cudaMemcpyDeviceToHost, b->stream));
     BATCH_CUDA(cudaStreamSynchronize(b->stream));
-    return LTL_OK;
+    return check_groups(b);
 }
 
 extern "C" int ltl_batch_upload(ltl_batch* b, int grid, const uint8_t* inner, size_t pitch) {
@@ -699,7 +847,7 @@ extern "C" int ltl_batch_download(ltl_batch* b, int grid, uint8_t* inner, size_t
     BATCH_CUDA(cudaMemcpy2DAsync(inner, pitch, b->staging + g.cell_off, g.n, g.n, g.n, cudaMemcpyDeviceToHost,
                                  b->stream));
     BATCH_CUDA(cudaStreamSynchronize(b->stream));
-    return LTL_OK;
+    return check_groups(b);
 }
 
 // Enqueue `steps` generations of every grid (stream-ordered on b->stream).
@@ -713,9 +861,19 @@ static cudaError_t enqueue_steps(ltl_batch* b, int steps, const char** what) {
         e = cudaMemsetAsync(b->d_next, 0, sizeof(int), b->stream);
         if (e == cudaSuccess) {
             *what = "persistent kernel launch";
-            k_batch_persist<<<b->persist_ctas, kPersistWarps * 32, b->persist_smem, b->stream>>>(
-                a0, a1, b->d_grids, b->d_rules, b->d_order, b->n_order, b->d_next, steps);
-            e = cudaGetLastError();
+            cudaLaunchConfig_t cfg{};
+            cfg.gridDim = dim3(b->persist_ctas);
+            cfg.blockDim = dim3(kPersistThreads);
+            cfg.dynamicSmemBytes = b->persist_smem;
+            cfg.stream = b->stream;
+            cudaLaunchAttribute at{};
+            at.id = cudaLaunchAttributeCooperative;
+            at.val.cooperative = b->grouped;
+            cfg.attrs = &at;
+            cfg.numAttrs = 1;
+            e = cudaLaunchKernelEx(&cfg, k_batch_persist, a0, a1, (const BatchGrid*)b->d_grids,
+                                   (const PackedRule*)b->d_rules, (const BatchGroup*)b->d_first, b->d_barriers,
+                                   (const int*)b->d_order, b->n_order, b->d_next, b->d_err, steps);
         }
         return e;
     }
@@ -764,6 +922,7 @@ extern "C" int ltl_batch_step(ltl_batch* b, int steps) {
     }
     if (steps == 0) return LTL_OK;
     BATCH_CUDA(cudaSetDevice(b->device));
+    b->unchecked = b->unchecked || (b->persistent && b->grouped);
     const char* what = "";
     if (b->no_graph) {
         cudaError_t e = enqueue_steps(b, steps, &what);
@@ -809,7 +968,7 @@ extern "C" int ltl_batch_synchronize(ltl_batch* b) {
     }
     BATCH_CUDA(cudaSetDevice(b->device));
     BATCH_CUDA(cudaStreamSynchronize(b->stream));
-    return LTL_OK;
+    return check_groups(b);
 }
 
 extern "C" int ltl_batch_info(const ltl_batch* b, long long* cells, long long* device_bytes, int* temporal_depth) {

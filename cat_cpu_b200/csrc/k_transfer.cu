@@ -18,7 +18,7 @@
 // src/CellularAutomata/CADataDomainComparator.tpp:8-27.
 #include <algorithm>
 
-#include "ltl_kernels.h"
+#include "packed_core.cuh"
 #include "transfer_core.cuh"
 
 namespace ltl {
@@ -30,8 +30,9 @@ constexpr int kTy = 8;     // rows per block pass
 constexpr int kRows = 4;   // rows per thread in flight
 
 // Byte rows -> word rows: thread = one 32-bit word of a row, kNonzero: a cell is
-// alive if its byte is not 0 (else by its bit 0).  Words past the cells get 0.
-template <bool kNonzero>
+// alive if its byte is not 0 (else by its bit 0).  Words past the cells get 0; bits
+// past them in the last word 0, or the row's first cells (kJoin, cols >= 64).
+template <bool kNonzero, bool kJoin>
 __global__ void __launch_bounds__(kTx * kTy)
 k_cells_to_words(const uint8_t* __restrict__ src, size_t sp, int rows, int cols, uint32_t* __restrict__ dst, size_t dp,
                  int nwords) {
@@ -53,9 +54,16 @@ k_cells_to_words(const uint8_t* __restrict__ src, size_t sp, int rows, int cols,
 #pragma unroll
         for (int k = 0; k < kRows; ++k) {
             const int r = r0 + k * kTy;
-            if (r < rows)
-                dst[(size_t)r * dp + w] =
-                    (cells16_to_bits<kNonzero>(a[k]) | (cells16_to_bits<kNonzero>(b[k]) << 16)) & mask;
+            if (r >= rows) continue;
+            uint32_t v = (cells16_to_bits<kNonzero>(a[k]) | (cells16_to_bits<kNonzero>(b[k]) << 16)) & mask;
+            if constexpr (kJoin) {
+                if (valid > 0 && valid < 32) {
+                    const uint8_t* p = src + (size_t)r * sp;
+                    v = join_word(v, cells16_to_bits<kNonzero>(load16(p, src, end)) |
+                                         (cells16_to_bits<kNonzero>(load16(p + 16, src, end)) << 16), cols);
+                }
+            }
+            dst[(size_t)r * dp + w] = v;
         }
     }
 }
@@ -269,8 +277,25 @@ cudaError_t launch_pack_rows(const uint8_t* src, size_t pitch, bool nonzero, con
                              int nrows, cudaStream_t s) {
     if (nrows <= 0) return cudaSuccess;
     uint32_t* d = word_origin(dst) + (size_t)row0 * dst.wpitch;
-    auto kernel = nonzero ? k_cells_to_words<true> : k_cells_to_words<false>;
+    const bool join = dst.n >= 64 && dst.n % 32 != 0;
+    auto kernel = nonzero ? (join ? k_cells_to_words<true, true> : k_cells_to_words<true, false>)
+                          : (join ? k_cells_to_words<false, true> : k_cells_to_words<false, false>);
     kernel<<<cover(dst.nw, nrows, kRows), kBlock, 0, s>>>(src, pitch, nrows, dst.n, d, dst.wpitch, dst.nw);
+    return cudaGetLastError();
+}
+
+// Rows copied in as words: join their last words.
+__global__ void k_join_rows(uint32_t* __restrict__ words, size_t pitch, int rows, int n, int nw) {
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= rows) return;
+    uint32_t* row = words + (size_t)r * pitch;
+    row[nw - 1] = join_word(row[nw - 1], row[0], n);
+}
+
+cudaError_t launch_join_rows(const PackedFrame& f, cudaStream_t s) {
+    if (f.n < 64 || f.n % 32 == 0) return cudaSuccess;
+    const int rows = f.nrows();
+    k_join_rows<<<(rows + 127) / 128, 128, 0, s>>>(word_origin(f), f.wpitch, rows, f.n, f.nw);
     return cudaGetLastError();
 }
 
@@ -287,7 +312,7 @@ cudaError_t launch_pack(const uint8_t* cells, size_t cell_pitch, int rows, int c
                         size_t word_pitch_words, cudaStream_t s) {
     if (rows == 0 || cols == 0) return cudaSuccess;
     const int nwords = 2 * ((cols + 63) / 64);  // 32-bit halves, little-endian
-    k_cells_to_words<true><<<cover(nwords, rows, kRows), kBlock, 0, s>>>(cells, cell_pitch, rows, cols,
+    k_cells_to_words<true, false><<<cover(nwords, rows, kRows), kBlock, 0, s>>>(cells, cell_pitch, rows, cols,
                                                                        (uint32_t*)words, 2 * word_pitch_words, nwords);
     return cudaGetLastError();
 }

@@ -433,11 +433,12 @@ extern "C" int ltl_upload_packed(ltl_ctx* c, const uint64_t* words, size_t word_
     LTL_CUDA(cudaSetDevice(c->device));
     if (keeps_packed(c)) {
         // straight into the packed frame: a little-endian uint64 row is its 32-bit
-        // word row; the steps mask the bits past n
+        // word row
         PackedFrame& f = cur_packed(c);
         LTL_CUDA(cudaMemcpy2DAsync(f.words + (size_t)f.HR * f.wpitch + f.HW, f.wpitch * sizeof(uint32_t), words,
                                    word_pitch_bytes, (size_t)f.nw * sizeof(uint32_t), c->rows,
                                    cudaMemcpyHostToDevice, c->stream));
+        LTL_CUDA(launch_join_rows(f, c->stream));
     } else {
         if (int r = pack_stage(c)) return r;
         const size_t spitch = (size_t)(c->n + 63) / 64;  // words

@@ -43,7 +43,9 @@ cudaError_t launch_plain_generic(const Frame& cur, const Frame& nxt, const Rule&
 // of word j / 32 (LSB first; two consecutive words are one little-endian uint64
 // of the PACK codec).  Inner row i is frame row HR + i, inner word w is frame
 // column HW + w.  No step reads a halo: rows and words wrap in the loads.  Bits
-// past n in a row's last word hold anything; readers mask them.
+// past n in a row's last word are copies of the row's first cells where n >= 64
+// (joined rows, see packed_core.cuh; uploads make them, the packed step keeps
+// them), else anything; other readers mask them.
 struct PackedFrame {
     uint32_t* words;
     int n;          // cells per side
@@ -85,6 +87,8 @@ cudaError_t launch_binarize(const Frame& f, cudaStream_t s);
 // by its bit 0.
 cudaError_t launch_pack_rows(const uint8_t* src, size_t pitch, bool nonzero, const PackedFrame& dst, int row0,
                              int nrows, cudaStream_t s);
+// Joins every row of a frame whose inner words were copied in from PACK words.
+cudaError_t launch_join_rows(const PackedFrame& f, cudaStream_t s);
 cudaError_t launch_unpack_rows(const PackedFrame& src, int row0, int nrows, uint8_t* dst, size_t pitch, cudaStream_t s);
 // A packed frame's inner words as PACK-coded rows (bits past n cleared).
 cudaError_t launch_frame_to_pack64(const PackedFrame& f, uint64_t* dst, size_t dst_pitch_words, cudaStream_t s);

@@ -29,7 +29,8 @@ def words_of(grid, wp, rng):
     nw = (n + 31) // 32
     padded = np.zeros((rows, nw * 32), dtype=np.uint8)
     padded[:, :n] = grid
-    padded[:, n:] = rng.integers(0, 2, size=(rows, nw * 32 - n))  # bits past n: anything
+    past = nw * 32 - n  # bits past n: the row's first cells from 64 cells on, else anything
+    padded[:, n:] = grid[:, :past] if n >= 64 else rng.integers(0, 2, size=(rows, past))
     out = rng.integers(0, 2**32, size=(rows, wp), dtype=np.uint32)
     out[:, :nw] = np.packbits(padded, axis=1, bitorder="little").view("<u4")
     return out
@@ -60,6 +61,9 @@ def check(host, grid, want, r, rule, words, ring, band, rng):
         return 0
     assert rc == 0, (n, rows, r, words, ring, band, rc)
     assert np.array_equal(cells_of(nxt, n), want), (n, rows, r, words, ring, band)
+    if n >= 64:  # the step keeps the rows joined
+        nw = (n + 31) // 32
+        assert np.array_equal(cells_of(nxt, 32 * nw)[:, n:], want[:, :32 * nw - n]), (n, rows, r, words, ring, band)
     return 1
 
 
@@ -99,6 +103,8 @@ def test_tiles_vs_oracle(host, radius):
             rc = host.packed_tiles_host(cur.ctypes.data_as(ctypes.c_void_p), nxt.ctypes.data_as(ctypes.c_void_p), wp, n,
                                         rows, radius, *rule, tr, tc, threads, band)
             assert rc == 0 and np.array_equal(cells_of(nxt, n), want), (n, rows, radius, tr, tc, rc)
+            if n >= 64:
+                assert np.array_equal(cells_of(nxt, 32 * nw)[:, n:], want[:, :32 * nw - n]), (n, rows, radius, tr, tc)
 
 
 def test_walk_on_strips(host):
