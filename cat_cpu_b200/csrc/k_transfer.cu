@@ -235,6 +235,20 @@ k_words_to_pack(const uint32_t* __restrict__ src, size_t sp, int rows, int n, ui
         dst[(size_t)r * dp + w] = valid > 0 ? __ldg(src + (size_t)r * sp + w) & mask : 0u;
 }
 
+// The other way, last words joined (kJoin).
+template <bool kJoin>
+__global__ void __launch_bounds__(kTx * kTy)
+k_pack_to_words(const uint32_t* __restrict__ src, size_t sp, int rows, int n, uint32_t* __restrict__ dst, size_t dp,
+                int nwords) {
+    const int w = blockIdx.x * kTx + threadIdx.x;
+    if (w >= nwords) return;
+    for (int r = blockIdx.y * kTy + threadIdx.y; r < rows; r += gridDim.y * kTy) {
+        uint32_t v = __ldg(src + (size_t)r * sp + w);
+        if (kJoin && w == nwords - 1) v = join_word(v, __ldg(src + (size_t)r * sp), n);
+        dst[(size_t)r * dp + w] = v;
+    }
+}
+
 // `items` threads along a row, `rows` rows, `per` rows per thread.  `cap`
 // bounds the blocks of a reduction (each ends in an atomic).
 dim3 cover(long long items, int rows, int per, long long cap = 0) {
@@ -284,21 +298,6 @@ cudaError_t launch_pack_rows(const uint8_t* src, size_t pitch, bool nonzero, con
     return cudaGetLastError();
 }
 
-// Rows copied in as words: join their last words.
-__global__ void k_join_rows(uint32_t* __restrict__ words, size_t pitch, int rows, int n, int nw) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= rows) return;
-    uint32_t* row = words + (size_t)r * pitch;
-    row[nw - 1] = join_word(row[nw - 1], row[0], n);
-}
-
-cudaError_t launch_join_rows(const PackedFrame& f, cudaStream_t s) {
-    if (f.n < 64 || f.n % 32 == 0) return cudaSuccess;
-    const int rows = f.nrows();
-    k_join_rows<<<(rows + 127) / 128, 128, 0, s>>>(word_origin(f), f.wpitch, rows, f.n, f.nw);
-    return cudaGetLastError();
-}
-
 cudaError_t launch_unpack_rows(const PackedFrame& src, int row0, int nrows, uint8_t* dst, size_t pitch,
                                cudaStream_t s) {
     if (nrows <= 0) return cudaSuccess;
@@ -329,6 +328,14 @@ cudaError_t launch_frame_to_pack64(const PackedFrame& f, uint64_t* dst, size_t d
     const int rows = f.nrows(), nwords = 2 * ((f.n + 63) / 64);
     k_words_to_pack<<<cover(nwords, rows, 1), kBlock, 0, s>>>(word_origin(f), f.wpitch, rows, f.n, (uint32_t*)dst,
                                                              2 * dst_pitch_words, nwords);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_pack64_to_frame(const uint64_t* src, size_t src_pitch_words, const PackedFrame& f, cudaStream_t s) {
+    const int rows = f.nrows();
+    auto kernel = f.n >= 64 && f.n % 32 != 0 ? k_pack_to_words<true> : k_pack_to_words<false>;
+    kernel<<<cover(f.nw, rows, 1), kBlock, 0, s>>>((const uint32_t*)src, 2 * src_pitch_words, rows, f.n, word_origin(f),
+                                                   f.wpitch, f.nw);
     return cudaGetLastError();
 }
 

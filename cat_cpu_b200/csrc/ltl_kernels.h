@@ -87,11 +87,11 @@ cudaError_t launch_binarize(const Frame& f, cudaStream_t s);
 // by its bit 0.
 cudaError_t launch_pack_rows(const uint8_t* src, size_t pitch, bool nonzero, const PackedFrame& dst, int row0,
                              int nrows, cudaStream_t s);
-// Joins every row of a frame whose inner words were copied in from PACK words.
-cudaError_t launch_join_rows(const PackedFrame& f, cudaStream_t s);
 cudaError_t launch_unpack_rows(const PackedFrame& src, int row0, int nrows, uint8_t* dst, size_t pitch, cudaStream_t s);
 // A packed frame's inner words as PACK-coded rows (bits past n cleared).
 cudaError_t launch_frame_to_pack64(const PackedFrame& f, uint64_t* dst, size_t dst_pitch_words, cudaStream_t s);
+// PACK-coded rows into a packed frame.
+cudaError_t launch_pack64_to_frame(const uint64_t* src, size_t src_pitch_words, const PackedFrame& f, cudaStream_t s);
 // PACK codec on callers' buffers (not 0 -> 1).
 cudaError_t launch_pack(const uint8_t* cells, size_t cell_pitch, int rows, int cols, uint64_t* words,
                         size_t word_pitch_words, cudaStream_t s);
