@@ -102,7 +102,8 @@ extern "C" int ltl_step_noalloc(const uint8_t* dev_in, size_t in_pitch, uint8_t*
     Frame fb{scratch + frame, n, H, pitch};
     const Rule rule{radius, smin, smax, bmin, bmax};
     int band_rows = 0;
-    if (!generic) band_rows = (int)tuning_lookup("plain", radius, n, "band_rows", plain_swar8_band_rows(n, device));
+    if (!generic) band_rows = (int)tuning_lookup("plain", radius, n, "band_rows", 0);
+    if (!generic && band_rows <= 0) band_rows = plain_swar8_band_rows(n, n, radius, 1, device);
     // The frames are not cleared.  The inner cells are written by the copy and
     // the halo by the halo fill before any step reads them.  The kernels also
     // read bytes outside the halo'd grid (the wide kernel's loads past the right

@@ -245,17 +245,34 @@ k_plain_swar8(const uint8_t* __restrict__ cur, uint8_t* __restrict__ nxt, int n,
 
 bool plain_swar8_supported(int radius) { return radius >= 1 && radius <= 5; }
 
-int plain_swar8_band_rows(int n, int device) {
+// Three generations per pass at R <= 2, two above (us per generation, 2 / 3: R = 1
+// 1024^2 4.0 / 3.3, 8192^2 20.0 / 18.4; R = 3 8192^2 23.4 / 25.6; R = 5 1024^2 5.1 / 5.7,
+// 8192^2 24.8 / 27.5).
+int plain_swar8_depth(int radius) { return radius <= 2 ? 3 : 2; }
+
+// Rows per band.  All bands of a pass run at once, k CTAs of four warps per SM; a band
+// walks its rows, 2R rows more per further generation of the pass, and a window start.
+// More CTAs per SM slow each other down, fewer walk longer: time of a row at k = 1 .. 4
+// 0.27, 0.36, 0.50, 0.64 us, fitted to R = 5 at depth 2 (1024^2 10.2 us a pass with 16
+// rows, 25.0 with 64; 4096^2 18.4 with 16 rows, 18.6 with 32, 25.4 with 64; 8192^2 49.6
+// with 64, 69 with 16).
+int plain_swar8_band_rows(int rows, int n, int radius, int depth, int device) {
+    static const double row_us[] = {0.27, 0.36, 0.50, 0.64};
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     const int strips = (n + kStripOut - 1) / kStripOut;
-    // Enough items for ~32 resident warps per SM, but bands of at least 96 rows:
-    // every band re-reads 2R+1 rows to start its vertical window.
-    long long target_items = (long long)sms * 32;
-    int bands = (int)std::max<long long>(1, target_items / std::max(strips, 1));
-    int rows = (n + bands - 1) / bands;
-    rows = std::max(96, std::min(rows, 512));
-    return rows;
+    double best = 0;
+    int best_rows = rows;
+    for (int k = 1; k <= 4; ++k) {
+        const int bands = std::max(1, sms * k * kPlainWarps / strips);
+        const int b = std::max(8, (rows + bands - 1) / bands);
+        const double t = row_us[k - 1] * (b + 2 * radius * (depth - 1) + 0.3 * (2 * radius + 1));
+        if (best == 0 || t < best) {
+            best = t;
+            best_rows = b;
+        }
+    }
+    return std::min(best_rows, std::max(rows, 1));
 }
 
 template <int R>

@@ -44,6 +44,10 @@ struct ltl_ctx {
     int rows = 0;    // rows (== n except for ltl_create_rect)
     Rule rule{};
     int variant = LTL_VARIANT_PLAIN;
+    // LTL_VARIANT_AUTO runs the bit-packed kernels where they are the fastest, but its
+    // info and parameters stay those of the plain variant that it always named
+    bool auto_packed = false;
+    int plain_depth = 1;        // auto_packed: the depth that info reports
     int depth = 1;
     Frame fa{}, fb{};
     bool cur_is_a = true;
@@ -57,7 +61,6 @@ struct ltl_ctx {
     int packed_band_rows = 0;   // packed: rows per work item (0: heuristic)
     // packed and tensor variants: the grid lives in packed frames between steps
     PackedFrame pa{}, pb{};
-    uint32_t* pwords = nullptr;
     size_t pwords_bytes = 0;
     bool runs = false;          // packed, small grid: many generations per launch
     PackedRun run{};            // barrier and error word of those launches
@@ -80,6 +83,7 @@ struct ltl_ctx {
 };
 
 static constexpr int kGraphPasses = 8;
+static constexpr int kAutoPackedRadius = 28;
 static constexpr int kRunSteps = 512;  // generations per launch of a small packed grid
 
 static Frame& cur_frame(ltl_ctx* c) { return c->cur_is_a ? c->fa : c->fb; }
@@ -111,10 +115,8 @@ static void release(ltl_ctx* c) {
         if (g) cudaGraphExecDestroy(g);
     if (c->tplan) tensor_plan_destroy(c->tplan);
     if (c->frames) cudaFree(c->frames);
-    if (c->pwords) cudaFree(c->pwords);
     if (c->pstage) cudaFree(c->pstage);
     if (c->bstage) cudaFree(c->bstage);
-    if (c->scratch) cudaFree(c->scratch);
     if (c->own_stream) cudaStreamDestroy(c->own_stream);
     delete c;
 }
@@ -151,6 +153,10 @@ static int create_impl(ltl_ctx** out, int device, int rows, int n, int radius, i
         ltl_set_error("ltl_create: n=%d too large", n);
         return LTL_EINVAL;
     }
+    // AUTO: bit-packed up to R = 28, ahead of the plain kernels there at every side
+    // (us per generation, plain / packed: 64^2 R = 1 20 / 0.5, 1024^2 R = 5 12.9 / 2.0,
+    // 16384^2 R = 5 87 / 44, R = 17 217 / 106, R = 28 232 / 167; R = 32 228 / 237)
+    const bool auto_packed = variant == LTL_VARIANT_AUTO && rows == n && radius <= kAutoPackedRadius;
     if (variant == LTL_VARIANT_AUTO) variant = LTL_VARIANT_PLAIN;
     if (variant != LTL_VARIANT_PLAIN && variant != LTL_VARIANT_TENSOR && variant != LTL_VARIANT_PACKED) {
         ltl_set_error("ltl_create: unknown variant %d", variant);
@@ -184,7 +190,7 @@ static int create_impl(ltl_ctx** out, int device, int rows, int n, int radius, i
     c->n = n;
     c->rows = rows;
     c->rule = Rule{radius, smin, smax, bmin, bmax};
-    c->variant = variant;
+    c->auto_packed = auto_packed;
     cudaError_t e = cudaSetDevice(device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) {
@@ -200,18 +206,31 @@ static int create_impl(ltl_ctx** out, int device, int rows, int n, int radius, i
     size_t frows = (size_t)rows + 2 * H + 1;  // +1 spare row: vector loads may run past the last frame row
     size_t one = round_up(frows * pitch, 4096);
     c->frames_bytes = 2 * one;
-    e = cudaMalloc(&c->frames, c->frames_bytes);
-    if (e == cudaSuccess) e = cudaMemsetAsync(c->frames, 0, c->frames_bytes, c->stream);
-    if (e == cudaSuccess) e = cudaMalloc(&c->scratch, 8 * sizeof(unsigned long long));
-    if (e == cudaSuccess) e = cudaMemsetAsync(c->scratch, 0, 8 * sizeof(unsigned long long), c->stream);
+    // packed and tensor: both steps wrap rows and words themselves; the packed step
+    // wants 16-byte aligned rows without a halo, the tensor step a halo word to exist
+    PackedFrame p{};
+    size_t pone = 0;
+    if (auto_packed || variant != LTL_VARIANT_PLAIN) {
+        p.n = n;
+        p.rows = rows;
+        p.nw = (n + 31) / 32;
+        p.HR = p.HW = variant == LTL_VARIANT_TENSOR ? 1 : 0;
+        p.wpitch = round_up((size_t)p.nw + (p.HW ? 2 * p.HW + 1 : 0), 4);
+        pone = round_up(((size_t)rows + 2 * p.HR) * p.wpitch * sizeof(uint32_t), 4096);
+        c->pwords_bytes = 2 * pone;
+    }
+    // one allocation (each costs a solver about 40 us): byte frames, packed frames, scratch
+    const size_t scratch_at = c->frames_bytes + c->pwords_bytes, bytes = scratch_at + 256;
+    e = cudaMalloc(&c->frames, bytes);
+    if (e == cudaSuccess) e = cudaMemsetAsync(c->frames, 0, bytes, c->stream);
     if (e == cudaSuccess) {
+        c->scratch = (unsigned long long*)(c->frames + scratch_at);
         // words 0..3: reductions; 4: barrier; 5: error word
         c->run.barrier = (GridBarrier*)(c->scratch + 4);
         c->run.err = (unsigned int*)(c->scratch + 5);
     }
     if (e != cudaSuccess) {
-        ltl_set_error("ltl_create: device allocation of %zu bytes failed: %s", c->frames_bytes,
-                      cudaGetErrorString(e));
+        ltl_set_error("ltl_create: device allocation of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
         release(c);
         return e == cudaErrorMemoryAllocation ? LTL_ENOMEM : LTL_ECUDA;
     }
@@ -219,15 +238,21 @@ static int create_impl(ltl_ctx** out, int device, int rows, int n, int radius, i
     c->fb = Frame{c->frames + one, n, H, pitch, rows};
 
     if (variant == LTL_VARIANT_PLAIN && plain_swar8_supported(radius)) {
-        // generations per pass: the tuning table's value, else 2 where the
-        // temporally blocked kernel applies (grids below 256 gain nothing)
-        const int want = (int)tuning_lookup("plain", radius, n, "depth", n >= 256 ? 2 : 1);
+        // generations per pass: the tuning table's value, else the built-in choice
+        const int want = (int)tuning_lookup("plain", radius, n, "depth", plain_swar8_depth(radius));
         if (want > 1 && plain_tb_supported(radius, want) && H >= want * radius) depth = want;
-        c->band_rows = (int)tuning_lookup("plain", radius, n, "band_rows", plain_swar8_band_rows(n, device));
+        c->band_rows = (int)tuning_lookup("plain", radius, n, "band_rows", 0);
+        if (c->band_rows <= 0) c->band_rows = plain_swar8_band_rows(rows, n, radius, depth, device);
         c->plain_wrap = plain_wrap_supported(n, rows);
     } else if (variant == LTL_VARIANT_PLAIN) {
         c->band_rows = (int)tuning_lookup("plain", radius, n, "band_rows", 0);  // 0: the launcher's choice
     }
+    if (auto_packed) {
+        c->plain_depth = depth;
+        depth = 1;
+        variant = LTL_VARIANT_PACKED;
+    }
+    c->variant = variant;
     if (variant == LTL_VARIANT_PACKED) c->packed_band_rows = (int)tuning_lookup("packed", radius, n, "band_rows", 0);
     if (variant == LTL_VARIANT_PLAIN) e = plain_prepare(radius);
     if (variant == LTL_VARIANT_PLAIN && e == cudaSuccess) e = plain_tb_prepare(radius);
@@ -237,29 +262,9 @@ static int create_impl(ltl_ctx** out, int device, int rows, int n, int radius, i
         return LTL_ECUDA;
     }
     if (variant == LTL_VARIANT_PACKED || variant == LTL_VARIANT_TENSOR) {
-        // both steps wrap rows and words themselves; the packed step wants 16-byte
-        // aligned rows without a halo, the tensor step a halo word to exist
-        PackedFrame p{};
-        p.n = n;
-        p.rows = rows;
-        p.nw = (n + 31) / 32;
-        p.HR = variant == LTL_VARIANT_PACKED ? 0 : 1;
-        p.HW = variant == LTL_VARIANT_PACKED ? 0 : 1;
-        p.wpitch = round_up((size_t)p.nw + (p.HW ? 2 * p.HW + 1 : 0), 4);
-        size_t prow = (size_t)rows + 2 * p.HR;
-        size_t pone = round_up(prow * p.wpitch * sizeof(uint32_t), 4096);
-        c->pwords_bytes = 2 * pone;
-        e = cudaMalloc(&c->pwords, c->pwords_bytes);
-        if (e == cudaSuccess) e = cudaMemsetAsync(c->pwords, 0, c->pwords_bytes, c->stream);
-        if (e != cudaSuccess) {
-            ltl_set_error("ltl_create: packed allocation failed: %s", cudaGetErrorString(e));
-            release(c);
-            return LTL_ENOMEM;
-        }
-        c->pa = p;
-        c->pa.words = c->pwords;
-        c->pb = p;
-        c->pb.words = (uint32_t*)((uint8_t*)c->pwords + pone);
+        c->pa = c->pb = p;
+        c->pa.words = (uint32_t*)(c->frames + c->frames_bytes);
+        c->pb.words = (uint32_t*)(c->frames + c->frames_bytes + pone);
         c->runs = variant == LTL_VARIANT_PACKED && packed_runs(p, radius);
         if (variant == LTL_VARIANT_PACKED && (e = packed_prepare(p, radius)) != cudaSuccess) {
             ltl_set_error("ltl_create: kernel setup failed: %s", cudaGetErrorString(e));
@@ -326,7 +331,7 @@ extern "C" int ltl_get_info(const ltl_ctx* c, ltl_info* info) {
         ltl_set_error("ltl_get_info: info is NULL");
         return LTL_EINVAL;
     }
-    info->variant = c->variant;
+    info->variant = c->auto_packed ? LTL_VARIANT_PLAIN : c->variant;
     info->n = c->n;
     info->rows = c->rows;
     info->radius = c->rule.radius;
@@ -336,7 +341,7 @@ extern "C" int ltl_get_info(const ltl_ctx* c, ltl_info* info) {
     info->bmax = c->rule.bmax;
     info->halo = c->fa.H;
     info->pitch = (long long)c->fa.pitch;
-    info->temporal_depth = c->depth;
+    info->temporal_depth = c->auto_packed ? c->plain_depth : c->depth;
     info->operand_bits = c->tplan ? tensor_plan_operand_bits(c->tplan) : 0;
     info->device_bytes = (long long)(c->frames_bytes + c->pwords_bytes);
     return LTL_OK;
@@ -552,7 +557,7 @@ extern "C" int ltl_upload_rows_device(ltl_ctx* c, int row0, int nrows, const uin
     LTL_CUDA(cudaSetDevice(c->device));
     if (keeps_packed(c)) {
         // straight into the packed frame
-        LTL_CUDA(launch_pack_rows(dev, pitch, false, cur_packed(c), row0, nrows, c->stream));
+        LTL_CUDA(launch_pack_rows(dev, pitch, c->auto_packed, cur_packed(c), row0, nrows, c->stream));
         return after_upload(c);
     }
     Frame& f = cur_frame(c);
@@ -785,8 +790,9 @@ extern "C" int ltl_set_param(ltl_ctx* c, const char* name, long long value) {
             ltl_set_error("ltl_set_param: band_rows must be 0 (built-in choice) or in [16, 4096]");
             return LTL_EINVAL;
         }
+        if (c->auto_packed) return LTL_OK;  // a shape of the plain kernels, which do not run
         if (c->variant == LTL_VARIANT_PLAIN && plain_swar8_supported(c->rule.radius))
-            c->band_rows = value ? (int)value : plain_swar8_band_rows(c->n, c->device);
+            c->band_rows = value ? (int)value : plain_swar8_band_rows(c->rows, c->n, c->rule.radius, c->depth, c->device);
         else if (c->variant == LTL_VARIANT_PLAIN) c->band_rows = (int)value;
         else if (c->variant == LTL_VARIANT_PACKED) c->packed_band_rows = (int)value;
         else {
@@ -797,7 +803,7 @@ extern "C" int ltl_set_param(ltl_ctx* c, const char* name, long long value) {
         return LTL_OK;
     }
     if (std::strcmp(name, "depth") == 0) {
-        if (c->variant != LTL_VARIANT_PLAIN) {
+        if (c->variant != LTL_VARIANT_PLAIN && !c->auto_packed) {
             ltl_set_error("ltl_set_param: depth applies to the plain variant");
             return LTL_EUNSUPPORTED;
         }
@@ -806,7 +812,7 @@ extern "C" int ltl_set_param(ltl_ctx* c, const char* name, long long value) {
                           value, c->rule.radius);
             return LTL_EINVAL;
         }
-        c->depth = (int)value;
+        (c->auto_packed ? c->plain_depth : c->depth) = (int)value;
         drop_graphs(c);
         return LTL_OK;
     }

@@ -22,7 +22,9 @@ cudaError_t plain_prepare(int radius);
 bool plain_wrap_supported(int n, int rows);
 cudaError_t launch_plain_swar8(const Frame& cur, const Frame& nxt, const Rule& rule, int band_rows, bool wrap,
                                cudaStream_t s);
-int plain_swar8_band_rows(int n, int device);
+// Built-in shape: generations per pass, and rows per work item at that depth.
+int plain_swar8_depth(int radius);
+int plain_swar8_band_rows(int rows, int n, int radius, int depth, int device);
 // Temporally blocked SWAR step: `depth` (2 or 3, depth * R <= 16) generations per
 // pass; the frames' halo must be at least depth * R.
 bool plain_tb_supported(int radius, int depth);

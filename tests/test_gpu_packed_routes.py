@@ -69,3 +69,29 @@ def test_captured_steps_replay(n, radius):
         torch.cuda.synchronize()
         assert np.array_equal(s.getCurrentState(), O.run(g, radius, rule, 8))
         del graph
+
+
+@pytest.mark.parametrize("n,radius", [(64, 1), (100, 5), (1000, 12), (300, 28), (300, 29)])
+def test_auto_names_plain_and_takes_its_parameters(n, radius):
+    """The default solver: same info, parameters and results on either side of the
+    radius where it changes kernels."""
+    import cat_cpu_b200 as C
+    rule = rule_of(radius)
+    g = (np.random.default_rng(n + radius).random((n, n)) < 0.45).astype(np.uint8)
+    with C.CUDASolver(n, radius, rule) as s, C.CUDASolver(n, radius, rule, variant=C.VARIANT_PLAIN) as p:
+        for field in ("variant", "halo", "pitch", "temporal_depth", "operand_bits", "radius", "n", "rows"):
+            assert getattr(s.info, field) == getattr(p.info, field), field
+        for solver in (s, p):
+            solver.set_param("band_rows", 32)
+            if radius <= 5:
+                solver.set_param("depth", 2)
+                assert solver.info.temporal_depth == 2
+            else:
+                with pytest.raises(C.LtlError):
+                    solver.set_param("depth", 2)
+            with pytest.raises(C.LtlError):
+                solver.set_param("wait_limit_ns", 10**9)
+            solver.setState(g)
+            solver.doSteps(5)
+            assert np.array_equal(solver.getCurrentState(), O.run(g, radius, rule, 5))
+            assert solver.population() == int(O.run(g, radius, rule, 5).sum())
