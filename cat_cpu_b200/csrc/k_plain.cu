@@ -20,46 +20,63 @@ namespace ltl {
 // Top/bottom bands copy 16-byte chunks whose columns are inner (same column in
 // the source row); everything else goes byte by byte.
 // ---------------------------------------------------------------------------
-__global__ void k_halo_rows(uint8_t* __restrict__ g, int n, int rows, int H, size_t pitch) {
-    const int band = blockIdx.y;                       // 0 .. 2H-1
-    const int r = band < H ? band : rows + band;       // frame row
-    const int src_r = H + wrap_mod(r - H, rows);
-    const int W = n + 2 * H;
-    const int nchunks = (W + 15) / 16;
-    uint8_t* dst_row = g + (size_t)r * pitch;
-    const uint8_t* src_row = g + (size_t)src_r * pitch;
-    for (int ch = blockIdx.x * blockDim.x + threadIdx.x; ch < nchunks; ch += gridDim.x * blockDim.x) {
-        int c0 = ch * 16;
-        if (c0 >= H && c0 + 16 <= H + n) {
-            *(uint4*)(dst_row + c0) = *(const uint4*)(src_row + c0);
+// One launch: the first 2H row_blocks blocks copy halo rows, the others fill the
+// column halos of the inner rows.  (As two launches a step of a small grid spent a
+// quarter of its time here: 512^2, R = 20, bands of 16 rows, 13.9 us a generation with
+// two, 12.3 with one.)
+constexpr int kHaloThreads = 128;
+
+__global__ void __launch_bounds__(kHaloThreads)
+k_halo(uint8_t* __restrict__ g, int n, int rows, int H, size_t pitch, int row_blocks) {
+    const int top = 2 * H * row_blocks;
+    if ((int)blockIdx.x < top) {
+        const int band = blockIdx.x / row_blocks;          // 0 .. 2H-1
+        const int r = band < H ? band : rows + band;       // frame row
+        const int src_r = H + wrap_mod(r - H, rows);
+        const int W = n + 2 * H;
+        const int nchunks = (W + 15) / 16;
+        uint8_t* dst_row = g + (size_t)r * pitch;
+        const uint8_t* src_row = g + (size_t)src_r * pitch;
+        for (int ch = (blockIdx.x - band * row_blocks) * kHaloThreads + threadIdx.x; ch < nchunks;
+             ch += row_blocks * kHaloThreads) {
+            int c0 = ch * 16;
+            if (c0 >= H && c0 + 16 <= H + n) {
+                *(uint4*)(dst_row + c0) = *(const uint4*)(src_row + c0);
+            } else {
+                for (int c = c0; c < c0 + 16 && c < W; ++c) dst_row[c] = src_row[H + wrap_mod(c - H, n)];
+            }
+        }
+        return;
+    }
+    // inner rows, four halo cells per thread; H is a multiple of 16, so the left
+    // halo's groups are aligned words
+    const int per_row = 2 * H / 4;
+    const long long total = (long long)rows * per_row;
+    const long long stride = (long long)(gridDim.x - top) * kHaloThreads;
+    for (long long t = (long long)(blockIdx.x - top) * kHaloThreads + threadIdx.x; t < total; t += stride) {
+        const int i = (int)(t / per_row);
+        const int k = 4 * (int)(t - (long long)i * per_row);
+        const int c = k < H ? k : n + k;  // frame column
+        uint8_t* row = g + (size_t)(H + i) * pitch;
+        uint32_t v = 0u;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v |= (uint32_t)row[H + wrap_mod(c + e - H, n)] << (8 * e);
+        if ((c & 3) == 0) {
+            *(uint32_t*)(row + c) = v;
         } else {
-            for (int c = c0; c < c0 + 16 && c < W; ++c) dst_row[c] = src_row[H + wrap_mod(c - H, n)];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) row[c + e] = (uint8_t)(v >> (8 * e));
         }
     }
 }
 
-__global__ void k_halo_cols(uint8_t* __restrict__ g, int n, int rows, int H, size_t pitch) {
-    // inner rows only; 2H halo bytes per row
-    const int per_row = 2 * H;
-    const long long total = (long long)rows * per_row;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-         t += (long long)gridDim.x * blockDim.x) {
-        int i = (int)(t / per_row);
-        int k = (int)(t % per_row);
-        int c = k < H ? k : n + k;  // frame column
-        uint8_t* row = g + (size_t)(H + i) * pitch;
-        row[c] = row[H + wrap_mod(c - H, n)];
-    }
-}
-
 cudaError_t launch_halo_fill(const Frame& f, cudaStream_t s) {
-    const int W = f.n + 2 * f.H;
-    const int nchunks = (W + 15) / 16;
-    dim3 g1((unsigned)std::min((nchunks + 127) / 128, 64), (unsigned)(2 * f.H));
-    k_halo_rows<<<g1, 128, 0, s>>>(f.base, f.n, f.nrows(), f.H, f.pitch);
-    long long total = (long long)f.nrows() * 2 * f.H;
-    int blocks = (int)std::min<long long>((total + 255) / 256, 4096);
-    k_halo_cols<<<blocks, 256, 0, s>>>(f.base, f.n, f.nrows(), f.H, f.pitch);
+    const int nchunks = (f.n + 2 * f.H + 15) / 16;
+    const int row_blocks = std::min((nchunks + kHaloThreads - 1) / kHaloThreads, 64);
+    const long long total = (long long)f.nrows() * 2 * f.H / 4;
+    const long long col_blocks = std::min<long long>((total + kHaloThreads - 1) / kHaloThreads, 4096);
+    k_halo<<<(unsigned)(2 * f.H * row_blocks + col_blocks), kHaloThreads, 0, s>>>(f.base, f.n, f.nrows(), f.H, f.pitch,
+                                                                              row_blocks);
     return cudaGetLastError();
 }
 
@@ -980,6 +997,31 @@ static cudaError_t launch_wide_rm(const Frame& cur, const Frame& nxt, const Rule
     return cudaGetLastError();
 }
 
+// Rows per band: the least of a model of one launch.  A CTA takes 0.11 us of an SM per
+// row (1.5 + 0.06 R rows more to start its window), and 0.26 us per row by itself; an SM holds
+// `resident` CTAs, and those past the last full load of all SMs end nearly alone.  So
+// large grids want long bands, and small ones enough CTAs.  Measured (us per generation,
+// bands of 16 / 32 / 48 / 64 rows): 512^2 R = 40 13.6 / 17.9 / 22.0 / 26.4; 4096^2 R = 12
+// 24.1 / 26.9 / 28.6 / 34.3; 6001^2 R = 64 52.4 / 47.3 / 45.3 / 48.6; 16384^2 R = 64 285
+// / 246 / 236 / 244.
+static int wide_band_rows(int rows, int tiles, int R, int resident) {
+    const int sms = 148;
+    double best = 0;
+    int best_rows = 64;
+    for (int b = 8; b <= 64; b += 4) {
+        const long long ctas = (long long)tiles * ((rows + b - 1) / b);
+        const double alone = 0.26 * b + 1.0, shared = 0.11 * (b + 1.5 + 0.06 * R);
+        const long long per_sm = (ctas + sms - 1) / sms;
+        const double t = per_sm <= resident ? std::max(per_sm * shared, alone)
+                                            : (double)ctas / sms * shared + 0.8 * alone;
+        if (best == 0 || t < best) {
+            best = t;
+            best_rows = b;
+        }
+    }
+    return best_rows;
+}
+
 cudaError_t launch_plain_generic(const Frame& cur, const Frame& nxt, const Rule& rule, int band_rows,
                                  cudaStream_t s) {
     const int n = cur.n, rows = cur.nrows(), R = rule.radius;
@@ -993,11 +1035,7 @@ cudaError_t launch_plain_generic(const Frame& cur, const Frame& nxt, const Rule&
     const int nt = wide_threads(R);
     const int T = (nt * cpt - 2 * R - cpt + 1) & ~3;
     const int tiles = (n + T - 1) / T;
-    // bands of 64 rows unless set: many CTAs per SM over the launch, so that
-    // their 2R+1-row starts (independent loads) overlap other CTAs' scans
-    // (measured on 16384^2 and 32768^2 for R = 6..200: within a few percent of
-    // the best height everywhere)
-    int band = band_rows > 0 ? band_rows : 64;
+    int band = band_rows > 0 ? band_rows : wide_band_rows(rows, tiles, R, nt == 128 ? 9 : (cpt == 8 ? 4 : 3));
     band = std::max(band, (rows + 65534) / 65535);  // grid y limit
     band = std::min(band + (band & 1), std::max(rows + (rows & 1), 2));  // even: row pairs never straddle bands
     const dim3 grid(tiles, (rows + band - 1) / band);

@@ -581,7 +581,7 @@ static cudaError_t enqueue_pass(ltl_ctx* c, int gens) {
         if (e == cudaSuccess) e = cudaEventRecord(e0, c->stream);
         if (e != cudaSuccess) return e;
     }
-    int step_kernels = 0, halo_kernels = 2;
+    int step_kernels = 0, halo_kernels = 1;
     switch (c->variant) {
         case LTL_VARIANT_PLAIN: {
             Frame& a = cur_frame(c);
