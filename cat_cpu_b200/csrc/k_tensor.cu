@@ -280,11 +280,19 @@ struct Cursor {
 // applies the rule to unit u - 1, the tensor core has the next unit's product 1
 // queued while the epilogue finishes the previous one.
 //
-// MODE: rule lanes and product-2 operand type (TcMode); FAST: n % 32 == 0 and
-// large enough that rows and words wrap with one correction; NG: product-1 K
+// How the X tiles are filled: kGather cell by cell (small sides); kFast (FAST below):
+// from words staged through shared memory, where n is large enough that rows and
+// words wrap with one correction; kFastSeam: the same with the tiles at the row's end
+// gathered, where 32 does not divide n.  (An instantiation of its own: with the test
+// and the gather in kFast's loop a 16384^2 step at R = 5 took 126.8 us, not 115.8.
+// Ragged sides before this form, all gathered: 13517^2 R = 9 180 us, now 105.)
+enum TcForm { kGather = 0, kFast = 1, kFastSeam = 2 };
+
+// MODE: rule lanes and product-2 operand type (TcMode); NG: product-1 K
 // steps = X groups of 32 columns per row.
-template <int MODE, bool FAST, int NG, bool XT>
+template <int MODE, int FORM, int NG, bool XT>
 __global__ void __launch_bounds__(kThreads, 1) k_tensor_step(const __grid_constant__ TcParams p) {
+    constexpr bool FAST = FORM != kGather;
     static_assert(!XT || (FAST && NG <= 5), "X in tensor memory: FAST tiles with at most 5 K steps");
     constexpr int kHBufs = XT ? 1 : 2;  // H buffers in TMEM (C has two either way)
     constexpr int kCBufs = 2;
@@ -541,6 +549,19 @@ __global__ void __launch_bounds__(kThreads, 1) k_tensor_step(const __grid_consta
         Cursor c;  // the unit being stored
         c.init(wk);
         bool ok = true;
+        // the NG groups of X row `row` of unit cc, rows and columns taken modulo n
+        uint32_t wg[NG];
+        auto gather = [&](const Cursor& cc) {
+            const int gr0 = cc.ty * p.Tr - R + 128 * cc.b + row;
+            const uint32_t* rp = p.src + (size_t)wrap_slow(gr0, p.n) * (size_t)p.wpitch;
+            int a = wrap_slow(cc.tx * kTc - p.PADC, p.n);
+#pragma unroll
+            for (int k = 0; k < NG; ++k) {
+                wg[k] = fetch32(rp, a, p.n);
+                a += 32;
+                while (a >= p.n) a -= p.n;
+            }
+        };
         // spreads X row `row` of unit c to the stage: group g from x_of(g)
         auto store = [&](const Cursor& cc, auto x_of) -> bool {
             if (cc.u >= S) {
@@ -604,26 +625,22 @@ __global__ void __launch_bounds__(kThreads, 1) k_tensor_step(const __grid_consta
                 }
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&bars[W_EMPTY + slot]);
-                ok = store(c, [&](int g) { return prmt(w[g], w[g + 1], 0x5432u); });
+                // where the row's end is inside a word, the tiles that reach over the seam
+                // are gathered cell by cell instead (the first and the last one or two of
+                // a row of tiles); all others read whole words as ever
+                const int x0 = c.tx * kTc - p.PADC;
+                if (FORM == kFastSeam && (x0 < 0 || x0 + 32 * NG > p.n)) {
+                    gather(c);
+                    ok = store(c, [&](int g) { return wg[g]; });
+                } else {
+                    ok = store(c, [&](int g) { return prmt(w[g], w[g + 1], 0x5432u); });
+                }
                 if (!ok) break;
             }
         } else {
-            uint32_t w[NG];
-            // the NG groups of X row `row` of unit cc, rows and columns taken modulo n
-            auto gather = [&](const Cursor& cc) {
-                const int gr0 = cc.ty * p.Tr - R + 128 * cc.b + row;
-                const uint32_t* rp = p.src + (size_t)wrap_slow(gr0, p.n) * (size_t)p.wpitch;
-                int a = wrap_slow(cc.tx * kTc - p.PADC, p.n);
-#pragma unroll
-                for (int k = 0; k < NG; ++k) {
-                    w[k] = fetch32(rp, a, p.n);
-                    a += 32;
-                    while (a >= p.n) a -= p.n;
-                }
-            };
             for (; c.u < units; c.next(wk)) {
                 gather(c);
-                ok = store(c, [&](int g) { return w[g]; });
+                ok = store(c, [&](int g) { return wg[g]; });
                 if (!ok) break;
             }
         }
@@ -832,31 +849,38 @@ struct TensorPlan {
 //   R 113..127   32-bit lanes, 13 K steps
 //   R 128        32-bit lanes on f32 counts, f16 product 2, 13 K steps
 template <int MODE, int NG>
-static TcKernel pick_fast(bool fast) {
-    return fast ? k_tensor_step<MODE, true, NG, false> : k_tensor_step<MODE, false, NG, false>;
+static TcKernel pick_form(int form) {
+    switch (form) {
+        case kFast: return k_tensor_step<MODE, kFast, NG, false>;
+        case kFastSeam: return k_tensor_step<MODE, kFastSeam, NG, false>;
+        default: return k_tensor_step<MODE, kGather, NG, false>;
+    }
 }
 // X in tensor memory: FAST tiles of 8- and 16-bit rule lanes with 5 K steps (R <= 16)
 static bool tensor_xt(int mode, bool fast, int ng) { return fast && ng == 5 && mode <= kLanes16; }
-static TcKernel pick_kernel(int mode, bool fast, int ng) {
-    if (tensor_xt(mode, fast, ng))
-        return mode == kLanes8 ? k_tensor_step<kLanes8, true, 5, true> : k_tensor_step<kLanes16, true, 5, true>;
+template <int MODE>
+static TcKernel pick_xt(int form) {
+    return form == kFast ? k_tensor_step<MODE, kFast, 5, true> : k_tensor_step<MODE, kFastSeam, 5, true>;
+}
+static TcKernel pick_kernel(int mode, int form, int ng) {
+    if (tensor_xt(mode, form != kGather, ng)) return mode == kLanes8 ? pick_xt<kLanes8>(form) : pick_xt<kLanes16>(form);
     switch (mode) {
-        case kLanes8: return ng == 5 ? pick_fast<kLanes8, 5>(fast) : nullptr;
+        case kLanes8: return ng == 5 ? pick_form<kLanes8, 5>(form) : nullptr;
         case kLanes16:
             switch (ng) {
-                case 5: return pick_fast<kLanes16, 5>(fast);
-                case 7: return pick_fast<kLanes16, 7>(fast);
-                case 9: return pick_fast<kLanes16, 9>(fast);
-                case 11: return pick_fast<kLanes16, 11>(fast);
+                case 5: return pick_form<kLanes16, 5>(form);
+                case 7: return pick_form<kLanes16, 7>(form);
+                case 9: return pick_form<kLanes16, 9>(form);
+                case 11: return pick_form<kLanes16, 11>(form);
                 default: return nullptr;
             }
         case kLanes32:
             switch (ng) {
-                case 11: return pick_fast<kLanes32, 11>(fast);
-                case 13: return pick_fast<kLanes32, 13>(fast);
+                case 11: return pick_form<kLanes32, 11>(form);
+                case 13: return pick_form<kLanes32, 13>(form);
                 default: return nullptr;
             }
-        case kF16: return ng == 13 ? pick_fast<kF16, 13>(fast) : nullptr;
+        case kF16: return ng == 13 ? pick_form<kF16, 13>(form) : nullptr;
         default: return nullptr;
     }
 }
@@ -985,7 +1009,7 @@ TensorPlan* tensor_plan_create(const PackedFrame& a, const PackedFrame& b, const
     // one correction wraps a row (rows span [-R, n + 128 nb)) and a word index
     // (words span [-4, nw + ng)); groups are word halves
     const int nb_of_r = R <= 32 ? 1 : (128 + 2 * R + 127) / 128;
-    const bool fast_ok = a.n % 32 == 0 && nw >= 4 && a.n >= 128 * nb_of_r + R;
+    const bool fast_ok = nw >= 4 && a.n >= 128 * nb_of_r + R;
     TensorGeometry G{};
     if (!tensor_geometry(R, fast_ok, G)) {
         snprintf(why, why_len, "no tile shape for R=%d", R);
@@ -1044,7 +1068,7 @@ TensorPlan* tensor_plan_create(const PackedFrame& a, const PackedFrame& b, const
         q.wait_ns = kWaitLimitNs;
         q.inject_missing_commit = 0;
     }
-    P->kernel = pick_kernel(G.mode, fast, G.ng);
+    P->kernel = pick_kernel(G.mode, !fast ? kGather : (a.n % 32 == 0 ? kFast : kFastSeam), G.ng);
     if (!P->kernel) {
         snprintf(why, why_len, "no kernel instantiation for R=%d", R);
         cudaFree(P->err);
