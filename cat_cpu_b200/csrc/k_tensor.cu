@@ -62,6 +62,7 @@
 #include <cstdio>
 #include <cstring>
 
+#include "grid_barrier.cuh"
 #include "ltl_kernels.h"
 #include "tc_ptx.cuh"
 
@@ -112,8 +113,10 @@ __host__ __device__ constexpr uint32_t c_col_xt(int buf) { return 128u + 128u * 
 __host__ __device__ constexpr uint32_t x_col(int stage, int ng) { return 384u + 8u * (uint32_t)(ng * stage); }
 
 struct TcParams {
-    const uint32_t* src;  // inner word (0, 0) of the current packed frame
+    uint32_t* src;        // inner word (0, 0) of the current packed frame
     uint32_t* dst;        // inner word (0, 0) of the next packed frame
+    int steps;            // generations; the frames change roles after each
+    GridBarrier* barrier; // counts the CTAs that have finished a generation
     long long wpitch;     // words per frame row
     int n, nw;
     int R, PADC;      // radius, column halo of a tile (16 mod 32)
@@ -143,7 +146,8 @@ enum Bar {
     DRAIN = C_EMPTY + 2,      // [2] per MMA-issuing warp
     W_FULL = DRAIN + 2,       // [kWordDepth] packed-word ring slots
     W_EMPTY = W_FULL + kWordDepth,
-    NBARS = W_EMPTY + kWordDepth
+    GEN_DONE = W_EMPTY + kWordDepth,  // every rule warp has stored its part of a generation
+    NBARS
 };
 
 // Rule lanes and product-2 operand type (the template parameter MODE):
@@ -206,18 +210,26 @@ __device__ __forceinline__ int wrap_slow(int v, int n) {
     return r < 0 ? r + n : r;
 }
 
+// A word of the grid: read-only where the launch runs one generation.
+template <bool RUN>
+__device__ __forceinline__ uint32_t ld_grid(const uint32_t* p) {
+    if constexpr (RUN) return *p;
+    else return __ldg(p);
+}
+
 // Cells a .. a+31 (modulo n) of one packed row, bit b = cell a+b; 0 <= a < n.
 // Bits past n in the row's last word are ignored.
-__device__ __forceinline__ uint32_t fetch32(const uint32_t* __restrict__ row, int a, int n) {
+template <bool RUN>
+__device__ __forceinline__ uint32_t fetch32(const uint32_t* row, int a, int n) {
     if (n >= 32) {
         const int w0 = a >> 5, s = a & 31;
         // row[w0 + 1] may be the right halo word (w0 = nw - 1): its bits are masked below
-        uint32_t v = __funnelshift_r(__ldg(row + w0), __ldg(row + w0 + 1), s);
+        uint32_t v = __funnelshift_r(ld_grid<RUN>(row + w0), ld_grid<RUN>(row + w0 + 1), s);
         const int valid = n - a;
-        if (valid < 32) v = (v & ((1u << valid) - 1u)) | (__ldg(row) << valid);
+        if (valid < 32) v = (v & ((1u << valid) - 1u)) | (ld_grid<RUN>(row) << valid);
         return v;
     }
-    const uint32_t w = __ldg(row);
+    const uint32_t w = ld_grid<RUN>(row);
     uint32_t v = 0u;
     int c = a;
     for (int b = 0; b < 32; ++b) {
@@ -228,29 +240,39 @@ __device__ __forceinline__ uint32_t fetch32(const uint32_t* __restrict__ row, in
 }
 
 // Position in this CTA's stream of work, advanced incrementally (no integer
-// division in the loops).  Tiles t = blockIdx.x + j * gridDim.x, units (X
-// blocks) u = j * nb + b.  The strides live in a Walk shared by the cursors
-// of a thread.
+// division in the loops).  A generation's tiles are t = blockIdx.x + k * gridDim.x,
+// k < mine; over all generations tiles j and units (X blocks) u = j * nb + b are
+// numbered through, so the rings and buffers run on from one generation to the
+// next.  The strides live in a Walk shared by the cursors of a thread.
 struct Walk {
-    int step_x, step_y, tiles_x, nb, stages;
+    int step_x, step_y, tiles_x, nb, stages, mine, tx0, ty0;
     __device__ explicit Walk(const TcParams& p) {
         tiles_x = p.tiles_x;
         nb = p.nb;
         stages = p.stages;
         step_y = (int)gridDim.x / tiles_x;
         step_x = (int)gridDim.x - step_y * tiles_x;
+        mine = my_tiles(p);
+        ty0 = (int)blockIdx.x / tiles_x;
+        tx0 = (int)blockIdx.x - ty0 * tiles_x;
+    }
+    static __device__ int my_tiles(const TcParams& p) {
+        const int ntiles = p.tiles_x * p.tiles_y;
+        return ntiles > (int)blockIdx.x ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
     }
 };
 
+template <bool RUN>
 struct Cursor {
     int u, b, j;  // unit, row block within the tile, tile count
     int st, sph;  // X ring stage of unit u and its phase parity ((u / stages) & 1)
+    int g, k;     // RUN: generation, tile within it
     int ty, tx;   // tile coordinates
 
     __device__ void init(const Walk& w) {
-        u = b = j = st = sph = 0;
-        ty = (int)blockIdx.x / w.tiles_x;
-        tx = (int)blockIdx.x - ty * w.tiles_x;
+        u = b = j = st = sph = g = k = 0;
+        ty = w.ty0;
+        tx = w.tx0;
     }
     __device__ void next(const Walk& w) {
         ++u;
@@ -261,6 +283,13 @@ struct Cursor {
         if (++b == w.nb) {
             b = 0;
             ++j;
+            if (RUN && ++k == w.mine) {
+                k = 0;
+                ++g;
+                tx = w.tx0;
+                ty = w.ty0;
+                return;
+            }
             tx += w.step_x;
             ty += w.step_y;
             if (tx >= w.tiles_x) {
@@ -288,9 +317,54 @@ struct Cursor {
 // Ragged sides before this form, all gathered: 13517^2 R = 9 180 us, now 105.)
 enum TcForm { kGather = 0, kFast = 1, kFastSeam = 2 };
 
+// Generations.  A launch runs p.steps of them; the prologue (operand matrices, TMEM,
+// barriers) and the launch itself are paid once.  Only the warps that read the grid
+// first (the loaders, or the unpack warps in kGather) wait between generations, for
+// every CTA's rule warps to have stored the one before: each CTA adds one to a device
+// counter (release) and they poll it (acquire, bounded).  All others run on, and see
+// the new grid through the barriers of the rings; the launch is cooperative.
+// Measured per generation, a launch each / as one launch: 512^2 R = 5 6.4 / 4.5 us,
+// 4096^2 R = 16 15.8 / 14.4; large grids keep single launches (tensor_plan_create).
+class GenWait {
+    GridBarrier* bar;
+    unsigned long long base;
+
+public:
+    // lane 0 of a reading warp, before it loads anything (its CTA cannot have arrived yet)
+    __device__ GenWait(const TcParams& p, int lane) : bar(p.barrier), base(0) {
+        if (lane == 0 && p.steps > 1) {
+            unsigned long long now;
+            asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(now) : "l"(&bar->arrived) : "memory");
+            base = now - now % gridDim.x;
+        }
+    }
+    // the whole warp: generation g may be read
+    __device__ bool wait(int g, int lane, uint64_t limit_ns) {
+        bool ok = true;
+        if (lane == 0) {
+            const unsigned long long target = base + (unsigned long long)g * gridDim.x;
+            const uint64_t t0 = globaltimer();
+            while (true) {
+                unsigned long long now;
+                asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(now) : "l"(&bar->arrived) : "memory");
+                if (now >= target) break;
+                if (globaltimer() - t0 > limit_ns) {
+                    ok = false;
+                    break;
+                }
+            }
+        }
+        return __shfl_sync(0xffffffffu, ok, 0);
+    }
+    static __device__ void arrive(const TcParams& p) {
+        asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(&p.barrier->arrived) : "memory");
+    }
+};
+
 // MODE: rule lanes and product-2 operand type (TcMode); NG: product-1 K
 // steps = X groups of 32 columns per row.
-template <int MODE, int FORM, int NG, bool XT>
+// RUN: many generations (p.steps), else one.
+template <int MODE, int FORM, int NG, bool XT, bool RUN>
 __global__ void __launch_bounds__(kThreads, 1) k_tensor_step(const __grid_constant__ TcParams p) {
     constexpr bool FAST = FORM != kGather;
     static_assert(!XT || (FAST && NG <= 5), "X in tensor memory: FAST tiles with at most 5 K steps");
@@ -314,9 +388,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_tensor_step(const __grid_consta
     constexpr int kXB = ATOMS * kAtomBytes;  // bytes of one X stage
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int ntiles = p.tiles_x * p.tiles_y;
-    const int mine = ntiles > (int)blockIdx.x ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
-    const int units = mine * nb;
+    const int tiles = RUN ? Walk::my_tiles(p) * p.steps : Walk::my_tiles(p);
+    const int units = tiles * nb;
     constexpr uint32_t kTmemCols = 512;
 
     if (tid == 0) {
@@ -337,6 +410,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tensor_step(const __grid_consta
             mbar_init(&bars[W_FULL + i], 32 * kLoadWarps);  // one cp.async-tracking arrival per loader thread
             mbar_init(&bars[W_EMPTY + i], kUnpackWarps);
         }
+        mbar_init(&bars[GEN_DONE], kRuleWarps);
         fence_mbar_init();
     }
     if (warp == 0) tmem_alloc(tmem_slot, kTmemCols);
@@ -403,7 +477,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tensor_step(const __grid_consta
             return __all_sync(0xffffffffu, mbar_wait(bar, ph, p.wait_ns, kSleepNs));
         };
         const Walk wk(p);
-        Cursor c;
+        Cursor<RUN> c;
         c.init(wk);
         bool ok = true;
         if (warp == 0) {
@@ -494,10 +568,19 @@ __global__ void __launch_bounds__(kThreads, 1) k_tensor_step(const __grid_consta
             uint32_t* ring = (uint32_t*)(smem + L.wr_off);  // [kWordDepth][128][RW]
             const int row_base = 64 * (warp - kLoadWarp0);
             const Walk wk(p);
-            Cursor c;
+            Cursor<RUN> c;
             c.init(wk);
             bool ok = true;
+            GenWait gens(p, RUN ? lane : 1);
+            int gen = 0;
+            const uint32_t* src = p.src;
             for (; c.u < units; c.next(wk)) {
+                if (RUN && c.g != gen) {
+                    gen = c.g;
+                    src = gen & 1 ? p.dst : p.src;
+                    ok = gens.wait(gen, lane, p.wait_ns);
+                    if (!ok) break;
+                }
                 const int slot = c.u & (kWordDepth - 1);
                 if (c.u >= kWordDepth) {
                     ok = __all_sync(0xffffffffu, mbar_wait(&bars[W_EMPTY + slot],
@@ -511,7 +594,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tensor_step(const __grid_consta
                 // whole 16-byte chunks: aligned start (rows are 16-byte aligned:
                 // wpitch % 4 == 0), no seam inside the needed words, the chunks'
                 // extra words still inside the frame row
-                const bool vec = ((uintptr_t)(p.src + wi0) & 15) == 0 && (p.wpitch & 3) == 0 &&
+                const bool vec = ((uintptr_t)(src + wi0) & 15) == 0 && (p.wpitch & 3) == 0 &&
                                  wi0 + NW1 <= p.nw && wi0 + RW <= p.wpitch - 1;
                 const int gr0 = c.ty * p.Tr - R + 128 * c.b;
 #pragma unroll
@@ -520,7 +603,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tensor_step(const __grid_consta
                     int gr = gr0 + row;
                     if (gr < 0) gr += p.n;
                     else if (gr >= p.n) gr -= p.n;
-                    const uint32_t* rp = p.src + (size_t)gr * (size_t)p.wpitch;
+                    const uint32_t* rp = src + (size_t)gr * (size_t)p.wpitch;
                     uint32_t* dr = d + row * RW;
                     if (vec) {
 #pragma unroll
@@ -546,24 +629,24 @@ __global__ void __launch_bounds__(kThreads, 1) k_tensor_step(const __grid_consta
         const int row = tid - 32 * kUnpackWarp0;
         const int sw = row & 7;
         const Walk wk(p);
-        Cursor c;  // the unit being stored
+        Cursor<RUN> c;  // the unit being stored
         c.init(wk);
         bool ok = true;
         // the NG groups of X row `row` of unit cc, rows and columns taken modulo n
         uint32_t wg[NG];
-        auto gather = [&](const Cursor& cc) {
+        auto gather = [&](const Cursor<RUN>& cc) {
             const int gr0 = cc.ty * p.Tr - R + 128 * cc.b + row;
-            const uint32_t* rp = p.src + (size_t)wrap_slow(gr0, p.n) * (size_t)p.wpitch;
+            const uint32_t* rp = (RUN && (cc.g & 1) ? p.dst : p.src) + (size_t)wrap_slow(gr0, p.n) * (size_t)p.wpitch;
             int a = wrap_slow(cc.tx * kTc - p.PADC, p.n);
 #pragma unroll
             for (int k = 0; k < NG; ++k) {
-                wg[k] = fetch32(rp, a, p.n);
+                wg[k] = fetch32<RUN>(rp, a, p.n);
                 a += 32;
                 while (a >= p.n) a -= p.n;
             }
         };
         // spreads X row `row` of unit c to the stage: group g from x_of(g)
-        auto store = [&](const Cursor& cc, auto x_of) -> bool {
+        auto store = [&](const Cursor<RUN>& cc, auto x_of) -> bool {
             if (cc.u >= S) {
                 bool wt = true;
                 if (lane == 0) wt = mbar_wait(&bars[X_EMPTY + cc.st], (uint32_t)(cc.sph ^ 1), p.wait_ns, kSleepNs);
@@ -638,7 +721,14 @@ __global__ void __launch_bounds__(kThreads, 1) k_tensor_step(const __grid_consta
                 if (!ok) break;
             }
         } else {
+            GenWait gens(p, RUN ? lane : 1);
+            int gen = 0;
             for (; c.u < units; c.next(wk)) {
+                if (RUN && c.g != gen) {
+                    gen = c.g;
+                    ok = gens.wait(gen, lane, p.wait_ns);
+                    if (!ok) break;
+                }
                 gather(c);
                 ok = store(c, [&](int g) { return wg[g]; });
                 if (!ok) break;
@@ -656,7 +746,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tensor_step(const __grid_consta
             return __all_sync(0xffffffffu, wt);
         };
         const Walk wk(p);
-        Cursor c;
+        Cursor<RUN> c;
         c.init(wk);
         bool ok = true;
         if (warp < kRuleWarp0) {
@@ -721,7 +811,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tensor_step(const __grid_consta
             const uint32_t lane_off = ((uint32_t)(q * 32) << 16) + (uint32_t)(kN1 * grp0);
             const uint32_t nlo0 = p.nlo0, dlo = p.dlo, hiH0 = p.hiH0, dhi = p.dhi;
             // output word e of this thread in the tile of cursor c (offset, or -1)
-            auto out_at = [&](const Cursor& cc, int e) -> long long {
+            auto out_at = [&](const Cursor<RUN>& cc, int e) -> long long {
                 const int gi = cc.ty * p.Tr + m;
                 const int wi = cc.tx * kChunks + grp0 + e;
                 if (m >= p.Tr || gi >= p.n || wi >= p.nw) return -1;
@@ -770,13 +860,24 @@ __global__ void __launch_bounds__(kThreads, 1) k_tensor_step(const __grid_consta
                 return acc;
             };
             // the centre words (the output words' own cells in the current grid) of
-            // the next tile are loaded while this one is processed
-            long long at0 = mine > 0 ? out_at(c, 0) : -1, at1 = mine > 0 ? out_at(c, 1) : -1;
-            uint32_t cw0 = at0 >= 0 ? __ldg(p.src + at0) : 0u, cw1 = at1 >= 0 ? __ldg(p.src + at1) : 0u;
-            for (int j = 0; j < mine && ok; ++j) {
+            // the next tile are loaded while this one is processed; those of a
+            // generation's first tile once its counts are there (the grid they come
+            // from is complete by then).  Plain loads: the grid changes under this launch.
+            const uint32_t* src = p.src;
+            uint32_t* dst = p.dst;
+            long long at0 = tiles > 0 ? out_at(c, 0) : -1, at1 = tiles > 0 ? out_at(c, 1) : -1;
+            uint32_t cw0 = 0u, cw1 = 0u;
+            auto load_centre = [&]() {
+                cw0 = at0 >= 0 ? ld_grid<RUN>(src + at0) : 0u;
+                cw1 = at1 >= 0 ? ld_grid<RUN>(src + at1) : 0u;
+            };
+            bool late = RUN;  // centre words not loaded yet
+            if (!late) load_centre();
+            for (int j = 0; j < tiles && ok; ++j) {
                 const int cb = j % kCBufs;
                 ok = wait_all(&bars[C_FULL + cb], (uint32_t)((j / kCBufs) & 1));
                 if (!ok) break;
+                if (RUN && late) load_centre();
                 fence_after();
                 uint32_t acc0, acc1;
                 if constexpr (MODE >= kLanes32) {
@@ -805,13 +906,28 @@ __global__ void __launch_bounds__(kThreads, 1) k_tensor_step(const __grid_consta
                     acc0 = rule16(va, cw0);
                     acc1 = rule16(vb, cw1);
                 }
-                if (at0 >= 0) p.dst[at0] = acc0;
-                if (at1 >= 0) p.dst[at1] = acc1;
+                if (at0 >= 0) dst[at0] = acc0;
+                if (at1 >= 0) dst[at1] = acc1;
+                const int gen = RUN ? c.g : 0;
                 for (int b = 0; b < nb; ++b) c.next(wk);
-                at0 = j + 1 < mine ? out_at(c, 0) : -1;
-                at1 = j + 1 < mine ? out_at(c, 1) : -1;
-                cw0 = at0 >= 0 ? __ldg(p.src + at0) : 0u;
-                cw1 = at1 >= 0 ? __ldg(p.src + at1) : 0u;
+                at0 = j + 1 < tiles ? out_at(c, 0) : -1;
+                at1 = j + 1 < tiles ? out_at(c, 1) : -1;
+                late = RUN && c.g != gen;
+                if (!late) {
+                    load_centre();
+                } else if (c.g < p.steps) {
+                    // this warp's part of the generation is stored; the first rule warp
+                    // reports the CTA's
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&bars[GEN_DONE]);
+                    if (warp == kRuleWarp0) {
+                        ok = wait_all(&bars[GEN_DONE], (uint32_t)(gen & 1));
+                        if (ok && lane == 0) GenWait::arrive(p);
+                    }
+                    uint32_t* t = const_cast<uint32_t*>(src);
+                    src = dst;
+                    dst = t;
+                }
             }
         }
         if (!ok && lane == 0) atomicOr(p.err, 8u);
@@ -832,11 +948,13 @@ using TcKernel = void (*)(TcParams);
 
 struct TensorPlan {
     TcParams prm[2];  // source frame a -> b, b -> a
-    TcKernel kernel;
+    TcKernel kernel, run;  // one generation, many
+    bool runs;             // small enough for many per launch
     int smem_bytes;
     int grid;
     int operand_bits;  // product-2 operand: 8 (u8) or 16 (f16)
     unsigned int* err;
+    GridBarrier* barrier;  // zero whenever no launch that failed has used it
 };
 
 // The instantiations that exist (R ranges as tensor_geometry lays them out):
@@ -848,39 +966,41 @@ struct TensorPlan {
 //   R 91..112    32-bit lanes, 11 K steps
 //   R 113..127   32-bit lanes, 13 K steps
 //   R 128        32-bit lanes on f32 counts, f16 product 2, 13 K steps
-template <int MODE, int NG>
+template <int MODE, int NG, bool RUN>
 static TcKernel pick_form(int form) {
     switch (form) {
-        case kFast: return k_tensor_step<MODE, kFast, NG, false>;
-        case kFastSeam: return k_tensor_step<MODE, kFastSeam, NG, false>;
-        default: return k_tensor_step<MODE, kGather, NG, false>;
+        case kFast: return k_tensor_step<MODE, kFast, NG, false, RUN>;
+        case kFastSeam: return k_tensor_step<MODE, kFastSeam, NG, false, RUN>;
+        default: return k_tensor_step<MODE, kGather, NG, false, RUN>;
     }
 }
 // X in tensor memory: FAST tiles of 8- and 16-bit rule lanes with 5 K steps (R <= 16)
 static bool tensor_xt(int mode, bool fast, int ng) { return fast && ng == 5 && mode <= kLanes16; }
-template <int MODE>
+template <int MODE, bool RUN>
 static TcKernel pick_xt(int form) {
-    return form == kFast ? k_tensor_step<MODE, kFast, 5, true> : k_tensor_step<MODE, kFastSeam, 5, true>;
+    return form == kFast ? k_tensor_step<MODE, kFast, 5, true, RUN> : k_tensor_step<MODE, kFastSeam, 5, true, RUN>;
 }
+template <bool RUN>
 static TcKernel pick_kernel(int mode, int form, int ng) {
-    if (tensor_xt(mode, form != kGather, ng)) return mode == kLanes8 ? pick_xt<kLanes8>(form) : pick_xt<kLanes16>(form);
+    if (tensor_xt(mode, form != kGather, ng))
+        return mode == kLanes8 ? pick_xt<kLanes8, RUN>(form) : pick_xt<kLanes16, RUN>(form);
     switch (mode) {
-        case kLanes8: return ng == 5 ? pick_form<kLanes8, 5>(form) : nullptr;
+        case kLanes8: return ng == 5 ? pick_form<kLanes8, 5, RUN>(form) : nullptr;
         case kLanes16:
             switch (ng) {
-                case 5: return pick_form<kLanes16, 5>(form);
-                case 7: return pick_form<kLanes16, 7>(form);
-                case 9: return pick_form<kLanes16, 9>(form);
-                case 11: return pick_form<kLanes16, 11>(form);
+                case 5: return pick_form<kLanes16, 5, RUN>(form);
+                case 7: return pick_form<kLanes16, 7, RUN>(form);
+                case 9: return pick_form<kLanes16, 9, RUN>(form);
+                case 11: return pick_form<kLanes16, 11, RUN>(form);
                 default: return nullptr;
             }
         case kLanes32:
             switch (ng) {
-                case 11: return pick_form<kLanes32, 11>(form);
-                case 13: return pick_form<kLanes32, 13>(form);
+                case 11: return pick_form<kLanes32, 11, RUN>(form);
+                case 13: return pick_form<kLanes32, 13, RUN>(form);
                 default: return nullptr;
             }
-        case kF16: return ng == 13 ? pick_form<kF16, 13>(form) : nullptr;
+        case kF16: return ng == 13 ? pick_form<kF16, 13, RUN>(form) : nullptr;
         default: return nullptr;
     }
 }
@@ -1057,18 +1177,26 @@ TensorPlan* tensor_plan_create(const PackedFrame& a, const PackedFrame& b, const
         q.hiH0 = hiH_d * bcast;
         q.dhi = hiH_s - hiH_d;
     }
-    if (cudaMalloc(&P->err, sizeof(unsigned int)) != cudaSuccess) {
+    // error word, then the barrier
+    unsigned long long* words = nullptr;
+    if (cudaMalloc(&words, 2 * sizeof(unsigned long long)) != cudaSuccess) {
         snprintf(why, why_len, "error-flag allocation failed");
         delete P;
         return nullptr;
     }
-    cudaMemset(P->err, 0, sizeof(unsigned int));
+    cudaMemset(words, 0, 2 * sizeof(unsigned long long));
+    P->err = (unsigned int*)words;
+    P->barrier = (GridBarrier*)(words + 1);
     for (auto& q : P->prm) {
         q.err = P->err;
+        q.barrier = P->barrier;
+        q.steps = 1;
         q.wait_ns = kWaitLimitNs;
         q.inject_missing_commit = 0;
     }
-    P->kernel = pick_kernel(G.mode, !fast ? kGather : (a.n % 32 == 0 ? kFast : kFastSeam), G.ng);
+    const int form = !fast ? kGather : (a.n % 32 == 0 ? kFast : kFastSeam);
+    P->kernel = pick_kernel<false>(G.mode, form, G.ng);
+    P->run = pick_kernel<true>(G.mode, form, G.ng);
     if (!P->kernel) {
         snprintf(why, why_len, "no kernel instantiation for R=%d", R);
         cudaFree(P->err);
@@ -1079,8 +1207,14 @@ TensorPlan* tensor_plan_create(const PackedFrame& a, const PackedFrame& b, const
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     P->grid = std::min(P->prm[0].tiles_x * P->prm[0].tiles_y, sms);
-    if (cudaFuncSetAttribute(P->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, P->smem_bytes) !=
-        cudaSuccess) {
+    // units of a generation per CTA: with many, the run's longer loops cost more than
+    // the launches (16384^2 R = 5 115 us per generation in launches of one, 128 in one
+    // launch; 8192^2 R = 5 33.5 / 34.3; 4096^2 R = 5 12.6 / 11.3, R = 100 33.5 / 32.5)
+    P->runs = (long long)P->prm[0].tiles_x * P->prm[0].tiles_y * G.nb <= 24ll * P->grid;
+    cudaError_t ae = cudaFuncSetAttribute(P->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, P->smem_bytes);
+    if (ae == cudaSuccess && P->runs)
+        ae = cudaFuncSetAttribute(P->run, cudaFuncAttributeMaxDynamicSharedMemorySize, P->smem_bytes);
+    if (ae != cudaSuccess) {
         snprintf(why, why_len, "cannot reserve %d bytes of shared memory", P->smem_bytes);
         cudaFree(P->err);
         delete P;
@@ -1106,10 +1240,26 @@ void tensor_plan_set_wait(TensorPlan* p, unsigned long long ns, int inject_missi
 int tensor_plan_operand_bits(const TensorPlan* p) { return p ? p->operand_bits : 0; }
 unsigned int* tensor_plan_error_flag(TensorPlan* p) { return p ? p->err : nullptr; }
 
-cudaError_t launch_tensor_pass(TensorPlan* p, bool src_is_a, cudaStream_t s) {
-    const int i = src_is_a ? 0 : 1;
-    p->kernel<<<p->grid, kThreads, p->smem_bytes, s>>>(p->prm[i]);
-    return cudaGetLastError();
+bool tensor_plan_runs(const TensorPlan* p) { return p->runs; }
+
+cudaError_t tensor_plan_reset(TensorPlan* p) {
+    return cudaMemset(p->err, 0, 2 * sizeof(unsigned long long));  // error word and barrier
+}
+
+cudaError_t launch_tensor_steps(TensorPlan* p, bool src_is_a, int steps, cudaStream_t s) {
+    TcParams q = p->prm[src_is_a ? 0 : 1];
+    q.steps = steps;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(p->grid);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = p->smem_bytes;
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeCooperative;
+    at.val.cooperative = steps > 1 && p->grid > 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, steps > 1 ? p->run : p->kernel, q);
 }
 
 }  // namespace ltl

@@ -84,7 +84,7 @@ struct ltl_ctx {
 
 static constexpr int kGraphPasses = 8;
 static constexpr int kAutoPackedRadius = 28;
-static constexpr int kRunSteps = 512;  // generations per launch of a small packed grid
+static constexpr int kRunSteps = 512;  // generations per launch of a small packed or tensor grid
 
 static Frame& cur_frame(ltl_ctx* c) { return c->cur_is_a ? c->fa : c->fb; }
 static Frame& nxt_frame(ltl_ctx* c) { return c->cur_is_a ? c->fb : c->fa; }
@@ -614,7 +614,7 @@ static cudaError_t enqueue_pass(ltl_ctx* c, int gens) {
         }
         case LTL_VARIANT_TENSOR: {
             // packed frames, torus wrap inside the kernel: no halo pass
-            e = launch_tensor_pass(c->tplan, c->cur_is_a, c->stream);
+            e = launch_tensor_steps(c->tplan, c->cur_is_a, gens, c->stream);
             step_kernels = 1;
             halo_kernels = 0;
             if (c->timing && e == cudaSuccess) e = cudaEventRecord(e1, c->stream);
@@ -656,10 +656,14 @@ static int build_graph(ltl_ctx* c, int which) {
 
 // One launch for up to kRunSteps generations (a kernel holds its SMs until its last).
 static cudaError_t enqueue_run(ltl_ctx* c, int steps) {
-    cudaError_t e = launch_packed_run(cur_packed(c), nxt_packed(c), c->rule, steps, c->run, c->stream);
-    if (e != cudaSuccess) return e;
-    c->run_unchecked = true;
-    if (steps % 2) c->cur_is_a = !c->cur_is_a;
+    cudaError_t e;
+    if (c->tplan) {
+        e = launch_tensor_steps(c->tplan, c->cur_is_a, steps, c->stream);
+    } else {
+        e = launch_packed_run(cur_packed(c), nxt_packed(c), c->rule, steps, c->run, c->stream);
+        if (e == cudaSuccess) c->run_unchecked = true;
+    }
+    if (e == cudaSuccess && steps % 2) c->cur_is_a = !c->cur_is_a;
     return e;
 }
 
@@ -671,7 +675,7 @@ extern "C" int ltl_step(ltl_ctx* c, int steps) {
     }
     if (steps == 0) return LTL_OK;
     LTL_CUDA(cudaSetDevice(c->device));
-    if (!c->timing && runs_packed(c)) {
+    if (!c->timing && (runs_packed(c) || (c->tplan && tensor_plan_runs(c->tplan)))) {
         for (; steps > 0; steps -= kRunSteps) LTL_CUDA(enqueue_run(c, std::min(steps, kRunSteps)));
         return LTL_OK;
     }
@@ -711,8 +715,7 @@ extern "C" int ltl_synchronize(ltl_ctx* c) {
         LTL_CUDA(cudaMemcpy(&flag, tensor_plan_error_flag(c->tplan), sizeof(flag), cudaMemcpyDeviceToHost));
         if (flag) {
             // clear it, so that the context stays usable after the caller re-uploads a state
-            const unsigned int zero = 0;
-            cudaMemcpy(tensor_plan_error_flag(c->tplan), &zero, sizeof(zero), cudaMemcpyHostToDevice);
+            tensor_plan_reset(c->tplan);
             ltl_set_error("tensor kernel reported a bounded-wait timeout (flag 0x%x); the grid state is "
                           "unspecified until the next upload",
                           flag);

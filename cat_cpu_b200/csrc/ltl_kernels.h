@@ -118,8 +118,12 @@ TensorPlan* tensor_plan_create(const PackedFrame& a, const PackedFrame& b, const
 void tensor_plan_destroy(TensorPlan* p);
 int tensor_plan_depth(const TensorPlan* p);
 int tensor_plan_operand_bits(const TensorPlan* p);
-// Advance one pass (tensor_plan_depth generations) from packed frame `src_is_a ? a : b`.
-cudaError_t launch_tensor_pass(TensorPlan* p, bool src_is_a, cudaStream_t s);
+// Advance `steps` generations in one launch, from packed frame `src_is_a ? a : b`
+// (steps > 1 only where tensor_plan_runs).
+bool tensor_plan_runs(const TensorPlan* p);
+cudaError_t launch_tensor_steps(TensorPlan* p, bool src_is_a, int steps, cudaStream_t s);
+// After a launch that set the error flag: clears it and the generations' barrier.
+cudaError_t tensor_plan_reset(TensorPlan* p);
 unsigned int* tensor_plan_error_flag(TensorPlan* p);
 // Limit of the kernel's bounded waits, and a test hook that withholds one
 // completion signal so that the waits run out (no fault, no hang: the kernel

@@ -23,6 +23,50 @@ def test_ragged_sides_vs_oracle(radius):
         g = (rng.random((n, n)) < 0.45).astype(np.uint8)
         with C.CUDASolver(n, radius, rule, variant=C.VARIANT_TENSOR) as s:
             s.setState(g)
-            s.doSteps(2)
+            for steps in (2, 1, 5):  # many generations per launch, and one
+                s.doSteps(steps)
+                s.synchronize()
+                g = O.run(g, radius, rule, steps)
+                assert np.array_equal(s.getCurrentState(), g), (n, radius, steps)
+
+
+def test_timeout_in_a_launch_of_many_generations():
+    """A withheld completion signal in one CTA: the others wait for its generation in
+    vain, every wait is bounded, the host sees LTL_ETIMEOUT, and the solver works on."""
+    import cat_cpu_b200 as C
+    n, r = 700, 5
+    g = (np.random.default_rng(1).random((n, n)) < 0.45).astype(np.uint8)
+    with C.CUDASolver(n, r, O.BOSCO_R5, variant=C.VARIANT_TENSOR) as s:
+        s.set_param("wait_limit_ns", 20_000_000)
+        s.set_param("inject_missing_commit", 1)
+        s.setState(g)
+        s.doSteps(4)
+        with pytest.raises(C.LtlError) as e:
             s.synchronize()
-            assert np.array_equal(s.getCurrentState(), O.run(g, radius, rule, 2)), (n, radius)
+        assert e.value.code == C.ltl.ETIMEOUT
+        s.set_param("inject_missing_commit", 0)
+        s.setState(g)
+        s.doSteps(6)
+        s.synchronize()
+        assert np.array_equal(s.getCurrentState(), O.run(g, r, O.BOSCO_R5, 6))
+
+
+def test_captured_generations_replay():
+    import torch
+    import cat_cpu_b200 as C
+    n, r = 500, 6
+    rule = O.scaled_rule(r)
+    g = (np.random.default_rng(2).random((n, n)) < 0.45).astype(np.uint8)
+    stream = torch.cuda.Stream()
+    with C.CUDASolver(n, r, rule, variant=C.VARIANT_TENSOR) as s:
+        s.set_stream(stream.cuda_stream)
+        s.setState(g)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            s.doSteps(4)
+        with torch.cuda.stream(stream):
+            graph.replay()
+            graph.replay()
+        torch.cuda.synchronize()
+        assert np.array_equal(s.getCurrentState(), O.run(g, r, rule, 8))
+        del graph
