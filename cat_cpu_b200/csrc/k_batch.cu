@@ -288,14 +288,14 @@ __global__ void k_batch_pack(const uint8_t* __restrict__ cells, uint32_t* __rest
         const int i = t / g.nw, w = t % g.nw;
         const uint8_t* p = c + (size_t)i * g.n + 32 * w;
         const int valid = g.n - 32 * w;
-        uint32_t v = cells16_to_bits<true>(load16(p, c, end));
-        if (valid > 16) v |= cells16_to_bits<true>(load16(p + 16, c, end)) << 16;
+        uint32_t v = cells16_to_bits<true>(load16<true>(p, c, end));
+        if (valid > 16) v |= cells16_to_bits<true>(load16<true>(p + 16, c, end)) << 16;
         if (valid < 32) {
             v &= (1u << valid) - 1u;
             if (g.n >= 64) {
                 const uint8_t* q = c + (size_t)i * g.n;
-                v = join_word(v, cells16_to_bits<true>(load16(q, c, end)) |
-                                     (cells16_to_bits<true>(load16(q + 16, c, end)) << 16), g.n);
+                v = join_word(v, cells16_to_bits<true>(load16<true>(q, c, end)) |
+                                     (cells16_to_bits<true>(load16<true>(q + 16, c, end)) << 16), g.n);
             }
         }
         arena[g.off + (size_t)i * g.wp + w] = v;
@@ -313,7 +313,7 @@ __global__ void k_batch_unpack(const uint32_t* __restrict__ arena, uint8_t* __re
         const int c = lead(row) + 16 * (t % vecs);
         if (c >= g.n) continue;
         const uint32_t bits = bits16_at(arena + g.off + (size_t)i * g.wp, c, g.nw);
-        store16(row + c, bits16_to_cells(bits), -c, g.n - c);
+        store16<true>(row + c, bits16_to_cells(bits), -c, g.n - c);
     }
 }
 

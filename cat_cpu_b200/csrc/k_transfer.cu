@@ -10,8 +10,9 @@
 // vectors that are aligned in the destination, and read an unaligned source as
 // aligned 32-bit words shifted together (load16).  Measured on B200, before
 // (one byte, or 64 strided bytes, per thread) and after: 16384^2 cells to PACK
-// words and back 2057 -> 131 us (604 MB, 4.6 TB/s); 16384^2 cells into a packed
-// frame and out again 1376 -> 152 us (the byte frame between is gone too).
+// words and back 2057 -> 107 us (604 MB, 5.6 TB/s; eight rows per thread 145);
+// 16384^2 cells into a packed frame and out again 1376 -> 117 us (the byte frame
+// between is gone too).
 //
 // Reference counterparts (kezada94/CAT_cpu): the host <-> solver copies of
 // src/CellularAutomata/Solvers/AMXSolver.cpp (CASolver.cpp:3-13) and
@@ -48,8 +49,8 @@ k_cells_to_words(const uint8_t* __restrict__ src, size_t sp, int rows, int cols,
             const int r = r0 + k * kTy;
             const uint8_t* p = src + (size_t)r * sp + 32 * (size_t)w;
             a[k] = b[k] = make_uint4(0u, 0u, 0u, 0u);
-            if (r < rows && valid > 0) a[k] = load16(p, src, end);
-            if (r < rows && valid > 16) b[k] = load16(p + 16, src, end);
+            if (r < rows && valid > 0) a[k] = load16<true>(p, src, end);
+            if (r < rows && valid > 16) b[k] = load16<true>(p + 16, src, end);
         }
 #pragma unroll
         for (int k = 0; k < kRows; ++k) {
@@ -59,8 +60,8 @@ k_cells_to_words(const uint8_t* __restrict__ src, size_t sp, int rows, int cols,
             if constexpr (kJoin) {
                 if (valid > 0 && valid < 32) {
                     const uint8_t* p = src + (size_t)r * sp;
-                    v = join_word(v, cells16_to_bits<kNonzero>(load16(p, src, end)) |
-                                         (cells16_to_bits<kNonzero>(load16(p + 16, src, end)) << 16), cols);
+                    v = join_word(v, cells16_to_bits<kNonzero>(load16<true>(p, src, end)) |
+                                         (cells16_to_bits<kNonzero>(load16<true>(p + 16, src, end)) << 16), cols);
                 }
             }
             dst[(size_t)r * dp + w] = v;
@@ -87,7 +88,7 @@ k_words_to_cells(const uint32_t* __restrict__ src, size_t sp, int nwords, int ro
             if (r >= rows) continue;
             uint8_t* row = dst + (size_t)r * dp;
             const int c = lead(row) + 16 * v;
-            if (c < cols) store16(row + c, bits16_to_cells(bits[k]), -c, cols - c);
+            if (c < cols) store16<true>(row + c, bits16_to_cells(bits[k]), -c, cols - c);
         }
     }
 }
@@ -106,7 +107,7 @@ k_copy_cells(const uint8_t* src, size_t sp, int rows, int cols, uint8_t* dst, si
             const int r = r0 + k * kTy;
             const int c = lead(dst + (size_t)r * dp) + 16 * v;
             a[k] = make_uint4(0u, 0u, 0u, 0u);
-            if (r < rows && c < cols) a[k] = load16(src + (size_t)r * sp + c, src, end);
+            if (r < rows && c < cols) a[k] = load16<false>(src + (size_t)r * sp + c, src, end);
         }
 #pragma unroll
         for (int k = 0; k < kRows; ++k) {
@@ -116,7 +117,7 @@ k_copy_cells(const uint8_t* src, size_t sp, int rows, int cols, uint8_t* dst, si
             const int c = lead(row) + 16 * v;
             if constexpr (kNonzero)
                 a[k] = make_uint4(nonzero4(a[k].x), nonzero4(a[k].y), nonzero4(a[k].z), nonzero4(a[k].w));
-            if (c < cols) store16(row + c, a[k], -c, cols - c);
+            if (c < cols) store16<false>(row + c, a[k], -c, cols - c);
         }
     }
 }
@@ -193,7 +194,7 @@ k_compare(GridRows g, const uint8_t* __restrict__ other, size_t op, unsigned lon
                 } else {
                     a[k] = __ldg((const uint4*)((const uint8_t*)g.inner + (size_t)r * g.pitch) + v);
                 }
-                b[k] = load16(other + (size_t)r * op + 16 * (size_t)v, other, end);
+                b[k] = load16<true>(other + (size_t)r * op + 16 * (size_t)v, other, end);
             }
 #pragma unroll
             for (int k = 0; k < kRows; ++k) {

@@ -33,10 +33,15 @@ __device__ __forceinline__ uint4 bits16_to_cells(uint32_t b) {
 }
 
 // The 16 bytes at p, of a buffer whose bytes are [lo, hi).  Bytes outside the
-// buffer come back as 0 and are not read.  p may have any alignment.
+// buffer come back as 0 and are not read.  p may have any alignment.  kStream: whole
+// vectors are marked to be evicted first (so are store16's): cells that become words,
+// or come from them, pass through once and would push the words out of L2 (16384^2
+// cells to words and back 136 us without marks or with those of the stores alone, 107
+// with both; compare 147 / 123).  A copy of cells is slower with them, 84 / 96.
+template <bool kStream>
 __device__ __forceinline__ uint4 load16(const uint8_t* p, const uint8_t* lo, const uint8_t* hi) {
     const uintptr_t a = (uintptr_t)p;
-    if ((a & 15) == 0 && p >= lo && p + 16 <= hi) return *(const uint4*)p;
+    if ((a & 15) == 0 && p >= lo && p + 16 <= hi) return kStream ? __ldcs((const uint4*)p) : *(const uint4*)p;
     const uint32_t* q = (const uint32_t*)(a & ~(uintptr_t)3);
     const int sh = 8 * (int)(a & 3);
     if ((const uint8_t*)q >= lo && (const uint8_t*)(q + 5) <= hi) {
@@ -53,9 +58,11 @@ __device__ __forceinline__ uint4 load16(const uint8_t* p, const uint8_t* lo, con
 
 // Bytes [from, to) of v to dst .. dst + 15 (dst 16-byte aligned; a whole vector
 // where from = 0 and to = 16).
+template <bool kStream>
 __device__ __forceinline__ void store16(uint8_t* dst, uint4 v, int from, int to) {
     if (from <= 0 && to >= 16) {
-        *(uint4*)dst = v;
+        if constexpr (kStream) __stcs((uint4*)dst, v);
+        else *(uint4*)dst = v;
         return;
     }
     const uint32_t w[4] = {v.x, v.y, v.z, v.w};
