@@ -29,14 +29,14 @@ constexpr int kTileThreads = 512;
 constexpr int kTileMaxRadius = 16;   // radii of the tile kernels
 constexpr size_t kTileSmem = 220 * 1024;
 
-// Words per lane and ring of the band walk, measured at 16384^2 (us): two words
-// per lane share their neighbours' loads and half the loop's bookkeeping (R = 1
-// 26 against 33, R = 5 53 / 58, R = 8 75 / 78), until the ring's share of shared
-// memory leaves too few warps (R = 12 104 / 96, R = 16 128 / 104).  From R = 29 on
-// a ring leaves one or two warps per SM, and counting the leaving row again is
-// cheaper (R = 32 283 against 340, R = 24 226 against 169).
-template <int R>
-constexpr int packed_words() { return R <= 8 ? 2 : 1; }
+// Words per lane of the band walk.  Two share their neighbours' loads and half the
+// loop's bookkeeping (16384^2, us, one / two: R = 1 33 / 26, R = 5 58 / 43, R = 9 75.5 /
+// 58.7, R = 12 84.3 / 72.8, R = 16 100.7 / 86.4).  Above R = 10 their ring leaves one CTA
+// per SM, which only rows without ragged lanes stand (12001^2 R = 12 59 / 72, R = 10 54 /
+// 49); above R = 16 it does not fit.
+constexpr int packed_words(int R, bool ragged) { return R <= (ragged ? 10 : 16) ? 2 : 1; }
+// Ring.  From R = 29 on it leaves one or two warps per SM, and counting the leaving row
+// again is cheaper (16384^2 R = 32 216 us against 340 with one, R = 24 226 against 144).
 template <int R>
 constexpr bool packed_ring() { return R <= 28; }
 
@@ -75,9 +75,11 @@ struct PackedSplit {
     }
 };
 
-// One generation.
+// One generation.  Two CTAs per SM are all that is asked of the compiler: left to
+// itself it keeps to 64 registers and pays in instructions (16384^2 R = 8 77.5 us
+// against 61.7, R = 12 91.9 / 84.7, R = 5 44.7 / 43.6).
 template <int R, int W, bool kRing, int EDGE>
-__global__ void __launch_bounds__(kPackedWarps * 32)
+__global__ void __launch_bounds__(kPackedWarps * 32, 2)
 k_packed_step(const uint32_t* __restrict__ cur, uint32_t* __restrict__ nxt, int wp, int n, int nw, int rows,
               PackedSplit split, const __grid_constant__ PackedRule pr) {
     extern __shared__ __align__(16) uint32_t ring_all[];
@@ -294,13 +296,21 @@ struct SmallLaunch {
     }
 };
 
+// f(launcher) of the band walk's form for a side.
+template <int R, class F>
+static cudaError_t with_walk(int n, F f) {
+    if (n < 64) return f(PackedLaunch<R, 1, kEdgeTiny>{});
+    if (packed_edge(n, 2) == kEdgeNone && packed_words(R, false) == 2)
+        return f(PackedLaunch<R, packed_words(R, false), kEdgeNone>{});
+    constexpr int W = packed_words(R, true);
+    if (packed_edge(n, W) == kEdgeNone) return f(PackedLaunch<R, W, kEdgeNone>{});
+    return f(PackedLaunch<R, W, kEdgeRagged>{});
+}
+
 template <int R>
 static cudaError_t launch_packed_r(const PackedFrame& c, const PackedFrame& x, const PackedRule& pr, int band_rows,
                                    cudaStream_t s) {
-    constexpr int W = packed_words<R>();
-    if (c.n < 64) return PackedLaunch<R, 1, kEdgeTiny>::step(c, x, pr, band_rows, s);
-    if (packed_edge(c.n, W) == kEdgeNone) return PackedLaunch<R, W, kEdgeNone>::step(c, x, pr, band_rows, s);
-    return PackedLaunch<R, W, kEdgeRagged>::step(c, x, pr, band_rows, s);
+    return with_walk<R>(c.n, [&](auto l) { return l.step(c, x, pr, band_rows, s); });
 }
 
 // Which kernel advances a grid, by its words and R.  Measured per generation (us, 48
@@ -360,10 +370,7 @@ static int device_sms() {
 // 3 us here, so not those of every form).
 template <int R>
 static cudaError_t prepare_packed_r(const PackedFrame& f, int sms) {
-    constexpr int W = packed_words<R>();
-    cudaError_t e = f.n < 64 ? PackedLaunch<R, 1, kEdgeTiny>::prepare()
-                             : (packed_edge(f.n, W) == kEdgeNone ? PackedLaunch<R, W, kEdgeNone>::prepare()
-                                                                : PackedLaunch<R, W, kEdgeRagged>::prepare());
+    cudaError_t e = with_walk<R>(f.n, [](auto l) { return l.prepare(); });
     if constexpr (R <= kTileMaxRadius) {
         const PackedRoute route = packed_route_r<R>(f.nrows(), f.nw, sms);
         if (e != cudaSuccess || route == kRouteWalk) return e;
