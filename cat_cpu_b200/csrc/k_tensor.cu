@@ -457,6 +457,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tensor_step(const __grid_consta
             *(uint4*)(bv + (((i >> 3) * 2 + half) * 128 + (i & 7) * 16)) = make_uint4(w[0], w[1], w[2], w[3]);
         }
     }
+    if constexpr (!RUN) chain_wait();  // the prologue above reads nothing of the grid
     fence_proxy_async();
     fence_before();
     __syncthreads();
@@ -1249,6 +1250,7 @@ cudaError_t tensor_plan_reset(TensorPlan* p) {
 cudaError_t launch_tensor_steps(TensorPlan* p, bool src_is_a, int steps, cudaStream_t s) {
     TcParams q = p->prm[src_is_a ? 0 : 1];
     q.steps = steps;
+    if (steps == 1) return launch_chained(p->kernel, dim3(p->grid), dim3(kThreads), p->smem_bytes, s, q);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(p->grid);
     cfg.blockDim = dim3(kThreads);
@@ -1256,10 +1258,10 @@ cudaError_t launch_tensor_steps(TensorPlan* p, bool src_is_a, int steps, cudaStr
     cfg.stream = s;
     cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeCooperative;
-    at.val.cooperative = steps > 1 && p->grid > 1;
+    at.val.cooperative = p->grid > 1;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, steps > 1 ? p->run : p->kernel, q);
+    return cudaLaunchKernelEx(&cfg, p->run, q);
 }
 
 }  // namespace ltl
