@@ -40,6 +40,11 @@ constexpr int packed_words(int R, bool ragged) { return R <= (ragged ? 10 : 16) 
 template <int R>
 constexpr bool packed_ring() { return R <= 28; }
 
+// Rows in flight per lane: two where few warps share an SM (the larger rings) and the
+// lane has no ragged words besides (16384^2 R = 8 58.9 -> 55.9, R = 12 72.7 -> 67.6, R = 5
+// 43.4 -> 43.5; 12001^2 R = 16 68.5 -> 72.1).
+constexpr bool packed_deep(int R, int W, int edge) { return edge == kEdgeNone && W == 2 && R >= 6; }
+
 // Rows per band.  All bands of a step run at once, k CTAs on each SM, and each
 // counts 2R+1 rows (at about 0.6 of an output row's cost) before its first output
 // row: more CTAs per SM keep the ALU busier, fewer repeat less.  Time of a row
@@ -86,7 +91,7 @@ k_packed_step(const uint32_t* __restrict__ cur, uint32_t* __restrict__ nxt, int 
     uint32_t* ring = ring_all + (kRing ? (threadIdx.x >> 5) * PackedRing<R, W>::WARP_WORDS : 0);
     int w0, r0, r1;
     if (split.item(blockIdx.x * (kPackedWarps * 32) + threadIdx.x, rows, W, w0, r0, r1))
-        packed_walk<R, W, kRing, EDGE, true>(cur, nxt, wp, n, nw, rows, r0, r1, w0, ring, threadIdx.x & 31, pr);
+        packed_walk<R, W, kRing, EDGE, true, packed_deep(R, W, EDGE)>(cur, nxt, wp, n, nw, rows, r0, r1, w0, ring, threadIdx.x & 31, pr);
 }
 
 // `steps` generations in one cooperative launch, a tile per CTA (packed_tile.cuh), a

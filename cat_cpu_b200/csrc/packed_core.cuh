@@ -457,7 +457,7 @@ struct RowReader {
 // cur, nxt: word 0 of row 0; wp words per row (a multiple of 4; the row's words
 // up to a multiple of W may be written).  kConst: cur is not written while the
 // kernel runs (read-only loads).  ring: this warp's ring.
-template <int R, int W, bool kRing, int EDGE, bool kConst>
+template <int R, int W, bool kRing, int EDGE, bool kConst, bool kDeep = false>
 __device__ __forceinline__ void packed_walk(const uint32_t* cur, uint32_t* nxt, int wp, int n, int nw, int rows, int r0,
                                             int r1, int w0, uint32_t* ring, int lane, const PackedRule& pr) {
     using Ring = PackedRing<R, W>;
@@ -516,8 +516,18 @@ __device__ __forceinline__ void packed_walk(const uint32_t* cur, uint32_t* nxt, 
     if constexpr ((2 * R + 1) % kChunk != 0) start_rows(std::integral_constant<int, (2 * R + 1) % kChunk>{});
     slot = ring;
     const uint32_t* const ring_end = ring + Ring::WARP_WORDS;
-    RowWords<W, EDGE> next;
+    // rows in flight: the next one, kDeep also the one after it (and its centre)
+    RowWords<W, EDGE> next, next2;
+    uint32_t cen2[W];
     if (r0 + 1 < r1) rd.load(pi, next);
+    if constexpr (kDeep) {
+        pi += wp;
+        ++ri;
+        wrap(pi, ri);
+        if (r0 + 2 < r1) rd.load(pi, next2);
+        pc += wp;
+        if (r0 + 1 < r1) rd.own(pc, cen2);
+    }
 #pragma unroll 1
     for (int r = r0;; ++r) {
         uint32_t val[W];
@@ -532,12 +542,20 @@ __device__ __forceinline__ void packed_walk(const uint32_t* cur, uint32_t* nxt, 
         if (r + 1 >= r1) break;
         pn += wp;
         pc += wp;
-        rd.own(pc, cen);
         RowWords<W, EDGE> x = next;
         pi += wp;
         ++ri;
         wrap(pi, ri);
-        if (r + 2 < r1) rd.load(pi, next);
+        if constexpr (kDeep) {
+#pragma unroll
+            for (int w = 0; w < W; ++w) cen[w] = cen2[w];
+            next = next2;
+            if (r + 2 < r1) rd.own(pc, cen2);
+            if (r + 3 < r1) rd.load(pi, next2);
+        } else {
+            rd.own(pc, cen);
+            if (r + 2 < r1) rd.load(pi, next);
+        }
         rd.fix(x);
         uint32_t in[W][PH], out[W][PH];
         if constexpr (kRing) {

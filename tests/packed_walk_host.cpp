@@ -46,8 +46,12 @@ static void grid_step(const uint32_t* cur, uint32_t* nxt, int wp, int n, int row
     int lane = 0;
     for (int r0 = 0; r0 < rows; r0 += band_rows)
         for (int g = 0; g < groups; ++g, lane = (lane + 1) % 32)
-            packed_walk<R, W, kRing, EDGE, true>(cur, nxt, wp, n, nw, rows, r0, std::min(r0 + band_rows, rows), W * g,
-                                                 (uint32_t*)ring.data(), lane, pr);
+            if (lane % 2)  // one or two rows in flight
+                packed_walk<R, W, kRing, EDGE, true, true>(cur, nxt, wp, n, nw, rows, r0, std::min(r0 + band_rows, rows),
+                                                           W * g, (uint32_t*)ring.data(), lane, pr);
+            else
+                packed_walk<R, W, kRing, EDGE, true>(cur, nxt, wp, n, nw, rows, r0, std::min(r0 + band_rows, rows), W * g,
+                                                     (uint32_t*)ring.data(), lane, pr);
 }
 
 template <int R, bool kRing>
