@@ -15,7 +15,7 @@
 // pipe cannot do either).  At R = 5 a word costs 67 such operations: window count
 // 23.5, moving B 21, rule 23.  Measured per generation at 16384^2, R = 5: 71.9 us
 // before (a halo'd frame, one word per lane, neighbours by shuffle, 90 operations and
-// as many again around them, 71% of the ALU), 44.3 now (about 84%).
+// as many again around them, 71% of the ALU), 43.5 now (81% in a cold launch).
 #include <algorithm>
 
 #include "grid_barrier.cuh"
@@ -50,7 +50,16 @@ constexpr bool packed_deep(int R, int W, int edge) { return edge == kEdgeNone &&
 // row: more CTAs per SM keep the ALU busier, fewer repeat less.  Time of a row
 // relative to three or more CTAs per SM, measured on B200 at R = 5 (16384^2: 50.6,
 // 44.6, 46.0 us at k = 2, 3, 4; 4096^2: k = 1 1.5 times): 1.5, 1.12, 1, 1.
-static int packed_band_rows(int rows, int groups, int R, int sms, int per_sm) {
+//
+// Small radii repeat little and wait for memory, so they take about 20 + 4R rows: as
+// many CTAs as an SM holds, or several waves of them (one CTA more than it holds would
+// be a wave of its own; 14001^2 R = 2 k = 5, 6, 7: 28.2, 30.8, 28.2 us).  us, long
+// bands / these: 10001^2 R = 1 14.1 / 12.6; 16001^2 R = 1 33.2 / 26.7, R = 4 49.4 / 47.1
+// (R = 5 no gain); 15040^2 R = 1 24.5 / 22.6; 16384^2 R = 3 35.8 / 36.5.  Beyond the L2
+// long bands cost up to twice as much, every one of them being at another place of the
+// grid: 32768^2 R = 1 173 / 91, R = 5 189 / 180; 20032^2 R = 1 61 / 40, R = 5 82 / 76;
+// 22016^2 R = 6 93 / 97.
+static int packed_band_rows(int rows, int groups, int R, bool ragged, bool beyond_l2, int sms, int per_sm) {
     static const double rate[] = {1.5, 1.12, 1.0, 1.0};
     double best = 0;
     int best_rows = rows;
@@ -62,6 +71,14 @@ static int packed_band_rows(int rows, int groups, int R, int sms, int per_sm) {
             best = t;
             best_rows = b;
         }
+    }
+    const int brief = 20 + 4 * R;
+    if (best_rows > brief && R <= (beyond_l2 ? 5 : ragged ? 4 : 2)) {
+        const long long lanes = (long long)sms * kPackedWarps * 32;
+        long long k = ((long long)rows * groups + brief * lanes - 1) / (brief * lanes);
+        if (k == per_sm + 1) k = per_sm;
+        const long long bands = std::max(1LL, k * lanes / groups);
+        best_rows = std::min(best_rows, (int)((rows + bands - 1) / bands));
     }
     return std::min(best_rows, rows);
 }
@@ -192,12 +209,15 @@ struct PackedLaunch {
     }
     template <class K>
     static PackedSplit split(K kernel, const PackedFrame& c, int band_rows, unsigned& ctas) {
-        int dev = 0, sms = 148, per_sm = 0;
+        int dev = 0, sms = 148, l2 = 126 << 20, per_sm = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kPackedWarps * 32, smem);
         const int rows = c.nrows(), groups = (c.nw + W - 1) / W;
-        if (band_rows <= 0) band_rows = packed_band_rows(rows, groups, R, sms, std::max(per_sm, 1));
+        const bool beyond_l2 = 8ll * rows * c.wpitch > l2 / 4 * 3ll;  // (both frames; a rest stays in it)
+        if (band_rows <= 0)
+            band_rows = packed_band_rows(rows, groups, R, EDGE != kEdgeNone, beyond_l2, sms, std::max(per_sm, 1));
         const int bands = (rows + band_rows - 1) / band_rows;
         const long long items = (long long)groups * bands;
         ctas = (unsigned)((items + kPackedWarps * 32 - 1) / (kPackedWarps * 32));

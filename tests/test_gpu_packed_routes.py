@@ -95,3 +95,31 @@ def test_auto_names_plain_and_takes_its_parameters(n, radius):
             solver.doSteps(5)
             assert np.array_equal(solver.getCurrentState(), O.run(g, radius, rule, 5))
             assert solver.population() == int(O.run(g, radius, rule, 5).sum())
+
+
+@pytest.mark.parametrize("n,radius", [(12001, 1), (12032, 2), (14001, 4), (20033, 5), (20032, 1)])
+def test_short_bands_vs_long_bands_and_plain(n, radius):
+    """Grids large enough for the band walk's short bands (within the L2, and with
+    frames that do not fit it): the same cells as with long bands and as the plain
+    solver's, which counts in another way."""
+    import torch
+    import cat_cpu_b200 as C
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(n)
+    g = (torch.rand((n, n), generator=gen, device="cuda") < 0.45).to(torch.uint8)
+    torch.cuda.synchronize()
+    got = []
+    for variant, band_rows in ((C.VARIANT_PACKED, 0), (C.VARIANT_PACKED, 500), (C.VARIANT_PLAIN, 0)):
+        out = torch.empty_like(g)
+        torch.cuda.synchronize()
+        with C.CUDASolver(n, radius, rule_of(radius), variant=variant) as s:
+            if band_rows:
+                s.set_param("band_rows", band_rows)
+            s.upload_device(g.data_ptr(), n)
+            s.doSteps(3)
+            s.download_device(out.data_ptr(), n)
+            s.synchronize()
+        got.append(out)
+    assert int(got[0].sum()) > 0
+    assert torch.equal(got[0], got[1])
+    assert torch.equal(got[0], got[2])
