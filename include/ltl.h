@@ -36,7 +36,8 @@ extern "C" {
 
 /* Stepping variants (the GPU analogues of the reference's solver codes,
  * CASolverFactory.cpp:10-119; the reference's own codes 0-6 are CPU solvers). */
-#define LTL_VARIANT_AUTO (-1)  /* pick the fastest exact variant for (n, R) */
+#define LTL_VARIANT_AUTO (-1)  /* the fastest exact kernels for (n, R): bit-packed up to R = 28, else plain;
+                                * ltl_get_info and ltl_set_param treat it as the plain variant */
 #define LTL_VARIANT_PLAIN 0    /* CUDA-core SWAR stencil, uint8 cells */
 #define LTL_VARIANT_TENSOR 1   /* tcgen05 banded products B_v * X * B_h, bit-packed grid */
 #define LTL_VARIANT_PACKED 2   /* bit-packed cells (64 per uint64), CUDA-core bit logic */
@@ -119,7 +120,9 @@ int ltl_upload_device(ltl_ctx* ctx, const uint8_t* dev_inner, size_t pitch);
 int ltl_download_device(ltl_ctx* ctx, uint8_t* dev_inner, size_t pitch);
 
 /* Advance `steps` generations (asynchronous on the context's stream).
- * Replaces CASolver::doSteps/doStep (CASolver.cpp:15-31): halo fill, step, swap. */
+ * Replaces CASolver::doSteps/doStep (CASolver.cpp:15-31): halo fill, step, swap.
+ * Small packed and tensor grids run a call's generations in one cooperative launch
+ * whose CTAs wait for one another (bounded: ltl_synchronize reports LTL_ETIMEOUT). */
 int ltl_step(ltl_ctx* ctx, int steps);
 
 /* Wait for all work queued on the context's stream; reports device-side error flags. */
@@ -185,10 +188,12 @@ int ltl_batch_upload_all(ltl_batch* b, const uint8_t* cells);
 int ltl_batch_download_all(ltl_batch* b, uint8_t* cells);
 int ltl_batch_step(ltl_batch* b, int steps);
 /* Batch shape parameters (autotuned; also read from the tuning table):
- *   "persistent"          1 (default): one persistent launch per rule class runs
- *                         every generation of an ltl_batch_step, each CTA taking
- *                         whole grids, largest first; 0: per-generation launches
- *                         (the two parameters below apply)
+ *   "persistent"          1 (default): one persistent launch runs every generation
+ *                         of an ltl_batch_step: large grids by groups of CTAs, the
+ *                         others by single CTAs, the most work first (a bounded wait
+ *                         between a group's CTAs: ltl_batch_synchronize and the
+ *                         downloads report LTL_ETIMEOUT if it ran out); 0:
+ *                         per-generation launches (the two parameters below apply)
  *   "stream_band_rows"    rows per work item of the streamed per-step kernels
  *   "resident_max_bytes"  shared-memory budget deciding which grids stay resident
  * Setting one rebuilds the work lists before the next step. */
@@ -203,7 +208,8 @@ int ltl_batch_info(const ltl_batch* b, long long* cells, long long* device_bytes
 /* Shape parameters (what cat_cpu_b200/autotune.py sweeps; the autotuned table
  * tuning/ltl_tuning.txt next to the library sets them at ltl_create):
  *   "band_rows"  rows per work item of the plain and packed step kernels
- *                (0: the built-in choice);
+ *                (0: the built-in choice; a set value also keeps small packed
+ *                grids on the kernel that has such bands);
  *   "depth"      generations per pass of the plain variant: 1, or 2..3 with
  *                depth * R <= 16 and R <= 5 (temporal blocking: one read and
  *                one write of the grid per pass).  ltl_step accepts any step
