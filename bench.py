@@ -51,9 +51,10 @@ REF_RULE_TAG = "R5_S32-56_B34-45"
 # workload (the bit-packed kernels are bound by logic operations on the ALU pipe,
 # the tensor kernel by hand-offs between its warp roles, not by HBM).
 LIMITER = {
-    "plain": {"pipe": "alu", "ncu_pct_of_peak": 72.0, "source": "profiles/k_plain_swar8_tb_n16384_r5.md"},
-    "packed": {"pipe": "alu", "ncu_pct_of_peak": 70.7, "source": "profiles/k_packed_step_n16384_r5.md"},
-    "tensor": {"pipe": "tensor", "ncu_pct_of_peak": 32.8, "issue_active_pct": 59.9,
+    "plain": {"pipe": "alu", "ncu_pct_of_peak": 65.6, "issue_active_pct": 71.1,
+              "source": "profiles/k_plain_swar8_tb_n16384_r5.md"},
+    "packed": {"pipe": "alu", "ncu_pct_of_peak": 80.7, "source": "profiles/k_packed_step_n16384_r5.md"},
+    "tensor": {"pipe": "tensor", "ncu_pct_of_peak": 33.0, "issue_active_pct": 60.4,
                "source": "profiles/k_tensor_step_n16384_r5.md"},
 }
 
