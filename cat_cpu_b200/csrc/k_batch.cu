@@ -284,8 +284,8 @@ __global__ void k_batch_pack(const uint8_t* __restrict__ cells, uint32_t* __rest
     const BatchGrid g = grids[first + blockIdx.y];
     const uint8_t* c = cells + g.cell_off;
     const uint8_t* end = c + (size_t)g.n * g.n;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < g.n * g.nw; t += gridDim.x * blockDim.x) {
-        const int i = t / g.nw, w = t % g.nw;
+    for (RowWalk t(blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, g.nw); t.row < g.n; t.next()) {
+        const int i = t.row, w = t.col;
         const uint8_t* p = c + (size_t)i * g.n + 32 * w;
         const int valid = g.n - 32 * w;
         uint32_t v = cells16_to_bits<true>(load16<true>(p, c, end));
@@ -307,10 +307,10 @@ __global__ void k_batch_unpack(const uint32_t* __restrict__ arena, uint8_t* __re
     const BatchGrid g = grids[first + blockIdx.y];
     uint8_t* dst = cells + g.cell_off;
     const int vecs = (g.n + 15) / 16 + 1;  // aligned vectors a row may touch
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < g.n * vecs; t += gridDim.x * blockDim.x) {
-        const int i = t / vecs;
+    for (RowWalk t(blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, vecs); t.row < g.n; t.next()) {
+        const int i = t.row;
         uint8_t* row = dst + (size_t)i * g.n;
-        const int c = lead(row) + 16 * (t % vecs);
+        const int c = lead(row) + 16 * t.col;
         if (c >= g.n) continue;
         const uint32_t bits = bits16_at(arena + g.off + (size_t)i * g.wp, c, g.nw);
         store16<true>(row + c, bits16_to_cells(bits), -c, g.n - c);

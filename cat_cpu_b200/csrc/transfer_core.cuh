@@ -80,6 +80,24 @@ __device__ __forceinline__ uint32_t bits16_at(const uint32_t* row, int c, int nw
     return __funnelshift_r(lo, hi, c & 31) & 0xffffu;
 }
 
+// Items `at`, at + stride, .. of an array of `width` items per row, in row-major order,
+// as rows and columns.  No item number is formed: the number of 16-cell vectors of a
+// grid passes 2^31 at 185,352 cells a side, that of its words at 262,144.
+struct RowWalk {
+    int row, col;
+    int width, rows_on, cols_on;  // what a stride moves
+    __host__ __device__ RowWalk(int at, int stride, int width_)
+        : row(at / width_), col(at % width_), width(width_), rows_on(stride / width_), cols_on(stride % width_) {}
+    __host__ __device__ void next() {
+        row += rows_on;
+        col += cols_on;
+        if (col >= width) {
+            col -= width;
+            ++row;
+        }
+    }
+};
+
 // Byte offset of the first 16-byte vector of a destination row relative to its
 // first cell: 0 if aligned, else negative (that vector starts before the row).
 __device__ __forceinline__ int lead(const uint8_t* p) { return -(int)((uintptr_t)p & 15); }
