@@ -29,24 +29,28 @@ namespace {
 constexpr int kTx = 32;    // threads along a row
 constexpr int kTy = 8;     // rows per block pass
 constexpr int kRows = 4;   // rows per thread in flight
+// (Rows are counted unsigned: a grid of blocks may pass the last of 2^31 - 1 rows.)
+
+// 16-byte vectors that a row of cells may touch.
+__host__ __device__ constexpr int vectors(int cols) { return (cols + 15) / 16 + 1; }
 
 // Byte rows -> word rows: thread = one 32-bit word of a row, kNonzero: a cell is
 // alive if its byte is not 0 (else by its bit 0).  Words past the cells get 0; bits
 // past them in the last word 0, or the row's first cells (kJoin, cols >= 64).
 template <bool kNonzero, bool kJoin>
 __global__ void __launch_bounds__(kTx * kTy)
-k_cells_to_words(const uint8_t* __restrict__ src, size_t sp, int rows, int cols, uint32_t* __restrict__ dst, size_t dp,
+k_cells_to_words(const uint8_t* __restrict__ src, size_t sp, unsigned rows, int cols, uint32_t* __restrict__ dst, size_t dp,
                  int nwords) {
     const int w = blockIdx.x * kTx + threadIdx.x;
     if (w >= nwords) return;
     const uint8_t* end = src + (size_t)(rows - 1) * sp + cols;
     const int valid = cols - 32 * w;
     const uint32_t mask = valid >= 32 ? 0xffffffffu : (valid > 0 ? (1u << valid) - 1u : 0u);
-    for (int r0 = blockIdx.y * (kTy * kRows) + threadIdx.y; r0 < rows; r0 += gridDim.y * (kTy * kRows)) {
+    for (unsigned r0 = blockIdx.y * (kTy * kRows) + threadIdx.y; r0 < rows; r0 += gridDim.y * (kTy * kRows)) {
         uint4 a[kRows], b[kRows];
 #pragma unroll
         for (int k = 0; k < kRows; ++k) {
-            const int r = r0 + k * kTy;
+            const unsigned r = r0 + k * kTy;
             const uint8_t* p = src + (size_t)r * sp + 32 * (size_t)w;
             a[k] = b[k] = make_uint4(0u, 0u, 0u, 0u);
             if (r < rows && valid > 0) a[k] = load16<true>(p, src, end);
@@ -54,7 +58,7 @@ k_cells_to_words(const uint8_t* __restrict__ src, size_t sp, int rows, int cols,
         }
 #pragma unroll
         for (int k = 0; k < kRows; ++k) {
-            const int r = r0 + k * kTy;
+            const unsigned r = r0 + k * kTy;
             if (r >= rows) continue;
             uint32_t v = (cells16_to_bits<kNonzero>(a[k]) | (cells16_to_bits<kNonzero>(b[k]) << 16)) & mask;
             if constexpr (kJoin) {
@@ -71,20 +75,21 @@ k_cells_to_words(const uint8_t* __restrict__ src, size_t sp, int rows, int cols,
 
 // Word rows -> byte rows: thread = one aligned 16-byte vector of the destination.
 __global__ void __launch_bounds__(kTx * kTy)
-k_words_to_cells(const uint32_t* __restrict__ src, size_t sp, int nwords, int rows, int cols, uint8_t* __restrict__ dst,
+k_words_to_cells(const uint32_t* __restrict__ src, size_t sp, int nwords, unsigned rows, int cols, uint8_t* __restrict__ dst,
                  size_t dp) {
     const int v = blockIdx.x * kTx + threadIdx.x;
-    for (int r0 = blockIdx.y * (kTy * kRows) + threadIdx.y; r0 < rows; r0 += gridDim.y * (kTy * kRows)) {
+    if (v >= vectors(cols)) return;
+    for (unsigned r0 = blockIdx.y * (kTy * kRows) + threadIdx.y; r0 < rows; r0 += gridDim.y * (kTy * kRows)) {
         uint32_t bits[kRows];
 #pragma unroll
         for (int k = 0; k < kRows; ++k) {
-            const int r = r0 + k * kTy;
+            const unsigned r = r0 + k * kTy;
             const int c = lead(dst + (size_t)r * dp) + 16 * v;
             bits[k] = r < rows && c < cols ? bits16_at(src + (size_t)r * sp, c, nwords) : 0u;
         }
 #pragma unroll
         for (int k = 0; k < kRows; ++k) {
-            const int r = r0 + k * kTy;
+            const unsigned r = r0 + k * kTy;
             if (r >= rows) continue;
             uint8_t* row = dst + (size_t)r * dp;
             const int c = lead(row) + 16 * v;
@@ -97,21 +102,22 @@ k_words_to_cells(const uint32_t* __restrict__ src, size_t sp, int nwords, int ro
 // src == dst is allowed: a thread reads only the vectors it writes.
 template <bool kNonzero>
 __global__ void __launch_bounds__(kTx * kTy)
-k_copy_cells(const uint8_t* src, size_t sp, int rows, int cols, uint8_t* dst, size_t dp) {
+k_copy_cells(const uint8_t* src, size_t sp, unsigned rows, int cols, uint8_t* dst, size_t dp) {
     const int v = blockIdx.x * kTx + threadIdx.x;
+    if (v >= vectors(cols)) return;
     const uint8_t* end = src + (size_t)(rows - 1) * sp + cols;
-    for (int r0 = blockIdx.y * (kTy * kRows) + threadIdx.y; r0 < rows; r0 += gridDim.y * (kTy * kRows)) {
+    for (unsigned r0 = blockIdx.y * (kTy * kRows) + threadIdx.y; r0 < rows; r0 += gridDim.y * (kTy * kRows)) {
         uint4 a[kRows];
 #pragma unroll
         for (int k = 0; k < kRows; ++k) {
-            const int r = r0 + k * kTy;
+            const unsigned r = r0 + k * kTy;
             const int c = lead(dst + (size_t)r * dp) + 16 * v;
             a[k] = make_uint4(0u, 0u, 0u, 0u);
             if (r < rows && c < cols) a[k] = load16<false>(src + (size_t)r * sp + c, src, end);
         }
 #pragma unroll
         for (int k = 0; k < kRows; ++k) {
-            const int r = r0 + k * kTy;
+            const unsigned r = r0 + k * kTy;
             if (r >= rows) continue;
             uint8_t* row = dst + (size_t)r * dp;
             const int c = lead(row) + 16 * v;
@@ -127,7 +133,8 @@ k_copy_cells(const uint8_t* src, size_t sp, int rows, int cols, uint8_t* dst, si
 struct GridRows {
     const void* inner;  // cell (0, 0): byte frame (16-byte aligned rows) or word frame
     size_t pitch;       // bytes or words
-    int n, rows;
+    int n;
+    unsigned rows;
 };
 
 __device__ __forceinline__ void keep_cells(uint4& v, int valid) {
@@ -148,11 +155,11 @@ __global__ void __launch_bounds__(kTx * kTy) k_population(GridRows g, unsigned l
     const int v = blockIdx.x * kTx + threadIdx.x;
     const int valid = g.n - kCells * v;
     if (valid > 0) {
-        for (int r0 = blockIdx.y * (kTy * kRows) + threadIdx.y; r0 < g.rows; r0 += gridDim.y * (kTy * kRows)) {
+        for (unsigned r0 = blockIdx.y * (kTy * kRows) + threadIdx.y; r0 < g.rows; r0 += gridDim.y * (kTy * kRows)) {
             uint32_t cnt = 0;
 #pragma unroll
             for (int k = 0; k < kRows; ++k) {
-                const int r = r0 + k * kTy;
+                const unsigned r = r0 + k * kTy;
                 if (r >= g.rows) continue;
                 if constexpr (kWords) {
                     uint32_t w = __ldg((const uint32_t*)g.inner + (size_t)r * g.pitch + v);
@@ -181,11 +188,11 @@ k_compare(GridRows g, const uint8_t* __restrict__ other, size_t op, unsigned lon
     const int valid = g.n - 16 * v;
     if (valid > 0) {
         const uint8_t* end = other + (size_t)(g.rows - 1) * op + g.n;
-        for (int r0 = blockIdx.y * (kTy * kRows) + threadIdx.y; r0 < g.rows; r0 += gridDim.y * (kTy * kRows)) {
+        for (unsigned r0 = blockIdx.y * (kTy * kRows) + threadIdx.y; r0 < g.rows; r0 += gridDim.y * (kTy * kRows)) {
             uint4 a[kRows], b[kRows];
 #pragma unroll
             for (int k = 0; k < kRows; ++k) {
-                const int r = r0 + k * kTy;
+                const unsigned r = r0 + k * kTy;
                 a[k] = b[k] = make_uint4(0u, 0u, 0u, 0u);
                 if (r >= g.rows) continue;
                 if constexpr (kWords) {
@@ -226,24 +233,24 @@ k_compare(GridRows g, const uint8_t* __restrict__ other, size_t op, unsigned lon
 // Inner words of a packed frame -> PACK-coded rows (uint64 word k of a row =
 // frame words 2k and 2k + 1), bits past n cleared.  Thread = one frame word.
 __global__ void __launch_bounds__(kTx * kTy)
-k_words_to_pack(const uint32_t* __restrict__ src, size_t sp, int rows, int n, uint32_t* __restrict__ dst, size_t dp,
+k_words_to_pack(const uint32_t* __restrict__ src, size_t sp, unsigned rows, int n, uint32_t* __restrict__ dst, size_t dp,
                 int nwords) {
     const int w = blockIdx.x * kTx + threadIdx.x;
     if (w >= nwords) return;
     const int valid = n - 32 * w;
     const uint32_t mask = valid >= 32 ? 0xffffffffu : (valid > 0 ? (1u << valid) - 1u : 0u);
-    for (int r = blockIdx.y * kTy + threadIdx.y; r < rows; r += gridDim.y * kTy)
+    for (unsigned r = blockIdx.y * kTy + threadIdx.y; r < rows; r += gridDim.y * kTy)
         dst[(size_t)r * dp + w] = valid > 0 ? __ldg(src + (size_t)r * sp + w) & mask : 0u;
 }
 
 // The other way, last words joined (kJoin).
 template <bool kJoin>
 __global__ void __launch_bounds__(kTx * kTy)
-k_pack_to_words(const uint32_t* __restrict__ src, size_t sp, int rows, int n, uint32_t* __restrict__ dst, size_t dp,
+k_pack_to_words(const uint32_t* __restrict__ src, size_t sp, unsigned rows, int n, uint32_t* __restrict__ dst, size_t dp,
                 int nwords) {
     const int w = blockIdx.x * kTx + threadIdx.x;
     if (w >= nwords) return;
-    for (int r = blockIdx.y * kTy + threadIdx.y; r < rows; r += gridDim.y * kTy) {
+    for (unsigned r = blockIdx.y * kTy + threadIdx.y; r < rows; r += gridDim.y * kTy) {
         uint32_t v = __ldg(src + (size_t)r * sp + w);
         if (kJoin && w == nwords - 1) v = join_word(v, __ldg(src + (size_t)r * sp), n);
         dst[(size_t)r * dp + w] = v;
@@ -263,24 +270,24 @@ const dim3 kBlock(kTx, kTy);
 constexpr long long kReduceBlocks = 148 * 16;
 
 GridRows byte_rows(const Frame& f) {
-    return GridRows{f.base + (size_t)f.H * f.pitch + f.H, f.pitch, f.n, f.nrows()};
+    return GridRows{f.base + (size_t)f.H * f.pitch + f.H, f.pitch, f.n, (unsigned)f.nrows()};
 }
 uint32_t* word_origin(const PackedFrame& f) { return f.words + (size_t)f.HR * f.wpitch + f.HW; }
-GridRows word_rows(const PackedFrame& f) { return GridRows{word_origin(f), f.wpitch, f.n, f.nrows()}; }
+GridRows word_rows(const PackedFrame& f) { return GridRows{word_origin(f), f.wpitch, f.n, (unsigned)f.nrows()}; }
 
 }  // namespace
 
 // --- byte buffers <-> byte frames -------------------------------------------
 cudaError_t launch_copy_in(const Frame& f, const uint8_t* src, size_t src_pitch, cudaStream_t s) {
     const int rows = f.nrows();
-    k_copy_cells<true><<<cover((f.n + 15) / 16 + 1, rows, kRows), kBlock, 0, s>>>(src, src_pitch, rows, f.n,
+    k_copy_cells<true><<<cover(vectors(f.n), rows, kRows), kBlock, 0, s>>>(src, src_pitch, rows, f.n,
                                                                                  f.inner(0, 0), f.pitch);
     return cudaGetLastError();
 }
 
 cudaError_t launch_copy_out(const Frame& f, uint8_t* dst, size_t dst_pitch, cudaStream_t s) {
     const int rows = f.nrows();
-    k_copy_cells<false><<<cover((f.n + 15) / 16 + 1, rows, kRows), kBlock, 0, s>>>(f.cinner(0, 0), f.pitch, rows, f.n,
+    k_copy_cells<false><<<cover(vectors(f.n), rows, kRows), kBlock, 0, s>>>(f.cinner(0, 0), f.pitch, rows, f.n,
                                                                                   dst, dst_pitch);
     return cudaGetLastError();
 }
@@ -302,7 +309,7 @@ cudaError_t launch_pack_rows(const uint8_t* src, size_t pitch, bool nonzero, con
 cudaError_t launch_unpack_rows(const PackedFrame& src, int row0, int nrows, uint8_t* dst, size_t pitch,
                                cudaStream_t s) {
     if (nrows <= 0) return cudaSuccess;
-    k_words_to_cells<<<cover((src.n + 15) / 16 + 1, nrows, kRows), kBlock, 0, s>>>(
+    k_words_to_cells<<<cover(vectors(src.n), nrows, kRows), kBlock, 0, s>>>(
         word_origin(src) + (size_t)row0 * src.wpitch, src.wpitch, src.nw, nrows, src.n, dst, pitch);
     return cudaGetLastError();
 }
@@ -320,7 +327,7 @@ cudaError_t launch_pack(const uint8_t* cells, size_t cell_pitch, int rows, int c
 cudaError_t launch_unpack(const uint64_t* words, size_t word_pitch_words, int rows, int cols, uint8_t* cells,
                           size_t cell_pitch, cudaStream_t s) {
     if (rows == 0 || cols == 0) return cudaSuccess;
-    k_words_to_cells<<<cover((cols + 15) / 16 + 1, rows, kRows), kBlock, 0, s>>>(
+    k_words_to_cells<<<cover(vectors(cols), rows, kRows), kBlock, 0, s>>>(
         (const uint32_t*)words, 2 * word_pitch_words, 2 * ((cols + 63) / 64), rows, cols, cells, cell_pitch);
     return cudaGetLastError();
 }

@@ -89,3 +89,36 @@ def test_batch_transfers():
         g = rng.integers(0, 2, size=(n, n + 5), dtype=np.uint8)
         b.upload(k, np.ascontiguousarray(g[:, :n]))
         assert np.array_equal(b.download(k), g[:, :n]), n
+
+
+@pytest.mark.parametrize("rows,cols", [(2**31 - 1, 1), (2**31 - 2**21 + 7, 3), (1, 2**31 - 64), (2, 2**31 - 600)])
+def test_codec_at_the_ends_of_its_range(rows, cols):
+    """As many rows, and as many cells in a row, as the arguments can say."""
+    import torch
+    import cat_cpu_b200 as C
+    L = C.lib()
+    nw = (cols + 63) // 64
+    cells = torch.zeros(rows * cols, dtype=torch.uint8, device="cuda")
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(cols)
+    for r0 in range(0, rows * cols, 2**28):
+        part = cells[r0:r0 + 2**28]
+        part.copy_(torch.randint(0, 2, part.shape, generator=gen, dtype=torch.uint8, device="cuda"))
+    words = torch.full((rows * nw,), -1, dtype=torch.int64, device="cuda")
+    torch.cuda.synchronize()
+    C.ltl.check(L.ltl_pack_device(_ptr(cells), cols, rows, cols, _ptr(words), 8 * nw, None))
+    torch.cuda.synchronize()
+    if rows > cols:  # a word per row
+        want = sum(cells.view(rows, cols)[:, j].to(torch.int64) << j for j in range(cols))
+        assert torch.equal(words, want)
+        del want
+    else:
+        bits = words.view(torch.uint8).view(rows, 8 * nw)
+        for b in range(8):  # bit b of byte k is cell 8 k + b
+            w = cells.view(rows, cols)[:, b::8]
+            assert torch.equal((bits[:, :w.shape[1]] >> b) & 1, w), b
+    back = torch.full_like(cells, 9)
+    torch.cuda.synchronize()
+    C.ltl.check(L.ltl_unpack_device(_ptr(words), 8 * nw, rows, cols, _ptr(back), cols, None))
+    torch.cuda.synchronize()
+    assert torch.equal(back, cells)
