@@ -681,7 +681,10 @@ extern "C" int ltl_step(ltl_ctx* c, int steps) {
     }
     int passes = steps / c->depth;
     const int rest = steps % c->depth;  // a last, shorter pass
-    while (!c->timing && passes >= kGraphPasses) {
+    // in a caller's capture the passes become nodes of the caller's graph, however many
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (!c->timing && passes >= kGraphPasses) LTL_CUDA(cudaStreamIsCapturing(c->stream, &capture));
+    while (!c->timing && capture == cudaStreamCaptureStatusNone && passes >= kGraphPasses) {
         int which = c->cur_is_a ? 0 : 1;
         if (!c->graph[which]) {
             if (int r = build_graph(c, which)) return r;

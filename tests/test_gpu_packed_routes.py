@@ -123,3 +123,33 @@ def test_short_bands_vs_long_bands_and_plain(n, radius):
     assert int(got[0].sum()) > 0
     assert torch.equal(got[0], got[1])
     assert torch.equal(got[0], got[2])
+
+
+@pytest.mark.parametrize("variant,n,radius,steps", [(-1, 700, 17, 10), (-1, 7000, 5, 14), (0, 1000, 5, 22), (0, 300, 1, 23),
+                                                    (1, 5200, 5, 16), (2, 700, 20, 8)])
+def test_captured_steps_of_many_passes(variant, n, radius, steps):
+    """As many passes in one captured call as the solver otherwise replays from a
+    graph of its own, also where it has made that graph before."""
+    import torch
+    import cat_cpu_b200 as C
+    rule = rule_of(radius)
+    g = (np.random.default_rng(n).random((n, n)) < 0.45).astype(np.uint8)
+    stream = torch.cuda.Stream()
+    with C.CUDASolver(n, radius, rule, variant=variant) as s, C.CUDASolver(n, radius, rule, variant=0) as one:
+        one.set_param("depth", 1)
+        one.setState(g)
+        one.doSteps(2 * steps)
+        want = one.getCurrentState()
+        s.set_stream(stream.cuda_stream)
+        for before in (0, 48):
+            s.doSteps(before)
+            s.setState(g)
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=stream):
+                s.doSteps(steps)
+                s.doSteps(steps)
+            with torch.cuda.stream(stream):
+                graph.replay()
+            torch.cuda.synchronize()
+            assert np.array_equal(s.getCurrentState(), want), before
+            del graph
