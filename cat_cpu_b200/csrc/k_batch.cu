@@ -511,6 +511,16 @@ static void batch_release(ltl_batch* b) {
 
 static uint32_t* cur_arena(ltl_batch* b);
 
+// A device copy of a table (allocated here).  Tables, and the words that a launch expects
+// to be zero, are written in the batch's own stream: that one waits for no other, so a
+// legacy-stream copy or memset could still be outstanding at the first launch.
+template <class T>
+static int to_device(ltl_batch* b, T** dst, const std::vector<T>& src) {
+    BATCH_CUDA(cudaMalloc(dst, sizeof(T) * src.size()));
+    BATCH_CUDA(cudaMemcpyAsync(*dst, src.data(), sizeof(T) * src.size(), cudaMemcpyHostToDevice, b->stream));
+    return LTL_OK;
+}
+
 // Work plan: which grids are resident, and the streamed work lists.  Rebuilt
 // when a shape parameter changes (the arenas' layout does not depend on it).
 static int batch_plan(ltl_batch* b) {
@@ -560,11 +570,10 @@ static int batch_plan(ltl_batch* b) {
         first.resize(b->persist_ctas, BatchGroup{0, 0, 0});
         b->n_order = (int)order.size();
         order.resize(count);  // (never empty)
-        BATCH_CUDA(cudaMalloc(&b->d_order, sizeof(int) * count));
-        BATCH_CUDA(cudaMemcpy(b->d_order, order.data(), sizeof(int) * count, cudaMemcpyHostToDevice));
-        BATCH_CUDA(cudaMalloc(&b->d_first, sizeof(BatchGroup) * first.size()));
-        BATCH_CUDA(cudaMemcpy(b->d_first, first.data(), sizeof(BatchGroup) * first.size(), cudaMemcpyHostToDevice));
-        BATCH_CUDA(cudaMemset(b->d_barriers, 0, sizeof(GridBarrier) * count));
+        if (int r = to_device(b, &b->d_order, order)) return r;
+        if (int r = to_device(b, &b->d_first, first)) return r;
+        BATCH_CUDA(cudaMemsetAsync(b->d_barriers, 0, sizeof(GridBarrier) * count, b->stream));
+        BATCH_CUDA(cudaStreamSynchronize(b->stream));
         return LTL_OK;
     }
     for (int i = 0; i < count; ++i) {
@@ -586,9 +595,7 @@ static int batch_plan(ltl_batch* b) {
         if (!c.streamed.empty()) BATCH_CUDA(batch_step_prepare_dispatch(c.rule.radius));
     for (auto& c : b->classes) {
         if (!c.resident.empty()) {
-            BATCH_CUDA(cudaMalloc(&c.d_resident, sizeof(int) * c.resident.size()));
-            BATCH_CUDA(cudaMemcpy(c.d_resident, c.resident.data(), sizeof(int) * c.resident.size(),
-                                  cudaMemcpyHostToDevice));
+            if (int r = to_device(b, &c.d_resident, c.resident)) return r;
         }
         std::vector<int4> items;
         for (int gi : c.streamed) {
@@ -600,10 +607,10 @@ static int batch_plan(ltl_batch* b) {
         }
         c.n_items = (int)items.size();
         if (!items.empty()) {
-            BATCH_CUDA(cudaMalloc(&c.d_items, sizeof(int4) * items.size()));
-            BATCH_CUDA(cudaMemcpy(c.d_items, items.data(), sizeof(int4) * items.size(), cudaMemcpyHostToDevice));
+            if (int r = to_device(b, &c.d_items, items)) return r;
         }
     }
+    BATCH_CUDA(cudaStreamSynchronize(b->stream));
     return LTL_OK;
 }
 
@@ -650,19 +657,17 @@ static int batch_build(ltl_batch* b, int flags) {
     b->persistent = !(flags & LTL_BATCH_STREAM_ALL) && tuning_lookup("batch", -1, 0, "persistent", 1) != 0;
     BATCH_CUDA(cudaMalloc(&b->d_next, sizeof(int)));
     BATCH_CUDA(cudaMalloc(&b->d_err, sizeof(unsigned int)));
-    BATCH_CUDA(cudaMemset(b->d_err, 0, sizeof(unsigned int)));
+    BATCH_CUDA(cudaMemsetAsync(b->d_err, 0, sizeof(unsigned int), b->stream));
     BATCH_CUDA(cudaMalloc(&b->d_barriers, sizeof(GridBarrier) * count));
     {
         std::vector<PackedRule> rules;
         for (auto& c : b->classes) rules.push_back(c.pr);
-        BATCH_CUDA(cudaMalloc(&b->d_rules, sizeof(PackedRule) * rules.size()));
-        BATCH_CUDA(cudaMemcpy(b->d_rules, rules.data(), sizeof(PackedRule) * rules.size(), cudaMemcpyHostToDevice));
+        if (int r = to_device(b, &b->d_rules, rules)) return r;
     }
-    BATCH_CUDA(cudaMalloc(&b->d_grids, sizeof(BatchGrid) * count));
-    BATCH_CUDA(cudaMemcpy(b->d_grids, b->grids.data(), sizeof(BatchGrid) * count, cudaMemcpyHostToDevice));
+    if (int r = to_device(b, &b->d_grids, b->grids)) return r;
     for (auto& a : b->arena) {
         BATCH_CUDA(cudaMalloc(&a, b->arena_words * sizeof(uint32_t)));
-        BATCH_CUDA(cudaMemset(a, 0, b->arena_words * sizeof(uint32_t)));
+        BATCH_CUDA(cudaMemsetAsync(a, 0, b->arena_words * sizeof(uint32_t), b->stream));
     }
     BATCH_CUDA(cudaMalloc(&b->staging, (size_t)std::max<long long>(cells, 1)));
     return batch_plan(b);
@@ -780,8 +785,9 @@ static int check_groups(ltl_batch* b) {
     BATCH_CUDA(cudaMemcpy(&flag, b->d_err, sizeof(flag), cudaMemcpyDeviceToHost));
     b->unchecked = false;
     if (!flag) return LTL_OK;
-    BATCH_CUDA(cudaMemset(b->d_err, 0, sizeof(flag)));
-    BATCH_CUDA(cudaMemset(b->d_barriers, 0, sizeof(GridBarrier) * b->grids.size()));
+    BATCH_CUDA(cudaMemsetAsync(b->d_err, 0, sizeof(flag), b->stream));
+    BATCH_CUDA(cudaMemsetAsync(b->d_barriers, 0, sizeof(GridBarrier) * b->grids.size(), b->stream));
+    BATCH_CUDA(cudaStreamSynchronize(b->stream));
     ltl_set_error("batch kernel reported a bounded-wait timeout; the grids are unspecified until the next upload");
     return LTL_ETIMEOUT;
 }

@@ -1112,8 +1112,8 @@ static bool tensor_geometry(int R, bool fast_ok, TensorGeometry& G) {
     return false;
 }
 
-TensorPlan* tensor_plan_create(const PackedFrame& a, const PackedFrame& b, const Rule& rule, int device, char* why,
-                               size_t why_len) {
+TensorPlan* tensor_plan_create(const PackedFrame& a, const PackedFrame& b, const Rule& rule, int device,
+                               GridBarrier* barrier, unsigned int* err, char* why, size_t why_len) {
     if (!tensor_supported(a.n, rule.radius, why, why_len)) return nullptr;
     int major = 0;
     cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device);
@@ -1178,19 +1178,9 @@ TensorPlan* tensor_plan_create(const PackedFrame& a, const PackedFrame& b, const
         q.hiH0 = hiH_d * bcast;
         q.dhi = hiH_s - hiH_d;
     }
-    // error word, then the barrier
-    unsigned long long* words = nullptr;
-    if (cudaMalloc(&words, 2 * sizeof(unsigned long long)) != cudaSuccess) {
-        snprintf(why, why_len, "error-flag allocation failed");
-        delete P;
-        return nullptr;
-    }
-    cudaMemset(words, 0, 2 * sizeof(unsigned long long));
-    P->err = (unsigned int*)words;
-    P->barrier = (GridBarrier*)(words + 1);
     for (auto& q : P->prm) {
-        q.err = P->err;
-        q.barrier = P->barrier;
+        q.err = err;
+        q.barrier = barrier;
         q.steps = 1;
         q.wait_ns = kWaitLimitNs;
         q.inject_missing_commit = 0;
@@ -1200,7 +1190,6 @@ TensorPlan* tensor_plan_create(const PackedFrame& a, const PackedFrame& b, const
     P->run = pick_kernel<true>(G.mode, form, G.ng);
     if (!P->kernel) {
         snprintf(why, why_len, "no kernel instantiation for R=%d", R);
-        cudaFree(P->err);
         delete P;
         return nullptr;
     }
@@ -1217,18 +1206,13 @@ TensorPlan* tensor_plan_create(const PackedFrame& a, const PackedFrame& b, const
         ae = cudaFuncSetAttribute(P->run, cudaFuncAttributeMaxDynamicSharedMemorySize, P->smem_bytes);
     if (ae != cudaSuccess) {
         snprintf(why, why_len, "cannot reserve %d bytes of shared memory", P->smem_bytes);
-        cudaFree(P->err);
         delete P;
         return nullptr;
     }
     return P;
 }
 
-void tensor_plan_destroy(TensorPlan* p) {
-    if (!p) return;
-    if (p->err) cudaFree(p->err);
-    delete p;
-}
+void tensor_plan_destroy(TensorPlan* p) { delete p; }
 
 int tensor_plan_depth(const TensorPlan*) { return 1; }
 
@@ -1239,13 +1223,8 @@ void tensor_plan_set_wait(TensorPlan* p, unsigned long long ns, int inject_missi
     }
 }
 int tensor_plan_operand_bits(const TensorPlan* p) { return p ? p->operand_bits : 0; }
-unsigned int* tensor_plan_error_flag(TensorPlan* p) { return p ? p->err : nullptr; }
 
 bool tensor_plan_runs(const TensorPlan* p) { return p->runs; }
-
-cudaError_t tensor_plan_reset(TensorPlan* p) {
-    return cudaMemset(p->err, 0, 2 * sizeof(unsigned long long));  // error word and barrier
-}
 
 cudaError_t launch_tensor_steps(TensorPlan* p, bool src_is_a, int steps, cudaStream_t s) {
     TcParams q = p->prm[src_is_a ? 0 : 1];

@@ -63,7 +63,7 @@ struct ltl_ctx {
     PackedFrame pa{}, pb{};
     size_t pwords_bytes = 0;
     bool runs = false;          // packed, small grid: many generations per launch
-    PackedRun run{};            // barrier and error word of those launches
+    PackedRun run{};            // barrier and error word of the launches whose CTAs wait (also the tensor step's)
     bool run_unchecked = false; // such a launch was made since its error word was last read
     uint8_t* bstage = nullptr;  // dense byte staging of the plain variant (made on first use)
     // PACK-coded staging rows of ltl_upload_packed / ltl_download_packed (made on first use)
@@ -273,7 +273,7 @@ static int create_impl(ltl_ctx** out, int device, int rows, int n, int radius, i
         }
     }
     if (variant == LTL_VARIANT_TENSOR) {
-        c->tplan = tensor_plan_create(c->pa, c->pb, c->rule, device, why, sizeof(why));
+        c->tplan = tensor_plan_create(c->pa, c->pb, c->rule, device, c->run.barrier, c->run.err, why, sizeof(why));
         if (!c->tplan) {
             ltl_set_error("ltl_create: tensor plan: %s", why);
             release(c);
@@ -698,30 +698,28 @@ extern "C" int ltl_step(ltl_ctx* c, int steps) {
     return LTL_OK;
 }
 
+// After a wait ran out (the stream is idle): zeroes the error word and the barrier, which
+// is at some count in between, in the stream that the next launch goes to.
+static int reset_waits(ltl_ctx* c) {
+    LTL_CUDA(cudaMemsetAsync(c->scratch + 4, 0, 2 * sizeof(unsigned long long), c->stream));
+    LTL_CUDA(cudaStreamSynchronize(c->stream));
+    return LTL_OK;
+}
+
 extern "C" int ltl_synchronize(ltl_ctx* c) {
     if (int r = check_ctx(c)) return r;
     LTL_CUDA(cudaSetDevice(c->device));
     LTL_CUDA(cudaStreamSynchronize(c->stream));
-    if (c->run_unchecked) {
+    if (c->run_unchecked || c->tplan) {
         unsigned int flag = 0;
         LTL_CUDA(cudaMemcpy(&flag, c->run.err, sizeof(flag), cudaMemcpyDeviceToHost));
         c->run_unchecked = false;
         if (flag) {
-            LTL_CUDA(cudaMemset(c->scratch + 4, 0, 2 * sizeof(unsigned long long)));
-            ltl_set_error("packed kernel reported a bounded-wait timeout; the grid state is unspecified until the "
-                          "next upload");
-            return LTL_ETIMEOUT;
-        }
-    }
-    if (c->tplan) {
-        unsigned int flag = 0;
-        LTL_CUDA(cudaMemcpy(&flag, tensor_plan_error_flag(c->tplan), sizeof(flag), cudaMemcpyDeviceToHost));
-        if (flag) {
-            // clear it, so that the context stays usable after the caller re-uploads a state
-            tensor_plan_reset(c->tplan);
-            ltl_set_error("tensor kernel reported a bounded-wait timeout (flag 0x%x); the grid state is "
-                          "unspecified until the next upload",
-                          flag);
+            // the context stays usable after the caller re-uploads a state
+            if (int r = reset_waits(c)) return r;
+            ltl_set_error("%s kernel reported a bounded-wait timeout (flag 0x%x); the grid state is unspecified until "
+                          "the next upload",
+                          c->tplan ? "tensor" : "packed", flag);
             return LTL_ETIMEOUT;
         }
     }

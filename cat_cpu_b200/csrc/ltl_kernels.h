@@ -113,8 +113,10 @@ cudaError_t launch_compare(const PackedFrame& f, const uint8_t* other, size_t ot
 // itself, so the packed halo is never read).  The frames need HW >= 1.
 struct TensorPlan;
 bool tensor_supported(int n, int radius, char* why, size_t why_len);
-TensorPlan* tensor_plan_create(const PackedFrame& a, const PackedFrame& b, const Rule& rule, int device, char* why,
-                               size_t why_len);
+// barrier, err: device words, zero before the plan's first launch; err is set when a
+// wait runs out, and both have to be zeroed then.
+TensorPlan* tensor_plan_create(const PackedFrame& a, const PackedFrame& b, const Rule& rule, int device,
+                               GridBarrier* barrier, unsigned int* err, char* why, size_t why_len);
 void tensor_plan_destroy(TensorPlan* p);
 int tensor_plan_depth(const TensorPlan* p);
 int tensor_plan_operand_bits(const TensorPlan* p);
@@ -122,9 +124,6 @@ int tensor_plan_operand_bits(const TensorPlan* p);
 // (steps > 1 only where tensor_plan_runs).
 bool tensor_plan_runs(const TensorPlan* p);
 cudaError_t launch_tensor_steps(TensorPlan* p, bool src_is_a, int steps, cudaStream_t s);
-// After a launch that set the error flag: clears it and the generations' barrier.
-cudaError_t tensor_plan_reset(TensorPlan* p);
-unsigned int* tensor_plan_error_flag(TensorPlan* p);
 // Limit of the kernel's bounded waits, and a test hook that withholds one
 // completion signal so that the waits run out (no fault, no hang: the kernel
 // returns after the limit with an error bit set).
