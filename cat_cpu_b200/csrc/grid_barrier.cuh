@@ -4,6 +4,8 @@
 
 #include <cstdint>
 
+#include "ltl_kernels.h"
+
 namespace ltl {
 
 // State of a barrier in device memory.  `arrived` only ever grows: it is a
@@ -14,17 +16,18 @@ struct GridBarrier {
     unsigned long long arrived;
 };
 
-constexpr unsigned long long kBarrierLimitNs = 2000000000ull;  // far above any generation's time
-
 // One CTA's view.  All threads of the CTA call wait(); it returns false once the
 // wait has run out (the CTA should then return: the others will run out too), and
-// sets *err.
+// sets *err.  That word stays set until the host has read it; the barrier is at some
+// count in between then, and has to be zeroed before the next launch that uses it.
 struct GridBarrierWait {
     unsigned long long* arrived;
     unsigned long long target;
+    unsigned long long limit_ns;
     unsigned int ctas;
 
-    __device__ __forceinline__ GridBarrierWait(GridBarrier* b, unsigned int ctas_) : arrived(&b->arrived), ctas(ctas_) {
+    __device__ __forceinline__ GridBarrierWait(GridBarrier* b, unsigned int ctas_, const BarrierLimit& limit)
+        : arrived(&b->arrived), limit_ns(limit.ns), ctas(ctas_ > 1 ? ctas_ + limit.missing : 1u) {
         if (threadIdx.x == 0 && ctas > 1) {
             unsigned long long now;
             asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(now) : "l"(arrived) : "memory");
@@ -48,7 +51,7 @@ struct GridBarrierWait {
                     if ((++tries & 1023) == 0) {
                         asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
                         if (t0 == 0) t0 = t;
-                        if (t - t0 > kBarrierLimitNs) {
+                        if (t - t0 > limit_ns) {
                             *(volatile unsigned int*)err = 1u;
                             late = 1;
                             break;

@@ -139,14 +139,21 @@ struct BatchGroup {
     int grid, rank, size;
 };
 
+// The groups' barriers (one per grid), the word set if a wait runs out, the waits' limit.
+struct BatchWaits {
+    GridBarrier* barriers;
+    unsigned int* err;
+    BarrierLimit limit;
+};
+
 // Not inlined: forms and radii that share one function share its registers (255 and
 // spills; one by one they fit the 128 that four CTAs per SM leave).
 template <int R, int W, int EDGE>
 __device__ __noinline__ bool persist_form(const BatchGrid& g, uint32_t* f0, uint32_t* f1, int steps, int rank,
-                                          int size, GridBarrier* barrier, unsigned int* err, const PackedRule& rule,
+                                          int size, const BatchWaits& waits, int grid, const PackedRule& rule,
                                           uint32_t* ring) {
     const PackedRule pr = rule;  // the masks the comparators use, kept in registers
-    GridBarrierWait group(barrier, size);
+    GridBarrierWait group(waits.barriers + grid, size, waits.limit);
     const int lanes = size * kPersistThreads, id = rank * kPersistThreads + threadIdx.x;
     const int groups = (g.nw + W - 1) / W;
     const int bands = min(g.n, max(1, lanes / groups));
@@ -160,7 +167,7 @@ __device__ __noinline__ bool persist_form(const BatchGrid& g, uint32_t* f0, uint
             packed_walk<R, W, true, EDGE, false>(src, dst, g.wp, g.n, g.nw, g.n, r0, min(r0 + band_rows, g.n),
                                                  W * (it - band * groups), ring, threadIdx.x & 31, pr);
         }
-        if (!group.wait(err)) return false;
+        if (!group.wait(waits.err)) return false;
     }
     return true;
 }
@@ -168,21 +175,21 @@ __device__ __noinline__ bool persist_form(const BatchGrid& g, uint32_t* f0, uint
 // All generations of one grid (radius R) by this CTA, or its part of them.
 template <int R>
 __device__ __forceinline__ bool persist_grid(const BatchGrid& g, uint32_t* a0, uint32_t* a1, int steps, int rank, int size,
-                             GridBarrier* barrier, unsigned int* err, const PackedRule& rule, uint32_t* ring_all) {
+                             const BatchWaits& waits, int grid, const PackedRule& rule, uint32_t* ring_all) {
     constexpr int W = persist_words(R);
     uint32_t* ring = ring_all + (threadIdx.x >> 5) * PackedRing<R, W>::WARP_WORDS;
     uint32_t* f0 = a0 + g.off;
     uint32_t* f1 = a1 + g.off;
-    if (g.n < 64) return persist_form<R, 1, kEdgeTiny>(g, f0, f1, steps, rank, size, barrier, err, rule, ring);
+    if (g.n < 64) return persist_form<R, 1, kEdgeTiny>(g, f0, f1, steps, rank, size, waits, grid, rule, ring);
     if (packed_edge(g.n, W) == kEdgeNone)
-        return persist_form<R, W, kEdgeNone>(g, f0, f1, steps, rank, size, barrier, err, rule, ring);
-    return persist_form<R, W, kEdgeRagged>(g, f0, f1, steps, rank, size, barrier, err, rule, ring);
+        return persist_form<R, W, kEdgeNone>(g, f0, f1, steps, rank, size, waits, grid, rule, ring);
+    return persist_form<R, W, kEdgeRagged>(g, f0, f1, steps, rank, size, waits, grid, rule, ring);
 }
 
 __global__ void __launch_bounds__(kPersistThreads, 4)
 k_batch_persist(uint32_t* a0, uint32_t* a1, const BatchGrid* __restrict__ grids, const PackedRule* __restrict__ rules,
-                const BatchGroup* __restrict__ first, GridBarrier* barriers, const int* __restrict__ order, int n_order,
-                int* next, unsigned int* err, int steps) {
+                const BatchGroup* __restrict__ first, const __grid_constant__ BatchWaits waits,
+                const int* __restrict__ order, int n_order, int* next, int steps) {
     extern __shared__ __align__(16) uint32_t ring_all[];
     __shared__ int s_item;
     BatchGroup task = first[blockIdx.x];
@@ -200,7 +207,7 @@ k_batch_persist(uint32_t* a0, uint32_t* a1, const BatchGrid* __restrict__ grids,
         switch (g.R) {
 #define LTL_C(r)                                                                                                    \
     case r:                                                                                                         \
-        ok = persist_grid<r>(g, a0, a1, steps, task.rank, task.size, barriers + task.grid, err, rules[g.cls],       \
+        ok = persist_grid<r>(g, a0, a1, steps, task.rank, task.size, waits, task.grid, rules[g.cls],       \
                              ring_all);                                                                             \
         break;
             LTL_BATCH_RADII(LTL_C)
@@ -280,8 +287,10 @@ static void batch_split(const std::vector<BatchCost>& grids, int ctas, std::vect
 // (memory-bound like k_transfer.cu's kernels: 16-byte vectors of cells.  A grid's
 // rows are n bytes apart in the staging buffer, so most rows start unaligned.)
 __global__ void k_batch_pack(const uint8_t* __restrict__ cells, uint32_t* __restrict__ arena,
-                             const BatchGrid* __restrict__ grids, int first) {
+                             const BatchGrid* __restrict__ grids, int first, GridBarrier* barriers) {
     const BatchGrid g = grids[first + blockIdx.y];
+    // (a group whose wait ran out leaves its barrier at some count in between)
+    if (blockIdx.x == 0 && threadIdx.x == 0) barriers[first + blockIdx.y].arrived = 0;
     const uint8_t* c = cells + g.cell_off;
     const uint8_t* end = c + (size_t)g.n * g.n;
     for (RowWalk t(blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, g.nw); t.row < g.n; t.next()) {
@@ -468,7 +477,8 @@ struct ltl_batch {
     int persist_ctas = 0;
     size_t persist_smem = 0;
     bool grouped = false;              // some grid has more than one CTA: cooperative launch
-    bool unchecked = false;            // a grouped launch was made since d_err was last read
+    bool waits = false;                // a grouped launch has been made (or captured): d_err is read
+    BarrierLimit limit{};
     cudaStream_t own = nullptr, stream = nullptr, aux = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr;
     // graph cache: (steps, parity) -> exec
@@ -698,6 +708,13 @@ extern "C" int ltl_batch_set_param(ltl_batch* b, const char* name, long long val
             return LTL_EINVAL;
         }
         b->resident_max = value;
+    } else if (std::strcmp(name, "inject_missing_arrival") == 0) {
+        if (value != 0 && (value < 1000000 || value > 10000000000ll)) {
+            ltl_set_error("ltl_batch_set_param: inject_missing_arrival must be 0 or a wait limit in [1e6, 1e10] ns");
+            return LTL_EINVAL;
+        }
+        b->limit = BarrierLimit{};
+        if (value) b->limit = BarrierLimit{(unsigned long long)value, 1u};
     } else {
         ltl_set_error("ltl_batch_set_param: unknown parameter '%s'", name);
         return LTL_EINVAL;
@@ -778,12 +795,13 @@ extern "C" int ltl_batch_set_stream(ltl_batch* b, void* stream) {
 static uint32_t* cur_arena(ltl_batch* b) { return b->arena[b->cur_is_a ? 0 : 1]; }
 static uint32_t* nxt_arena(ltl_batch* b) { return b->arena[b->cur_is_a ? 1 : 0]; }
 
-// After the stream was waited for: did a group's barrier wait run out?
-static int check_groups(ltl_batch* b) {
-    if (!b->unchecked) return LTL_OK;
+// Waits for the stream; did a group's barrier wait run out since this was last asked?
+// (Asked again after every launch and every replay of a caller's graph with one in it, of
+// which the host knows nothing.)
+static int wait_groups(ltl_batch* b) {
     unsigned int flag = 0;
-    BATCH_CUDA(cudaMemcpy(&flag, b->d_err, sizeof(flag), cudaMemcpyDeviceToHost));
-    b->unchecked = false;
+    if (b->waits) BATCH_CUDA(cudaMemcpyAsync(&flag, b->d_err, sizeof(flag), cudaMemcpyDeviceToHost, b->stream));
+    BATCH_CUDA(cudaStreamSynchronize(b->stream));
     if (!flag) return LTL_OK;
     BATCH_CUDA(cudaMemsetAsync(b->d_err, 0, sizeof(flag), b->stream));
     BATCH_CUDA(cudaMemsetAsync(b->d_barriers, 0, sizeof(GridBarrier) * b->grids.size(), b->stream));
@@ -802,7 +820,7 @@ extern "C" int ltl_batch_upload_all(ltl_batch* b, const uint8_t* cells) {
     const int count = (int)b->grids.size();
     for (int first = 0; first < count; first += 65535) {
         dim3 g(16, (unsigned)std::min(65535, count - first));
-        k_batch_pack<<<g, 256, 0, b->stream>>>(b->staging, cur_arena(b), b->d_grids, first);
+        k_batch_pack<<<g, 256, 0, b->stream>>>(b->staging, cur_arena(b), b->d_grids, first, b->d_barriers);
     }
     BATCH_CUDA(cudaGetLastError());
     BATCH_CUDA(cudaStreamSynchronize(b->stream));
@@ -822,8 +840,7 @@ extern "C" int ltl_batch_download_all(ltl_batch* b, uint8_t* cells) {
     }
     BATCH_CUDA(cudaGetLastError());
     BATCH_CUDA(cudaMemcpyAsync(cells, b->staging, (size_t)b->total_cells, cudaMemcpyDeviceToHost, b->stream));
-    BATCH_CUDA(cudaStreamSynchronize(b->stream));
-    return check_groups(b);
+    return wait_groups(b);
 }
 
 extern "C" int ltl_batch_upload(ltl_batch* b, int grid, const uint8_t* inner, size_t pitch) {
@@ -835,7 +852,7 @@ extern "C" int ltl_batch_upload(ltl_batch* b, int grid, const uint8_t* inner, si
     const BatchGrid& g = b->grids[grid];
     BATCH_CUDA(cudaMemcpy2DAsync(b->staging + g.cell_off, g.n, inner, pitch, g.n, g.n, cudaMemcpyHostToDevice,
                                  b->stream));
-    k_batch_pack<<<dim3(16, 1), 256, 0, b->stream>>>(b->staging, cur_arena(b), b->d_grids, grid);
+    k_batch_pack<<<dim3(16, 1), 256, 0, b->stream>>>(b->staging, cur_arena(b), b->d_grids, grid, b->d_barriers);
     BATCH_CUDA(cudaGetLastError());
     BATCH_CUDA(cudaStreamSynchronize(b->stream));
     return LTL_OK;
@@ -852,8 +869,7 @@ extern "C" int ltl_batch_download(ltl_batch* b, int grid, uint8_t* inner, size_t
     BATCH_CUDA(cudaGetLastError());
     BATCH_CUDA(cudaMemcpy2DAsync(inner, pitch, b->staging + g.cell_off, g.n, g.n, g.n, cudaMemcpyDeviceToHost,
                                  b->stream));
-    BATCH_CUDA(cudaStreamSynchronize(b->stream));
-    return check_groups(b);
+    return wait_groups(b);
 }
 
 // Enqueue `steps` generations of every grid (stream-ordered on b->stream).
@@ -878,8 +894,9 @@ static cudaError_t enqueue_steps(ltl_batch* b, int steps, const char** what) {
             cfg.attrs = &at;
             cfg.numAttrs = 1;
             e = cudaLaunchKernelEx(&cfg, k_batch_persist, a0, a1, (const BatchGrid*)b->d_grids,
-                                   (const PackedRule*)b->d_rules, (const BatchGroup*)b->d_first, b->d_barriers,
-                                   (const int*)b->d_order, b->n_order, b->d_next, b->d_err, steps);
+                                   (const PackedRule*)b->d_rules, (const BatchGroup*)b->d_first,
+                                   BatchWaits{b->d_barriers, b->d_err, b->limit}, (const int*)b->d_order, b->n_order,
+                                   b->d_next, steps);
         }
         return e;
     }
@@ -928,7 +945,7 @@ extern "C" int ltl_batch_step(ltl_batch* b, int steps) {
     }
     if (steps == 0) return LTL_OK;
     BATCH_CUDA(cudaSetDevice(b->device));
-    b->unchecked = b->unchecked || (b->persistent && b->grouped);
+    b->waits = b->waits || (b->persistent && b->grouped);
     const char* what = "";
     if (b->no_graph) {
         cudaError_t e = enqueue_steps(b, steps, &what);
@@ -973,8 +990,7 @@ extern "C" int ltl_batch_synchronize(ltl_batch* b) {
         return LTL_EINVAL;
     }
     BATCH_CUDA(cudaSetDevice(b->device));
-    BATCH_CUDA(cudaStreamSynchronize(b->stream));
-    return check_groups(b);
+    return wait_groups(b);
 }
 
 extern "C" int ltl_batch_info(const ltl_batch* b, long long* cells, long long* device_bytes, int* temporal_depth) {

@@ -121,9 +121,9 @@ struct TileSplit {
 template <int R, int EDGE>
 __global__ void __launch_bounds__(kTileThreads, 1)
 k_packed_tiles(uint32_t* a, uint32_t* b, int steps, int wp, int n, int nw, int rows, TileSplit split,
-               GridBarrier* barrier, unsigned int* err, const __grid_constant__ PackedRule pr) {
+               const __grid_constant__ PackedRun run, const __grid_constant__ PackedRule pr) {
     extern __shared__ __align__(16) uint32_t counts[];
-    GridBarrierWait all(barrier, gridDim.x);
+    GridBarrierWait all(run.barrier, gridDim.x, run.limit);
     const int step = kTileThreads / split.tile_words;  // rows of the tile that the CTA's threads take at once
     const int first = threadIdx.x / split.tile_words, col = threadIdx.x - first * split.tile_words;
     const int ty = blockIdx.x / split.tiles_x;
@@ -137,7 +137,7 @@ k_packed_tiles(uint32_t* a, uint32_t* b, int steps, int wp, int n, int nw, int r
         if (works) tile_counts<R, EDGE, false>(cur, wp, n, nw, rows, r0, tr, w0, first, step, counts + col);
         __syncthreads();
         if (works && b0 < tr) tile_rows<R, false>(cur, nxt, wp, r0, b0, min(b0 + band, tr), w0, counts + col, pr);
-        if (s + 1 < steps && !all.wait(err)) return;
+        if (s + 1 < steps && !all.wait(run.err)) return;
     }
 }
 
@@ -150,13 +150,13 @@ k_packed_tiles(uint32_t* a, uint32_t* b, int steps, int wp, int n, int nw, int r
 template <int R, int EDGE>
 __global__ void __launch_bounds__(kTileThreads, 1)
 k_packed_small(uint32_t* a, uint32_t* b, int steps, int blocks, int wp, int n, int nw, int rows, int band_rows,
-               GridBarrier* barrier, unsigned int* err, const __grid_constant__ PackedRule pr) {
+               const __grid_constant__ PackedRun run, const __grid_constant__ PackedRule pr) {
     extern __shared__ __align__(16) uint32_t counts[];
     const bool whole = gridDim.x == 1;
     const int ext_max = whole ? rows : band_rows + 2 * R * ((steps + blocks - 1) / blocks);
     uint32_t* s_in = counts + (size_t)(whole ? rows + 2 * R : ext_max) * PackedTile<R>::ROW;
     uint32_t* s_out = s_in + (size_t)ext_max * kTileStride;
-    GridBarrierWait all(barrier, gridDim.x);
+    GridBarrierWait all(run.barrier, gridDim.x, run.limit);
     const int step = kTileThreads / nw;
     const int first = threadIdx.x / nw, col = threadIdx.x - first * nw;
     const bool works = first < step;
@@ -189,7 +189,7 @@ k_packed_small(uint32_t* a, uint32_t* b, int steps, int blocks, int wp, int n, i
         if (works)
             for (int i = first; i < tr; i += step) nxt[(size_t)(r0 + i) * wp + col] = s_in[(halo + i) * kTileStride + col];
         s += d;
-        if (s < steps && !all.wait(err)) return;
+        if (s < steps && !all.wait(run.err)) return;
         const uint32_t* t = cur;
         cur = nxt;
         nxt = (uint32_t*)t;
@@ -275,8 +275,7 @@ struct TileLaunch {
                            const PackedRun& run, cudaStream_t s) {
         const TileSplit sp = split(c.nrows(), c.nw, sms);
         return launch_group(k_packed_tiles<R, EDGE>, (unsigned)sp.tiles, PackedTile<R>::bytes(sp.tile_rows), steps > 1,
-                            s, c.words, x.words, steps, (int)c.wpitch, c.n, c.nw, c.nrows(), sp, run.barrier,
-                            run.err, pr);
+                            s, c.words, x.words, steps, (int)c.wpitch, c.n, c.nw, c.nrows(), sp, run, pr);
     }
 };
 
@@ -317,7 +316,7 @@ struct SmallLaunch {
         if (ctas == 1) blocks = 1;
         depth = (steps + blocks - 1) / blocks;
         return launch_group(k_packed_small<R, EDGE>, ctas, bytes(rows, tr, depth), blocks > 1, s, c.words, x.words,
-                            steps, blocks, (int)c.wpitch, c.n, c.nw, rows, tr, run.barrier, run.err, pr);
+                            steps, blocks, (int)c.wpitch, c.n, c.nw, rows, tr, run, pr);
     }
 };
 

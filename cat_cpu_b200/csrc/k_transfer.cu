@@ -19,6 +19,7 @@
 // src/CellularAutomata/CADataDomainComparator.tpp:8-27.
 #include <algorithm>
 
+#include "grid_barrier.cuh"
 #include "packed_core.cuh"
 #include "transfer_core.cuh"
 
@@ -31,6 +32,11 @@ constexpr int kTy = 8;     // rows per block pass
 constexpr int kRows = 4;   // rows per thread in flight
 // (Rows are counted unsigned: a grid of blocks may pass the last of 2^31 - 1 rows.)
 
+// A barrier that the grid's launches use, back to zero as the grid comes in.
+__device__ __forceinline__ void reset_barrier(GridBarrier* barrier) {
+    if (barrier && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && threadIdx.y == 0) barrier->arrived = 0;
+}
+
 // 16-byte vectors that a row of cells may touch.
 __host__ __device__ constexpr int vectors(int cols) { return (cols + 15) / 16 + 1; }
 
@@ -40,7 +46,8 @@ __host__ __device__ constexpr int vectors(int cols) { return (cols + 15) / 16 + 
 template <bool kNonzero, bool kJoin>
 __global__ void __launch_bounds__(kTx * kTy)
 k_cells_to_words(const uint8_t* __restrict__ src, size_t sp, unsigned rows, int cols, uint32_t* __restrict__ dst, size_t dp,
-                 int nwords) {
+                 int nwords, GridBarrier* barrier) {
+    reset_barrier(barrier);
     const int w = blockIdx.x * kTx + threadIdx.x;
     if (w >= nwords) return;
     const uint8_t* end = src + (size_t)(rows - 1) * sp + cols;
@@ -247,7 +254,8 @@ k_words_to_pack(const uint32_t* __restrict__ src, size_t sp, unsigned rows, int 
 template <bool kJoin>
 __global__ void __launch_bounds__(kTx * kTy)
 k_pack_to_words(const uint32_t* __restrict__ src, size_t sp, unsigned rows, int n, uint32_t* __restrict__ dst, size_t dp,
-                int nwords) {
+                int nwords, GridBarrier* barrier) {
+    reset_barrier(barrier);
     const int w = blockIdx.x * kTx + threadIdx.x;
     if (w >= nwords) return;
     for (unsigned r = blockIdx.y * kTy + threadIdx.y; r < rows; r += gridDim.y * kTy) {
@@ -296,13 +304,14 @@ cudaError_t launch_binarize(const Frame& f, cudaStream_t s) { return launch_copy
 
 // --- byte buffers <-> packed frames -----------------------------------------
 cudaError_t launch_pack_rows(const uint8_t* src, size_t pitch, bool nonzero, const PackedFrame& dst, int row0,
-                             int nrows, cudaStream_t s) {
+                             int nrows, GridBarrier* barrier, cudaStream_t s) {
     if (nrows <= 0) return cudaSuccess;
     uint32_t* d = word_origin(dst) + (size_t)row0 * dst.wpitch;
     const bool join = dst.n >= 64 && dst.n % 32 != 0;
     auto kernel = nonzero ? (join ? k_cells_to_words<true, true> : k_cells_to_words<true, false>)
                           : (join ? k_cells_to_words<false, true> : k_cells_to_words<false, false>);
-    kernel<<<cover(dst.nw, nrows, kRows), kBlock, 0, s>>>(src, pitch, nrows, dst.n, d, dst.wpitch, dst.nw);
+    kernel<<<cover(dst.nw, nrows, kRows), kBlock, 0, s>>>(src, pitch, nrows, dst.n, d, dst.wpitch, dst.nw,
+                                                              barrier);
     return cudaGetLastError();
 }
 
@@ -320,7 +329,8 @@ cudaError_t launch_pack(const uint8_t* cells, size_t cell_pitch, int rows, int c
     if (rows == 0 || cols == 0) return cudaSuccess;
     const int nwords = 2 * ((cols + 63) / 64);  // 32-bit halves, little-endian
     k_cells_to_words<true, false><<<cover(nwords, rows, kRows), kBlock, 0, s>>>(cells, cell_pitch, rows, cols,
-                                                                       (uint32_t*)words, 2 * word_pitch_words, nwords);
+                                                                       (uint32_t*)words, 2 * word_pitch_words, nwords,
+                                                                       nullptr);
     return cudaGetLastError();
 }
 
@@ -339,11 +349,12 @@ cudaError_t launch_frame_to_pack64(const PackedFrame& f, uint64_t* dst, size_t d
     return cudaGetLastError();
 }
 
-cudaError_t launch_pack64_to_frame(const uint64_t* src, size_t src_pitch_words, const PackedFrame& f, cudaStream_t s) {
+cudaError_t launch_pack64_to_frame(const uint64_t* src, size_t src_pitch_words, const PackedFrame& f,
+                                   GridBarrier* barrier, cudaStream_t s) {
     const int rows = f.nrows();
     auto kernel = f.n >= 64 && f.n % 32 != 0 ? k_pack_to_words<true> : k_pack_to_words<false>;
     kernel<<<cover(f.nw, rows, 1), kBlock, 0, s>>>((const uint32_t*)src, 2 * src_pitch_words, rows, f.n, word_origin(f),
-                                                   f.wpitch, f.nw);
+                                                   f.wpitch, f.nw, barrier);
     return cudaGetLastError();
 }
 

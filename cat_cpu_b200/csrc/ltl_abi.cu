@@ -64,7 +64,6 @@ struct ltl_ctx {
     size_t pwords_bytes = 0;
     bool runs = false;          // packed, small grid: many generations per launch
     PackedRun run{};            // barrier and error word of the launches whose CTAs wait (also the tensor step's)
-    bool run_unchecked = false; // such a launch was made since its error word was last read
     uint8_t* bstage = nullptr;  // dense byte staging of the plain variant (made on first use)
     // PACK-coded staging rows of ltl_upload_packed / ltl_download_packed (made on first use)
     uint64_t* pstage = nullptr;
@@ -119,6 +118,31 @@ static void release(ltl_ctx* c) {
     if (c->bstage) cudaFree(c->bstage);
     if (c->own_stream) cudaStreamDestroy(c->own_stream);
     delete c;
+}
+
+// Solvers with launches whose CTAs wait for one another, or warps for their barriers.
+static bool has_waits(const ltl_ctx* c) { return c->runs || c->tplan; }
+
+// After the stream was waited for: `flag` is the error word.  If a wait ran out, zeroes it
+// and the barrier, in the stream that the next launch goes to.
+static int report_waits(ltl_ctx* c, unsigned int flag) {
+    if (!flag) return LTL_OK;
+    LTL_CUDA(cudaMemsetAsync(c->scratch + 4, 0, 2 * sizeof(unsigned long long), c->stream));
+    LTL_CUDA(cudaStreamSynchronize(c->stream));
+    ltl_set_error("%s kernel reported a bounded-wait timeout (flag 0x%x); the grid state is unspecified until the "
+                  "next upload",
+                  c->tplan ? "tensor" : "packed", flag);
+    return LTL_ETIMEOUT;
+}
+
+// Ends every call that waits for results: waits for the stream and reports a wait that ran
+// out in any launch before, replays of a caller's graph included (so no host flag says
+// whether to look).
+static int finish(ltl_ctx* c) {
+    unsigned int flag = 0;
+    if (has_waits(c)) LTL_CUDA(cudaMemcpyAsync(&flag, c->run.err, sizeof(flag), cudaMemcpyDeviceToHost, c->stream));
+    LTL_CUDA(cudaStreamSynchronize(c->stream));
+    return report_waits(c, flag);
 }
 
 static void drop_graphs(ltl_ctx* c) {
@@ -364,7 +388,7 @@ static int after_upload(ltl_ctx* c) {
 // Cells from a device buffer into the current frame (not 0 -> 1).
 static int take_cells(ltl_ctx* c, const uint8_t* dev, size_t pitch) {
     if (keeps_packed(c))
-        LTL_CUDA(launch_pack_rows(dev, pitch, true, cur_packed(c), 0, c->rows, c->stream));
+        LTL_CUDA(launch_pack_rows(dev, pitch, true, cur_packed(c), 0, c->rows, c->run.barrier, c->stream));
     else
         LTL_CUDA(launch_copy_in(cur_frame(c), dev, pitch, c->stream));
     return after_upload(c);
@@ -439,8 +463,7 @@ extern "C" int ltl_download(ltl_ctx* c, uint8_t* inner, size_t pitch) {
         LTL_CUDA(cudaMemcpy2DAsync(inner, pitch, f.inner(0, 0), f.pitch, c->n, c->rows, cudaMemcpyDeviceToHost,
                                    c->stream));
     }
-    LTL_CUDA(cudaStreamSynchronize(c->stream));
-    return LTL_OK;
+    return finish(c);
 }
 
 // ---------------------------------------------------------------------------
@@ -482,7 +505,7 @@ extern "C" int ltl_upload_packed(ltl_ctx* c, const uint64_t* words, size_t word_
     LTL_CUDA(copy_rows(c->pstage, spitch * 8, words, word_pitch_bytes, spitch * 8, c->rows, cudaMemcpyHostToDevice,
                        c->stream));
     if (keeps_packed(c)) {
-        LTL_CUDA(launch_pack64_to_frame(c->pstage, spitch, cur_packed(c), c->stream));
+        LTL_CUDA(launch_pack64_to_frame(c->pstage, spitch, cur_packed(c), c->run.barrier, c->stream));
     } else {
         Frame& f = cur_frame(c);
         LTL_CUDA(launch_unpack(c->pstage, spitch, c->rows, c->n, f.inner(0, 0), f.pitch, c->stream));
@@ -506,8 +529,7 @@ extern "C" int ltl_download_packed(ltl_ctx* c, uint64_t* words, size_t word_pitc
     }
     LTL_CUDA(copy_rows(words, word_pitch_bytes, c->pstage, spitch * 8, spitch * 8, c->rows, cudaMemcpyDeviceToHost,
                        c->stream));
-    LTL_CUDA(cudaStreamSynchronize(c->stream));
-    return LTL_OK;
+    return finish(c);
 }
 
 extern "C" int ltl_download_device(ltl_ctx* c, uint8_t* dev_inner, size_t pitch) {
@@ -557,7 +579,7 @@ extern "C" int ltl_upload_rows_device(ltl_ctx* c, int row0, int nrows, const uin
     LTL_CUDA(cudaSetDevice(c->device));
     if (keeps_packed(c)) {
         // straight into the packed frame
-        LTL_CUDA(launch_pack_rows(dev, pitch, c->auto_packed, cur_packed(c), row0, nrows, c->stream));
+        LTL_CUDA(launch_pack_rows(dev, pitch, c->auto_packed, cur_packed(c), row0, nrows, nullptr, c->stream));
         return after_upload(c);
     }
     Frame& f = cur_frame(c);
@@ -661,7 +683,6 @@ static cudaError_t enqueue_run(ltl_ctx* c, int steps) {
         e = launch_tensor_steps(c->tplan, c->cur_is_a, steps, c->stream);
     } else {
         e = launch_packed_run(cur_packed(c), nxt_packed(c), c->rule, steps, c->run, c->stream);
-        if (e == cudaSuccess) c->run_unchecked = true;
     }
     if (e == cudaSuccess && steps % 2) c->cur_is_a = !c->cur_is_a;
     return e;
@@ -698,32 +719,10 @@ extern "C" int ltl_step(ltl_ctx* c, int steps) {
     return LTL_OK;
 }
 
-// After a wait ran out (the stream is idle): zeroes the error word and the barrier, which
-// is at some count in between, in the stream that the next launch goes to.
-static int reset_waits(ltl_ctx* c) {
-    LTL_CUDA(cudaMemsetAsync(c->scratch + 4, 0, 2 * sizeof(unsigned long long), c->stream));
-    LTL_CUDA(cudaStreamSynchronize(c->stream));
-    return LTL_OK;
-}
-
 extern "C" int ltl_synchronize(ltl_ctx* c) {
     if (int r = check_ctx(c)) return r;
     LTL_CUDA(cudaSetDevice(c->device));
-    LTL_CUDA(cudaStreamSynchronize(c->stream));
-    if (c->run_unchecked || c->tplan) {
-        unsigned int flag = 0;
-        LTL_CUDA(cudaMemcpy(&flag, c->run.err, sizeof(flag), cudaMemcpyDeviceToHost));
-        c->run_unchecked = false;
-        if (flag) {
-            // the context stays usable after the caller re-uploads a state
-            if (int r = reset_waits(c)) return r;
-            ltl_set_error("%s kernel reported a bounded-wait timeout (flag 0x%x); the grid state is unspecified until "
-                          "the next upload",
-                          c->tplan ? "tensor" : "packed", flag);
-            return LTL_ETIMEOUT;
-        }
-    }
-    return LTL_OK;
+    return finish(c);
 }
 
 extern "C" int ltl_population(ltl_ctx* c, uint64_t* live) {
@@ -735,11 +734,11 @@ extern "C" int ltl_population(ltl_ctx* c, uint64_t* live) {
     LTL_CUDA(cudaSetDevice(c->device));
     LTL_CUDA(keeps_packed(c) ? launch_population(cur_packed(c), c->scratch, c->stream)
                              : launch_population(cur_frame(c), c->scratch, c->stream));
-    unsigned long long v = 0;
-    LTL_CUDA(cudaMemcpyAsync(&v, c->scratch, sizeof(v), cudaMemcpyDeviceToHost, c->stream));
+    unsigned long long v[6];  // with the error word
+    LTL_CUDA(cudaMemcpyAsync(v, c->scratch, sizeof(v), cudaMemcpyDeviceToHost, c->stream));
     LTL_CUDA(cudaStreamSynchronize(c->stream));
-    *live = v;
-    return LTL_OK;
+    *live = v[0];
+    return report_waits(c, (unsigned int)v[5]);
 }
 
 extern "C" int ltl_compare_device(ltl_ctx* c, const uint8_t* dev_expected, size_t pitch, uint64_t* mismatches,
@@ -752,12 +751,12 @@ extern "C" int ltl_compare_device(ltl_ctx* c, const uint8_t* dev_expected, size_
     LTL_CUDA(cudaSetDevice(c->device));
     LTL_CUDA(keeps_packed(c) ? launch_compare(cur_packed(c), dev_expected, pitch, c->scratch, c->stream)
                              : launch_compare(cur_frame(c), dev_expected, pitch, c->scratch, c->stream));
-    unsigned long long v[2] = {0, 0};
+    unsigned long long v[6];  // with the error word
     LTL_CUDA(cudaMemcpyAsync(v, c->scratch, sizeof(v), cudaMemcpyDeviceToHost, c->stream));
     LTL_CUDA(cudaStreamSynchronize(c->stream));
     *mismatches = v[0];
     if (first_index) *first_index = v[0] ? (int64_t)v[1] : -1;
-    return LTL_OK;
+    return report_waits(c, (unsigned int)v[5]);
 }
 
 extern "C" int ltl_pack_device(const uint8_t* dev_cells, size_t cell_pitch, int rows, int cols,
@@ -836,6 +835,19 @@ extern "C" int ltl_set_param(ltl_ctx* c, const char* name, long long value) {
         }
         tensor_plan_set_wait(c->tplan, c->wait_ns, c->inject ? 1 : 0);
         drop_graphs(c);
+        return LTL_OK;
+    }
+    if (std::strcmp(name, "inject_missing_arrival") == 0) {
+        if (c->variant != LTL_VARIANT_PACKED || c->auto_packed) {
+            ltl_set_error("ltl_set_param: %s applies to the packed variant", name);
+            return LTL_EUNSUPPORTED;
+        }
+        if (value != 0 && (value < 1000000 || value > 10000000000ll)) {
+            ltl_set_error("ltl_set_param: inject_missing_arrival must be 0 or a wait limit in [1e6, 1e10] ns");
+            return LTL_EINVAL;
+        }
+        c->run.limit = BarrierLimit{};
+        if (value) c->run.limit = BarrierLimit{(unsigned long long)value, 1u};
         return LTL_OK;
     }
     ltl_set_error("ltl_set_param: unknown parameter '%s'", name);

@@ -9,6 +9,15 @@
 
 namespace ltl {
 
+struct GridBarrier;  // grid_barrier.cuh
+
+// Limit of a barrier wait.  missing = 1: the barrier expects one CTA more than there are,
+// so that every wait runs out (how the failure path is tested).
+struct BarrierLimit {
+    unsigned long long ns = 2000000000ull;  // far above any generation's time
+    unsigned int missing = 0;
+};
+
 // K5: refresh the torus halo of a frame (every halo cell <- its inner source).
 cudaError_t launch_halo_fill(const Frame& f, cudaStream_t s);
 
@@ -67,11 +76,11 @@ cudaError_t launch_packed_step(const PackedFrame& cur, const PackedFrame& nxt, c
 // Grids that are advanced many generations per launch (packed_runs: small ones, by
 // sides and radius alone): `steps` generations from cur, to nxt if `steps` is odd,
 // else back in cur; both frames are written.
-struct GridBarrier;
 struct PackedRun {
     GridBarrier* barrier = nullptr;  // device, zero at first; one per grid, which always has the same CTAs
     unsigned int* err = nullptr;     // device, zero at first; set if a barrier wait ran out: the grid
                                      // is then unspecified and the barrier has to be zeroed
+    BarrierLimit limit{};
 };
 bool packed_runs(const PackedFrame& f, int radius);
 cudaError_t launch_packed_run(const PackedFrame& cur, const PackedFrame& nxt, const Rule& rule, int steps,
@@ -86,14 +95,16 @@ cudaError_t launch_copy_out(const Frame& f, uint8_t* dst, size_t dst_pitch, cuda
 cudaError_t launch_binarize(const Frame& f, cudaStream_t s);
 // Inner rows [row0, row0 + nrows) of a packed frame from / to a buffer whose row
 // i is frame row row0 + i.  nonzero: a cell is alive if its byte is not 0, else
-// by its bit 0.
+// by its bit 0.  barrier (where a whole grid comes in, else null): zeroed, since a run
+// whose wait ran out leaves it at some count in between.
 cudaError_t launch_pack_rows(const uint8_t* src, size_t pitch, bool nonzero, const PackedFrame& dst, int row0,
-                             int nrows, cudaStream_t s);
+                             int nrows, GridBarrier* barrier, cudaStream_t s);
 cudaError_t launch_unpack_rows(const PackedFrame& src, int row0, int nrows, uint8_t* dst, size_t pitch, cudaStream_t s);
 // A packed frame's inner words as PACK-coded rows (bits past n cleared).
 cudaError_t launch_frame_to_pack64(const PackedFrame& f, uint64_t* dst, size_t dst_pitch_words, cudaStream_t s);
-// PACK-coded rows into a packed frame.
-cudaError_t launch_pack64_to_frame(const uint64_t* src, size_t src_pitch_words, const PackedFrame& f, cudaStream_t s);
+// PACK-coded rows into a packed frame (barrier as in launch_pack_rows).
+cudaError_t launch_pack64_to_frame(const uint64_t* src, size_t src_pitch_words, const PackedFrame& f,
+                                   GridBarrier* barrier, cudaStream_t s);
 // PACK codec on callers' buffers (not 0 -> 1).
 cudaError_t launch_pack(const uint8_t* cells, size_t cell_pitch, int rows, int cols, uint64_t* words,
                         size_t word_pitch_words, cudaStream_t s);

@@ -122,7 +122,10 @@ int ltl_download_device(ltl_ctx* ctx, uint8_t* dev_inner, size_t pitch);
 /* Advance `steps` generations (asynchronous on the context's stream).
  * Replaces CASolver::doSteps/doStep (CASolver.cpp:15-31): halo fill, step, swap.
  * Small packed and tensor grids run a call's generations in one cooperative launch
- * whose CTAs wait for one another (bounded: ltl_synchronize reports LTL_ETIMEOUT). */
+ * whose CTAs wait for one another.  Every wait is bounded: if one runs out, the next of
+ * ltl_synchronize, ltl_download, ltl_download_packed, ltl_population and
+ * ltl_compare_device returns LTL_ETIMEOUT (once), and the grid is unspecified until
+ * it is uploaded again.  The stream-ordered downloads report nothing themselves. */
 int ltl_step(ltl_ctx* ctx, int steps);
 
 /* Wait for all work queued on the context's stream; reports device-side error flags. */
@@ -196,6 +199,8 @@ int ltl_batch_step(ltl_batch* b, int steps);
  *                         per-generation launches (the two parameters below apply)
  *   "stream_band_rows"    rows per work item of the streamed per-step kernels
  *   "resident_max_bytes"  shared-memory budget deciding which grids stay resident
+ *   "inject_missing_arrival"  0, or the limit in ns (1e6 to 1e10) of the groups' waits,
+ *                         which then all run out (used by the failure-detection test)
  * Setting one rebuilds the work lists before the next step. */
 int ltl_batch_set_param(ltl_batch* b, const char* name, long long value);
 int ltl_batch_synchronize(ltl_batch* b);
@@ -220,7 +225,10 @@ int ltl_batch_info(const ltl_batch* b, long long* cells, long long* device_bytes
  *   "wait_limit_ns"          limit of each wait (default 2e9);
  *   "inject_missing_commit"  1 = withhold one completion signal, so the next
  *                            pass's waits run out and ltl_synchronize returns
- *                            LTL_ETIMEOUT (used by the failure-detection test). */
+ *                            LTL_ETIMEOUT (used by the failure-detection test).
+ * and of the packed variant's launches of many generations:
+ *   "inject_missing_arrival" 0, or the limit in ns (1e6 to 1e10) of waits that then all
+ *                            run out, since the barrier expects a CTA too many. */
 int ltl_set_param(ltl_ctx* ctx, const char* name, long long value);
 
 /* Kernel timing for benchmarks (the reference times whole runs with a
