@@ -147,7 +147,9 @@ enum Bar {
     W_FULL = DRAIN + 2,       // [kWordDepth] packed-word ring slots
     W_EMPTY = W_FULL + kWordDepth,
     GEN_DONE = W_EMPTY + kWordDepth,  // every rule warp has stored its part of a generation
-    NBARS
+    NBARS,
+    GEN_READY = NBARS + 1  // the warps that wait for the other CTAs' generation have seen it (in the
+                           // second half of the 16 bytes that hold the TMEM address)
 };
 
 // Rule lanes and product-2 operand type (the template parameter MODE):
@@ -321,10 +323,11 @@ enum TcForm { kGather = 0, kFast = 1, kFastSeam = 2 };
 // barriers) and the launch itself are paid once.  Only the warps that read the grid
 // first (the loaders, or the unpack warps in kGather) wait between generations, for
 // every CTA's rule warps to have stored the one before: each CTA adds one to a device
-// counter (release) and they poll it (acquire, bounded).  All others run on, and see
-// the new grid through the barriers of the rings; the launch is cooperative.
-// Measured per generation, a launch each / as one launch: 512^2 R = 5 6.4 / 4.5 us,
-// 4096^2 R = 16 15.8 / 14.4; large grids keep single launches (tensor_plan_create).
+// counter (release) and they poll it (acquire, bounded).  They pass that on to the warps
+// that read grid words besides them (centre words, tiles over the seam) through GEN_READY;
+// the rings' own barriers order shared memory alone.  The launch is cooperative.
+// Measured per generation, a launch each / as one launch: 512^2 R = 5 6.4 / 4.2 us,
+// 4096^2 R = 16 15.8 / 14.2; large grids keep single launches (tensor_plan_create).
 class GenWait {
     GridBarrier* bar;
     unsigned long long base;
@@ -338,8 +341,9 @@ public:
             base = now - now % gridDim.x;
         }
     }
-    // the whole warp: generation g may be read
-    __device__ bool wait(int g, int lane, uint64_t limit_ns) {
+    // the whole warp: generation g may be read, by this warp and by those that wait for
+    // phase g - 1 of `ready`
+    __device__ bool wait(int g, int lane, uint64_t limit_ns, uint64_t* ready) {
         bool ok = true;
         if (lane == 0) {
             const unsigned long long target = base + (unsigned long long)g * gridDim.x;
@@ -354,7 +358,10 @@ public:
                 }
             }
         }
-        return __shfl_sync(0xffffffffu, ok, 0);
+        ok = __shfl_sync(0xffffffffu, ok, 0);
+        __syncwarp();  // (the shuffle orders no memory)
+        if (ok && lane == 0) mbar_arrive(ready);
+        return ok;
     }
     static __device__ void arrive(const TcParams& p) {
         asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(&p.barrier->arrived) : "memory");
@@ -411,6 +418,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tensor_step(const __grid_consta
             mbar_init(&bars[W_EMPTY + i], kUnpackWarps);
         }
         mbar_init(&bars[GEN_DONE], kRuleWarps);
+        if constexpr (RUN) mbar_init(&bars[GEN_READY], FAST ? kLoadWarps : kUnpackWarps);
         fence_mbar_init();
     }
     if (warp == 0) tmem_alloc(tmem_slot, kTmemCols);
@@ -579,7 +587,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tensor_step(const __grid_consta
                 if (RUN && c.g != gen) {
                     gen = c.g;
                     src = gen & 1 ? p.dst : p.src;
-                    ok = gens.wait(gen, lane, p.wait_ns);
+                    ok = gens.wait(gen, lane, p.wait_ns, &bars[GEN_READY]);
                     if (!ok) break;
                 }
                 const int slot = c.u & (kWordDepth - 1);
@@ -714,6 +722,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_tensor_step(const __grid_consta
                 // a row of tiles); all others read whole words as ever
                 const int x0 = c.tx * kTc - p.PADC;
                 if (FORM == kFastSeam && (x0 < 0 || x0 + 32 * NG > p.n)) {
+                    if (RUN && c.g > 0) {  // (its words are not those that came through the ring)
+                        ok = __all_sync(0xffffffffu, mbar_wait(&bars[GEN_READY], (uint32_t)((c.g - 1) & 1), p.wait_ns,
+                                                               kSleepNs));
+                        if (!ok) break;
+                    }
                     gather(c);
                     ok = store(c, [&](int g) { return wg[g]; });
                 } else {
@@ -727,7 +740,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tensor_step(const __grid_consta
             for (; c.u < units; c.next(wk)) {
                 if (RUN && c.g != gen) {
                     gen = c.g;
-                    ok = gens.wait(gen, lane, p.wait_ns);
+                    ok = gens.wait(gen, lane, p.wait_ns, &bars[GEN_READY]);
                     if (!ok) break;
                 }
                 gather(c);
@@ -862,8 +875,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_tensor_step(const __grid_consta
             };
             // the centre words (the output words' own cells in the current grid) of
             // the next tile are loaded while this one is processed; those of a
-            // generation's first tile once its counts are there (the grid they come
-            // from is complete by then).  Plain loads: the grid changes under this launch.
+            // generation's first tile once the grid they come from is complete.  Plain
+            // loads: the grid changes under this launch.
             const uint32_t* src = p.src;
             uint32_t* dst = p.dst;
             long long at0 = tiles > 0 ? out_at(c, 0) : -1, at1 = tiles > 0 ? out_at(c, 1) : -1;
@@ -876,9 +889,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_tensor_step(const __grid_consta
             if (!late) load_centre();
             for (int j = 0; j < tiles && ok; ++j) {
                 const int cb = j % kCBufs;
+                if (RUN && late) {
+                    ok = c.g == 0 || wait_all(&bars[GEN_READY], (uint32_t)((c.g - 1) & 1));
+                    if (!ok) break;
+                    load_centre();
+                }
                 ok = wait_all(&bars[C_FULL + cb], (uint32_t)((j / kCBufs) & 1));
                 if (!ok) break;
-                if (RUN && late) load_centre();
                 fence_after();
                 uint32_t acc0, acc1;
                 if constexpr (MODE >= kLanes32) {
@@ -1199,7 +1216,7 @@ TensorPlan* tensor_plan_create(const PackedFrame& a, const PackedFrame& b, const
     P->grid = std::min(P->prm[0].tiles_x * P->prm[0].tiles_y, sms);
     // units of a generation per CTA: with many, the run's longer loops cost more than
     // the launches (16384^2 R = 5 115 us per generation in launches of one, 128 in one
-    // launch; 8192^2 R = 5 33.5 / 34.3; 4096^2 R = 5 12.6 / 11.3, R = 100 33.5 / 32.5)
+    // launch; 8192^2 R = 5 33.5 / 34.3; 4096^2 R = 5 12.6 / 11.5, R = 100 33.5 / 32.5)
     P->runs = (long long)P->prm[0].tiles_x * P->prm[0].tiles_y * G.nb <= 24ll * P->grid;
     cudaError_t ae = cudaFuncSetAttribute(P->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, P->smem_bytes);
     if (ae == cudaSuccess && P->runs)
