@@ -465,11 +465,14 @@ __global__ void __launch_bounds__(kThreads, 1) k_tensor_step(const __grid_consta
             *(uint4*)(bv + (((i >> 3) * 2 + half) * 128 + (i & 7) * 16)) = make_uint4(w[0], w[1], w[2], w[3]);
         }
     }
-    if constexpr (!RUN) chain_wait();  // the prologue above reads nothing of the grid
     fence_proxy_async();
     fence_before();
     __syncthreads();
     fence_after();
+    // The prologue above reads nothing of the grid.  Only now, with the CTA's tensor memory
+    // allocated, may the next launch start: one of its CTAs that came to this SM before the
+    // allocation would take the memory, and wait for this launch, which waits for the memory.
+    if constexpr (!RUN) chain_wait();
     const uint32_t tmem = *tmem_slot;
 
     if (warp < kLoadWarp0) {
@@ -964,6 +967,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_tensor_step(const __grid_consta
 // ---------------------------------------------------------------------------
 using TcKernel = void (*)(TcParams);
 
+// More than half of an SM's 228 KB: a CTA takes all of the SM's tensor memory, and two
+// launches of many generations that shared SMs could each hold it where the other waits
+// for it.  (The registers keep CTAs apart as well, but that is the compiler's choice.)
+constexpr int kSmemFloor = 116 * 1024;
+
 struct TensorPlan {
     TcParams prm[2];  // source frame a -> b, b -> a
     TcKernel kernel, run;  // one generation, many
@@ -1210,7 +1218,8 @@ TensorPlan* tensor_plan_create(const PackedFrame& a, const PackedFrame& b, const
         delete P;
         return nullptr;
     }
-    P->smem_bytes = smem_layout(G.stages, G.ng, G.nb, fast, G.mode, tensor_xt(G.mode, fast, G.ng)).total + 1024;
+    P->smem_bytes = std::max(smem_layout(G.stages, G.ng, G.nb, fast, G.mode, tensor_xt(G.mode, fast, G.ng)).total + 1024,
+                             kSmemFloor);
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     P->grid = std::min(P->prm[0].tiles_x * P->prm[0].tiles_y, sms);

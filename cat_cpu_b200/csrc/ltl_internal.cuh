@@ -104,7 +104,7 @@ __device__ __forceinline__ int wrap_mod(int v, int n) {
 // stream still runs its last CTAs, and waits there for that one's end (chain_wait, before
 // anything of the grid is touched).  Hides the launch and the prologue behind the tail.
 // For kernels of one CTA per SM: the tensor step at 8192^2 R = 5 33.5 -> 32.0 us, 16384^2
-// 115.4 -> 114.3.  Where several CTAs share an SM the early ones crowd the SMs that are
+// 115.4 -> 114.3 (30.3 and 108.2 since it waits after its prologue's block barrier).  Where several CTAs share an SM the early ones crowd the SMs that are
 // done first, and the step is as long as the fullest SM (band walk 16384^2 R = 2 31 ->
 // 43 us, plain R = 64 6001^2 39 -> 50), so those kernels are launched plainly.
 template <class... P, class... A>
