@@ -41,6 +41,7 @@ struct BatchGrid {
 constexpr int kBatchWarps = 4;
 constexpr int kResThreads = 1024;
 constexpr int kResSmemLimit = 220 * 1024;
+constexpr int kBatchMaxRadius = 16;
 
 // ---------------------------------------------------------------------------
 // Per-step kernel for the streamed grids of one rule class.
@@ -389,8 +390,8 @@ static cudaError_t batch_resident_dispatch(int R, const uint32_t* src, uint32_t*
 }
 
 template <int R>
-static cudaError_t prepare_resident_r(size_t smem) {
-    return cudaFuncSetAttribute(k_batch_resident<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+static cudaError_t prepare_resident_r() {
+    return cudaFuncSetAttribute(k_batch_resident<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, kResSmemLimit);
 }
 
 static cudaError_t batch_step_prepare_dispatch(int R) {
@@ -403,10 +404,10 @@ static cudaError_t batch_step_prepare_dispatch(int R) {
     }
 }
 
-static cudaError_t batch_prepare_dispatch(int R, size_t smem) {
+static cudaError_t batch_prepare_dispatch(int R) {
     switch (R) {
 #define LTL_C(r) \
-    case r: return prepare_resident_r<r>(smem);
+    case r: return prepare_resident_r<r>();
         LTL_BATCH_RADII(LTL_C)
 #undef LTL_C
         default: return cudaErrorInvalidValue;
@@ -556,8 +557,10 @@ static int batch_plan(ltl_batch* b) {
     if (b->persistent) {
         size_t smem = 0;
         for (const BatchGrid& g : b->grids) smem = std::max(smem, persist_ring_dispatch(g.R));
-        // always raised: the kernel's own static shared memory counts against the default 48 KiB too
-        BATCH_CUDA(cudaFuncSetAttribute(k_batch_persist, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        // the limit of the kernel, not of this batch: another one's launches need theirs
+        size_t most = 0;
+        for (int r = 1; r <= kBatchMaxRadius; ++r) most = std::max(most, persist_ring_dispatch(r));
+        BATCH_CUDA(cudaFuncSetAttribute(k_batch_persist, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
         int per_sm = 0;
         BATCH_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_persist, kPersistThreads, smem));
         per_sm = std::max(per_sm, 1);
@@ -596,11 +599,8 @@ static int batch_plan(ltl_batch* b) {
             c.streamed.push_back(i);
         }
     }
-    // one shared-memory limit per kernel instantiation (radius): the largest any class of that radius needs
-    std::map<int, size_t> smem_by_radius;
     for (auto& c : b->classes)
-        if (!c.resident.empty()) smem_by_radius[c.rule.radius] = std::max(smem_by_radius[c.rule.radius], c.res_smem);
-    for (auto& kv : smem_by_radius) BATCH_CUDA(batch_prepare_dispatch(kv.first, kv.second));
+        if (!c.resident.empty()) BATCH_CUDA(batch_prepare_dispatch(c.rule.radius));
     for (auto& c : b->classes)
         if (!c.streamed.empty()) BATCH_CUDA(batch_step_prepare_dispatch(c.rule.radius));
     for (auto& c : b->classes) {
@@ -734,7 +734,7 @@ extern "C" int ltl_batch_create(ltl_batch** out, int device, const ltl_grid_desc
             ltl_set_error("ltl_batch_create: grid %d: need n >= radius >= 1 (n=%d, radius=%d)", i, d.n, d.radius);
             return LTL_EINVAL;
         }
-        if (d.radius > 16) {
+        if (d.radius > kBatchMaxRadius) {
             ltl_set_error("ltl_batch_create: grid %d: batched grids support radius <= 16 (got %d)", i, d.radius);
             return LTL_EUNSUPPORTED;
         }

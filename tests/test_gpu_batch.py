@@ -146,3 +146,24 @@ def test_batch_errors():
     with pytest.raises(C.LtlError) as e:
         C.Batch([(4, 5, (1, 2, 3, 4))])
     assert e.value.code == C.ltl.EINVAL
+
+
+@pytest.mark.parametrize("resident", [0, 1])
+def test_batches_of_large_and_small_shared_memory(resident):
+    """A batch that needs little shared memory, made after one that needs much, leaves
+    that one's launches as they were."""
+    import cat_cpu_b200 as C
+    rng = np.random.default_rng(12)
+    made = []
+    for n, r in ((320, 16), (640, 2), (320, 2), (64, 1)):
+        b = C.Batch([(n, r, O.scaled_rule(r))])
+        if resident:
+            b.set_param("persistent", 0)
+            b.set_param("resident_max_bytes", 220 * 1024)
+        g = (rng.random((n, n)) < 0.45).astype(np.uint8)
+        b.upload_all(g.ravel())
+        made.append((b, n, r, g))
+    for b, n, r, g in made:
+        b.step(3)
+        assert np.array_equal(b.download_all().reshape(n, n), O.run(g, r, O.scaled_rule(r), 3)), (n, r)
+        b.close()
