@@ -64,7 +64,6 @@ struct ltl_ctx {
     size_t pwords_bytes = 0;
     bool runs = false;          // packed, small grid: many generations per launch
     PackedRun run{};            // barrier and error word of the launches whose CTAs wait (also the tensor step's)
-    uint8_t* bstage = nullptr;  // dense byte staging of the plain variant (made on first use)
     // PACK-coded staging rows of ltl_upload_packed / ltl_download_packed (made on first use)
     uint64_t* pstage = nullptr;
     // tensor variant
@@ -115,7 +114,6 @@ static void release(ltl_ctx* c) {
     if (c->tplan) tensor_plan_destroy(c->tplan);
     if (c->frames) cudaFree(c->frames);
     if (c->pstage) cudaFree(c->pstage);
-    if (c->bstage) cudaFree(c->bstage);
     if (c->own_stream) cudaStreamDestroy(c->own_stream);
     delete c;
 }
@@ -397,17 +395,12 @@ static int take_cells(ltl_ctx* c, const uint8_t* dev, size_t pitch) {
 // Dense device staging for a host transfer of uint8 cells, or null where the copy
 // engine moves the rows itself: it does so at full speed only where they are dense
 // on both sides or a multiple of 16 bytes (3001^2 cells row by row 1330 us, as one
-// dense copy and a kernel 490).
-static int byte_stage(ltl_ctx* c, size_t host_pitch, uint8_t** stage) {
-    *stage = nullptr;
-    if (host_pitch != (size_t)c->n) return LTL_OK;
-    if (keeps_packed(c)) {
-        *stage = c->frames;  // holds no state, and is larger than the dense grid
-    } else if (c->n % 16 != 0) {
-        if (!c->bstage) LTL_CUDA(cudaMalloc(&c->bstage, (size_t)c->rows * c->n));
-        *stage = c->bstage;
-    }
-    return LTL_OK;
+// dense copy and a kernel 490).  A byte frame that holds no state now, and is larger
+// than the dense grid: transfers need no memory of their own.
+static uint8_t* byte_stage(ltl_ctx* c, size_t host_pitch) {
+    if (host_pitch != (size_t)c->n) return nullptr;
+    if (keeps_packed(c)) return c->frames;
+    return c->n % 16 != 0 ? nxt_frame(c).base : nullptr;
 }
 
 extern "C" int ltl_upload(ltl_ctx* c, const uint8_t* inner, size_t pitch) {
@@ -418,11 +411,14 @@ extern "C" int ltl_upload(ltl_ctx* c, const uint8_t* inner, size_t pitch) {
     }
     LTL_CUDA(cudaSetDevice(c->device));
     Frame& f = cur_frame(c);
-    uint8_t* stage;
-    if (int r = byte_stage(c, pitch, &stage)) return r;
+    uint8_t* const stage = byte_stage(c, pitch);
     if (stage) {
-        LTL_CUDA(cudaMemcpyAsync(stage, inner, (size_t)c->rows * c->n, cudaMemcpyHostToDevice, c->stream));
+        const size_t bytes = (size_t)c->rows * c->n;
+        LTL_CUDA(cudaMemcpyAsync(stage, inner, bytes, cudaMemcpyHostToDevice, c->stream));
         if (int r = take_cells(c, stage, c->n)) return r;
+        // the plain steps read bytes of the frame that no cell is written to (and drop what
+        // comes of them): they may be 0 or 1, the caller's bytes anything
+        if (!keeps_packed(c)) LTL_CUDA(cudaMemsetAsync(stage, 0, bytes, c->stream));
     } else {
         LTL_CUDA(cudaMemcpy2DAsync(f.inner(0, 0), f.pitch, inner, pitch, c->n, c->rows, cudaMemcpyHostToDevice,
                                    c->stream));
@@ -451,8 +447,7 @@ extern "C" int ltl_download(ltl_ctx* c, uint8_t* inner, size_t pitch) {
     }
     LTL_CUDA(cudaSetDevice(c->device));
     Frame& f = cur_frame(c);
-    uint8_t* stage;
-    if (int r = byte_stage(c, pitch, &stage)) return r;
+    uint8_t* const stage = byte_stage(c, pitch);
     if (stage) {
         LTL_CUDA(keeps_packed(c) ? launch_unpack_rows(cur_packed(c), 0, c->rows, stage, c->n, c->stream)
                                  : launch_copy_out(f, stage, c->n, c->stream));
