@@ -64,7 +64,8 @@ struct ltl_ctx {
     size_t pwords_bytes = 0;
     bool runs = false;          // packed, small grid: many generations per launch
     PackedRun run{};            // barrier and error word of the launches whose CTAs wait (also the tensor step's)
-    // PACK-coded staging rows of ltl_upload_packed / ltl_download_packed (made on first use)
+    // the plain variant's PACK-coded staging rows of ltl_upload_packed / ltl_download_packed
+    // (made on first use; the others have a byte frame to spare, see pack_stage)
     uint64_t* pstage = nullptr;
     // tensor variant
     TensorPlan* tplan = nullptr;
@@ -227,12 +228,15 @@ static int create_impl(ltl_ctx** out, int device, int rows, int n, int radius, i
     size_t pitch = pitch_for(n, H);
     size_t frows = (size_t)rows + 2 * H + 1;  // +1 spare row: vector loads may run past the last frame row
     size_t one = round_up(frows * pitch, 4096);
-    c->frames_bytes = 2 * one;
+    // the plain variant's two grids; the others', which are in packed frames, stage host
+    // transfers in one
+    const bool packs = auto_packed || variant != LTL_VARIANT_PLAIN;
+    c->frames_bytes = packs ? one : 2 * one;
     // packed and tensor: both steps wrap rows and words themselves; the packed step
     // wants 16-byte aligned rows without a halo, the tensor step a halo word to exist
     PackedFrame p{};
     size_t pone = 0;
-    if (auto_packed || variant != LTL_VARIANT_PLAIN) {
+    if (packs) {
         p.n = n;
         p.rows = rows;
         p.nw = (n + 31) / 32;
@@ -257,7 +261,7 @@ static int create_impl(ltl_ctx** out, int device, int rows, int n, int radius, i
         return e == cudaErrorMemoryAllocation ? LTL_ENOMEM : LTL_ECUDA;
     }
     c->fa = Frame{c->frames, n, H, pitch, rows};
-    c->fb = Frame{c->frames + one, n, H, pitch, rows};
+    c->fb = Frame{packs ? c->frames : c->frames + one, n, H, pitch, rows};
 
     if (variant == LTL_VARIANT_PLAIN && plain_swar8_supported(radius)) {
         // generations per pass: the tuning table's value, else the built-in choice
@@ -370,7 +374,7 @@ extern "C" int ltl_get_info(const ltl_ctx* c, ltl_info* info) {
 }
 
 // The packed and tensor variants hold the grid in the packed frames only; their
-// byte frames are staging for host transfers.
+// byte frame is staging for host transfers.
 static bool keeps_packed(const ltl_ctx* c) {
     return c->variant == LTL_VARIANT_PACKED || c->variant == LTL_VARIANT_TENSOR;
 }
@@ -479,14 +483,20 @@ static cudaError_t copy_rows(void* dst, size_t dpitch, const void* src, size_t s
     return cudaMemcpy2DAsync(dst, dpitch, src, spitch, width, rows, kind, s);
 }
 
-static int pack_stage(ltl_ctx* c) {
-    if (c->pstage) return LTL_OK;
-    const size_t bytes = (size_t)c->rows * 8 * ((c->n + 63) / 64);
-    cudaError_t e = cudaMalloc(&c->pstage, std::max<size_t>(bytes, 8));
-    if (e != cudaSuccess) {
-        ltl_set_error("packed transfer staging allocation failed: %s", cudaGetErrorString(e));
-        return LTL_ENOMEM;
+static int pack_stage(ltl_ctx* c, uint64_t** stage) {
+    if (keeps_packed(c)) {
+        *stage = (uint64_t*)c->frames;  // (holds no state, and is larger)
+        return LTL_OK;
     }
+    if (!c->pstage) {
+        const size_t bytes = (size_t)c->rows * 8 * ((c->n + 63) / 64);
+        cudaError_t e = cudaMalloc(&c->pstage, std::max<size_t>(bytes, 8));
+        if (e != cudaSuccess) {
+            ltl_set_error("packed transfer staging allocation failed: %s", cudaGetErrorString(e));
+            return LTL_ENOMEM;
+        }
+    }
+    *stage = c->pstage;
     return LTL_OK;
 }
 
@@ -494,16 +504,17 @@ extern "C" int ltl_upload_packed(ltl_ctx* c, const uint64_t* words, size_t word_
     if (int r = check_ctx(c)) return r;
     if (int r = pack_args(c, "ltl_upload_packed", words, word_pitch_bytes)) return r;
     LTL_CUDA(cudaSetDevice(c->device));
-    if (int r = pack_stage(c)) return r;
+    uint64_t* stage;
+    if (int r = pack_stage(c, &stage)) return r;
     const size_t spitch = (size_t)(c->n + 63) / 64;  // words
     // through dense staging: as one copy where the caller's rows are dense too
-    LTL_CUDA(copy_rows(c->pstage, spitch * 8, words, word_pitch_bytes, spitch * 8, c->rows, cudaMemcpyHostToDevice,
+    LTL_CUDA(copy_rows(stage, spitch * 8, words, word_pitch_bytes, spitch * 8, c->rows, cudaMemcpyHostToDevice,
                        c->stream));
     if (keeps_packed(c)) {
-        LTL_CUDA(launch_pack64_to_frame(c->pstage, spitch, cur_packed(c), c->run.barrier, c->stream));
+        LTL_CUDA(launch_pack64_to_frame(stage, spitch, cur_packed(c), c->run.barrier, c->stream));
     } else {
         Frame& f = cur_frame(c);
-        LTL_CUDA(launch_unpack(c->pstage, spitch, c->rows, c->n, f.inner(0, 0), f.pitch, c->stream));
+        LTL_CUDA(launch_unpack(stage, spitch, c->rows, c->n, f.inner(0, 0), f.pitch, c->stream));
     }
     if (int r = after_upload(c)) return r;
     LTL_CUDA(cudaStreamSynchronize(c->stream));
@@ -514,15 +525,16 @@ extern "C" int ltl_download_packed(ltl_ctx* c, uint64_t* words, size_t word_pitc
     if (int r = check_ctx(c)) return r;
     if (int r = pack_args(c, "ltl_download_packed", words, word_pitch_bytes)) return r;
     LTL_CUDA(cudaSetDevice(c->device));
-    if (int r = pack_stage(c)) return r;
+    uint64_t* stage;
+    if (int r = pack_stage(c, &stage)) return r;
     const size_t spitch = (size_t)(c->n + 63) / 64;  // words
     if (keeps_packed(c)) {
-        LTL_CUDA(launch_frame_to_pack64(cur_packed(c), c->pstage, spitch, c->stream));
+        LTL_CUDA(launch_frame_to_pack64(cur_packed(c), stage, spitch, c->stream));
     } else {
         Frame& f = cur_frame(c);
-        LTL_CUDA(launch_pack(f.inner(0, 0), f.pitch, c->rows, c->n, c->pstage, spitch, c->stream));
+        LTL_CUDA(launch_pack(f.inner(0, 0), f.pitch, c->rows, c->n, stage, spitch, c->stream));
     }
-    LTL_CUDA(copy_rows(words, word_pitch_bytes, c->pstage, spitch * 8, spitch * 8, c->rows, cudaMemcpyDeviceToHost,
+    LTL_CUDA(copy_rows(words, word_pitch_bytes, stage, spitch * 8, spitch * 8, c->rows, cudaMemcpyDeviceToHost,
                        c->stream));
     return finish(c);
 }

@@ -19,7 +19,8 @@ def fill_memory():
     return held
 
 
-@pytest.mark.parametrize("variant,n,packed_too", [(0, 16001, False)])
+@pytest.mark.parametrize("variant,n,packed_too", [(0, 16001, False), (2, 16001, True), (-1, 16001, True), (1, 16001, True),
+                                                  (-1, 16384, True)])
 def test_transfers_when_memory_is_taken(variant, n, packed_too):
     """16001^2 cells are 256 MB, in the PACK coding 32 MB."""
     import torch
@@ -56,3 +57,11 @@ def test_transfers_when_memory_is_taken(variant, n, packed_too):
             torch.cuda.empty_cache()
         assert np.array_equal(got[0], g) and np.array_equal(got[1], want[1])
         assert not packed_too or np.array_equal(got[2], C.pack_grid(g))
+
+
+@pytest.mark.parametrize("n,radius", [(64, 1), (1000, 5), (4097, 28), (16384, 5)])
+def test_default_solver_holds_no_more_than_the_plain_one(n, radius):
+    import cat_cpu_b200 as C
+    rule = (2, 3, 3, 3)
+    with C.CUDASolver(n, radius, rule) as s, C.CUDASolver(n, radius, rule, variant=C.VARIANT_PLAIN) as p:
+        assert s.info.device_bytes <= p.info.device_bytes
