@@ -390,28 +390,28 @@ static int device_sms() {
     return sms;
 }
 
-// Attributes of the kernels that a grid's calls may launch (each one costs about
-// 3 us here, so not those of every form).
+// Attributes of the kernel that a grid's calls launch, and of no other: setting one loads
+// the kernel.
 template <int R>
-static cudaError_t prepare_packed_r(const PackedFrame& f, int sms) {
-    cudaError_t e = with_walk<R>(f.n, [](auto l) { return l.prepare(); });
+static cudaError_t prepare_packed_r(const PackedFrame& f, bool walk, int sms) {
+    if (walk) return with_walk<R>(f.n, [](auto l) { return l.prepare(); });
     if constexpr (R <= kTileMaxRadius) {
         const PackedRoute route = packed_route_r<R>(f.nrows(), f.nw, sms);
-        if (e != cudaSuccess || route == kRouteWalk) return e;
+        if (route == kRouteWalk) return cudaErrorInvalidValue;
         switch (packed_edge(f.n, 1)) {
             case kEdgeNone: return prepare_packed_edge<R, kEdgeNone>(route);
             case kEdgeRagged: return prepare_packed_edge<R, kEdgeRagged>(route);
             default: return prepare_packed_edge<R, kEdgeTiny>(route);
         }
     }
-    return e;
+    return cudaErrorInvalidValue;
 }
 
-cudaError_t packed_prepare(const PackedFrame& f, int radius) {
+cudaError_t packed_prepare(const PackedFrame& f, int radius, bool walk) {
     const int sms = device_sms();
     switch (radius) {
 #define LTL_PP(r) \
-    case r: return prepare_packed_r<r>(f, sms);
+    case r: return prepare_packed_r<r>(f, walk, sms);
         LTL_PACKED_RADII(LTL_PP)
 #undef LTL_PP
         default: return cudaSuccess;

@@ -119,6 +119,9 @@ static void release(ltl_ctx* c) {
     delete c;
 }
 
+// Small packed grids, unless the caller set the band walk's shape.
+static bool runs_packed(const ltl_ctx* c) { return c->runs && c->packed_band_rows <= 0; }
+
 // Solvers with launches whose CTAs wait for one another, or warps for their barriers.
 static bool has_waits(const ltl_ctx* c) { return c->runs || c->tplan; }
 
@@ -292,7 +295,7 @@ static int create_impl(ltl_ctx** out, int device, int rows, int n, int radius, i
         c->pa.words = (uint32_t*)(c->frames + c->frames_bytes);
         c->pb.words = (uint32_t*)(c->frames + c->frames_bytes + pone);
         c->runs = variant == LTL_VARIANT_PACKED && packed_runs(p, radius);
-        if (variant == LTL_VARIANT_PACKED && (e = packed_prepare(p, radius)) != cudaSuccess) {
+        if (variant == LTL_VARIANT_PACKED && (e = packed_prepare(p, radius, !runs_packed(c))) != cudaSuccess) {
             ltl_set_error("ltl_create: kernel setup failed: %s", cudaGetErrorString(e));
             release(c);
             return LTL_ECUDA;
@@ -595,9 +598,6 @@ extern "C" int ltl_upload_rows_device(ltl_ctx* c, int row0, int nrows, const uin
     return after_upload(c);
 }
 
-// Small packed grids, unless the caller set the band walk's shape.
-static bool runs_packed(const ltl_ctx* c) { return c->runs && c->packed_band_rows <= 0; }
-
 // One pass = `gens` generations (c->depth, or fewer for the remainder of a
 // step count; only the temporally blocked plain kernel takes more than 1).
 // Leaves the result in nxt and swaps.
@@ -804,8 +804,11 @@ extern "C" int ltl_set_param(ltl_ctx* c, const char* name, long long value) {
         if (c->variant == LTL_VARIANT_PLAIN && plain_swar8_supported(c->rule.radius))
             c->band_rows = value ? (int)value : plain_swar8_band_rows(c->rows, c->n, c->rule.radius, c->depth, c->device);
         else if (c->variant == LTL_VARIANT_PLAIN) c->band_rows = (int)value;
-        else if (c->variant == LTL_VARIANT_PACKED) c->packed_band_rows = (int)value;
-        else {
+        else if (c->variant == LTL_VARIANT_PACKED) {
+            c->packed_band_rows = (int)value;
+            LTL_CUDA(cudaSetDevice(c->device));
+            LTL_CUDA(packed_prepare(c->pa, c->rule.radius, !runs_packed(c)));
+        } else {
             ltl_set_error("ltl_set_param: band_rows applies to the plain and packed variants");
             return LTL_EUNSUPPORTED;
         }

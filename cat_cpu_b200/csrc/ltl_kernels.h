@@ -68,8 +68,9 @@ struct PackedFrame {
     __host__ __device__ int nrows() const { return rows ? rows : n; }
 };
 bool packed_supported(int n, int radius);
-// as plain_prepare, for a grid's frames
-cudaError_t packed_prepare(const PackedFrame& f, int radius);
+// as plain_prepare, for a grid's frames: before the first launch_packed_step (walk) or
+// launch_packed_run
+cudaError_t packed_prepare(const PackedFrame& f, int radius, bool walk);
 // band_rows <= 0: built-in heuristic; > 0: rows per work item (tuning table / ltl_set_param)
 cudaError_t launch_packed_step(const PackedFrame& cur, const PackedFrame& nxt, const Rule& rule, int band_rows,
                                cudaStream_t s);

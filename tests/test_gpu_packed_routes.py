@@ -153,3 +153,18 @@ def test_captured_steps_of_many_passes(variant, n, radius, steps):
             torch.cuda.synchronize()
             assert np.array_equal(s.getCurrentState(), want), before
             del graph
+
+
+@pytest.mark.parametrize("n,radius", [(200, 12), (1000, 12), (1000, 16), (3001, 8)])
+def test_changes_between_the_walk_and_the_runs(n, radius):
+    """A set band height keeps a small grid on the band walk, 0 gives it back."""
+    import cat_cpu_b200 as C
+    rule = rule_of(radius)
+    g = (np.random.default_rng(n).random((n, n)) < 0.45).astype(np.uint8)
+    with C.CUDASolver(n, radius, rule, variant=C.VARIANT_PACKED) as s:
+        s.setState(g)
+        for band in (0, 64, 0, 100):
+            s.set_param("band_rows", band)
+            s.doSteps(9)
+            g = O.run(g, radius, rule, 9)
+            assert np.array_equal(s.getCurrentState(), g), (n, radius, band)
