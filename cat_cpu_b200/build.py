@@ -2,8 +2,8 @@
 
     python -m cat_cpu_b200.build [--force] [--jobs N] [--verbose]
 
-Every .cu / .cpp under cat_cpu_b200/csrc is compiled separately (objects in
-cat_cpu_b200/_build/) and linked into cat_cpu_b200/libltl_b200.so.  Objects are
+Every .cu / .cpp under cat_cpu_b200/csrc is compiled separately (some in parts,
+PARTS below; objects in cat_cpu_b200/_build/) and linked into cat_cpu_b200/libltl_b200.so.  Objects are
 rebuilt when their source or any header under csrc/ or include/ is newer.
 """
 import argparse
@@ -22,6 +22,10 @@ PROG = os.path.join(PKG, "ltl_prog")
 HOST = os.path.join(PKG, "host")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 
+# Sources compiled in parts, each a CUDA module of its own that a program loads when it
+# first uses it: {file: [(part, extra flags)]}.
+PARTS = {"k_packed_radius.cu": [(f"r{r}", [f"-DLTL_RADIUS={r}"]) for r in range(1, 33)]}
+
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-O3", "-lineinfo", "-std=c++17", "-ccbin", "g++", "-Xcompiler", "-fPIC,-O3",
           "--expt-relaxed-constexpr", "-I", os.path.join(ROOT, "include"), "-I", CSRC]
@@ -37,12 +41,13 @@ def headers():
                   glob.glob(os.path.join(ROOT, "include", "*.h")))
 
 
-def _compile(src, force, verbose, extra):
-    obj = os.path.join(BUILD, os.path.basename(src) + ".o")
+def _compile(job, force, verbose, extra):
+    src, part, flags = job
+    obj = os.path.join(BUILD, os.path.basename(src) + (f".{part}" if part else "") + ".o")
     newest_dep = max([os.path.getmtime(src)] + [os.path.getmtime(h) for h in headers()])
     if not force and os.path.exists(obj) and os.path.getmtime(obj) >= newest_dep:
         return obj, None
-    cmd = [NVCC] + ARCH + COMMON + extra + ["-c", src, "-o", obj]
+    cmd = [NVCC] + ARCH + COMMON + flags + extra + ["-c", src, "-o", obj]
     if src.endswith(".cpp"):
         cmd = [NVCC] + COMMON + ["-x", "c++", "-c", src, "-o", obj]
     if verbose:
@@ -58,11 +63,14 @@ def _compile(src, force, verbose, extra):
 def build(force=False, jobs=None, verbose=False, ptxas_verbose=False):
     os.makedirs(BUILD, exist_ok=True)
     extra = ["-Xptxas", "-v"] if ptxas_verbose else []
-    srcs = sources()
-    jobs = jobs or min(len(srcs), os.cpu_count() or 4)
+    # parts last: a whole file takes longer than a part
+    todo = [(s, "", []) for s in sources() if os.path.basename(s) not in PARTS]
+    for s in sources():
+        todo += [(s, part, flags) for part, flags in PARTS.get(os.path.basename(s), [])]
+    jobs = jobs or min(len(todo), os.cpu_count() or 4)
     objs, errors = [], []
     with cf.ThreadPoolExecutor(jobs) as ex:
-        for obj, err in ex.map(lambda s: _compile(s, force, verbose or ptxas_verbose, extra), srcs):
+        for obj, err in ex.map(lambda job: _compile(job, force, verbose or ptxas_verbose, extra), todo):
             objs.append(obj)
             if err:
                 errors.append(err)
