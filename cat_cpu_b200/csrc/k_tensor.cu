@@ -1227,9 +1227,10 @@ TensorPlan* tensor_plan_create(const PackedFrame& a, const PackedFrame& b, const
     // the launches (16384^2 R = 5 115 us per generation in launches of one, 128 in one
     // launch; 8192^2 R = 5 33.5 / 34.3; 4096^2 R = 5 12.6 / 11.5, R = 100 33.5 / 32.5)
     P->runs = (long long)P->prm[0].tiles_x * P->prm[0].tiles_y * G.nb <= 24ll * P->grid;
-    cudaError_t ae = cudaFuncSetAttribute(P->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, P->smem_bytes);
+    // the kernel's limit, not this plan's: plans of other radii launch the same kernel with more
+    cudaError_t ae = cudaFuncSetAttribute(P->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
     if (ae == cudaSuccess && P->runs)
-        ae = cudaFuncSetAttribute(P->run, cudaFuncAttributeMaxDynamicSharedMemorySize, P->smem_bytes);
+        ae = cudaFuncSetAttribute(P->run, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
     if (ae != cudaSuccess) {
         snprintf(why, why_len, "cannot reserve %d bytes of shared memory", P->smem_bytes);
         delete P;

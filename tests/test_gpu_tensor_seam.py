@@ -70,3 +70,24 @@ def test_captured_generations_replay():
         torch.cuda.synchronize()
         assert np.array_equal(s.getCurrentState(), O.run(g, r, rule, 8))
         del graph
+
+
+def test_solvers_of_large_and_small_shared_memory():
+    """Radii that share a kernel and differ in the shared memory they launch it with, made
+    in falling order of that and stepped afterwards."""
+    import cat_cpu_b200 as C
+    rng = np.random.default_rng(7)
+    made = []
+    for n, r in ((700, 48), (700, 33), (700, 17), (700, 127), (700, 113), (512, 90), (300, 90), (640, 32), (500, 80), (500, 49)):
+        N = (2 * r + 1) ** 2
+        rule = (N // 3, N // 2, int(0.4 * N), int(0.46 * N))
+        s = C.CUDASolver(n, r, rule, variant=C.VARIANT_TENSOR)
+        g = (rng.random((n, n)) < 0.45).astype(np.uint8)
+        s.setState(g)
+        made.append((s, n, r, rule, g))
+    for s, n, r, rule, g in made:
+        s.doSteps(3)
+        s.doSteps(1)
+        s.synchronize()
+        assert np.array_equal(s.getCurrentState(), O.run(g, r, rule, 4)), (n, r)
+        s.close()
