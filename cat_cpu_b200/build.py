@@ -25,6 +25,7 @@ NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 # Sources compiled in parts, each a CUDA module of its own that a program loads when it
 # first uses it: {file: [(part, extra flags)]}.
 PARTS = {
+    "k_batch_radius.cu": [(f"r{r}", [f"-DLTL_RADIUS={r}"]) for r in range(1, 17)],
     "k_packed_radius.cu": [(f"r{r}", [f"-DLTL_RADIUS={r}"]) for r in range(1, 33)],
     "k_tensor_set.cu": [(f"{m}_{k}", [f"-DLTL_TENSOR_MODE=k{m}", f"-DLTL_TENSOR_NG={k}"])
                         for m, k in (("Lanes8", 5), ("Lanes16", 5), ("Lanes16", 7), ("Lanes16", 9), ("Lanes16", 11),
