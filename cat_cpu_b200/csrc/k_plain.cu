@@ -279,28 +279,56 @@ bool plain_swar8_supported(int radius) { return radius >= 1 && radius <= 5; }
 // 8192^2 24.8 / 27.5).
 int plain_swar8_depth(int radius) { return radius <= 2 ? 3 : 2; }
 
+// CTAs of the one-generation kernel that an SM holds.
+template <int R>
+static int swar8_resident_r() {
+    int ctas = 0;
+    const int smem = kPlainWarps * kRingRows * 32 * (int)sizeof(uint4);
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, k_plain_swar8<R>, kPlainWarps * 32, smem) != cudaSuccess)
+        ctas = 0;
+    return std::max(ctas, 1);
+}
+static int swar8_resident(int radius) {
+    switch (radius) {
+        case 1: return swar8_resident_r<1>();
+        case 2: return swar8_resident_r<2>();
+        case 3: return swar8_resident_r<3>();
+        case 4: return swar8_resident_r<4>();
+        default: return swar8_resident_r<5>();
+    }
+}
+
 // Rows per band.  All bands of a pass run at once, k CTAs of four warps per SM; a band
 // walks its rows, 2R rows more per further generation of the pass, and a window start.
 // More CTAs per SM slow each other down, fewer walk longer: time of a row at k = 1 .. 4
 // 0.27, 0.36, 0.50, 0.64 us, fitted to R = 5 at depth 2 (1024^2 10.2 us a pass with 16
 // rows, 25.0 with 64; 4096^2 18.4 with 16 rows, 18.6 with 32, 25.4 with 64; 8192^2 49.6
 // with 64, 69 with 16).
+//
+// One generation per pass (single steps, and what a step count leaves over) has three CTAs
+// of its kernel on an SM, and wants whole loads of them: 8192^2 R = 4 49.5, 39.2, 51.6 us at
+// 2, 3 and 4 per SM and 41.2 at 6, 16384^2 R = 1 161, 125, 166 and 125; so 0.32, 0.35 and 0.41
+// us a row at 1 to 3.  Bands of more than 700 rows are halved: 32768^2 R = 1 551 us in one
+// load, 473 in two (24000^2 250 / 252).
 int plain_swar8_band_rows(int rows, int n, int radius, int depth, int device) {
-    static const double row_us[] = {0.27, 0.36, 0.50, 0.64};
+    static const double row_us[] = {0.27, 0.36, 0.50, 0.64}, one_row_us[] = {0.32, 0.35, 0.41};
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     const int strips = (n + kStripOut - 1) / kStripOut;
+    const double* row = depth == 1 ? one_row_us : row_us;
+    const int most = depth == 1 ? std::min(swar8_resident(radius), 3) : 4;
     double best = 0;
     int best_rows = rows;
-    for (int k = 1; k <= 4; ++k) {
+    for (int k = 1; k <= most; ++k) {
         const int bands = std::max(1, sms * k * kPlainWarps / strips);
         const int b = std::max(8, (rows + bands - 1) / bands);
-        const double t = row_us[k - 1] * (b + 2 * radius * (depth - 1) + 0.3 * (2 * radius + 1));
+        const double t = row[k - 1] * (b + 2 * radius * (depth - 1) + 0.3 * (2 * radius + 1));
         if (best == 0 || t < best) {
             best = t;
             best_rows = b;
         }
     }
+    if (depth == 1 && best_rows > 700) best_rows = (best_rows + 1) / 2;
     return std::min(best_rows, std::max(rows, 1));
 }
 

@@ -56,7 +56,8 @@ struct ltl_ctx {
     unsigned long long* scratch = nullptr;
     cudaStream_t own_stream = nullptr;
     cudaStream_t stream = nullptr;
-    int band_rows = 64;         // plain: rows per work item
+    int band_rows = 0;          // plain: rows per work item (0: built-in choice)
+    int swar_bands[4] = {};     // plain R <= 5: that choice, by generations per pass
     bool plain_wrap = false;    // plain R <= 5: kernels apply the torus wrap, no halo refresh
     int packed_band_rows = 0;   // packed: rows per work item (0: heuristic)
     // packed and tensor variants: the grid lives in packed frames between steps
@@ -271,7 +272,6 @@ static int create_impl(ltl_ctx** out, int device, int rows, int n, int radius, i
         const int want = (int)tuning_lookup("plain", radius, n, "depth", plain_swar8_depth(radius));
         if (want > 1 && plain_tb_supported(radius, want) && H >= want * radius) depth = want;
         c->band_rows = (int)tuning_lookup("plain", radius, n, "band_rows", 0);
-        if (c->band_rows <= 0) c->band_rows = plain_swar8_band_rows(rows, n, radius, depth, device);
         c->plain_wrap = plain_wrap_supported(n, rows);
     } else if (variant == LTL_VARIANT_PLAIN) {
         c->band_rows = (int)tuning_lookup("plain", radius, n, "band_rows", 0);  // 0: the launcher's choice
@@ -284,6 +284,8 @@ static int create_impl(ltl_ctx** out, int device, int rows, int n, int radius, i
     c->variant = variant;
     if (variant == LTL_VARIANT_PACKED) c->packed_band_rows = (int)tuning_lookup("packed", radius, n, "band_rows", 0);
     if (variant == LTL_VARIANT_PLAIN) e = plain_prepare(radius);
+    if (variant == LTL_VARIANT_PLAIN && e == cudaSuccess && plain_swar8_supported(radius))
+        for (int d = 1; d <= 3; ++d) c->swar_bands[d] = plain_swar8_band_rows(rows, n, radius, d, device);
     if (variant == LTL_VARIANT_PLAIN && e == cudaSuccess) e = plain_tb_prepare(radius);
     if (e != cudaSuccess) {
         ltl_set_error("ltl_create: kernel setup failed: %s", cudaGetErrorString(e));
@@ -615,11 +617,12 @@ static cudaError_t enqueue_pass(ltl_ctx* c, int gens) {
         case LTL_VARIANT_PLAIN: {
             Frame& a = cur_frame(c);
             Frame& b = nxt_frame(c);
+            const int band = c->band_rows > 0 ? c->band_rows : c->swar_bands[gens];
             if (gens > 1) {
-                e = launch_plain_tb(a, b, c->rule, c->band_rows, gens, c->plain_wrap, c->stream);
+                e = launch_plain_tb(a, b, c->rule, band, gens, c->plain_wrap, c->stream);
                 step_kernels = 1;
             } else if (plain_swar8_supported(c->rule.radius)) {
-                e = launch_plain_swar8(a, b, c->rule, c->band_rows, c->plain_wrap, c->stream);
+                e = launch_plain_swar8(a, b, c->rule, band, c->plain_wrap, c->stream);
                 step_kernels = 1;
             } else {
                 e = launch_plain_generic(a, b, c->rule, c->band_rows, c->stream);
@@ -801,9 +804,7 @@ extern "C" int ltl_set_param(ltl_ctx* c, const char* name, long long value) {
             return LTL_EINVAL;
         }
         if (c->auto_packed) return LTL_OK;  // a shape of the plain kernels, which do not run
-        if (c->variant == LTL_VARIANT_PLAIN && plain_swar8_supported(c->rule.radius))
-            c->band_rows = value ? (int)value : plain_swar8_band_rows(c->rows, c->n, c->rule.radius, c->depth, c->device);
-        else if (c->variant == LTL_VARIANT_PLAIN) c->band_rows = (int)value;
+        if (c->variant == LTL_VARIANT_PLAIN) c->band_rows = (int)value;
         else if (c->variant == LTL_VARIANT_PACKED) {
             c->packed_band_rows = (int)value;
             LTL_CUDA(cudaSetDevice(c->device));
