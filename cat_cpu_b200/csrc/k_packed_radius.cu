@@ -41,6 +41,20 @@ constexpr int packed_words(int R, bool ragged) { return R <= (ragged ? 10 : 16) 
 // again is cheaper (16384^2 R = 32 216 us against 340 with one, R = 24 226 against 144).
 template <int R>
 constexpr bool packed_ring() { return R <= 28; }
+// From R = 19 on the ring leaves one CTA per SM, whose four warps are too few to wait for
+// memory: beyond the L2, and on rows with ragged lanes from half that size, large grids
+// do without (us, ring / none: 32768^2 R = 20 868 / 617, R = 28 883 / 721; 33000^2 R = 20
+// 1191 / 688; 20032^2 R = 28 303 / 281; 18496^2 R = 20 186 / 194, R = 28 201 / 235; 14001^2
+// R = 19 153 / 129, R = 28 171 / 168; 12001^2 R = 19 113 / 99, R = 28 126 / 131).
+constexpr bool packed_far_ringless(int R) { return R >= 19 && R <= 28; }
+
+// Both frames of a grid against eighths of the L2.
+static bool packed_beyond_l2(const PackedFrame& f, int eighths = 6) {  // (a rest of them stays in it)
+    int dev = 0, l2 = 126 << 20;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev);
+    return 8ll * f.nrows() * f.wpitch > l2 / 8 * (long long)eighths;
+}
 
 // Rows in flight per lane: two where few warps share an SM (the larger rings) and the
 // lane has no ragged words besides (16384^2 R = 8 58.9 -> 55.9, R = 12 72.7 -> 67.6, R = 5
@@ -198,9 +212,8 @@ k_packed_small(uint32_t* a, uint32_t* b, int steps, int blocks, int wp, int n, i
     }
 }
 
-template <int R, int W, int EDGE>
+template <int R, int W, int EDGE, bool kRing = packed_ring<R>()>
 struct PackedLaunch {
-    static constexpr bool kRing = packed_ring<R>();
     static constexpr int smem = kRing ? kPackedWarps * PackedRing<R, W>::WARP_WORDS * 4 : 0;
 
     static cudaError_t prepare() {
@@ -209,15 +222,13 @@ struct PackedLaunch {
     }
     template <class K>
     static PackedSplit split(K kernel, const PackedFrame& c, int band_rows, unsigned& ctas) {
-        int dev = 0, sms = 148, l2 = 126 << 20, per_sm = 0;
+        int dev = 0, sms = 148, per_sm = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kPackedWarps * 32, smem);
         const int rows = c.nrows(), groups = (c.nw + W - 1) / W;
-        const bool beyond_l2 = 8ll * rows * c.wpitch > l2 / 4 * 3ll;  // (both frames; a rest stays in it)
         if (band_rows <= 0)
-            band_rows = packed_band_rows(rows, groups, R, EDGE != kEdgeNone, beyond_l2, sms, std::max(per_sm, 1));
+            band_rows = packed_band_rows(rows, groups, R, EDGE != kEdgeNone, packed_beyond_l2(c), sms, std::max(per_sm, 1));
         const int bands = (rows + band_rows - 1) / band_rows;
         const long long items = (long long)groups * bands;
         ctas = (unsigned)((items + kPackedWarps * 32 - 1) / (kPackedWarps * 32));
@@ -320,9 +331,15 @@ struct SmallLaunch {
     }
 };
 
-// f(launcher) of the band walk's form for a side.
+// f(launcher) of the band walk's form for a grid.
 template <int R, class F>
-static cudaError_t with_walk(int n, F f) {
+static cudaError_t with_walk(const PackedFrame& frame, F f) {
+    const int n = frame.n;
+    if constexpr (packed_far_ringless(R)) {
+        const bool whole = packed_edge(n, 1) == kEdgeNone;
+        if (n >= 64 && packed_beyond_l2(frame, whole ? 6 : 3))
+            return whole ? f(PackedLaunch<R, 1, kEdgeNone, false>{}) : f(PackedLaunch<R, 1, kEdgeRagged, false>{});
+    }
     if (n < 64) return f(PackedLaunch<R, 1, kEdgeTiny>{});
     if (packed_edge(n, 2) == kEdgeNone && packed_words(R, false) == 2)
         return f(PackedLaunch<R, packed_words(R, false), kEdgeNone>{});
@@ -334,7 +351,7 @@ static cudaError_t with_walk(int n, F f) {
 template <int R>
 cudaError_t PackedOps<R>::step(const PackedFrame& c, const PackedFrame& x, const PackedRule& pr, int band_rows,
                                cudaStream_t s) {
-    return with_walk<R>(c.n, [&](auto l) { return l.step(c, x, pr, band_rows, s); });
+    return with_walk<R>(c, [&](auto l) { return l.step(c, x, pr, band_rows, s); });
 }
 
 // Which kernel advances a grid, by its words and R.  Measured per generation (us, 48
@@ -392,7 +409,7 @@ bool PackedOps<R>::runs(const PackedFrame& f, int sms) {
 
 template <int R>
 cudaError_t PackedOps<R>::prepare(const PackedFrame& f, bool walk, int sms) {
-    if (walk) return with_walk<R>(f.n, [](auto l) { return l.prepare(); });
+    if (walk) return with_walk<R>(f, [](auto l) { return l.prepare(); });
     if constexpr (R <= kTileMaxRadius) {
         const PackedRoute route = packed_route_r<R>(f.nrows(), f.nw, sms);
         if (route == kRouteWalk) return cudaErrorInvalidValue;

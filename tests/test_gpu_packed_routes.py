@@ -168,3 +168,30 @@ def test_changes_between_the_walk_and_the_runs(n, radius):
             s.doSteps(9)
             g = O.run(g, radius, rule, 9)
             assert np.array_equal(s.getCurrentState(), g), (n, radius, band)
+
+
+@pytest.mark.parametrize("rows,n,radius", [(13000, 15001, 19), (14001, 14001, 28), (19616, 19616, 20), (19616, 19616, 28),
+                                           (1500000, 60, 19)])
+def test_large_grids_without_the_ring_vs_plain(rows, n, radius):
+    """Radii whose ring leaves one CTA per SM, where grids are too large for that; and rows
+    of fewer than 64 cells, which keep it."""
+    import torch
+    import cat_cpu_b200 as C
+    N = (2 * radius + 1) ** 2
+    rule = (int(0.45 * N), N, int(0.45 * N), N)  # above the mean count: domains of both kinds
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(n)
+    g = (torch.rand((rows, n), generator=gen, device="cuda") < 0.45).to(torch.uint8)
+    torch.cuda.synchronize()
+    got = []
+    for variant in (C.VARIANT_PACKED, C.VARIANT_PLAIN):
+        out = torch.empty_like(g)
+        torch.cuda.synchronize()
+        with C.CUDASolver(n, radius, rule, variant=variant, rows=rows) as s:
+            s.upload_device(g.data_ptr(), n)
+            s.doSteps(9)
+            s.download_device(out.data_ptr(), n)
+            s.synchronize()
+        got.append(out)
+    assert 0 < int(got[0].sum()) < rows * n
+    assert torch.equal(got[0], got[1])
