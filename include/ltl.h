@@ -36,8 +36,9 @@ extern "C" {
 
 /* Stepping variants (the GPU analogues of the reference's solver codes,
  * CASolverFactory.cpp:10-119; the reference's own codes 0-6 are CPU solvers). */
-#define LTL_VARIANT_AUTO (-1)  /* the fastest exact kernels for (n, R): bit-packed up to R = 28, else plain;
-                                * ltl_get_info and ltl_set_param treat it as the plain variant */
+#define LTL_VARIANT_AUTO (-1)  /* bit-packed kernels up to R = 23 (to 28 from n = 2048 on where 32 divides
+                                * n), plain ones above; ltl_get_info names it plain either way, and
+                                * ltl_set_param takes the plain variant's parameters */
 #define LTL_VARIANT_PLAIN 0    /* CUDA-core SWAR stencil, uint8 cells */
 #define LTL_VARIANT_TENSOR 1   /* tcgen05 banded products B_v * X * B_h, bit-packed grid */
 #define LTL_VARIANT_PACKED 2   /* bit-packed cells (64 per uint64), CUDA-core bit logic */

@@ -195,3 +195,17 @@ def test_large_grids_without_the_ring_vs_plain(rows, n, radius):
         got.append(out)
     assert 0 < int(got[0].sum()) < rows * n
     assert torch.equal(got[0], got[1])
+
+
+@pytest.mark.parametrize("n,radius", [(2016, 23), (2016, 24), (2048, 24), (2048, 28), (2080, 29), (2049, 28)])
+def test_default_solver_where_it_changes_kernels(n, radius):
+    import cat_cpu_b200 as C
+    rule = rule_of(radius)
+    g = (np.random.default_rng(n + radius).random((n, n)) < 0.45).astype(np.uint8)
+    with C.CUDASolver(n, radius, rule) as s, C.CUDASolver(n, radius, rule, variant=C.VARIANT_PLAIN) as p:
+        for solver in (s, p):
+            solver.setState(g)
+            solver.doSteps(2)
+        assert np.array_equal(s.getCurrentState(), p.getCurrentState())
+        assert s.info.variant == p.info.variant == C.VARIANT_PLAIN
+        assert s.population() == p.population() > 0
