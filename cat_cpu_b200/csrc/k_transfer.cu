@@ -32,6 +32,13 @@ constexpr int kTy = 8;     // rows per block pass
 constexpr int kRows = 4;   // rows per thread in flight
 // (Rows are counted unsigned: a grid of blocks may pass the last of 2^31 - 1 rows.)
 
+// A block's threads along a row and rows: constants, unless rows are narrow (see shape;
+// 16384^2 cells to words and back 113 us with them read from the launch, 107 so).
+template <bool kNarrow>
+__device__ __forceinline__ unsigned tx() { return kNarrow ? blockDim.x : kTx; }
+template <bool kNarrow>
+__device__ __forceinline__ unsigned ty() { return kNarrow ? blockDim.y : kTy; }
+
 // A barrier that the grid's launches use, back to zero as the grid comes in.
 __device__ __forceinline__ void reset_barrier(GridBarrier* barrier) {
     if (barrier && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && threadIdx.y == 0) barrier->arrived = 0;
@@ -43,21 +50,21 @@ __host__ __device__ constexpr int vectors(int cols) { return (cols + 15) / 16 + 
 // Byte rows -> word rows: thread = one 32-bit word of a row, kNonzero: a cell is
 // alive if its byte is not 0 (else by its bit 0).  Words past the cells get 0; bits
 // past them in the last word 0, or the row's first cells (kJoin, cols >= 64).
-template <bool kNonzero, bool kJoin>
+template <bool kNonzero, bool kJoin, bool kNarrow>
 __global__ void __launch_bounds__(kTx * kTy)
 k_cells_to_words(const uint8_t* __restrict__ src, size_t sp, unsigned rows, int cols, uint32_t* __restrict__ dst, size_t dp,
                  int nwords, GridBarrier* barrier) {
     reset_barrier(barrier);
-    const int w = blockIdx.x * kTx + threadIdx.x;
+    const int w = blockIdx.x * tx<kNarrow>() + threadIdx.x;
     if (w >= nwords) return;
     const uint8_t* end = src + (size_t)(rows - 1) * sp + cols;
     const int valid = cols - 32 * w;
     const uint32_t mask = valid >= 32 ? 0xffffffffu : (valid > 0 ? (1u << valid) - 1u : 0u);
-    for (unsigned r0 = blockIdx.y * (kTy * kRows) + threadIdx.y; r0 < rows; r0 += gridDim.y * (kTy * kRows)) {
+    for (unsigned r0 = blockIdx.y * (ty<kNarrow>() * kRows) + threadIdx.y; r0 < rows; r0 += gridDim.y * (ty<kNarrow>() * kRows)) {
         uint4 a[kRows], b[kRows];
 #pragma unroll
         for (int k = 0; k < kRows; ++k) {
-            const unsigned r = r0 + k * kTy;
+            const unsigned r = r0 + k * ty<kNarrow>();
             const uint8_t* p = src + (size_t)r * sp + 32 * (size_t)w;
             a[k] = b[k] = make_uint4(0u, 0u, 0u, 0u);
             if (r < rows && valid > 0) a[k] = load16<true>(p, src, end);
@@ -65,7 +72,7 @@ k_cells_to_words(const uint8_t* __restrict__ src, size_t sp, unsigned rows, int 
         }
 #pragma unroll
         for (int k = 0; k < kRows; ++k) {
-            const unsigned r = r0 + k * kTy;
+            const unsigned r = r0 + k * ty<kNarrow>();
             if (r >= rows) continue;
             uint32_t v = (cells16_to_bits<kNonzero>(a[k]) | (cells16_to_bits<kNonzero>(b[k]) << 16)) & mask;
             if constexpr (kJoin) {
@@ -81,22 +88,23 @@ k_cells_to_words(const uint8_t* __restrict__ src, size_t sp, unsigned rows, int 
 }
 
 // Word rows -> byte rows: thread = one aligned 16-byte vector of the destination.
+template <bool kNarrow>
 __global__ void __launch_bounds__(kTx * kTy)
 k_words_to_cells(const uint32_t* __restrict__ src, size_t sp, int nwords, unsigned rows, int cols, uint8_t* __restrict__ dst,
                  size_t dp) {
-    const int v = blockIdx.x * kTx + threadIdx.x;
+    const int v = blockIdx.x * tx<kNarrow>() + threadIdx.x;
     if (v >= vectors(cols)) return;
-    for (unsigned r0 = blockIdx.y * (kTy * kRows) + threadIdx.y; r0 < rows; r0 += gridDim.y * (kTy * kRows)) {
+    for (unsigned r0 = blockIdx.y * (ty<kNarrow>() * kRows) + threadIdx.y; r0 < rows; r0 += gridDim.y * (ty<kNarrow>() * kRows)) {
         uint32_t bits[kRows];
 #pragma unroll
         for (int k = 0; k < kRows; ++k) {
-            const unsigned r = r0 + k * kTy;
+            const unsigned r = r0 + k * ty<kNarrow>();
             const int c = lead(dst + (size_t)r * dp) + 16 * v;
             bits[k] = r < rows && c < cols ? bits16_at(src + (size_t)r * sp, c, nwords) : 0u;
         }
 #pragma unroll
         for (int k = 0; k < kRows; ++k) {
-            const unsigned r = r0 + k * kTy;
+            const unsigned r = r0 + k * ty<kNarrow>();
             if (r >= rows) continue;
             uint8_t* row = dst + (size_t)r * dp;
             const int c = lead(row) + 16 * v;
@@ -107,24 +115,24 @@ k_words_to_cells(const uint32_t* __restrict__ src, size_t sp, int nwords, unsign
 
 // Byte rows -> byte rows (kNonzero: every byte that is not 0 becomes 1).
 // src == dst is allowed: a thread reads only the vectors it writes.
-template <bool kNonzero>
+template <bool kNonzero, bool kNarrow>
 __global__ void __launch_bounds__(kTx * kTy)
 k_copy_cells(const uint8_t* src, size_t sp, unsigned rows, int cols, uint8_t* dst, size_t dp) {
-    const int v = blockIdx.x * kTx + threadIdx.x;
+    const int v = blockIdx.x * tx<kNarrow>() + threadIdx.x;
     if (v >= vectors(cols)) return;
     const uint8_t* end = src + (size_t)(rows - 1) * sp + cols;
-    for (unsigned r0 = blockIdx.y * (kTy * kRows) + threadIdx.y; r0 < rows; r0 += gridDim.y * (kTy * kRows)) {
+    for (unsigned r0 = blockIdx.y * (ty<kNarrow>() * kRows) + threadIdx.y; r0 < rows; r0 += gridDim.y * (ty<kNarrow>() * kRows)) {
         uint4 a[kRows];
 #pragma unroll
         for (int k = 0; k < kRows; ++k) {
-            const unsigned r = r0 + k * kTy;
+            const unsigned r = r0 + k * ty<kNarrow>();
             const int c = lead(dst + (size_t)r * dp) + 16 * v;
             a[k] = make_uint4(0u, 0u, 0u, 0u);
             if (r < rows && c < cols) a[k] = load16<false>(src + (size_t)r * sp + c, src, end);
         }
 #pragma unroll
         for (int k = 0; k < kRows; ++k) {
-            const unsigned r = r0 + k * kTy;
+            const unsigned r = r0 + k * ty<kNarrow>();
             if (r >= rows) continue;
             uint8_t* row = dst + (size_t)r * dp;
             const int c = lead(row) + 16 * v;
@@ -239,39 +247,64 @@ k_compare(GridRows g, const uint8_t* __restrict__ other, size_t op, unsigned lon
 
 // Inner words of a packed frame -> PACK-coded rows (uint64 word k of a row =
 // frame words 2k and 2k + 1), bits past n cleared.  Thread = one frame word.
+template <bool kNarrow>
 __global__ void __launch_bounds__(kTx * kTy)
 k_words_to_pack(const uint32_t* __restrict__ src, size_t sp, unsigned rows, int n, uint32_t* __restrict__ dst, size_t dp,
                 int nwords) {
-    const int w = blockIdx.x * kTx + threadIdx.x;
+    const int w = blockIdx.x * tx<kNarrow>() + threadIdx.x;
     if (w >= nwords) return;
     const int valid = n - 32 * w;
     const uint32_t mask = valid >= 32 ? 0xffffffffu : (valid > 0 ? (1u << valid) - 1u : 0u);
-    for (unsigned r = blockIdx.y * kTy + threadIdx.y; r < rows; r += gridDim.y * kTy)
+    for (unsigned r = blockIdx.y * ty<kNarrow>() + threadIdx.y; r < rows; r += gridDim.y * ty<kNarrow>())
         dst[(size_t)r * dp + w] = valid > 0 ? __ldg(src + (size_t)r * sp + w) & mask : 0u;
 }
 
 // The other way, last words joined (kJoin).
-template <bool kJoin>
+template <bool kJoin, bool kNarrow>
 __global__ void __launch_bounds__(kTx * kTy)
 k_pack_to_words(const uint32_t* __restrict__ src, size_t sp, unsigned rows, int n, uint32_t* __restrict__ dst, size_t dp,
                 int nwords, GridBarrier* barrier) {
     reset_barrier(barrier);
-    const int w = blockIdx.x * kTx + threadIdx.x;
+    const int w = blockIdx.x * tx<kNarrow>() + threadIdx.x;
     if (w >= nwords) return;
-    for (unsigned r = blockIdx.y * kTy + threadIdx.y; r < rows; r += gridDim.y * kTy) {
+    for (unsigned r = blockIdx.y * ty<kNarrow>() + threadIdx.y; r < rows; r += gridDim.y * ty<kNarrow>()) {
         uint32_t v = __ldg(src + (size_t)r * sp + w);
         if (kJoin && w == nwords - 1) v = join_word(v, __ldg(src + (size_t)r * sp), n);
         dst[(size_t)r * dp + w] = v;
     }
 }
 
-// `items` threads along a row, `rows` rows, `per` rows per thread.  `cap`
-// bounds the blocks of a reduction (each ends in an atomic).
-dim3 cover(long long items, int rows, int per, long long cap = 0) {
+// Grid and block of a kernel without a reduction: `items` threads along a row (a power of
+// two up to kTx, so that rows of a few cells do not leave a warp to one or two threads:
+// 100,000 rows of 3 cells packed 26 us with a warp per row, 10 so), `per` rows per thread.
+struct Shape {
+    dim3 grid, block;
+    bool narrow;
+};
+Shape shape(long long items, int rows, int per) {
+    unsigned tx = kTx;
+    while (tx > 1 && tx / 2 >= items) tx /= 2;
+    const unsigned ty = kTx * kTy / tx;
+    const long long gy = std::max<long long>(1, ((long long)rows + ty * per - 1) / (ty * per));
+    return {dim3((unsigned)std::max<long long>(1, (items + tx - 1) / tx), (unsigned)std::min<long long>(gy, 65535)),
+            dim3(tx, ty), tx < kTx};
+}
+
+// The same for a reduction, whose warps are rows; `cap` bounds its blocks (each ends in an
+// atomic).
+dim3 cover(long long items, int rows, int per, long long cap) {
     const long long gx = std::max<long long>(1, (items + kTx - 1) / kTx);
     long long gy = std::max<long long>(1, ((long long)rows + kTy * per - 1) / (kTy * per));
-    if (cap > 0) gy = std::min(gy, std::max<long long>(1, cap / gx));
+    gy = std::min(gy, std::max<long long>(1, cap / gx));
     return dim3((unsigned)gx, (unsigned)std::min<long long>(gy, 65535));
+}
+
+auto cells_to_words(bool nonzero, bool join, bool narrow) {
+    if (narrow)
+        return nonzero ? (join ? k_cells_to_words<true, true, true> : k_cells_to_words<true, false, true>)
+                       : (join ? k_cells_to_words<false, true, true> : k_cells_to_words<false, false, true>);
+    return nonzero ? (join ? k_cells_to_words<true, true, false> : k_cells_to_words<true, false, false>)
+                   : (join ? k_cells_to_words<false, true, false> : k_cells_to_words<false, false, false>);
 }
 
 const dim3 kBlock(kTx, kTy);
@@ -288,14 +321,16 @@ GridRows word_rows(const PackedFrame& f) { return GridRows{word_origin(f), f.wpi
 // --- byte buffers <-> byte frames -------------------------------------------
 cudaError_t launch_copy_in(const Frame& f, const uint8_t* src, size_t src_pitch, cudaStream_t s) {
     const int rows = f.nrows();
-    k_copy_cells<true><<<cover(vectors(f.n), rows, kRows), kBlock, 0, s>>>(src, src_pitch, rows, f.n,
+    const Shape b = shape(vectors(f.n), rows, kRows);
+    (b.narrow ? k_copy_cells<true, true> : k_copy_cells<true, false>)<<<b.grid, b.block, 0, s>>>(src, src_pitch, rows, f.n,
                                                                                  f.inner(0, 0), f.pitch);
     return cudaGetLastError();
 }
 
 cudaError_t launch_copy_out(const Frame& f, uint8_t* dst, size_t dst_pitch, cudaStream_t s) {
     const int rows = f.nrows();
-    k_copy_cells<false><<<cover(vectors(f.n), rows, kRows), kBlock, 0, s>>>(f.cinner(0, 0), f.pitch, rows, f.n,
+    const Shape b = shape(vectors(f.n), rows, kRows);
+    (b.narrow ? k_copy_cells<false, true> : k_copy_cells<false, false>)<<<b.grid, b.block, 0, s>>>(f.cinner(0, 0), f.pitch, rows, f.n,
                                                                                   dst, dst_pitch);
     return cudaGetLastError();
 }
@@ -308,9 +343,9 @@ cudaError_t launch_pack_rows(const uint8_t* src, size_t pitch, bool nonzero, con
     if (nrows <= 0) return cudaSuccess;
     uint32_t* d = word_origin(dst) + (size_t)row0 * dst.wpitch;
     const bool join = dst.n >= 64 && dst.n % 32 != 0;
-    auto kernel = nonzero ? (join ? k_cells_to_words<true, true> : k_cells_to_words<true, false>)
-                          : (join ? k_cells_to_words<false, true> : k_cells_to_words<false, false>);
-    kernel<<<cover(dst.nw, nrows, kRows), kBlock, 0, s>>>(src, pitch, nrows, dst.n, d, dst.wpitch, dst.nw,
+    const Shape b = shape(dst.nw, nrows, kRows);
+    auto kernel = cells_to_words(nonzero, join, b.narrow);
+    kernel<<<b.grid, b.block, 0, s>>>(src, pitch, nrows, dst.n, d, dst.wpitch, dst.nw,
                                                               barrier);
     return cudaGetLastError();
 }
@@ -318,7 +353,8 @@ cudaError_t launch_pack_rows(const uint8_t* src, size_t pitch, bool nonzero, con
 cudaError_t launch_unpack_rows(const PackedFrame& src, int row0, int nrows, uint8_t* dst, size_t pitch,
                                cudaStream_t s) {
     if (nrows <= 0) return cudaSuccess;
-    k_words_to_cells<<<cover(vectors(src.n), nrows, kRows), kBlock, 0, s>>>(
+    const Shape b = shape(vectors(src.n), nrows, kRows);
+    (b.narrow ? k_words_to_cells<true> : k_words_to_cells<false>)<<<b.grid, b.block, 0, s>>>(
         word_origin(src) + (size_t)row0 * src.wpitch, src.wpitch, src.nw, nrows, src.n, dst, pitch);
     return cudaGetLastError();
 }
@@ -328,7 +364,8 @@ cudaError_t launch_pack(const uint8_t* cells, size_t cell_pitch, int rows, int c
                         size_t word_pitch_words, cudaStream_t s) {
     if (rows == 0 || cols == 0) return cudaSuccess;
     const int nwords = 2 * ((cols + 63) / 64);  // 32-bit halves, little-endian
-    k_cells_to_words<true, false><<<cover(nwords, rows, kRows), kBlock, 0, s>>>(cells, cell_pitch, rows, cols,
+    const Shape b = shape(nwords, rows, kRows);
+    (b.narrow ? k_cells_to_words<true, false, true> : k_cells_to_words<true, false, false>)<<<b.grid, b.block, 0, s>>>(cells, cell_pitch, rows, cols,
                                                                        (uint32_t*)words, 2 * word_pitch_words, nwords,
                                                                        nullptr);
     return cudaGetLastError();
@@ -337,14 +374,16 @@ cudaError_t launch_pack(const uint8_t* cells, size_t cell_pitch, int rows, int c
 cudaError_t launch_unpack(const uint64_t* words, size_t word_pitch_words, int rows, int cols, uint8_t* cells,
                           size_t cell_pitch, cudaStream_t s) {
     if (rows == 0 || cols == 0) return cudaSuccess;
-    k_words_to_cells<<<cover(vectors(cols), rows, kRows), kBlock, 0, s>>>(
+    const Shape b = shape(vectors(cols), rows, kRows);
+    (b.narrow ? k_words_to_cells<true> : k_words_to_cells<false>)<<<b.grid, b.block, 0, s>>>(
         (const uint32_t*)words, 2 * word_pitch_words, 2 * ((cols + 63) / 64), rows, cols, cells, cell_pitch);
     return cudaGetLastError();
 }
 
 cudaError_t launch_frame_to_pack64(const PackedFrame& f, uint64_t* dst, size_t dst_pitch_words, cudaStream_t s) {
     const int rows = f.nrows(), nwords = 2 * ((f.n + 63) / 64);
-    k_words_to_pack<<<cover(nwords, rows, 1), kBlock, 0, s>>>(word_origin(f), f.wpitch, rows, f.n, (uint32_t*)dst,
+    const Shape b = shape(nwords, rows, 1);
+    (b.narrow ? k_words_to_pack<true> : k_words_to_pack<false>)<<<b.grid, b.block, 0, s>>>(word_origin(f), f.wpitch, rows, f.n, (uint32_t*)dst,
                                                              2 * dst_pitch_words, nwords);
     return cudaGetLastError();
 }
@@ -352,8 +391,11 @@ cudaError_t launch_frame_to_pack64(const PackedFrame& f, uint64_t* dst, size_t d
 cudaError_t launch_pack64_to_frame(const uint64_t* src, size_t src_pitch_words, const PackedFrame& f,
                                    GridBarrier* barrier, cudaStream_t s) {
     const int rows = f.nrows();
-    auto kernel = f.n >= 64 && f.n % 32 != 0 ? k_pack_to_words<true> : k_pack_to_words<false>;
-    kernel<<<cover(f.nw, rows, 1), kBlock, 0, s>>>((const uint32_t*)src, 2 * src_pitch_words, rows, f.n, word_origin(f),
+    const Shape b = shape(f.nw, rows, 1);
+    const bool join = f.n >= 64 && f.n % 32 != 0;
+    auto kernel = b.narrow ? (join ? k_pack_to_words<true, true> : k_pack_to_words<false, true>)
+                           : (join ? k_pack_to_words<true, false> : k_pack_to_words<false, false>);
+    kernel<<<b.grid, b.block, 0, s>>>((const uint32_t*)src, 2 * src_pitch_words, rows, f.n, word_origin(f),
                                                    f.wpitch, f.nw, barrier);
     return cudaGetLastError();
 }

@@ -122,3 +122,32 @@ def test_codec_at_the_ends_of_its_range(rows, cols):
     C.ltl.check(L.ltl_unpack_device(_ptr(words), 8 * nw, rows, cols, _ptr(back), cols, None))
     torch.cuda.synchronize()
     assert torch.equal(back, cells)
+
+
+@pytest.mark.parametrize("cols", [1, 3, 15, 17, 40, 65, 130])
+def test_many_narrow_rows(cols):
+    """Rows narrower than a warp: several to a warp, many blocks of them."""
+    import torch
+    import cat_cpu_b200 as C
+    L = C.lib()
+    rows, nw = 100003, (cols + 63) // 64
+    cells = (np.random.default_rng(cols).random((rows, cols)) < 0.5).astype(np.uint8)
+    dev = torch.from_numpy(cells * 3).cuda()
+    words = torch.full((rows, nw), -1, dtype=torch.int64, device="cuda")
+    back = torch.full((rows, cols), 9, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    C.ltl.check(L.ltl_pack_device(_ptr(dev), cols, rows, cols, _ptr(words), 8 * nw, None))
+    C.ltl.check(L.ltl_unpack_device(_ptr(words), 8 * nw, rows, cols, _ptr(back), cols, None))
+    torch.cuda.synchronize()
+    assert np.array_equal(words.cpu().numpy().view(np.uint64), C.pack_grid(cells))
+    assert np.array_equal(back.cpu().numpy(), cells)
+    for variant in (0, 2):  # into frames and out
+        with C.CUDASolver(cols, 1, (2, 3, 3, 3), variant=variant, rows=rows) as s:
+            s.setState(cells)
+            assert np.array_equal(s.getCurrentState(), cells)
+            s.setStatePacked(C.pack_grid(cells))
+            assert np.array_equal(s.getCurrentStatePacked(), C.pack_grid(cells))
+            s.upload_device(dev.data_ptr(), cols)
+            s.download_device(back.data_ptr(), cols)
+            s.synchronize()
+            assert np.array_equal(back.cpu().numpy(), cells)
