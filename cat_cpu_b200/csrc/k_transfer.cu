@@ -44,6 +44,12 @@ __device__ __forceinline__ void reset_barrier(GridBarrier* barrier) {
     if (barrier && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && threadIdx.y == 0) barrier->arrived = 0;
 }
 
+// Rows on their way to the host after a wait may have run out (err: the word that this
+// sets): the first cell, or 32 cells, become a mark, which tells the host to look.
+__device__ __forceinline__ bool marks(const unsigned int* err, unsigned row, int item) {
+    return err && row == 0 && item == 0 && *(const volatile unsigned int*)err != 0u;
+}
+
 // 16-byte vectors that a row of cells may touch.
 __host__ __device__ constexpr int vectors(int cols) { return (cols + 15) / 16 + 1; }
 
@@ -91,7 +97,7 @@ k_cells_to_words(const uint8_t* __restrict__ src, size_t sp, unsigned rows, int 
 template <bool kNarrow>
 __global__ void __launch_bounds__(kTx * kTy)
 k_words_to_cells(const uint32_t* __restrict__ src, size_t sp, int nwords, unsigned rows, int cols, uint8_t* __restrict__ dst,
-                 size_t dp) {
+                 size_t dp, const unsigned int* err) {
     const int v = blockIdx.x * tx<kNarrow>() + threadIdx.x;
     if (v >= vectors(cols)) return;
     for (unsigned r0 = blockIdx.y * (ty<kNarrow>() * kRows) + threadIdx.y; r0 < rows; r0 += gridDim.y * (ty<kNarrow>() * kRows)) {
@@ -109,6 +115,7 @@ k_words_to_cells(const uint32_t* __restrict__ src, size_t sp, int nwords, unsign
             uint8_t* row = dst + (size_t)r * dp;
             const int c = lead(row) + 16 * v;
             if (c < cols) store16<true>(row + c, bits16_to_cells(bits[k]), -c, cols - c);
+            if (marks(err, r, v)) row[0] = kMarkCell;
         }
     }
 }
@@ -250,13 +257,15 @@ k_compare(GridRows g, const uint8_t* __restrict__ other, size_t op, unsigned lon
 template <bool kNarrow>
 __global__ void __launch_bounds__(kTx * kTy)
 k_words_to_pack(const uint32_t* __restrict__ src, size_t sp, unsigned rows, int n, uint32_t* __restrict__ dst, size_t dp,
-                int nwords) {
+                int nwords, const unsigned int* err) {
     const int w = blockIdx.x * tx<kNarrow>() + threadIdx.x;
     if (w >= nwords) return;
     const int valid = n - 32 * w;
     const uint32_t mask = valid >= 32 ? 0xffffffffu : (valid > 0 ? (1u << valid) - 1u : 0u);
     for (unsigned r = blockIdx.y * ty<kNarrow>() + threadIdx.y; r < rows; r += gridDim.y * ty<kNarrow>())
-        dst[(size_t)r * dp + w] = valid > 0 ? __ldg(src + (size_t)r * sp + w) & mask : 0u;
+        dst[(size_t)r * dp + w] = marks(err, r, w) ? kMarkCells
+                                  : valid > 0      ? __ldg(src + (size_t)r * sp + w) & mask
+                                                   : 0u;
 }
 
 // The other way, last words joined (kJoin).
@@ -351,11 +360,11 @@ cudaError_t launch_pack_rows(const uint8_t* src, size_t pitch, bool nonzero, con
 }
 
 cudaError_t launch_unpack_rows(const PackedFrame& src, int row0, int nrows, uint8_t* dst, size_t pitch,
-                               cudaStream_t s) {
+                               const unsigned int* err, cudaStream_t s) {
     if (nrows <= 0) return cudaSuccess;
     const Shape b = shape(vectors(src.n), nrows, kRows);
     (b.narrow ? k_words_to_cells<true> : k_words_to_cells<false>)<<<b.grid, b.block, 0, s>>>(
-        word_origin(src) + (size_t)row0 * src.wpitch, src.wpitch, src.nw, nrows, src.n, dst, pitch);
+        word_origin(src) + (size_t)row0 * src.wpitch, src.wpitch, src.nw, nrows, src.n, dst, pitch, err);
     return cudaGetLastError();
 }
 
@@ -376,15 +385,17 @@ cudaError_t launch_unpack(const uint64_t* words, size_t word_pitch_words, int ro
     if (rows == 0 || cols == 0) return cudaSuccess;
     const Shape b = shape(vectors(cols), rows, kRows);
     (b.narrow ? k_words_to_cells<true> : k_words_to_cells<false>)<<<b.grid, b.block, 0, s>>>(
-        (const uint32_t*)words, 2 * word_pitch_words, 2 * ((cols + 63) / 64), rows, cols, cells, cell_pitch);
+        (const uint32_t*)words, 2 * word_pitch_words, 2 * ((cols + 63) / 64), rows, cols, cells, cell_pitch,
+        nullptr);
     return cudaGetLastError();
 }
 
-cudaError_t launch_frame_to_pack64(const PackedFrame& f, uint64_t* dst, size_t dst_pitch_words, cudaStream_t s) {
+cudaError_t launch_frame_to_pack64(const PackedFrame& f, uint64_t* dst, size_t dst_pitch_words, const unsigned int* err,
+                                   cudaStream_t s) {
     const int rows = f.nrows(), nwords = 2 * ((f.n + 63) / 64);
     const Shape b = shape(nwords, rows, 1);
     (b.narrow ? k_words_to_pack<true> : k_words_to_pack<false>)<<<b.grid, b.block, 0, s>>>(word_origin(f), f.wpitch, rows, f.n, (uint32_t*)dst,
-                                                             2 * dst_pitch_words, nwords);
+                                                             2 * dst_pitch_words, nwords, err);
     return cudaGetLastError();
 }
 

@@ -124,6 +124,7 @@ static bool runs_packed(const ltl_ctx* c) { return c->runs && c->packed_band_row
 
 // Solvers with launches whose CTAs wait for one another, or warps for their barriers.
 static bool has_waits(const ltl_ctx* c) { return c->runs || c->tplan; }
+static const unsigned int* wait_word(const ltl_ctx* c) { return has_waits(c) ? c->run.err : nullptr; }
 
 // After the stream was waited for: `flag` is the error word.  If a wait ran out, zeroes it
 // and the barrier, in the stream that the next launch goes to.
@@ -137,9 +138,10 @@ static int report_waits(ltl_ctx* c, unsigned int flag) {
     return LTL_ETIMEOUT;
 }
 
-// Ends every call that waits for results: waits for the stream and reports a wait that ran
-// out in any launch before, replays of a caller's graph included (so no host flag says
-// whether to look).
+// Waits for the stream and reports a wait that ran out in any launch before, replays of a
+// caller's graph included (so no host flag says whether to look).  Calls that bring results
+// back see the word with these instead, since a copy of four bytes takes 10 us: reductions
+// copy it with their sums, downloads find a mark where the grid begins.
 static int finish(ltl_ctx* c) {
     unsigned int flag = 0;
     if (has_waits(c)) LTL_CUDA(cudaMemcpyAsync(&flag, c->run.err, sizeof(flag), cudaMemcpyDeviceToHost, c->stream));
@@ -466,16 +468,17 @@ extern "C" int ltl_download(ltl_ctx* c, uint8_t* inner, size_t pitch) {
     Frame& f = cur_frame(c);
     uint8_t* const stage = byte_stage(c, pitch);
     if (stage) {
-        LTL_CUDA(keeps_packed(c) ? launch_unpack_rows(cur_packed(c), 0, c->rows, stage, c->n, c->stream)
+        LTL_CUDA(keeps_packed(c) ? launch_unpack_rows(cur_packed(c), 0, c->rows, stage, c->n, wait_word(c), c->stream)
                                  : launch_copy_out(f, stage, c->n, c->stream));
         LTL_CUDA(cudaMemcpyAsync(inner, stage, (size_t)c->rows * c->n, cudaMemcpyDeviceToHost, c->stream));
     } else {
         if (keeps_packed(c))
-            LTL_CUDA(launch_unpack_rows(cur_packed(c), 0, c->rows, f.inner(0, 0), f.pitch, c->stream));
+            LTL_CUDA(launch_unpack_rows(cur_packed(c), 0, c->rows, f.inner(0, 0), f.pitch, wait_word(c), c->stream));
         LTL_CUDA(cudaMemcpy2DAsync(inner, pitch, f.inner(0, 0), f.pitch, c->n, c->rows, cudaMemcpyDeviceToHost,
                                    c->stream));
     }
-    return finish(c);
+    LTL_CUDA(cudaStreamSynchronize(c->stream));
+    return has_waits(c) && inner[0] == kMarkCell ? finish(c) : LTL_OK;
 }
 
 // ---------------------------------------------------------------------------
@@ -542,14 +545,15 @@ extern "C" int ltl_download_packed(ltl_ctx* c, uint64_t* words, size_t word_pitc
     if (int r = pack_stage(c, &stage)) return r;
     const size_t spitch = (size_t)(c->n + 63) / 64;  // words
     if (keeps_packed(c)) {
-        LTL_CUDA(launch_frame_to_pack64(cur_packed(c), stage, spitch, c->stream));
+        LTL_CUDA(launch_frame_to_pack64(cur_packed(c), stage, spitch, wait_word(c), c->stream));
     } else {
         Frame& f = cur_frame(c);
         LTL_CUDA(launch_pack(f.inner(0, 0), f.pitch, c->rows, c->n, stage, spitch, c->stream));
     }
     LTL_CUDA(copy_rows(words, word_pitch_bytes, stage, spitch * 8, spitch * 8, c->rows, cudaMemcpyDeviceToHost,
                        c->stream));
-    return finish(c);
+    LTL_CUDA(cudaStreamSynchronize(c->stream));
+    return has_waits(c) && (uint32_t)words[0] == kMarkCells ? finish(c) : LTL_OK;
 }
 
 extern "C" int ltl_download_device(ltl_ctx* c, uint8_t* dev_inner, size_t pitch) {
@@ -560,7 +564,7 @@ extern "C" int ltl_download_device(ltl_ctx* c, uint8_t* dev_inner, size_t pitch)
     }
     LTL_CUDA(cudaSetDevice(c->device));
     if (keeps_packed(c))
-        LTL_CUDA(launch_unpack_rows(cur_packed(c), 0, c->rows, dev_inner, pitch, c->stream));
+        LTL_CUDA(launch_unpack_rows(cur_packed(c), 0, c->rows, dev_inner, pitch, nullptr, c->stream));
     else
         LTL_CUDA(launch_copy_out(cur_frame(c), dev_inner, pitch, c->stream));
     return LTL_OK;
@@ -583,7 +587,7 @@ extern "C" int ltl_download_rows_device(ltl_ctx* c, int row0, int nrows, uint8_t
     LTL_CUDA(cudaSetDevice(c->device));
     if (keeps_packed(c)) {
         // straight from the packed frame: only the asked rows are unpacked
-        LTL_CUDA(launch_unpack_rows(cur_packed(c), row0, nrows, dev, pitch, c->stream));
+        LTL_CUDA(launch_unpack_rows(cur_packed(c), row0, nrows, dev, pitch, nullptr, c->stream));
         return LTL_OK;
     }
     Frame& f = cur_frame(c);

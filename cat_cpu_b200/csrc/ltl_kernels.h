@@ -100,9 +100,15 @@ cudaError_t launch_binarize(const Frame& f, cudaStream_t s);
 // whose wait ran out leaves it at some count in between.
 cudaError_t launch_pack_rows(const uint8_t* src, size_t pitch, bool nonzero, const PackedFrame& dst, int row0,
                              int nrows, GridBarrier* barrier, cudaStream_t s);
-cudaError_t launch_unpack_rows(const PackedFrame& src, int row0, int nrows, uint8_t* dst, size_t pitch, cudaStream_t s);
-// A packed frame's inner words as PACK-coded rows (bits past n cleared).
-cudaError_t launch_frame_to_pack64(const PackedFrame& f, uint64_t* dst, size_t dst_pitch_words, cudaStream_t s);
+// err (or null): if that word is set, dst's first cell becomes kMarkCell.
+constexpr uint8_t kMarkCell = 0xff;
+constexpr uint32_t kMarkCells = 0x5ac3a53cu;
+cudaError_t launch_unpack_rows(const PackedFrame& src, int row0, int nrows, uint8_t* dst, size_t pitch,
+                               const unsigned int* err, cudaStream_t s);
+// A packed frame's inner words as PACK-coded rows (bits past n cleared); err as above, the
+// first 32 cells become kMarkCells.
+cudaError_t launch_frame_to_pack64(const PackedFrame& f, uint64_t* dst, size_t dst_pitch_words, const unsigned int* err,
+                                   cudaStream_t s);
 // PACK-coded rows into a packed frame (barrier as in launch_pack_rows).
 cudaError_t launch_pack64_to_frame(const uint64_t* src, size_t src_pitch_words, const PackedFrame& f,
                                    GridBarrier* barrier, cudaStream_t s);
