@@ -1,6 +1,7 @@
-"""Shape autotuner: sweeps the kernels' work-item shapes on the device and writes
-the winners to cat_cpu_b200/tuning/ltl_tuning.txt, which libltl_b200 reads at
-ltl_create / ltl_batch_create.
+"""Shape autotuner: sweeps the kernels' work-item shapes on the device, against the
+shapes that are built in, and writes those that beat them to
+cat_cpu_b200/tuning/ltl_tuning.txt, which libltl_b200 reads at ltl_create /
+ltl_batch_create.
 
     python -m cat_cpu_b200.autotune [--quick] [--out DIR]
 
@@ -9,7 +10,8 @@ This is the analogue of the reference project's region-count landscape search
 scripts/extractBestRegionSize.py): here the swept shapes are
   plain / packed   band_rows: rows a warp walks down per work item (the vertical
                    window is restarted once per band, so longer bands re-read less
-                   but leave fewer items to balance over 148 SMs);
+                   but leave fewer items to balance over 148 SMs); 0 is the
+                   built-in choice, which follows the grid's sides;
   plain            depth: generations per pass of the temporally blocked kernel
                    (1, 2 or 3), swept jointly with band_rows;
   batch            persistent: one launch per call that runs every generation of
@@ -17,7 +19,10 @@ scripts/extractBestRegionSize.py): here the swept shapes are
                    latter stream_band_rows of the streamed per-step kernels and
                    resident_max_bytes: which grids are kept in shared memory for
                    a whole multi-step launch and which are streamed each step.
-The full landscape (every candidate's time) is written next to the table.
+A line of the table holds for a class of sides, so a shape gets one only if it is
+faster than the built-in choice at every side of the class that was timed, and by
+more than MARGIN on average.  The full landscape (every candidate's time) is written
+next to the table.
 """
 import argparse
 import concurrent.futures as cf
@@ -27,6 +32,19 @@ import time
 import numpy as np
 
 PKG = os.path.dirname(os.path.abspath(__file__))
+MARGIN = 0.03
+
+
+def choose(times, builtin):
+    """The candidate to write for a class of sides, or None to leave it to the built-in
+    choice.  times: {side: {candidate: ms}}, `builtin` among the candidates."""
+    gains = {}
+    for cand in next(iter(times.values())):
+        ratio = [t[cand] / t[builtin] for t in times.values()]
+        if cand != builtin and max(ratio) < 1:
+            gains[cand] = float(np.exp(np.mean(np.log(ratio))))
+    best = min(gains, key=gains.get, default=None)
+    return best if best is not None and gains[best] < 1 - MARGIN else None
 
 
 def _time_steps(torch, solver, stream, steps, reps=3):
@@ -53,13 +71,15 @@ def size_class(n):
 
 
 def tune_single(torch, C, variant, n, radius, rule, candidates, steps, depths=(1,)):
-    """Times every (depth, band_rows) pair; `steps` should be a multiple of every depth."""
+    """{(depth, band_rows): ms per step} and the built-in pair; `steps` should be a multiple
+    of every depth."""
     vcode = {"plain": C.VARIANT_PLAIN, "packed": C.VARIANT_PACKED}[variant]
     g = C.generate_state(n, 12345, 0.5, 1)
     stream = torch.cuda.Stream()
     s = C.CUDASolver(n, radius, rule, variant=vcode)
     s.set_stream(stream.cuda_stream)
-    rows = []
+    builtin = (s.info.temporal_depth, 0)
+    times = {}
     try:
         for d in depths:
             if variant == "plain":
@@ -68,12 +88,10 @@ def tune_single(torch, C, variant, n, radius, rule, candidates, steps, depths=(1
                 s.set_param("band_rows", br)
                 s.setState(g)
                 s.doSteps(12)
-                ms = _time_steps(torch, s, stream, steps)
-                rows.append(((d, br), ms))
+                times[(d, br)] = _time_steps(torch, s, stream, steps)
     finally:
         s.close()
-    best = min(rows, key=lambda x: x[1])
-    return best, rows
+    return times, builtin
 
 
 def tune_batch(torch, C, band_candidates, resident_candidates, steps):
@@ -107,8 +125,7 @@ def tune_batch(torch, C, band_candidates, resident_candidates, steps):
             rows.append(((pers, br, rm), a.elapsed_time(e)))
     finally:
         b.close()
-    best = min(rows, key=lambda x: x[1])
-    return best, rows
+    return dict(rows), cands[0]
 
 
 def main():
@@ -116,37 +133,44 @@ def main():
     ap.add_argument("--quick", action="store_true", help="fewer candidates")
     ap.add_argument("--out", default=os.path.join(PKG, "tuning"))
     args = ap.parse_args()
+    os.environ["LTL_TUNING_FILE"] = os.devnull  # the built-in choices, not an earlier table's
     import torch
     import cat_cpu_b200 as C
     from cat_cpu_b200.workloads import scaled_rule, BOSCO_R5
 
     os.makedirs(args.out, exist_ok=True)
     dev = torch.cuda.get_device_name(0)
-    table = [f"# autotuned on {dev} by cat_cpu_b200/autotune.py, {time.strftime('%Y-%m-%d %H:%M:%S')}"]
+    table = [f"# shapes that beat the built-in ones on {dev}: cat_cpu_b200/autotune.py, {time.strftime('%Y-%m-%d %H:%M:%S')}"]
     land = [f"# landscape ({dev}): candidate -> ms per step (single grids) or per 256-step batch run"]
-    plain_c = [64, 128, 256, 512] if args.quick else [64, 96, 128, 192, 256, 384, 512]
-    packed_c = [0, 32, 64, 128] if args.quick else [0, 32, 48, 64, 96, 128, 192, 256]  # 0: built-in choice
-    jobs = [("plain", 16384, 5, BOSCO_R5, plain_c), ("plain", 4096, 5, BOSCO_R5, plain_c),
-            ("packed", 16384, 5, BOSCO_R5, packed_c), ("packed", 32768, 5, BOSCO_R5, packed_c)]
-    for r in (1, 2, 4, 8, 16, 32):
-        if not args.quick or r in (1, 8):
-            jobs.append(("packed", 32768, r, scaled_rule(r), packed_c))
-    for variant, n, r, rule, cands in jobs:
+    bands = [0, 16, 64, 256] if args.quick else [0, 16, 32, 48, 64, 96, 128, 192, 256, 384, 512]  # 0: built-in
+    sides = [(1024, 4096), (8192, 16384), (32768,)]  # of each class
+    jobs = [("plain", 5), ("packed", 5)] + ([] if args.quick else [("plain", 1)] + [("packed", r) for r in (1, 2, 8, 16, 32)])
+    for variant, r in jobs:
+        rule = BOSCO_R5 if r == 5 else scaled_rule(r)
         depths = [d for d in (1, 2, 3) if d == 1 or (r <= 5 and d * r <= 16)] if variant == "plain" else [1]
-        ((d, br), ms), rows = tune_single(torch, C, variant, n, r, rule, cands, 24, depths)
-        lo, hi = size_class(n)
-        extra = f" depth={d}" if variant == "plain" else ""
-        table.append(f"variant={variant} radius={r} nmin={lo} nmax={hi} band_rows={br}{extra}")
-        land.append(f"{variant} n={n} R={r} (depth, band_rows): " + ", ".join(f"{c}:{t:.4f}" for c, t in rows) +
-                    f"  -> {(d, br)}")
-        print(land[-1], flush=True)
+        for ns in sides:
+            times = {}
+            for n in ns:
+                times[n], builtin = tune_single(torch, C, variant, n, r, rule, bands, 24, depths)
+                land.append(f"{variant} n={n} R={r} (depth, band_rows): " +
+                            ", ".join(f"{c}:{t:.4f}" for c, t in times[n].items()) + f"  built-in {builtin}")
+                print(land[-1], flush=True)
+            best = choose(times, builtin)
+            if best is not None:
+                lo, hi = size_class(ns[0])
+                extra = f" depth={best[0]}" if variant == "plain" else ""
+                table.append(f"variant={variant} radius={r} nmin={lo} nmax={hi} band_rows={best[1]}{extra}")
+                print("->", table[-1], flush=True)
     band_c = [32, 64, 128] if args.quick else [32, 48, 64, 96, 128]
     res_c = [0, 225280] if args.quick else [0, 65536, 131072, 225280]
-    ((pers, br, rm), ms), rows = tune_batch(torch, C, band_c, res_c, 256)
-    table.append(f"variant=batch radius=* persistent={pers} stream_band_rows={br} resident_max_bytes={rm}")
+    times, builtin = tune_batch(torch, C, band_c, res_c, 256)
     land.append("batch (persistent, stream_band_rows, resident_max_bytes): " +
-                ", ".join(f"{c}:{t:.2f}" for c, t in rows) + f"  -> {(pers, br, rm)}")
+                ", ".join(f"{c}:{t:.2f}" for c, t in times.items()))
     print(land[-1], flush=True)
+    # of the per-generation shapes the best one is written in any case: callers choose that mode
+    pers = choose({0: times}, builtin) is None
+    _, br, rm = min((c for c in times if c[0] == 0), key=times.get)
+    table.append(f"variant=batch radius=* persistent={int(pers)} stream_band_rows={br} resident_max_bytes={rm}")
     with open(os.path.join(args.out, "ltl_tuning.txt"), "w") as f:
         f.write("\n".join(table) + "\n")
     with open(os.path.join(args.out, "landscape.txt"), "w") as f:
