@@ -103,7 +103,7 @@ __device__ __forceinline__ bool persist_grid(const BatchGrid& g, uint32_t* a0, u
     uint32_t* ring = ring_all + (threadIdx.x >> 5) * PackedRing<R, W>::WARP_WORDS;
     uint32_t* f0 = a0 + g.off;
     uint32_t* f1 = a1 + g.off;
-    if (g.n < 64) return persist_form<R, 1, kEdgeTiny>(g, f0, f1, steps, rank, size, waits, grid, rule, ring);
+    if (!packed_two_words(g.n)) return persist_form<R, 1, kEdgeTiny>(g, f0, f1, steps, rank, size, waits, grid, rule, ring);
     if (packed_edge(g.n, W) == kEdgeNone)
         return persist_form<R, W, kEdgeNone>(g, f0, f1, steps, rank, size, waits, grid, rule, ring);
     return persist_form<R, W, kEdgeRagged>(g, f0, f1, steps, rank, size, waits, grid, rule, ring);

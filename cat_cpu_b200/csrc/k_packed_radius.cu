@@ -340,7 +340,7 @@ static cudaError_t with_walk(const PackedFrame& frame, F f) {
         if (n >= 64 && packed_beyond_l2(frame, whole ? 6 : 3))
             return whole ? f(PackedLaunch<R, 1, kEdgeNone, false>{}) : f(PackedLaunch<R, 1, kEdgeRagged, false>{});
     }
-    if (n < 64) return f(PackedLaunch<R, 1, kEdgeTiny>{});
+    if (!packed_two_words(n)) return f(PackedLaunch<R, 1, kEdgeTiny>{});
     if (packed_edge(n, 2) == kEdgeNone && packed_words(R, false) == 2)
         return f(PackedLaunch<R, packed_words(R, false), kEdgeNone>{});
     constexpr int W = packed_words(R, true);

@@ -344,8 +344,6 @@ cudaError_t launch_copy_out(const Frame& f, uint8_t* dst, size_t dst_pitch, cuda
     return cudaGetLastError();
 }
 
-cudaError_t launch_binarize(const Frame& f, cudaStream_t s) { return launch_copy_in(f, f.inner(0, 0), f.pitch, s); }
-
 // --- byte buffers <-> packed frames -----------------------------------------
 cudaError_t launch_pack_rows(const uint8_t* src, size_t pitch, bool nonzero, const PackedFrame& dst, int row0,
                              int nrows, GridBarrier* barrier, cudaStream_t s) {

@@ -92,8 +92,6 @@ cudaError_t launch_packed_run(const PackedFrame& cur, const PackedFrame& nxt, co
 // Byte frame <- / -> caller's buffer; in, every byte that is not 0 becomes 1.
 cudaError_t launch_copy_in(const Frame& f, const uint8_t* src, size_t src_pitch, cudaStream_t s);
 cudaError_t launch_copy_out(const Frame& f, uint8_t* dst, size_t dst_pitch, cudaStream_t s);
-// Every inner byte of the frame that is not 0 becomes 1.
-cudaError_t launch_binarize(const Frame& f, cudaStream_t s);
 // Inner rows [row0, row0 + nrows) of a packed frame from / to a buffer whose row
 // i is frame row row0 + i.  nonzero: a cell is alive if its byte is not 0, else
 // by its bit 0.  barrier (where a whole grid comes in, else null): zeroed, since a run

@@ -319,8 +319,9 @@ enum PackedEdge {
 __host__ __device__ inline int packed_edge(int n, int W) {
     return n < 64 ? kEdgeTiny : (n % (32 * W) == 0 ? kEdgeNone : kEdgeRagged);
 }
-// Two words per lane need a row of more than two words, or exactly two whole ones.
-__host__ __device__ inline bool packed_two_words(int n) { return n >= 64 && (n + 31) / 32 > 2; }
+// Two words per lane need a row of more than two words, or exactly two whole ones (one
+// lane is the row's first and its last then).
+__host__ __device__ inline bool packed_two_words(int n) { return n >= 64; }
 
 // The ring of one warp: 2R+1 rows of PH planes of W words per lane, laid out so
 // that a lane's planes are 16-byte vectors and a warp's vectors are contiguous.
