@@ -103,7 +103,9 @@ extern "C" int ltl_step_noalloc(const uint8_t* dev_in, size_t in_pitch, uint8_t*
     const Rule rule{radius, smin, smax, bmin, bmax};
     int band_rows = 0;
     if (!generic) band_rows = (int)tuning_lookup("plain", radius, n, "band_rows", 0);
-    if (!generic && band_rows <= 0) band_rows = plain_swar8_band_rows(n, n, radius, 1, device);
+    if (band_rows <= 0)
+        band_rows = generic ? plain_generic_band_rows(n, n, radius, device)
+                            : plain_swar8_band_rows(n, n, radius, 1, device);
     // The frames are not cleared.  The inner cells are written by the copy and
     // the halo by the halo fill before any step reads them.  The kernels also
     // read bytes outside the halo'd grid (the wide kernel's loads past the right
@@ -118,7 +120,7 @@ extern "C" int ltl_step_noalloc(const uint8_t* dev_in, size_t in_pitch, uint8_t*
     Frame* cur = &fa;
     Frame* nxt = &fb;
     for (int i = 0; i < steps && e == cudaSuccess; ++i) {
-        e = generic ? launch_plain_generic(*cur, *nxt, rule, 0, s)
+        e = generic ? launch_plain_generic(*cur, *nxt, rule, band_rows, s)
                     : launch_plain_swar8(*cur, *nxt, rule, band_rows, false, s);
         if (e == cudaSuccess) e = launch_halo_fill(*nxt, s);
         Frame* t = cur;

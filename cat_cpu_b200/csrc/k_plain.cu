@@ -1044,8 +1044,7 @@ static cudaError_t launch_wide_rm(const Frame& cur, const Frame& nxt, const Rule
 // bands of 16 / 32 / 48 / 64 rows): 512^2 R = 40 13.6 / 17.9 / 22.0 / 26.4; 4096^2 R = 12
 // 24.1 / 26.9 / 28.6 / 34.3; 6001^2 R = 64 52.4 / 47.3 / 45.3 / 48.6; 16384^2 R = 64 285
 // / 246 / 236 / 244.
-static int wide_band_rows(int rows, int tiles, int R, int resident) {
-    const int sms = 148;
+static int wide_band_rows(int rows, int tiles, int R, int sms, int resident) {
     double best = 0;
     int best_rows = 64;
     for (int b = 8; b <= 64; b += 4) {
@@ -1062,6 +1061,33 @@ static int wide_band_rows(int rows, int tiles, int R, int resident) {
     return best_rows;
 }
 
+// Outputs per tile, so that the prefix reads of the last output group, up to
+// P[T - 4 + (R + cpt - 1) + R + 4], stay inside P[0 .. NT cpt].
+static int wide_outputs(int R) {
+    const int cpt = plain_wide_cols_per_thread(R);
+    return (wide_threads(R) * cpt - 2 * R - cpt + 1) & ~3;
+}
+
+// CTAs that an SM holds of the kernel for a radius.
+template <bool PAIR, int CPT, int NT>
+static int wide_resident() {
+    int ctas = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, k_plain_wide<PAIR, CPT, 0, NT>, NT, 0) != cudaSuccess)
+        ctas = 0;
+    return std::max(ctas, 1);
+}
+
+int plain_generic_band_rows(int rows, int n, int radius, int device) {
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    const int T = wide_outputs(radius);
+    const int resident = radius <= kWidePairMaxRadius              ? wide_resident<true, 8, 128>()
+                         : wide_threads(radius) == 128             ? wide_resident<false, 8, 128>()
+                         : plain_wide_cols_per_thread(radius) == 8 ? wide_resident<false, 8, 256>()
+                                                                   : wide_resident<false, 16, 256>();
+    return wide_band_rows(rows, (n + T - 1) / T, radius, sms, resident);
+}
+
 cudaError_t launch_plain_generic(const Frame& cur, const Frame& nxt, const Rule& rule, int band_rows,
                                  cudaStream_t s) {
     const int n = cur.n, rows = cur.nrows(), R = rule.radius;
@@ -1070,12 +1096,10 @@ cudaError_t launch_plain_generic(const Frame& cur, const Frame& nxt, const Rule&
     const int cpt = plain_wide_cols_per_thread(R);
     if (cur.H < (int)round_up((size_t)R, (size_t)cpt) || (cur.H & 15) || (cur.pitch & 63))
         return cudaErrorInvalidValue;
-    // T: outputs per tile, so that the prefix reads of the last output group,
-    // up to P[T - 4 + (R + cpt - 1) + R + 4], stay inside P[0 .. NT cpt]
     const int nt = wide_threads(R);
-    const int T = (nt * cpt - 2 * R - cpt + 1) & ~3;
+    const int T = wide_outputs(R);
     const int tiles = (n + T - 1) / T;
-    int band = band_rows > 0 ? band_rows : wide_band_rows(rows, tiles, R, nt == 128 ? 9 : (cpt == 8 ? 4 : 3));
+    int band = band_rows > 0 ? band_rows : 64;
     band = std::max(band, (rows + 65534) / 65535);  // grid y limit
     band = std::min(band + (band & 1), std::max(rows + (rows & 1), 2));  // even: row pairs never straddle bands
     const dim3 grid(tiles, (rows + band - 1) / band);

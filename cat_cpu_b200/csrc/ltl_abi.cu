@@ -57,7 +57,7 @@ struct ltl_ctx {
     cudaStream_t own_stream = nullptr;
     cudaStream_t stream = nullptr;
     int band_rows = 0;          // plain: rows per work item (0: built-in choice)
-    int swar_bands[4] = {};     // plain R <= 5: that choice, by generations per pass
+    int built_in_bands[4] = {}; // that choice, by generations per pass
     bool plain_wrap = false;    // plain R <= 5: kernels apply the torus wrap, no halo refresh
     int packed_band_rows = 0;   // packed: rows per work item (0: heuristic)
     // packed and tensor variants: the grid lives in packed frames between steps
@@ -294,8 +294,11 @@ static int create_impl(ltl_ctx** out, int device, int rows, int n, int radius, i
     c->variant = variant;
     if (variant == LTL_VARIANT_PACKED) c->packed_band_rows = (int)tuning_lookup("packed", radius, n, "band_rows", 0);
     if (variant == LTL_VARIANT_PLAIN) e = plain_prepare(radius);
-    if (variant == LTL_VARIANT_PLAIN && e == cudaSuccess && plain_swar8_supported(radius))
-        for (int d = 1; d <= 3; ++d) c->swar_bands[d] = plain_swar8_band_rows(rows, n, radius, d, device);
+    if (variant == LTL_VARIANT_PLAIN && e == cudaSuccess) {
+        if (!plain_swar8_supported(radius)) c->built_in_bands[1] = plain_generic_band_rows(rows, n, radius, device);
+        else
+            for (int d = 1; d <= 3; ++d) c->built_in_bands[d] = plain_swar8_band_rows(rows, n, radius, d, device);
+    }
     if (variant == LTL_VARIANT_PLAIN && e == cudaSuccess) e = plain_tb_prepare(radius);
     if (e != cudaSuccess) {
         ltl_set_error("ltl_create: kernel setup failed: %s", cudaGetErrorString(e));
@@ -629,7 +632,7 @@ static cudaError_t enqueue_pass(ltl_ctx* c, int gens) {
         case LTL_VARIANT_PLAIN: {
             Frame& a = cur_frame(c);
             Frame& b = nxt_frame(c);
-            const int band = c->band_rows > 0 ? c->band_rows : c->swar_bands[gens];
+            const int band = c->band_rows > 0 ? c->band_rows : c->built_in_bands[gens];
             if (gens > 1) {
                 e = launch_plain_tb(a, b, c->rule, band, gens, c->plain_wrap, c->stream);
                 step_kernels = 1;
@@ -637,7 +640,7 @@ static cudaError_t enqueue_pass(ltl_ctx* c, int gens) {
                 e = launch_plain_swar8(a, b, c->rule, band, c->plain_wrap, c->stream);
                 step_kernels = 1;
             } else {
-                e = launch_plain_generic(a, b, c->rule, c->band_rows, c->stream);
+                e = launch_plain_generic(a, b, c->rule, band, c->stream);
                 step_kernels = 1;
             }
             if (c->timing && e == cudaSuccess) e = cudaEventRecord(e1, c->stream);

@@ -44,8 +44,9 @@ cudaError_t launch_plain_tb(const Frame& cur, const Frame& nxt, const Rule& rule
 // K1 generic path (R up to 2038): one fused kernel (vertical window sums in
 // registers, a prefix scan per row, or per pair of rows, in shared memory, the
 // rule); needs a halo of at least R rounded up to plain_wide_cols_per_thread(R).
-// band_rows: rows per CTA (0: built-in choice).
+// band_rows: rows per CTA (plain_generic_band_rows: built-in choice).
 bool plain_generic_supported(int radius);
+int plain_generic_band_rows(int rows, int n, int radius, int device);
 int plain_wide_cols_per_thread(int radius);
 cudaError_t launch_plain_generic(const Frame& cur, const Frame& nxt, const Rule& rule, int band_rows,
                                  cudaStream_t s);
