@@ -283,16 +283,18 @@ k_pack_to_words(const uint32_t* __restrict__ src, size_t sp, unsigned rows, int 
     }
 }
 
-// Grid and block of a kernel without a reduction: `items` threads along a row (a power of
-// two up to kTx, so that rows of a few cells do not leave a warp to one or two threads:
-// 100,000 rows of 3 cells packed 26 us with a warp per row, 10 so), `per` rows per thread.
+// Grid and block of a kernel without a reduction: `items` threads along a row, `per` rows per
+// thread.  Where rows of a few cells would leave a warp to one or two threads, and are more
+// than the SMs take at once, a block has fewer threads along a row (a power of two; 100,000
+// rows of 3 cells packed 26 us with a warp per row, 10 so; a pass over 64^2 15.0 / 15.7).
 struct Shape {
     dim3 grid, block;
     bool narrow;
 };
 Shape shape(long long items, int rows, int per) {
     unsigned tx = kTx;
-    while (tx > 1 && tx / 2 >= items) tx /= 2;
+    if (rows > 148 * 8 * kTy * per)
+        while (tx > 1 && tx / 2 >= items) tx /= 2;
     const unsigned ty = kTx * kTy / tx;
     const long long gy = std::max<long long>(1, ((long long)rows + ty * per - 1) / (ty * per));
     return {dim3((unsigned)std::max<long long>(1, (items + tx - 1) / tx), (unsigned)std::min<long long>(gy, 65535)),

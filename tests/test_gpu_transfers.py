@@ -130,7 +130,7 @@ def test_many_narrow_rows(cols):
     import torch
     import cat_cpu_b200 as C
     L = C.lib()
-    rows, nw = 100003, (cols + 63) // 64
+    rows, nw = 100003, (cols + 63) // 64  # (more than a load of the SMs)
     cells = (np.random.default_rng(cols).random((rows, cols)) < 0.5).astype(np.uint8)
     dev = torch.from_numpy(cells * 3).cuda()
     words = torch.full((rows, nw), -1, dtype=torch.int64, device="cuda")
