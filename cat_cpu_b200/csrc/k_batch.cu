@@ -403,6 +403,7 @@ static void batch_release(ltl_batch* b) {
     do {                                                                                           \
         cudaError_t e_ = (call);                                                                   \
         if (e_ != cudaSuccess) {                                                                   \
+            cudaGetLastError(); /* reported here, not by the next launch */                        \
             ltl_set_error("%s failed: %s", #call, cudaGetErrorString(e_));                         \
             return e_ == cudaErrorMemoryAllocation ? LTL_ENOMEM : LTL_ECUDA;                       \
         }                                                                                          \
@@ -838,6 +839,7 @@ extern "C" int ltl_batch_step(ltl_batch* b, int steps) {
     if (b->no_graph) {
         cudaError_t e = enqueue_steps(b, steps, &what);
         if (e != cudaSuccess) {
+            cudaGetLastError();
             ltl_set_error("ltl_batch_step: %s failed: %s", what, cudaGetErrorString(e));
             return LTL_ECUDA;
         }
@@ -862,6 +864,7 @@ extern "C" int ltl_batch_step(ltl_batch* b, int steps) {
         cudaError_t e3 = cudaGraphInstantiate(&ex, g, 0);
         cudaGraphDestroy(g);
         if (e3 != cudaSuccess) {
+            cudaGetLastError();
             ltl_set_error("ltl_batch_step: graph instantiate failed: %s", cudaGetErrorString(e3));
             return LTL_ECUDA;
         }

@@ -129,6 +129,7 @@ extern "C" int ltl_step_noalloc(const uint8_t* dev_in, size_t in_pitch, uint8_t*
     }
     if (e == cudaSuccess) e = launch_copy_out(*cur, dev_out, out_pitch, s);
     if (e != cudaSuccess) {
+        cudaGetLastError();
         ltl_set_error("ltl_step_noalloc: launch failed: %s", cudaGetErrorString(e));
         return LTL_ECUDA;
     }

@@ -32,6 +32,7 @@ void ltl_set_error(const char* fmt, ...) {
     do {                                                                                   \
         cudaError_t e_ = (call);                                                           \
         if (e_ != cudaSuccess) {                                                           \
+            cudaGetLastError(); /* reported here, not by the next launch */                \
             ltl_set_error("%s failed: %s (%s:%d)", #call, cudaGetErrorString(e_), __FILE__, \
                           __LINE__);                                                       \
             return e_ == cudaErrorMemoryAllocation ? LTL_ENOMEM : LTL_ECUDA;               \
@@ -168,6 +169,13 @@ static bool auto_packs(int n, int radius) {
     return radius <= 23 || (radius <= 28 && n % 32 == 0 && n >= 2048);
 }
 
+// A solver that could not be made: the error that says why is not left to be taken for
+// the next launch's, of this or another solver.
+static void release_failed(ltl_ctx* c) {
+    release(c);
+    cudaGetLastError();
+}
+
 // rows x n torus (rows == n unless a rectangular form is asked for: plain and packed)
 static int create_impl(ltl_ctx** out, int device, int rows, int n, int radius, int smin, int smax, int bmin,
                        int bmax, int variant) {
@@ -232,7 +240,7 @@ static int create_impl(ltl_ctx** out, int device, int rows, int n, int radius, i
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) {
         ltl_set_error("ltl_create: %s", cudaGetErrorString(e));
-        release(c);
+        release_failed(c);
         return LTL_ECUDA;
     }
     c->stream = c->own_stream;
@@ -271,7 +279,7 @@ static int create_impl(ltl_ctx** out, int device, int rows, int n, int radius, i
     }
     if (e != cudaSuccess) {
         ltl_set_error("ltl_create: device allocation of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
-        release(c);
+        release_failed(c);
         return e == cudaErrorMemoryAllocation ? LTL_ENOMEM : LTL_ECUDA;
     }
     c->fa = Frame{c->frames, n, H, pitch, rows};
@@ -302,7 +310,7 @@ static int create_impl(ltl_ctx** out, int device, int rows, int n, int radius, i
     if (variant == LTL_VARIANT_PLAIN && e == cudaSuccess) e = plain_tb_prepare(radius);
     if (e != cudaSuccess) {
         ltl_set_error("ltl_create: kernel setup failed: %s", cudaGetErrorString(e));
-        release(c);
+        release_failed(c);
         return LTL_ECUDA;
     }
     if (variant == LTL_VARIANT_PACKED || variant == LTL_VARIANT_TENSOR) {
@@ -312,7 +320,7 @@ static int create_impl(ltl_ctx** out, int device, int rows, int n, int radius, i
         c->runs = variant == LTL_VARIANT_PACKED && packed_runs(p, radius);
         if (variant == LTL_VARIANT_PACKED && (e = packed_prepare(p, radius, !runs_packed(c))) != cudaSuccess) {
             ltl_set_error("ltl_create: kernel setup failed: %s", cudaGetErrorString(e));
-            release(c);
+            release_failed(c);
             return LTL_ECUDA;
         }
     }
@@ -320,7 +328,7 @@ static int create_impl(ltl_ctx** out, int device, int rows, int n, int radius, i
         c->tplan = tensor_plan_create(c->pa, c->pb, c->rule, device, c->run.barrier, c->run.err, why, sizeof(why));
         if (!c->tplan) {
             ltl_set_error("ltl_create: tensor plan: %s", why);
-            release(c);
+            release_failed(c);
             return LTL_EUNSUPPORTED;
         }
         depth = tensor_plan_depth(c->tplan);
@@ -329,7 +337,7 @@ static int create_impl(ltl_ctx** out, int device, int rows, int n, int radius, i
     e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) {
         ltl_set_error("ltl_create: %s", cudaGetErrorString(e));
-        release(c);
+        release_failed(c);
         return LTL_ECUDA;
     }
     *out = c;
@@ -511,6 +519,7 @@ static int pack_stage(ltl_ctx* c, uint64_t** stage) {
         const size_t bytes = (size_t)c->rows * 8 * ((c->n + 63) / 64);
         cudaError_t e = cudaMalloc(&c->pstage, std::max<size_t>(bytes, 8));
         if (e != cudaSuccess) {
+            cudaGetLastError();
             ltl_set_error("packed transfer staging allocation failed: %s", cudaGetErrorString(e));
             return LTL_ENOMEM;
         }
@@ -687,6 +696,7 @@ static int build_graph(ltl_ctx* c, int which) {
     cudaError_t e2 = cudaStreamEndCapture(c->stream, &g);
     c->cur_is_a = saved;
     if (e != cudaSuccess || e2 != cudaSuccess) {
+        cudaGetLastError();
         if (g) cudaGraphDestroy(g);
         ltl_set_error("graph capture failed: %s", cudaGetErrorString(e != cudaSuccess ? e : e2));
         return LTL_ECUDA;
@@ -694,6 +704,7 @@ static int build_graph(ltl_ctx* c, int which) {
     cudaError_t e3 = cudaGraphInstantiate(&c->graph[which], g, 0);
     cudaGraphDestroy(g);
     if (e3 != cudaSuccess) {
+        cudaGetLastError();
         c->graph[which] = nullptr;
         ltl_set_error("graph instantiate failed: %s", cudaGetErrorString(e3));
         return LTL_ECUDA;

@@ -65,3 +65,20 @@ def test_default_solver_holds_no_more_than_the_plain_one(n, radius):
     rule = (2, 3, 3, 3)
     with C.CUDASolver(n, radius, rule) as s, C.CUDASolver(n, radius, rule, variant=C.VARIANT_PLAIN) as p:
         assert s.info.device_bytes <= p.info.device_bytes
+
+
+@pytest.mark.parametrize("variant", [0, 1, 2])
+def test_a_solver_that_does_not_fit_leaves_others_alone(variant):
+    import cat_cpu_b200 as C
+    from oracle import oracle as O
+    g = (np.random.default_rng(2).random((500, 500)) < 0.45).astype(np.uint8)
+    rule = O.scaled_rule(3)
+    with C.CUDASolver(500, 3, rule, variant=variant) as s:
+        s.setState(g)
+        for make in (lambda: C.CUDASolver(450000, 3, rule, variant=0), lambda: C.Batch([(400000, 3, rule)])):
+            with pytest.raises(C.LtlError) as e:
+                make()
+            assert e.value.code == C.ltl.ENOMEM
+            s.doSteps(1)
+            g = O.run(g, 3, rule, 1)
+            assert np.array_equal(s.getCurrentState(), g)
