@@ -5,18 +5,17 @@
 // src/CellularAutomata/Solvers/HostSolver.tpp:58-140); the reference runs one
 // grid per process (CPUBenchmark.cpp:63-85).  Design:
 //   - every grid is stored bit-packed (packed_core.cuh) in one device arena,
-//     two arenas ping-pong;
-//   - grids are grouped into rule classes (radius + rule); each class gets its
-//     own kernel instantiation, with the rule's bit masks in the constant bank;
-//   - "resident" grids (small enough that two packed copies fit in one SM's
-//     shared memory) are advanced all requested steps in ONE launch: a CTA loads
-//     the grid once and writes it back after the last step (temporal blocking
-//     of the whole run);
-//   - larger grids are advanced one generation per launch by a persistent
-//     kernel that walks a (grid, row band, word strip) work list; the whole step
-//     loop is captured in a CUDA graph, and the resident launches run
-//     concurrently on a forked stream.  No form has a halo: the walk wraps rows
-//     and words in its loads.
+//     two arenas ping-pong; no form has a halo, the walk wraps rows and words in
+//     its loads;
+//   - persistent mode (the default): one launch runs every generation of every
+//     grid of a call (k_batch_persist below);
+//   - per-generation mode (k_batch_radius.cu): grids are grouped into rule classes
+//     (radius + rule), each a kernel instantiation with its masks in the constant
+//     bank.  "Resident" grids, whose two packed copies fit in one SM's shared memory,
+//     are advanced all steps of a call in one launch; the others one generation per
+//     launch over a (grid, row band, word strip) work list, with the resident
+//     launches beside them on a forked stream;
+//   - either way a call is a CUDA graph, made for its step count and starting arena.
 #include <algorithm>
 #include <cstring>
 #include <map>
@@ -25,6 +24,7 @@
 
 #include "../../include/ltl.h"
 #include "batch_ops.h"
+#include "batch_split.h"
 #include "grid_barrier.cuh"
 #include "packed_core.cuh"
 #include "transfer_core.cuh"
@@ -49,14 +49,6 @@ namespace ltl {
 // (without transfers): 52 and 70 ms with one CTA of eight warps per grid, 3.8 and
 // 42 ms so.
 // ---------------------------------------------------------------------------
-constexpr int kPersistWarps = 4;
-constexpr int kPersistThreads = kPersistWarps * 32;
-
-// Words per lane.  The shared memory of a CTA is the largest ring of any radius in the
-// batch: with two words at R = 6 to 8 it would be 61 to 87 KB and leave two CTAs per SM
-// to every grid of the batch (the 1024-grid ensemble of R 1..8: 61.9 ms against 48.8).
-constexpr int persist_words(int R) { return R <= 5 ? 2 : 1; }
-
 // A CTA's first task: its rank in the group of grid `grid` (size 0: none).
 struct BatchGroup {
     int grid, rank, size;
@@ -69,13 +61,15 @@ struct BatchWaits {
     BarrierLimit limit;
 };
 
-// Not inlined: forms and radii that share one function share its registers (255 and
-// spills; one by one they fit the 128 that four CTAs per SM leave).
+// Not inlined: forms and radii that share one function share its registers (255, and
+// spills in the walk's loop).  One by one they are held to the 128 that four CTAs per SM
+// leave, at 20 to 100 bytes of spills in most, and are faster so (168 registers and three
+// CTAs: 48.6 ms against 42.2 for the 1024-grid ensemble).
 template <int R, int W, int EDGE>
 __device__ __noinline__ bool persist_form(const BatchGrid& g, uint32_t* f0, uint32_t* f1, int steps, int rank,
                                           int size, const BatchWaits& waits, int grid, const PackedRule& rule,
                                           uint32_t* ring) {
-    const PackedRule pr = rule;  // the masks the comparators use, kept in registers
+    const PackedRule pr = rule;  // the masks the comparators use: loaded once, as far as registers go
     GridBarrierWait group(waits.barriers + grid, size, waits.limit);
     const int lanes = size * kPersistThreads, id = rank * kPersistThreads + threadIdx.x;
     const int groups = (g.nw + W - 1) / W;
@@ -147,61 +141,6 @@ k_batch_persist(uint32_t* a0, uint32_t* a1, const BatchGrid* __restrict__ grids,
 template <int R>
 static size_t persist_ring_bytes() {
     return (size_t)kPersistWarps * PackedRing<R, persist_words(R)>::WARP_WORDS * 4;
-}
-
-// Which grids get groups of CTAs.  Model of one generation (us) by `size` CTAs on a
-// chip that holds `per_sm` CTAs on each SM: a band's rows, 0.6 of a row for each of the
-// 2R+1 rows that it counts first, and a group barrier.  A row of one CTA among three or
-// more per SM takes `row` times their number; the rates and rows are fitted to single
-// grids at 16384^2 (k_packed.cu).
-struct BatchCost {
-    int n, groups, R;
-    double row;
-    BatchCost(int n_, int nw, int R_, int per_sm) : n(n_), R(R_) {
-        static const double rate[] = {1.5, 1.12, 1.0};
-        const int W = n < 64 ? 1 : persist_words(R);
-        groups = (nw + W - 1) / W;
-        row = per_sm * rate[std::min(per_sm, 3) - 1] * (W == 2 ? 0.098 + 0.0156 * R : 0.090 + 0.0063 * R);
-    }
-    double start() const { return 0.6 * (2 * R + 1); }
-    static constexpr double kBarrier = 1.3, kSingle = 0.3;
-    double time(int size) const {
-        const int lanes = size * kPersistThreads;
-        const int bands = std::min(n, std::max(1, lanes / groups));
-        const int turns = groups > lanes ? (groups + lanes - 1) / lanes : 1;
-        return turns * row * (start() + (n + bands - 1) / bands) + (size > 1 ? kBarrier : kSingle);
-    }
-    // CTAs that bring a generation under t, 0 if none do
-    int size_for(double t) const {
-        if (time(1) <= t) return 1;
-        const int b = (int)((t - kBarrier) / row - start());
-        if (b < 1) return 0;
-        return (int)(((long long)((n + b - 1) / b) * groups + kPersistThreads - 1) / kPersistThreads);
-    }
-};
-
-// The smallest common time t for which all grids fit into `ctas` CTAs: groups side
-// by side, and the sum of all CTAs' time within ctas * t.  sizes: CTAs per grid.
-static void batch_split(const std::vector<BatchCost>& grids, int ctas, std::vector<int>& sizes) {
-    auto fits = [&](double t) {
-        double area = 0;
-        long long grouped = 0;
-        for (const BatchCost& g : grids) {
-            const int k = g.size_for(t);
-            if (k == 0) return false;
-            area += k * g.time(k);
-            if (k > 1) grouped += k;
-        }
-        return grouped <= ctas && area <= ctas * t;
-    };
-    double hi = 0, lo = 0;
-    for (const BatchCost& g : grids) hi += g.time(1);  // one CTA each, one after the other
-    for (int i = 0; i < 24 && hi - lo > 0.01 * hi; ++i) {
-        const double t = 0.5 * (lo + hi);
-        (fits(t) ? hi : lo) = t;
-    }
-    sizes.assign(grids.size(), 1);
-    for (size_t i = 0; i < grids.size(); ++i) sizes[i] = std::max(1, grids[i].size_for(hi));
 }
 
 // ---------------------------------------------------------------------------

@@ -169,7 +169,7 @@ k_packed_small(uint32_t* a, uint32_t* b, int steps, int blocks, int wp, int n, i
                const __grid_constant__ PackedRun run, const __grid_constant__ PackedRule pr) {
     extern __shared__ __align__(16) uint32_t counts[];
     const bool whole = gridDim.x == 1;
-    const int ext_max = whole ? rows : band_rows + 2 * R * ((steps + blocks - 1) / blocks);
+    const int ext_max = whole ? rows : band_rows + 2 * R * block_generations(steps, blocks);
     uint32_t* s_in = counts + (size_t)(whole ? rows + 2 * R : ext_max) * PackedTile<R>::ROW;
     uint32_t* s_out = s_in + (size_t)ext_max * kTileStride;
     GridBarrierWait all(run.barrier, gridDim.x, run.limit);
@@ -180,7 +180,7 @@ k_packed_small(uint32_t* a, uint32_t* b, int steps, int blocks, int wp, int n, i
     const uint32_t* cur = a;
     uint32_t* nxt = b;
     for (int s = 0; s < steps; --blocks) {
-        const int d = (steps - s + blocks - 1) / blocks;
+        const int d = block_generations(steps - s, blocks);
         const int halo = whole ? 0 : R * d, ext = tr + 2 * halo;
         if (works)
             for (int i = first; i < ext; i += step) {
@@ -322,10 +322,8 @@ struct SmallLaunch {
         const int reach = c.nw <= 4 ? 28 : 18;
         int depth = std::min(steps, std::max(1, std::min(12, (2 * reach + R - 1) / (2 * R))));
         while (tr < rows && depth > 1 && (bytes(rows, tr, depth) > kTileSmem || R * depth > rows)) --depth;
-        int blocks = (steps + depth - 1) / depth;
-        if (blocks % 2 != steps % 2) ++blocks;  // (then blocks < steps)
-        if (ctas == 1) blocks = 1;
-        depth = (steps + blocks - 1) / blocks;
+        const int blocks = ctas == 1 ? 1 : run_blocks(steps, depth);
+        depth = block_generations(steps, blocks);
         return launch_group(k_packed_small<R, EDGE>, ctas, bytes(rows, tr, depth), blocks > 1, s, c.words, x.words,
                             steps, blocks, (int)c.wpitch, c.n, c.nw, rows, tr, run, pr);
     }

@@ -1,5 +1,5 @@
 // packed_core.cuh -- bit-sliced building blocks shared by the packed kernels
-// (single grid: k_packed.cu, batched: k_batch.cu).
+// (single grid: k_packed_radius.cu, batched: k_batch.cu, k_batch_radius.cu).
 //
 // Cells are bits of 32-bit words (cell j of a row = bit j % 32 of word j / 32).
 // A count over many cells is kept "bit-sliced": plane i holds bit i of the count

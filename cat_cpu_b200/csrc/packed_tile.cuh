@@ -17,6 +17,16 @@ namespace ltl {
 constexpr int kTileWords = 32;   // words per tile row at most
 constexpr int kTileStride = 33;  // shared-memory words per plane of a row: rows of narrow tiles spread over the banks
 
+// Blocks of generations between barriers: of `steps` generations, at most `depth` to a
+// block.  Odd or even as `steps` is, so that the grid ends in the frame where single
+// generations would have left it.
+inline int run_blocks(int steps, int depth) {
+    const int blocks = (steps + depth - 1) / depth;
+    return blocks + (blocks % 2 != steps % 2);  // (more only where blocks < steps)
+}
+// Generations of the next block, with `left` of them in `blocks` blocks to come.
+__host__ __device__ constexpr int block_generations(int left, int blocks) { return (left + blocks - 1) / blocks; }
+
 template <int R>
 struct PackedTile {
     static constexpr int PH = bits_for(2 * R + 1);
