@@ -51,10 +51,10 @@ REF_RULE_TAG = "R5_S32-56_B34-45"
 # workload (the bit-packed kernels are bound by logic operations on the ALU pipe,
 # the tensor kernel by hand-offs between its warp roles, not by HBM).
 LIMITER = {
-    "plain": {"pipe": "alu", "ncu_pct_of_peak": 65.6, "issue_active_pct": 71.1,
+    "plain": {"pipe": "alu", "ncu_pct_of_peak": 65.5, "issue_active_pct": 71.0,
               "source": "profiles/k_plain_swar8_tb_n16384_r5.md"},
-    "packed": {"pipe": "alu", "ncu_pct_of_peak": 80.7, "source": "profiles/k_packed_step_n16384_r5.md"},
-    "tensor": {"pipe": "tensor", "ncu_pct_of_peak": 33.0, "issue_active_pct": 60.4,
+    "packed": {"pipe": "alu", "ncu_pct_of_peak": 80.8, "source": "profiles/k_packed_step_n16384_r5.md"},
+    "tensor": {"pipe": "tensor", "ncu_pct_of_peak": 34.7, "issue_active_pct": 63.3,
                "source": "profiles/k_tensor_step_n16384_r5.md"},
 }
 
@@ -656,8 +656,8 @@ def main():
                     "U[0.2,0.6] (mt19937_64 seed 4), 256 steps per ltl_batch_step call, bit-packed",
         "grid_steps_per_s": round(world * br["grids"] * br["steps"] / (b_ms * 1e-3), 1),
         "gcups": round(b_gcups, 2), "ms": round(b_ms, 3), "cells": br["cells"],
-        "mode": "persistent: one launch per rule class per ltl_batch_step call runs all 256 generations, "
-                "each CTA advancing whole grids (largest first) with the grid held in L1/L2",
+        "mode": "persistent: one launch per ltl_batch_step call runs all 256 generations, large grids by groups "
+                "of CTAs, the others by single CTAs (the most work first), held in L1/L2",
         "grids_all_steps_in_one_launch": br["resident_grids"],
         "roofline": {"bound": "hbm", "bytes_per_update": 0.25, "achieved": round(b_gcups * 0.25, 1),
                      "peak": peak, "unit": "GB/s", "frac": round(b_gcups * 0.25 / peak, 4),

@@ -158,13 +158,13 @@ static void drop_graphs(ltl_ctx* c) {
 }
 
 // Whether LTL_VARIANT_AUTO runs the bit-packed kernels or the plain ones.  us per generation,
-// plain / packed: up to R = 23 packed is ahead, or within 3%, at every side (64^2 R = 1 8 /
-// 0.5, 1024^2 R = 5 4.4 / 2.0, 16384^2 R = 5 78 / 44, R = 17 200 / 105; 1001^2 R = 20 10.4 / 9.7,
-// 6001^2 R = 22 39.0 / 39.0; the worst is 1500^2 R = 23, 12.1 / 13.3).  From R = 24 to 28 it
+// plain / packed: up to R = 23 packed is ahead, or within 3%, at nearly every side (64^2 R = 1
+// 2.4 / 0.5, 1024^2 R = 5 4.4 / 2.0, 16384^2 R = 5 78 / 44, R = 20 211 / 139; 1001^2 R = 20 10.4 /
+// 9.7, 6001^2 R = 22 39.0 / 39.0; the worst is 1500^2 R = 23, 12.1 / 13.3).  From R = 24 to 28 it
 // is on large whole sides only (4096^2 R = 24 25.3 / 18.8, R = 28 26.2 / 21.3, 16384^2 R = 28
 // 228 / 152; 2048^2 R = 24 12.6 / 12.8, 512^2 R = 24 8.2 / 11.6; ragged 3001^2 R = 24 18.0 /
 // 19.3, 6001^2 R = 26 37.7 / 41.6, 33000^2 R = 28 779 / 832).  Above 28 neither is ahead
-// everywhere (16384^2 R = 32 228 / 217, 4096^2 R = 29 26 / 28, 64^2 R = 29 9.5 / 9.8): plain.
+// everywhere (16384^2 R = 29 231 / 193, R = 32 228 / 217, 512^2 R = 29 10.3 / 14.2): plain.
 static bool auto_packs(int n, int radius) {
     return radius <= 23 || (radius <= 28 && n % 32 == 0 && n >= 2048);
 }

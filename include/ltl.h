@@ -46,7 +46,7 @@ extern "C" {
 typedef struct ltl_ctx ltl_ctx;
 
 typedef struct {
-    int variant;          /* variant actually used */
+    int variant;          /* variant (LTL_VARIANT_AUTO: LTL_VARIANT_PLAIN, see there) */
     int n, radius;
     int smin, smax, bmin, bmax;
     int halo;             /* halo width of the device grid (cells) */
