@@ -155,7 +155,9 @@ __global__ void k_batch_pack(const uint8_t* __restrict__ cells, uint32_t* __rest
     if (blockIdx.x == 0 && threadIdx.x == 0) barriers[first + blockIdx.y].arrived = 0;
     const uint8_t* c = cells + g.cell_off;
     const uint8_t* end = c + (size_t)g.n * g.n;
-    for (RowWalk t(blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, g.nw); t.row < g.n; t.next()) {
+    const int at = blockIdx.x * blockDim.x + threadIdx.x;
+    if (at >= (long long)g.n * g.nw) return;  // (most threads of a small grid: before the walk's divisions)
+    for (RowWalk t(at, gridDim.x * blockDim.x, g.nw); t.row < g.n; t.next()) {
         const int i = t.row, w = t.col;
         const uint8_t* p = c + (size_t)i * g.n + 32 * w;
         const int valid = g.n - 32 * w;
@@ -178,7 +180,9 @@ __global__ void k_batch_unpack(const uint32_t* __restrict__ arena, uint8_t* __re
     const BatchGrid g = grids[first + blockIdx.y];
     uint8_t* dst = cells + g.cell_off;
     const int vecs = (g.n + 15) / 16 + 1;  // aligned vectors a row may touch
-    for (RowWalk t(blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, vecs); t.row < g.n; t.next()) {
+    const int at = blockIdx.x * blockDim.x + threadIdx.x;
+    if (at >= (long long)g.n * vecs) return;
+    for (RowWalk t(at, gridDim.x * blockDim.x, vecs); t.row < g.n; t.next()) {
         const int i = t.row;
         uint8_t* row = dst + (size_t)i * g.n;
         const int c = lead(row) + 16 * t.col;
@@ -305,7 +309,8 @@ struct ltl_batch {
     int persist_ctas = 0;
     size_t persist_smem = 0;
     bool grouped = false;              // some grid has more than one CTA: cooperative launch
-    bool waits = false;                // a grouped launch has been made (or captured): d_err is read
+    bool unchecked = false;            // a grouped launch was made since d_err was last read
+    bool captured = false;             // one was captured: replays come unseen, so d_err is always read
     BarrierLimit limit{};
     cudaStream_t own = nullptr, stream = nullptr, aux = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr;
@@ -624,12 +629,12 @@ static uint32_t* cur_arena(ltl_batch* b) { return b->arena[b->cur_is_a ? 0 : 1];
 static uint32_t* nxt_arena(ltl_batch* b) { return b->arena[b->cur_is_a ? 1 : 0]; }
 
 // Waits for the stream; did a group's barrier wait run out since this was last asked?
-// (Asked again after every launch and every replay of a caller's graph with one in it, of
-// which the host knows nothing.)
 static int wait_groups(ltl_batch* b) {
     unsigned int flag = 0;
-    if (b->waits) BATCH_CUDA(cudaMemcpyAsync(&flag, b->d_err, sizeof(flag), cudaMemcpyDeviceToHost, b->stream));
+    if (b->unchecked || b->captured)
+        BATCH_CUDA(cudaMemcpyAsync(&flag, b->d_err, sizeof(flag), cudaMemcpyDeviceToHost, b->stream));
     BATCH_CUDA(cudaStreamSynchronize(b->stream));
+    b->unchecked = false;
     if (!flag) return LTL_OK;
     BATCH_CUDA(cudaMemsetAsync(b->d_err, 0, sizeof(flag), b->stream));
     BATCH_CUDA(cudaMemsetAsync(b->d_barriers, 0, sizeof(GridBarrier) * b->grids.size(), b->stream));
@@ -773,7 +778,12 @@ extern "C" int ltl_batch_step(ltl_batch* b, int steps) {
     }
     if (steps == 0) return LTL_OK;
     BATCH_CUDA(cudaSetDevice(b->device));
-    b->waits = b->waits || (b->persistent && b->grouped);
+    if (b->persistent && b->grouped) {
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        if (b->no_graph) BATCH_CUDA(cudaStreamIsCapturing(b->stream, &capture));
+        b->unchecked = true;
+        b->captured = b->captured || capture != cudaStreamCaptureStatusNone;
+    }
     const char* what = "";
     if (b->no_graph) {
         cudaError_t e = enqueue_steps(b, steps, &what);

@@ -145,3 +145,26 @@ def test_arguments():
     for variant in (C.VARIANT_AUTO, C.VARIANT_PLAIN, C.VARIANT_TENSOR):
         with C.CUDASolver(300, 5, O.BOSCO_R5, variant=variant) as s, pytest.raises(C.LtlError):
             s.set_param("inject_missing_arrival", 10**7)
+
+
+def test_replays_of_a_captured_batch_report():
+    import torch
+    import cat_cpu_b200 as C
+    n, r = 1000, 5
+    flat = (np.random.default_rng(3).random(n * n) < 0.45).astype(np.uint8)
+    stream = torch.cuda.Stream()
+    b = C.Batch([(n, r, rule_of(r))], flags=2)  # launched directly, so that it can be captured
+    b.set_param("inject_missing_arrival", 5_000_000)
+    b.set_stream(stream.cuda_stream)
+    b.upload_all(flat)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        b.step(4)
+    b.synchronize()  # nothing has run
+    for _ in range(2):
+        b.upload_all(flat)
+        with torch.cuda.stream(stream):
+            graph.replay()
+        times_out(b.download_all)
+    del graph
+    b.close()
