@@ -156,7 +156,12 @@ TensorPlan* tensor_plan_create(const PackedFrame& a, const PackedFrame& b, const
     // one correction wraps a row (rows span [-R, n + 128 nb)) and a word index
     // (words span [-4, nw + ng)); groups are word halves
     const int nb_of_r = R <= 32 ? 1 : (128 + 2 * R + 127) / 128;
-    const bool fast_ok = nw >= 4 && a.n >= 128 * nb_of_r + R;
+    // where 32 does not divide n, rows of fewer tiles than this are gathered: too many of them
+    // reach over the seam (us per generation, staged / gathered: 1000^2 R = 5 5.9 / 4.8, R = 113
+    // 19.6 / 12.4, 1500^2 R = 8 7.0 / 6.7, R = 90 16.2 / 12.9; 2001^2 R = 8 7.1 / 7.0, R = 16 7.9 /
+    // 8.8, R = 90 19.9 / 22.3, R = 113 24.2 / 22.3; 3001^2 R = 64 20 / 28)
+    constexpr int kSeamTiles = 16;
+    const bool fast_ok = nw >= 4 && a.n >= 128 * nb_of_r + R && (a.n % 32 == 0 || (a.n + kTc - 1) / kTc >= kSeamTiles);
     TensorGeometry G{};
     if (!tensor_geometry(R, fast_ok, G)) {
         snprintf(why, why_len, "no tile shape for R=%d", R);

@@ -91,3 +91,22 @@ def test_solvers_of_large_and_small_shared_memory():
         s.synchronize()
         assert np.array_equal(s.getCurrentState(), O.run(g, r, rule, 4)), (n, r)
         s.close()
+
+
+@pytest.mark.parametrize("radius", [1, 5, 6, 16, 17, 33, 60, 91, 113, 128])
+def test_staged_ragged_sides_vs_oracle(radius):
+    """Around the side from which ragged rows are staged, with the row's end early, late and
+    in the middle of a word and of a tile."""
+    import cat_cpu_b200 as C
+    rng = np.random.default_rng(50 + radius)
+    N = (2 * radius + 1) ** 2
+    rule = (int(0.45 * N), N, int(0.45 * N), N)  # above the mean count: domains of both kinds
+    for n in (1919, 1921, 1950, 2047, 2049, 2079, 2191):
+        g = (rng.random((n, n)) < 0.45).astype(np.uint8)
+        with C.CUDASolver(n, radius, rule, variant=C.VARIANT_TENSOR) as s:
+            s.setState(g)
+            for steps in (2, 1):  # many generations per launch, and one
+                s.doSteps(steps)
+                s.synchronize()
+                g = O.run(g, radius, rule, steps)
+                assert np.array_equal(s.getCurrentState(), g), (n, radius, steps)

@@ -10,8 +10,8 @@ from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
 
-# bands in several CTAs, tiles, tensor
-SOLVERS = [("packed", 300, 5), ("packed", 2048, 8), ("tensor", 700, 5)]
+# bands in several CTAs, tiles, tensor: gathered, staged with and without a seam
+SOLVERS = [("packed", 300, 5), ("packed", 2048, 8), ("tensor", 700, 5), ("tensor", 2001, 5), ("tensor", 704, 5)]
 RULE = {5: O.BOSCO_R5}
 
 
